@@ -1252,7 +1252,7 @@ static int stats_of(clotho_ctx* ctx, uint32_t idx, clotho_stats* out, uint32_t* 
         uint32_t* d_counts = nullptr;
         CK(pool_alloc(ctx, &d_counts, counts.size() * 4));
         CK(cudaMemsetAsync(d_counts, 0, counts.size() * 4, ctx->stream));
-        if (S && s.W) launch_stats(cfg(ctx), ctx->d_pops[0], idx, d_counts, s.W);
+        launch_margins(cfg(ctx), ctx->d_pops[0], idx, S, s.W, d_counts, nullptr);
         CK(cudaMemcpyAsync(counts.data(), d_counts, counts.size() * 4, cudaMemcpyDeviceToHost, ctx->stream));
         CK(cudaFreeAsync(d_counts, ctx->stream));
         ctx->launches += 1;
@@ -1299,13 +1299,12 @@ static int margins_of(clotho_ctx* ctx, uint32_t idx, uint32_t* col, uint32_t* ro
     uint32_t* d = nullptr;
     CK(pool_alloc(ctx, &d, (ncol + nrow) * 4));
     CK(cudaMemsetAsync(d, 0, (ncol + nrow) * 4, ctx->stream));
-    if (col && S && s.W) launch_stats(cfg(ctx), ctx->d_pops[0], idx, d, s.W);
-    if (row && S) launch_row_counts(cfg(ctx), ctx->d_pops[0], idx, d + ncol, S);
+    launch_margins(cfg(ctx), ctx->d_pops[0], idx, S, s.W, col ? d : nullptr, row ? d + ncol : nullptr);
     if (col && s.A) CK(cudaMemcpyAsync(col, d, (size_t)s.A * 4, cudaMemcpyDeviceToHost, ctx->stream));
     if (row && S) CK(cudaMemcpyAsync(row, d + ncol, (size_t)S * 4, cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaFreeAsync(d, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
-    ctx->launches += (col ? 1 : 0) + (row ? 1 : 0);
+    ctx->launches += (col || row) ? 1 : 0;
     return check_launch(ctx, "margins");
 }
 

@@ -315,8 +315,8 @@ void launch_cdf(const LaunchCfg&, const PopDev* pops, uint32_t npops, uint32_t m
 void launch_end(const LaunchCfg&, const PopDev* pops, uint32_t npops);
 void launch_seed_rows(const LaunchCfg&, const PopDev* pops, uint32_t npops, const uint32_t* thr,
                       uint64_t seed, uint32_t A);
-void launch_stats(const LaunchCfg&, const PopDev* pops, uint32_t p, uint32_t* counts, uint32_t A);
-void launch_row_counts(const LaunchCfg&, const PopDev* pops, uint32_t p, uint32_t* counts, uint32_t S);
+void launch_margins(const LaunchCfg&, const PopDev* pops, uint32_t p, uint32_t S, uint32_t W, uint32_t* colc,
+                    uint32_t* rowc);
 // device accumulators of the pairwise-difference kernel
 struct PairwiseOut {
     unsigned long long count, total, sumsq;
