@@ -67,15 +67,15 @@ std::vector<size_t> sizes_of(const Geometry& g) {
         A * 4, A * 8, A * 4, A * 16,     // free_list, pos, age, eff (traits padded to 4)
         g.FXcap * 8ull, g.FXcap * 4ull, g.FXcap * T * 4ull,
         S * 32, S * 32, N * 32, N * 8, N * 8,    // zg[0], zg[1], zi, fit, cdf
-        (N / 1024 + 8) * 8, ((S > g.NB ? S : g.NB) / 1024 + 8) * 4ull, ((S > g.NB ? S : g.NB) / 1024 + 8) * 4ull,
-        (S + 1) * 4 * 2ull,              // row_cnt, row_off
+        (N / 1024 + 8) * 8, (N / 128 + 64) * 8, (kPoisTab + 1) * 8, (kPoisTab + 1) * 8, ((S > g.NB ? S : g.NB) / 1024 + 8) * 4ull, ((S > g.NB ? S : g.NB) / 1024 + 8) * 4ull,
+        (S + 1) * 4, (S + 1) * 4,        // row_cnt, row_off
         S * 4, g.Mcap * 4ull, g.Mcap * 4ull,  // row_cur, row_mut, mut_slot
-        (g.NB + 1ull) * 4 * 2, g.NB * 4ull, A * 8, A * 4, A * 4,  // bcnt+boff, bcur, bpos, bslot, rank
+        (g.NB + 1ull) * 4, (g.NB + 1ull) * 4, g.NB * 4ull, A * 8, A * 4, A * 4,  // bcnt, boff, bcur, bpos, bslot, rank
         g.table ? A * 4 : 0,                            // inv
         g.table ? (A / 64 + 1) * W * 8 : 0,             // suf
         g.table ? S * 16 : 0,                           // plan_row
-        g.table ? (S + 1) * 4 * 2 : 0,                  // ord_cnt + ord_off
-        g.table ? S * 4 : 0,                            // ord_cur
+        g.table ? N * 4 : 0,                            // ord_cnt
+        g.table ? N * 4 : 0,                            // ord_cur
         g.table ? S * 4 : 0,                            // ord_pos
         g.table ? g.EVcap * 4ull : 0,                   // plan_go
         g.table ? g.EVcap * 4ull : 0,                   // plan_cr
@@ -96,11 +96,6 @@ struct clotho_ctx {
     int num_sms = 152;
     cudaStream_t stream = nullptr, copy_stream = nullptr;
     cudaStream_t own_stream = nullptr;  // the context's own compute stream (stream may be the caller's)
-    // a step's parent selection and row ordering run on side_stream beside the allele-space work (mutation
-    // counts, free space, new alleles, ranks, suffix tables), forked after the step's header and joined
-    // before the row plans; a captured step keeps the two branches as parallel graph branches
-    cudaStream_t side_stream = nullptr;
-    cudaEvent_t fork_ev = nullptr, join_ev = nullptr;
     // populations' device tables come from the context's own stream-ordered pool, which keeps freed
     // blocks for the next population (a serving loop adds and removes populations every few steps)
     cudaMemPool_t pool = nullptr;
@@ -254,18 +249,16 @@ int alloc_pop(clotho_ctx* ctx, const clotho_desc& d, PopHost** out) {
     b.fx_pos = (double*)ptr[k++]; b.fx_age = (uint32_t*)ptr[k++]; b.fx_eff = (float*)ptr[k++];
     b.zg[0] = (double*)ptr[k++]; b.zg[1] = (double*)ptr[k++];
     b.zi = (double*)ptr[k++]; b.fit = (double*)ptr[k++]; b.cdf = (double*)ptr[k++];
-    b.scan_part = (double*)ptr[k++]; b.scan_upart = (uint32_t*)ptr[k++]; b.scan_opart = (uint32_t*)ptr[k++];
-    b.row_cnt = (uint32_t*)ptr[k++];
-    b.row_off = b.row_cnt + (g.Scap + 1);
+    b.scan_part = (double*)ptr[k++]; b.scan_wsum = (double*)ptr[k++];
+    b.pois_mu = (double*)ptr[k++]; b.pois_rho = (double*)ptr[k++];
+    b.scan_upart = (uint32_t*)ptr[k++]; b.scan_opart = (uint32_t*)ptr[k++];
+    b.row_cnt = (uint32_t*)ptr[k++]; b.row_off = (uint32_t*)ptr[k++];
     b.row_cur = (uint32_t*)ptr[k++]; b.row_mut = (uint32_t*)ptr[k++]; b.mut_slot = (uint32_t*)ptr[k++];
-    b.bcnt = (uint32_t*)ptr[k++];
-    b.boff = b.bcnt + (g.NB + 1);
+    b.bcnt = (uint32_t*)ptr[k++]; b.boff = (uint32_t*)ptr[k++];
     b.bcur = (uint32_t*)ptr[k++]; b.bpos = (double*)ptr[k++]; b.bslot = (uint32_t*)ptr[k++];
     b.rank = (uint32_t*)ptr[k++]; b.inv = (uint32_t*)ptr[k++]; b.suf = (uint64_t*)ptr[k++];
     b.plan_row = (uint4*)ptr[k++];
-    b.ord_cnt = (uint32_t*)ptr[k++];
-    b.ord_off = b.ord_cnt ? b.ord_cnt + (g.Scap + 1) : nullptr;
-    b.ord_cur = (uint32_t*)ptr[k++]; b.ord_pos = (uint32_t*)ptr[k++];
+    b.ord_cnt = (uint32_t*)ptr[k++]; b.ord_cur = (uint32_t*)ptr[k++]; b.ord_pos = (uint32_t*)ptr[k++];
     b.plan_go = (uint32_t*)ptr[k++]; b.plan_cr = (uint32_t*)ptr[k++];
     b.plan_mut = (uint2*)ptr[k++]; b.plan_z = (double*)ptr[k++];
     b.colcnt = (uint32_t*)ptr[k++];
@@ -287,6 +280,7 @@ int alloc_pop(clotho_ctx* ctx, const clotho_desc& d, PopHost** out) {
     }
     p->dev[2] = p->dev[0];
     p->dev[2].mode = kModePhilox;
+    launch_pois_tables(ctx->stream, b);
     *out = p;
     return 0;
 }
@@ -392,16 +386,7 @@ bool count_on(clotho_ctx* ctx, uint32_t fuse) {
 // The generation kernel over every population: one launch when all populations use the same build; in a
 // batch that mixes them, one launch per build (bitmap, chunk-mask, interval), each over its own populations,
 // so every population runs the build it runs alone.
-// ordered: the rows' processing order is already enqueued (the fused step's side branch).
-void launch_gen(clotho_ctx* ctx, const PopDev* pops, uint32_t npops, uint32_t fuse, bool ordered = false) {
-    if (ctx->n_suf > 0) {  // per-row crossover plans of the suffix-table classifier (other populations skip it)
-        if (!ordered) {
-            launch_order(cfg(ctx), pops, npops, ctx->maxS);
-            ctx->launches += 5;  // order count, 3-kernel scan, order scatter
-        }
-        launch_row_plan(cfg(ctx), pops, npops, ctx->maxS);
-        ctx->launches += 1;
-    }
+void launch_gen(clotho_ctx* ctx, const PopDev* pops, uint32_t npops, uint32_t fuse) {
     const int prof = ctx->profiling ? (ctx->phase_clocks ? 2 : 1) : 0;
     const uint32_t kinds = (ctx->n_bm > 0) + (ctx->n_cm > 0) + (ctx->n_iv > 0);
     const bool mixed = kinds > 1;
@@ -461,13 +446,17 @@ int require_ready(clotho_ctx* ctx) {
     return 0;
 }
 
-// Make accF/accV of every population hold the AND/OR of its parent rows
-// (called right after k_begin when the previous step did not fuse them).
+PrepSizes prep_sizes(const clotho_ctx* ctx) {
+    return PrepSizes{ctx->maxS, ctx->maxN, ctx->maxNB, ctx->maxA, ctx->n_suf > 0};
+}
+
+// Make accF/accV of every population hold the AND/OR of its current rows
+// (called before a step when the previous one did not fuse them).
 void ensure_parent_acc(clotho_ctx* ctx, const PopDev* pops, uint32_t npops) {
     bool need = false;
     for (PopHost* p : ctx->pops) need |= !p->acc_valid;
     if (need) {
-        launch_fs_reduce(cfg(ctx), pops, npops, ctx->maxW, 1u);
+        launch_fs_reduce(cfg(ctx), pops, npops, ctx->maxW, 0u);
         ctx->launches += 1;
     }
 }
@@ -478,38 +467,14 @@ void enqueue_fused_step(clotho_ctx* ctx, uint32_t set, bool philox) {
     const PopDev* pops = ctx->d_pops[set];
     LaunchCfg L = cfg(ctx);
     ctx->pairs_set = set == 1u ? 1u : 0u;  // the device-drawn set (2) shares set 0's buffers
-    launch_begin(L, pops, n, ctx->d_hdr[set], ctx->d_ctl);
     ensure_parent_acc(ctx, pops, n);
-    // side branch: parents (from the parent generation's fitness) and the rows' processing order (from the
-    // parents) read only the step header and the pairs, and write only the pairs, the ordering arrays and
-    // their own scan partials, none of which the main branch touches before the join
-    auto note = [ctx](cudaError_t e) {
-        if (e != cudaSuccess && ctx->launch_err == cudaSuccess) ctx->launch_err = e;
-    };
-    LaunchCfg Ls = L;
-    Ls.stream = ctx->side_stream;
-    note(cudaEventRecord(ctx->fork_ev, L.stream));
-    note(cudaStreamWaitEvent(ctx->side_stream, ctx->fork_ev, 0));
-    if (philox) launch_select_philox(Ls, pops, n);
-    if (ctx->n_suf > 0) {
-        launch_order(Ls, pops, n, ctx->maxS);
-        ctx->launches += 5;  // order count, 3-kernel scan, order scatter
-    }
-    note(cudaEventRecord(ctx->join_ev, ctx->side_stream));
-    // main branch: the child's allele space
-    if (philox) launch_mut_counts_philox(L, pops, n, ctx->maxS);
-    launch_fs_finalize(L, pops, n, count_on(ctx, kFuseMut | kFusePheno | kFuseFs));
-    if (!philox) launch_mut_csr_tape(L, pops, n, ctx->maxS);
-    launch_mut_resolve(L, pops, n);
-    launch_ranks(L, pops, n, ctx->maxNB, ctx->maxW_suf, ctx->n_suf > 0);
-    note(cudaStreamWaitEvent(L.stream, ctx->join_ev, 0));
-    launch_gen(ctx, pops, n, kFuseMut | kFusePheno | kFuseFs, true);
-    launch_individuals(L, pops, n);
-    launch_cdf(L, pops, n, ctx->maxN);
-    launch_end(L, pops, n);
-    // begin, mutation counts or CSR (4 or 6), finalize, resolve, ranks (6, + suffix table), selection (device
-    // draws), individuals, 3-kernel prefix sum, end; launch_gen and ensure_parent_acc count their own
-    ctx->launches += 19u + (philox ? 0u : 1u) + (ctx->n_suf > 0 ? 1u : 0u);
+    const PrepSizes z = prep_sizes(ctx);
+    const uint32_t what = kStepBegin | kStepMut | kStepOrder | (philox ? kStepSelect : kStepTape);
+    ctx->launches += launch_prep(L, pops, n, z, ctx->d_hdr[set], ctx->d_ctl, what,
+                                 count_on(ctx, kFuseMut | kFusePheno | kFuseFs));
+    ctx->launches += launch_plan(L, pops, n, z, ctx->maxW_suf);
+    launch_gen(ctx, pops, n, kFuseMut | kFusePheno | kFuseFs);
+    ctx->launches += launch_fitness(L, pops, n, ctx->maxN, true);
     for (PopHost* p : ctx->pops) p->acc_valid = true;
 }
 
@@ -569,16 +534,13 @@ int clotho_create(const clotho_desc* desc, clotho_ctx** out) {
         return CLOTHO_E_CUDA;
     }
     cudaDeviceGetAttribute(&ctx->num_sms, cudaDevAttrMultiProcessorCount, ctx->device);
-    if (init_recip_step() || init_recip_gen()) {  // constant tables of this device
+    if (init_recip_prep() || init_recip_gen()) {  // constant tables of this device
         cudaGetLastError();
         delete ctx;
         return CLOTHO_E_CUDA;
     }
     if (cudaStreamCreateWithFlags(&ctx->own_stream, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaStreamCreateWithFlags(&ctx->copy_stream, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaStreamCreateWithFlags(&ctx->side_stream, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaEventCreateWithFlags(&ctx->fork_ev, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&ctx->join_ev, cudaEventDisableTiming) != cudaSuccess) {
+        cudaStreamCreateWithFlags(&ctx->copy_stream, cudaStreamNonBlocking) != cudaSuccess) {
         cudaGetLastError();
         clotho_destroy(ctx);  // releases whichever stream was made
         return CLOTHO_E_CUDA;
@@ -652,7 +614,6 @@ int clotho_destroy(clotho_ctx* ctx) {
     if (!ctx) return CLOTHO_E_ARG;
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
     if (ctx->copy_stream) cudaStreamSynchronize(ctx->copy_stream);
-    if (ctx->side_stream) cudaStreamSynchronize(ctx->side_stream);
     for (PopHost* p : ctx->pops) free_pop(ctx, p);
     ctx->pops.clear();
     if (ctx->own_stream) cudaStreamSynchronize(ctx->own_stream);
@@ -678,9 +639,6 @@ int clotho_destroy(clotho_ctx* ctx) {
     if (ctx->t1) cudaEventDestroy(ctx->t1);
     if (ctx->own_stream) cudaStreamDestroy(ctx->own_stream);
     if (ctx->copy_stream) cudaStreamDestroy(ctx->copy_stream);
-    if (ctx->side_stream) cudaStreamDestroy(ctx->side_stream);
-    if (ctx->fork_ev) cudaEventDestroy(ctx->fork_ev);
-    if (ctx->join_ev) cudaEventDestroy(ctx->join_ev);
     delete ctx;
     return 0;
 }
@@ -788,9 +746,7 @@ static int finish_start(clotho_ctx* ctx) {
     LaunchCfg L = cfg(ctx);
     launch_fs_reduce(L, ctx->d_pops[0], 1, ctx->maxW, 0u);
     launch_phenotype(L, ctx->d_pops[0], 1);
-    launch_individuals(L, ctx->d_pops[0], 1);
-    launch_cdf(L, ctx->d_pops[0], 1, ctx->maxN);
-    ctx->launches += 6;
+    ctx->launches += 2 + launch_fitness(L, ctx->d_pops[0], 1, ctx->maxN, false);
     int rc = check_launch(ctx, "start");
     if (rc) return rc;
     CK(cudaStreamSynchronize(ctx->stream));
@@ -989,9 +945,10 @@ int clotho_crossover(clotho_ctx* ctx, const uint8_t* swap, const uint32_t* ev_of
     if ((rc = h2d(ctx, D.swap, swap, 2ull * N, ctx->stream))) return rc;
     if ((rc = h2d(ctx, D.ev_off, ev_off, 2ull * N + 1, ctx->stream))) return rc;
     if ((rc = h2d(ctx, D.ev_pos, ev_pos, (size_t)ev_total, ctx->stream))) return rc;
-    // item prefix is already set by begin; ranks over the current positions
-    launch_ranks(cfg(ctx), ctx->d_pops[0], 1, ctx->maxNB, ctx->maxW, ctx->n_suf > 0);
-    ctx->launches += 6u + (ctx->n_suf > 0 ? 1u : 0u);
+    // item prefix is already set by begin; the rows' order, ranks over the current positions
+    const PrepSizes z = prep_sizes(ctx);
+    ctx->launches += launch_prep(cfg(ctx), ctx->d_pops[0], 1, z, nullptr, ctx->d_ctl, kStepOrder, false);
+    ctx->launches += launch_plan(cfg(ctx), ctx->d_pops[0], 1, z, ctx->maxW);
     launch_gen(ctx, ctx->d_pops[0], 1, 0u);
     if ((rc = check_launch(ctx, "crossover"))) return rc;
     CK(cudaStreamSynchronize(ctx->stream));
@@ -1026,9 +983,7 @@ int clotho_phenotype(clotho_ctx* ctx) {
 
 int clotho_fitness(clotho_ctx* ctx) {
     if (!ctx) return CLOTHO_E_ARG;
-    launch_individuals(cfg(ctx), ctx->d_pops[0], 1);
-    launch_cdf(cfg(ctx), ctx->d_pops[0], 1, ctx->maxN);
-    ctx->launches += 4;
+    ctx->launches += launch_fitness(cfg(ctx), ctx->d_pops[0], 1, ctx->maxN, false);
     return check_launch(ctx, "fitness");
 }
 

@@ -77,9 +77,12 @@ struct PopDev {
     double*   zi;          // [Ncap * 4] per-individual phenotypes
     double*   fit;         // [Ncap]
     double*   cdf;         // [Ncap]
-    double*   scan_part;   // [Ncap / 1024 + 2]
-    uint32_t* scan_upart;  // [Scap / 1024 + 2]
-    uint32_t* scan_opart;  // [Scap / 1024 + 2] the row-ordering scan's own partials (it runs beside the others)
+    double*   scan_part;   // [Ncap / 4096 + 2] offsets of the fitness sum's 4,096-individual chunks
+    double*   scan_wsum;   // [Ncap / 128 + 64] fitness sums of 128 individuals
+    double*   pois_mu;     // [kPoisTab + 1] Poisson(mu) CDF F_0 .. F_{kPoisTab-1}, then p_{kPoisTab-1}
+    double*   pois_rho;    // [kPoisTab + 1] the same of Poisson(rho)
+    uint32_t* scan_upart;  // [max(Scap, NB) / 1024 + 2] chunk sums
+    uint32_t* scan_opart;  // [Scap / 1024 + 2] the row-ordering scan's own chunk sums (it runs beside the others)
     uint32_t* pairs;       // [2 * Ncap]
     uint8_t*  swap;        // [Scap]
     uint32_t* ev_off;      // [Scap + 1]
@@ -90,20 +93,19 @@ struct PopDev {
     uint32_t* mut_slot;    // [Mcap]
     uint32_t* row_cnt;     // [Scap + 1] per-row mutation counts (zero between steps)
     uint32_t* row_off;     // [Scap + 1] exclusive prefix of row_cnt
-    uint32_t* row_cur;     // [Scap] scatter cursors (zero between steps)
+    uint32_t* row_cur;     // [Scap] scatter cursors of the tape's new alleles
     uint32_t* row_mut;     // [Mcap] mutation indices grouped by row
     uint32_t* bcnt;        // [NB + 1] positions per bucket (zero between steps)
     uint32_t* boff;        // [NB + 1] exclusive prefix of bcnt
-    uint32_t* bcur;        // [NB] bucket scatter cursors (zero between steps)
+    uint32_t* bcur;        // [NB] bucket scatter cursors
     double*   bpos;        // [Acap] positions grouped by bucket
     uint32_t* bslot;       // [Acap] slot of each bpos entry
     uint32_t* rank;        // [Acap] rank of each slot (position, then slot index) among the A slots
     uint32_t* inv;         // [Acap] slot of each rank (Acap <= kTableMaxSlots, else null)
     uint64_t* suf;         // [(Acap/64 + 1) * Wcap] suffix table of the crossover classifier (Acap <= kTableMaxSlots, else null)
     uint4*    plan_row;    // [Scap] crossover plans in processing order: row, top strand, event base, events | flags << 30
-    uint32_t* ord_cnt;     // [Scap + 1] rows per ordering key (zero between steps)
-    uint32_t* ord_off;     // [Scap + 1] exclusive prefix of ord_cnt
-    uint32_t* ord_cur;     // [Scap] scatter cursors (zero between steps)
+    uint32_t* ord_cnt;     // [Ncap] rows per parent individual (zero between steps)
+    uint32_t* ord_cur;     // [Ncap] scatter cursors: the exclusive prefix of ord_cnt
     uint32_t* ord_pos;     // [Scap] processing position of each row
     uint32_t* plan_go;     // [EVcap] table row offset per planned event (with suf)
     uint32_t* plan_cr;     // [EVcap] correction ranks per planned event: first | count << 20 (with suf)
@@ -234,7 +236,30 @@ __device__ inline uint32_t poisson_inv(double u, double lambda, double e) {
     return k;
 }
 
-__device__ inline uint32_t lane_id() { return threadIdx.x & 31u; }
+constexpr uint32_t kPoisTab = 64;     // entries of a population's Poisson CDF tables (made with it)
+
+// poisson_inv(u, lambda, exp(-lambda)) from the table cdf[k] = F_k of the same recurrence: the first k with
+// u <= F_k (u and F_k are non-negative, so their bit patterns compare as integers); past the table the
+// recurrence goes on from (p, F) at k = kPoisTab - 1, as poisson_inv would.
+__device__ __forceinline__ uint32_t poisson_tab(double u, const double* cdf, double plast, double lambda) {
+    uint32_t k = 0;
+    while (k < kPoisTab && lt_nonneg(cdf[k], u)) ++k;
+    if (k < kPoisTab) return k;
+    k = kPoisTab - 1u;
+    double pk = plast, F = cdf[k];
+    while (u > F && k < 4096u) {
+        ++k;
+        poisson_step(pk, F, lambda, k);
+    }
+    return k;
+}
+
+// Programmatic dependent launch: a kernel launched with launch_k may be resident before its predecessor in the
+// stream ends.  pdl_wait returns when the predecessor has ended and its writes are visible; every block of every
+// such kernel calls it before it touches memory (so a predecessor's end means that all before it ended, too).
+// pdl_go lets the successor's blocks in as this kernel's leave.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_go() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // Monotone bucket of a position in [0,1) (values outside are clamped).
 // floor(x * NB) for x in (0, 1), from the bits with integer operations: 0 for
@@ -286,15 +311,46 @@ inline uint32_t blocks_for(uint64_t n, uint32_t per_block) {
     const uint64_t b = (n + per_block - 1) / per_block;
     return b < 1 ? 1u : (b > 0x7fffffffull ? 0x7fffffffu : (uint32_t)b);
 }
+// Launch with the programmatic dependency of pdl_wait / pdl_go.
+template <class... P, class... A>
+inline cudaError_t launch_smem_k(const LaunchCfg& L, void (*k)(P...), dim3 grid, dim3 block, size_t smem, A... a) {
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c{};
+    c.gridDim = grid;
+    c.blockDim = block;
+    c.dynamicSmemBytes = smem;
+    c.stream = L.stream;
+    c.attrs = &at;
+    c.numAttrs = 1;
+    return cudaLaunchKernelEx(&c, k, static_cast<P>(a)...);
+}
+template <class... P, class... A>
+inline cudaError_t launch_k(const LaunchCfg& L, void (*k)(P...), dim3 grid, dim3 block, A... a) {
+    return launch_smem_k(L, k, grid, block, 0, a...);
+}
+
 // which: 0 = current child rows, 1 = parent rows of the step in progress
 void launch_fs_reduce(const LaunchCfg&, const PopDev* pops, uint32_t npops, uint32_t maxW, uint32_t which);
-// count_on: the step's generation kernel counts columns for the populations that asked (see
-// generation_counts_fit); their counts are zeroed here and marked valid
-void launch_fs_finalize(const LaunchCfg&, const PopDev* pops, uint32_t npops, bool count_on = false);
-void launch_begin(const LaunchCfg&, const PopDev* pops, uint32_t npops, const uint32_t* hdr,
-                  WorkCtl* ctl);
-void launch_mut_csr_tape(const LaunchCfg&, const PopDev* pops, uint32_t npops, uint32_t maxS);
-void launch_mut_counts_philox(const LaunchCfg&, const PopDev* pops, uint32_t npops, uint32_t maxS);
+// staged API: the step header; the free-space analysis and the child's allele count
+void launch_begin(const LaunchCfg&, const PopDev* pops, uint32_t npops, const uint32_t* hdr, WorkCtl* ctl);
+void launch_fs_finalize(const LaunchCfg&, const PopDev* pops, uint32_t npops);
+
+// What launch_prep does.  Begin: header and free space; Mut: mutation counts and slots (Tape: of tapes);
+// Order: the rows' processing order (Select: with parents drawn on the device); position buckets always.
+constexpr uint32_t kStepBegin = 1u, kStepMut = 2u, kStepOrder = 4u, kStepSelect = 8u, kStepTape = 16u;
+struct PrepSizes {
+    uint32_t maxS, maxN, maxNB, maxA;   // largest capacities of the batch
+    bool tables;                        // some population has a suffix table
+};
+// hdr: null in the staged API, where k_begin has set the sizes.  count_on: the step's generation kernel counts
+// columns for the populations that asked (see generation_counts_fit); their counts are zeroed here and marked
+// valid.  Returns the launches made.
+uint32_t launch_prep(const LaunchCfg&, const PopDev* pops, uint32_t npops, const PrepSizes&, const uint32_t* hdr,
+                     WorkCtl* ctl, uint32_t what, bool count_on);
+// Poisson tables of one population (the device copy of its descriptor)
+void launch_pois_tables(cudaStream_t s, const PopDev& P);
 void launch_mut_resolve(const LaunchCfg&, const PopDev* pops, uint32_t npops);
 void launch_select_philox(const LaunchCfg&, const PopDev* pops, uint32_t npops);
 // Generation-kernel builds: suffix-table masks in per-warp bitmaps (capacity <= kSufMaxSlots), chunk by
@@ -310,8 +366,8 @@ cudaError_t launch_generation(const LaunchCfg&, const PopDev* pops, uint32_t npo
 bool generation_counts_fit(uint32_t maxW, uint32_t maxA);
 void launch_mut_scatter(const LaunchCfg&, const PopDev* pops, uint32_t npops);
 void launch_phenotype(const LaunchCfg&, const PopDev* pops, uint32_t npops);
-void launch_individuals(const LaunchCfg&, const PopDev* pops, uint32_t npops);
-void launch_cdf(const LaunchCfg&, const PopDev* pops, uint32_t npops, uint32_t maxN);
+// individual phenotypes, fitness and its prefix sum; end: and the step's end.  Returns the launches made.
+uint32_t launch_fitness(const LaunchCfg&, const PopDev* pops, uint32_t npops, uint32_t maxN, bool end);
 void launch_end(const LaunchCfg&, const PopDev* pops, uint32_t npops);
 void launch_seed_rows(const LaunchCfg&, const PopDev* pops, uint32_t npops, const uint32_t* thr,
                       uint64_t seed, uint32_t A);
@@ -324,16 +380,10 @@ struct PairwiseOut {
 };
 void launch_pairwise(const LaunchCfg&, const PopDev* pops, uint32_t p, const uint32_t* sample, uint32_t n,
                      uint32_t* dist, PairwiseOut* out);
-void launch_ranks(const LaunchCfg&, const PopDev* pops, uint32_t npops, uint32_t maxNB, uint32_t maxW, bool suf);
-void launch_uscan_buckets(const LaunchCfg&, const PopDev* pops, uint32_t npops, uint32_t maxNB);
-void launch_uscan_order(const LaunchCfg&, const PopDev* pops, uint32_t npops, uint32_t maxS);
-
-void launch_plan(const LaunchCfg&, const PopDev* pops, uint32_t npops, uint32_t maxS);
-// the two halves of launch_plan: the rows' processing order (by parent; needs only the pairs and the step
-// header) and the per-row plans (needs the ranks, the suffix tables and the new alleles as well)
-void launch_order(const LaunchCfg&, const PopDev* pops, uint32_t npops, uint32_t maxS);
-void launch_row_plan(const LaunchCfg&, const PopDev* pops, uint32_t npops, uint32_t maxS);
-int init_recip_step();  // k_step.cu's copy of the reciprocal table
+// After launch_prep: the slots' ranks, the suffix tables and (tables: some population has one) the rows' plans.
+// Returns the launches made.
+uint32_t launch_plan(const LaunchCfg&, const PopDev* pops, uint32_t npops, const PrepSizes&, uint32_t maxW);
+int init_recip_prep();  // k_prep.cu's copy of the reciprocal table
 int init_recip_gen();   // k_generation.cu's copy
 
 // crossover-plan row flags

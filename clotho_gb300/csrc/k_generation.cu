@@ -1365,6 +1365,8 @@ k_generation(const PopDev* __restrict__ pops, uint32_t npops, WorkCtl* __restric
         }
         __syncwarp();
     }
+    pdl_wait();
+    pdl_go();
     const bool do_mut = (fuse & kFuseMut) != 0, do_ph = (fuse & kFusePheno) != 0, do_fs = (fuse & kFuseFs) != 0;
     uint64_t* const cplanes =
         CNT ? reinterpret_cast<uint64_t*>(reinterpret_cast<WarpSmem*>(s_dyn + (3u + kWarps) * maxW) + kWarps) : nullptr;
@@ -1621,12 +1623,11 @@ cudaError_t launch_generation(const LaunchCfg& L, const PopDev* pops, uint32_t n
     // 128 words: its narrow build (copy rows by direct loads)
     const bool narrow = L.narrow_ok && maxW <= 64u * kDirectCopyChunks;
     const int si = cm ? 7 : suf ? (profile == 2 ? (narrow ? 4 : 2) : cnt ? (narrow ? 6 : 5) : narrow ? 3 : 1) : 0;
-    const void* fns[8] = {(const void*)k_generation<false, false, false>, (const void*)k_generation<true, false, false>,
-                          (const void*)k_generation<true, true, false>, (const void*)k_generation<true, false, true>,
-                          (const void*)k_generation<true, true, true>,
-                          (const void*)k_generation<true, false, false, true>,
-                          (const void*)k_generation<true, false, true, true>,
-                          (const void*)k_generation<true, false, false, false, true>};
+    using Kernel = void (*)(const PopDev*, uint32_t, WorkCtl*, uint32_t, int, uint32_t, uint32_t, uint32_t);
+    static const Kernel fns[8] = {k_generation<false, false, false>,      k_generation<true, false, false>,
+                                  k_generation<true, true, false>,        k_generation<true, false, true>,
+                                  k_generation<true, true, true>,         k_generation<true, false, false, true>,
+                                  k_generation<true, false, true, true>,  k_generation<true, false, false, false, true>};
     // static shared memory is above 48 KB on its own, so the opt-in attribute is always needed; it is a
     // property of the function on each device, so it is kept per device (host threads share the table)
     {
@@ -1639,144 +1640,70 @@ cudaError_t launch_generation(const LaunchCfg& L, const PopDev* pops, uint32_t n
         std::lock_guard<std::mutex> lock(mu);
         size_t& c = configured[dev][si];
         if (smem > c || c == 0) {
-            e = cudaFuncSetAttribute(fns[si], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            e = cudaFuncSetAttribute((const void*)fns[si], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
             if (e != cudaSuccess) return e;
             c = smem > 0 ? smem : 1;
         }
     }
-    switch (si) {
-        case 7:
-            k_generation<true, false, false, false, true><<<L.num_sms, kGenThreads, smem, L.stream>>>(
-                pops, npops, ctl, fuse, profile, maxW, acc_words, mx);
-            break;
-        case 6:
-            k_generation<true, false, true, true><<<L.num_sms, kGenThreads, smem, L.stream>>>(pops, npops, ctl, fuse,
-                                                                                              profile, maxW, 0u, mx);
-            break;
-        case 5:
-            k_generation<true, false, false, true><<<L.num_sms, kGenThreads, smem, L.stream>>>(pops, npops, ctl, fuse,
-                                                                                               profile, maxW, 0u, mx);
-            break;
-        case 4:
-            k_generation<true, true, true><<<L.num_sms, kGenThreads, smem, L.stream>>>(pops, npops, ctl, fuse,
-                                                                                       profile, maxW, 0u, mx);
-            break;
-        case 3:
-            k_generation<true, false, true><<<L.num_sms, kGenThreads, smem, L.stream>>>(pops, npops, ctl, fuse,
-                                                                                        profile, maxW, 0u, mx);
-            break;
-        case 2:
-            k_generation<true, true, false><<<L.num_sms, kGenThreads, smem, L.stream>>>(pops, npops, ctl, fuse,
-                                                                                        profile, maxW, 0u, mx);
-            break;
-        case 1:
-            k_generation<true, false, false><<<L.num_sms, kGenThreads, smem, L.stream>>>(pops, npops, ctl, fuse,
-                                                                                        profile, maxW, 0u, mx);
-            break;
-        default:
-            k_generation<false, false, false><<<L.num_sms, kGenThreads, smem, L.stream>>>(pops, npops, ctl, fuse,
-                                                                                         profile, maxW, acc_words, mx);
-    }
-    return cudaSuccess;
+    return launch_smem_k(L, fns[si], dim3(L.num_sms), dim3(kGenThreads), smem, pops, npops, ctl, fuse, profile, maxW,
+                         (suf && !cm) ? 0u : acc_words, mx);
 }
 
 // ---------------------------------------------------------------------------
 constexpr uint32_t kPlanSmemEv = 16;  // breakpoints of a row the plan kernel ranks in shared memory
-constexpr uint32_t kPoisTab = 64;     // entries of the plan kernel's Poisson CDF table
-
-// poisson_inv(u, rho, exp(-rho)) from the table cdf[k] = F_k of the same recurrence: the first k with
-// u <= F_k (u and F_k are non-negative, so their bit patterns compare as integers); past the table the
-// recurrence goes on from (p, F) at k = kPoisTab - 1, as poisson_inv would.
-__device__ __forceinline__ uint32_t poisson_tab(double u, const double* cdf, double plast, double lambda) {
-    uint32_t k = 0;
-    while (k < kPoisTab && lt_nonneg(cdf[k], u)) ++k;
-    if (k < kPoisTab) return k;
-    k = kPoisTab - 1u;
-    double pk = plast, F = cdf[k];
-    while (u > F && k < 4096u) {
-        ++k;
-        poisson_step(pk, F, lambda, k);
-    }
-    return k;
-}
-
-// Processing order of the offspring rows (parent-major): rows are sorted by
-// parent individual, so rows reading the same parent strands run side by side
-// and the second read of a strand is an L2 hit.  Counting sort by key; the
-// order inside one key does not matter (rows are independent).  Keys 0 and 2
-// (by gamete parity first) are kept for measurement.
-#ifndef CLOTHO_ORDER_KEY
-#define CLOTHO_ORDER_KEY 1
-#endif
-__device__ __forceinline__ uint32_t order_key(const PopDev& P, uint32_t g, uint32_t N, uint32_t pN) {
-    uint32_t pind = P.pairs[g];
-    if (pind >= pN) pind = 0;
-#if CLOTHO_ORDER_KEY == 1
-    return pind;                                  // parent only
-#elif CLOTHO_ORDER_KEY == 2
-    return (g & 1u) * N + (g >> 1);               // even rows, then odd rows
-#else
-    return (g & 1u) * N + pind;                   // parity, then parent
-#endif
-}
-
-__global__ void k_ord_count(const PopDev* __restrict__ pops, uint32_t npops) {
-    for (uint32_t p = blockIdx.z; p < npops; p += gridDim.z) {
-        const PopDev& P = pops[p];
-        if (!P.plan_row) continue;
-        const uint32_t N = P.st->N, pN = P.st->pN, S = 2u * N;
-        for (uint32_t g = blockIdx.x * blockDim.x + threadIdx.x; g < S; g += gridDim.x * blockDim.x)
-            atomicAdd(&P.ord_cnt[order_key(P, g, N, pN)], 1u);
-    }
-}
-
-__global__ void k_ord_scatter(const PopDev* __restrict__ pops, uint32_t npops) {
-    for (uint32_t p = blockIdx.z; p < npops; p += gridDim.z) {
-        const PopDev& P = pops[p];
-        if (!P.plan_row) continue;
-        const uint32_t N = P.st->N, pN = P.st->pN, S = 2u * N;
-        for (uint32_t g = blockIdx.x * blockDim.x + threadIdx.x; g < S; g += gridDim.x * blockDim.x) {
-            const uint32_t key = order_key(P, g, N, pN);
-            P.ord_pos[g] = P.ord_off[key] + atomicAdd(&P.ord_cur[key], 1u);
-        }
-    }
-}
-
 // ---------------------------------------------------------------------------
+// Position ranks of the slots [0, A) and the rows' plans, side by side (both need only the
+// position buckets).
+//
+// A slot's rank = slots in lower buckets + slots of its own bucket with a smaller position
+// (or the same position and a lower slot index).  inv is the inverse map (rank -> slot).
+//
 // Per-row crossover plans for the suffix-table classifier, one thread per row:
 // the top strand (parent individual and strand swap), the breakpoint count,
 // and for every breakpoint its nearest table row and correction ranks; plus
 // the direction of the phenotype gather.  Device-drawn breakpoints get their
-// plan entries from a block-aggregated counter; tape rows use the tape's own
+// plan entries from a warp-aggregated counter; tape rows use the tape's own
 // event offsets.
-__global__ void __launch_bounds__(256) k_row_plan(const PopDev* __restrict__ pops, uint32_t npops) {
+__device__ __forceinline__ void slot_ranks(const PopDev& P, uint32_t block, uint32_t blocks) {
+    const uint32_t A = P.st->A;
+    for (uint32_t s = block * 256u + threadIdx.x; s < A; s += blocks * 256u) {
+        const double x = P.pos[s];
+        const uint32_t b = pos_bucket(x, P.NB);
+        const uint32_t k0 = P.boff[b], k1 = P.boff[b + 1u];
+        uint32_t r = k0;
+        for (uint32_t k = k0; k < k1; ++k) {
+            const double y = P.bpos[k];
+            r += (y < x || (y == x && P.bslot[k] < s)) ? 1u : 0u;
+        }
+        P.rank[s] = r;
+        if (P.inv) P.inv[r] = s;
+    }
+}
+
+__global__ void __launch_bounds__(256, 4) k_plan(const PopDev* __restrict__ pops, uint32_t npops, uint32_t nrank) {
     const uint32_t lane = threadIdx.x & 31u;
     // a thread's thresholds (up to kPlanSmemEv) stay in shared memory while they are ranked
     // against each other; longer lists use their global slots
     __shared__ uint32_t s_cr[256][kPlanSmemEv + 1];
-    // the population's Poisson(rho) CDF, built by the same FP64 recurrence as poisson_inv and
-    // searched with integer compares, so a breakpoint count costs no FP64 work
-    __shared__ double s_cdf[kPoisTab];
-    __shared__ double s_plast;
+    // the population's Poisson(rho) CDF, searched with integer compares, so a breakpoint count costs no FP64 work
+    __shared__ double s_cdf[kPoisTab + 1];
+    pdl_wait();
+    pdl_go();
     for (uint32_t p = blockIdx.z; p < npops; p += gridDim.z) {
         const PopDev& P = pops[p];
-        if (!P.plan_row) continue;
+        // blocks [0, nrank) rank the slots, the rest (a single block: the same) plan the rows
+        const bool alone = gridDim.x == 1u;
+        if (alone || blockIdx.x < nrank) slot_ranks(P, alone ? 0u : blockIdx.x, alone ? 1u : nrank);
+        if (!P.plan_row || (!alone && blockIdx.x < nrank)) continue;
+        const uint32_t bx = alone ? 0u : blockIdx.x - nrank, nb = alone ? 1u : gridDim.x - nrank;
         __syncthreads();  // the previous population's table is no longer read
-        if (threadIdx.x == 0) {
-            double pk = P.exp_neg_rho, F = pk;
-            s_cdf[0] = F;
-            for (uint32_t k = 1; k < kPoisTab; ++k) {
-                poisson_step(pk, F, P.rho, k);
-                s_cdf[k] = F;
-            }
-            s_plast = pk;
-        }
+        if (threadIdx.x <= kPoisTab) s_cdf[threadIdx.x] = P.pois_rho[threadIdx.x];
         __syncthreads();
         const DevStatus st = *P.st;
         const uint32_t S = 2u * st.N, A = st.A, Se = (S + 1u) >> 1;
         const bool philox = P.mode == kModePhilox;
         const bool q1 = (P.flags & 1u) != 0;
-        for (uint32_t v0 = blockIdx.x * blockDim.x; v0 < S; v0 += gridDim.x * blockDim.x) {
+        for (uint32_t v0 = bx * 256u; v0 < S; v0 += nb * 256u) {
             const uint32_t v = v0 + threadIdx.x;
             const bool live = v < S;
             // even gametes on the first half of the threads, odd ones on the second:
@@ -1793,7 +1720,7 @@ __global__ void __launch_bounds__(256) k_row_plan(const PopDev* __restrict__ pop
                 }
                 if (philox) {
                     const U4 x = philox4x32(g, 0u, st.gen, kStreamGamete, P.seed);
-                    E = (q1 && (g & 1u)) ? 0u : poisson_tab(u01(x.x, x.y), s_cdf, s_plast, P.rho);
+                    E = (q1 && (g & 1u)) ? 0u : poisson_tab(u01(x.x, x.y), s_cdf, s_cdf[kPoisTab], P.rho);
                     swap = lt_nonneg(u01(x.z, x.w), P.bias);
                     if (E > kMaxEvDevice) {
                         atomicOr(&P.st->err, kErrEvents);
@@ -1892,68 +1819,6 @@ __global__ void __launch_bounds__(256) k_row_plan(const PopDev* __restrict__ pop
 
 int init_recip_gen() { return fill_recip_table(); }
 
-void launch_order(const LaunchCfg& L, const PopDev* pops, uint32_t npops, uint32_t maxS) {
-    const dim3 g = pop_grid(npops, blocks_for(maxS, 256), L.num_sms, 8);
-    k_ord_count<<<g, 256, 0, L.stream>>>(pops, npops);
-    launch_uscan_order(L, pops, npops, maxS);
-    k_ord_scatter<<<g, 256, 0, L.stream>>>(pops, npops);
-}
-
-void launch_row_plan(const LaunchCfg& L, const PopDev* pops, uint32_t npops, uint32_t maxS) {
-    k_row_plan<<<pop_grid(npops, blocks_for(maxS, 256), L.num_sms, 8), 256, 0, L.stream>>>(pops, npops);
-}
-
-void launch_plan(const LaunchCfg& L, const PopDev* pops, uint32_t npops, uint32_t maxS) {
-    launch_order(L, pops, npops, maxS);
-    launch_row_plan(L, pops, npops, maxS);
-}
-
-// ---------------------------------------------------------------------------
-// Position ranks for the crossover classifiers, rebuilt every generation over
-// the slots [0, A): counting sort of positions into NB buckets, then each
-// slot's rank = slots in lower buckets + slots of its own bucket with a
-// smaller position (or the same position and a lower slot index).  inv is the
-// inverse map (rank -> slot); suf is the suffix table of the classifier.
-__global__ void k_rank_count(const PopDev* __restrict__ pops, uint32_t npops) {
-    for (uint32_t p = blockIdx.z; p < npops; p += gridDim.z) {
-        const PopDev& P = pops[p];
-        const uint32_t A = P.st->A;
-        for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < A; s += gridDim.x * blockDim.x)
-            atomicAdd(&P.bcnt[pos_bucket(P.pos[s], P.NB)], 1u);
-    }
-}
-__global__ void k_rank_scatter(const PopDev* __restrict__ pops, uint32_t npops) {
-    for (uint32_t p = blockIdx.z; p < npops; p += gridDim.z) {
-        const PopDev& P = pops[p];
-        const uint32_t A = P.st->A;
-        for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < A; s += gridDim.x * blockDim.x) {
-            const double x = P.pos[s];
-            const uint32_t b = pos_bucket(x, P.NB);
-            const uint32_t k = P.boff[b] + atomicAdd(&P.bcur[b], 1u);
-            P.bpos[k] = x;
-            P.bslot[k] = s;
-        }
-    }
-}
-__global__ void k_rank_final(const PopDev* __restrict__ pops, uint32_t npops) {
-    for (uint32_t p = blockIdx.z; p < npops; p += gridDim.z) {
-        const PopDev& P = pops[p];
-        const uint32_t A = P.st->A;
-        for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < A; s += gridDim.x * blockDim.x) {
-            const double x = P.pos[s];
-            const uint32_t b = pos_bucket(x, P.NB);
-            const uint32_t k0 = P.boff[b], k1 = P.boff[b + 1u];
-            uint32_t r = k0;
-            for (uint32_t k = k0; k < k1; ++k) {
-                const double y = P.bpos[k];
-                r += (y < x || (y == x && P.bslot[k] < s)) ? 1u : 0u;
-            }
-            P.rank[s] = r;
-            if (P.inv) P.inv[r] = s;
-        }
-    }
-}
-
 // suf[g * Wcap + w] = bits of word w whose slot has rank >= 64 g, for
 // g = 0 .. ceil(A/64) (the last row is empty).  A unit of work is 32 words and
 // every kSufSlices-th table row; the units are spread over the whole grid from
@@ -1962,6 +1827,8 @@ constexpr uint32_t kSufSlices = 16;
 __global__ void __launch_bounds__(256) k_suf_build(const PopDev* __restrict__ pops, uint32_t npops) {
     __shared__ uint32_t s_grp[32][65];  // (rank >> 6) + 1 per slot, 0 beyond A
     const uint32_t tx = threadIdx.x & 31u, ty = threadIdx.x >> 5;
+    pdl_wait();
+    pdl_go();
     for (uint32_t p = blockIdx.z; p < npops; p += gridDim.z) {
         const PopDev& P = pops[p];
         if (!P.suf) continue;
@@ -1988,17 +1855,16 @@ __global__ void __launch_bounds__(256) k_suf_build(const PopDev* __restrict__ po
     }
 }
 
-void launch_ranks(const LaunchCfg& L, const PopDev* pops, uint32_t npops, uint32_t maxNB, uint32_t maxW,
-                  bool suf) {
-    const dim3 g = pop_grid(npops, L.num_sms * 2u, L.num_sms, 2);
-    k_rank_count<<<g, 256, 0, L.stream>>>(pops, npops);
-    launch_uscan_buckets(L, pops, npops, maxNB);
-    k_rank_scatter<<<g, 256, 0, L.stream>>>(pops, npops);
-    k_rank_final<<<g, 256, 0, L.stream>>>(pops, npops);
-    if (suf) {
-        const uint32_t units = (maxW + 31u) / 32u * kSufSlices;
-        k_suf_build<<<pop_grid(npops, units, L.num_sms, 4), 256, 0, L.stream>>>(pops, npops);
-    }
+uint32_t launch_plan(const LaunchCfg& L, const PopDev* pops, uint32_t npops, const PrepSizes& z, uint32_t maxW) {
+    const uint32_t nr = blocks_for(z.maxA, 256), np = z.tables ? blocks_for(z.maxS, 256) : 0u;
+    const dim3 g = pop_grid(npops, nr + np, L.num_sms, 8);
+    // a slot's rank is a quarter of a row's plan at most
+    const uint32_t nrank = z.tables ? std::max(1u, std::min(nr, g.x / 4u)) : g.x;
+    launch_k(L, k_plan, g, dim3(256), pops, npops, nrank);
+    if (!z.tables) return 1u;
+    const uint32_t units = (maxW + 31u) / 32u * kSufSlices;
+    launch_k(L, k_suf_build, pop_grid(npops, units, L.num_sms, 4), dim3(256), pops, npops);
+    return 2u;
 }
 
 // ---------------------------------------------------------------------------

@@ -1,0 +1,535 @@
+// k_prep.cu -- everything a generation needs before its rows are written, in six
+// kernels: step header, free space, mutation counts and slots, parents, the rows'
+// processing order, and the position buckets of the crossover ranks (the ranks
+// themselves and the rows' plans are k_plan, k_generation.cu).
+//
+// A small population's step is bound by its launches: every dependent launch costs
+// 3 to 4 us however little it does.  So work that does not depend on each other
+// shares a launch (free space beside the mutation counts and the parent draws; both
+// prefix sums beside the new alleles; the rows' order beside the bucket counts), a
+// scan is one kernel (each block sums what lies before its chunk itself, as long as
+// that is at most kDirectScan counts; above, one more launch leaves chunk sums), and
+// every kernel is launched with programmatic dependent launch: its blocks are
+// resident when their predecessor ends.
+//
+// All kernels walk every population of the batch on blockIdx.z; sizes are read from
+// the device status words.
+#include "step.cuh"
+
+#include <algorithm>
+
+namespace clotho {
+
+namespace {
+
+constexpr uint32_t kChunk = 1024;  // counts a scan chunk: 256 threads x 4, or one a thread of a 1,024-thread block
+
+// The step's offspring count: from the header, or (staged calls, after k_begin) from the status.
+__device__ __forceinline__ uint32_t step_N(const PopDev& P, const uint32_t* hdr, uint32_t p) {
+    return hdr ? min(hdr[2u * p], P.Ncap) : P.st->N;
+}
+
+// The rows' ordering keys are parent individuals; rows of an empty parent generation all have key 0.
+__device__ __forceinline__ uint32_t order_keys(uint32_t pN) { return max(pN, 1u); }
+
+// Sum of v over a block of 256 threads, in every thread.
+__device__ __forceinline__ uint32_t block_sum_256(uint32_t v, uint32_t* s8) {
+    v = __reduce_add_sync(0xffffffffu, v);
+    __syncthreads();
+    if ((threadIdx.x & 31u) == 0u) s8[threadIdx.x >> 5] = v;
+    __syncthreads();
+    uint32_t t = 0;
+#pragma unroll
+    for (uint32_t i = 0; i < 8; ++i) t += s8[i];
+    return t;
+}
+
+// One chunk of an exclusive prefix sum over cnt[0, L): off (and cur, when given: scatter cursors) of the
+// chunk's elements.  What lies before the chunk is summed from the counts (direct) or from the chunk sums.
+// Returns the inclusive total at the chunk's end, in every thread.
+__device__ __forceinline__ uint32_t scan_chunk(const uint32_t* cnt, const uint32_t* part, bool direct, uint32_t L,
+                                               uint32_t c, uint32_t* off, uint32_t* cur, uint32_t* s8) {
+    uint32_t v = 0;
+    if (direct) {
+        const uint4* q = reinterpret_cast<const uint4*>(cnt);
+        for (uint32_t i = threadIdx.x; i < c * (kChunk / 4u); i += 256u) {
+            const uint4 x = q[i];
+            v += (x.x + x.y) + (x.z + x.w);
+        }
+    } else {
+        for (uint32_t i = threadIdx.x; i < c; i += 256u) v += part[i];
+    }
+    uint32_t run = block_sum_256(v, s8);
+    const uint32_t b = c * kChunk + threadIdx.x * 4u;
+    uint32_t x[4];
+    if (b + 4u <= L) {
+        const uint4 q = *reinterpret_cast<const uint4*>(cnt + b);
+        x[0] = q.x; x[1] = q.y; x[2] = q.z; x[3] = q.w;
+    } else {
+#pragma unroll
+        for (uint32_t k = 0; k < 4; ++k) x[k] = (b + k < L) ? cnt[b + k] : 0u;
+    }
+    const uint32_t s = (x[0] + x[1]) + (x[2] + x[3]);
+    uint32_t incl = s;
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= (uint32_t)o) incl += y;
+    }
+    __syncthreads();  // block_sum_256's reads of s8 are done
+    if (lane == 31u) s8[warp] = incl;
+    __syncthreads();
+    uint32_t total = run;
+#pragma unroll
+    for (uint32_t i = 0; i < 8; ++i) {
+        if (i < warp) run += s8[i];
+        total += s8[i];
+    }
+    run += incl - s;
+    const uint32_t o4[4] = {run, run + x[0], run + x[0] + x[1], run + x[0] + x[1] + x[2]};
+    if (b + 4u <= L) {
+        if (off) *reinterpret_cast<uint4*>(off + b) = make_uint4(o4[0], o4[1], o4[2], o4[3]);
+        if (cur) *reinterpret_cast<uint4*>(cur + b) = make_uint4(o4[0], o4[1], o4[2], o4[3]);
+    } else {
+#pragma unroll
+        for (uint32_t k = 0; k < 4; ++k)
+            if (b + k < L) {
+                if (off) off[b + k] = o4[k];
+                if (cur) cur[b + k] = o4[k];
+            }
+    }
+    return total;
+}
+
+// Parents of individual k (SelectionGenerator::update, general_fitness_selection_generator.hpp:45-69): uniform
+// when every fitness is equal, else the FP64 inclusive prefix sum and an upper_bound per draw.
+__device__ __forceinline__ uint2 draw_parents(const PopDev& P, uint32_t k, uint32_t Np, uint32_t gen, bool uni,
+                                              double total) {
+    const U4 x = philox4x32(k, 0u, gen, kStreamSelect, P.seed);
+    const double u[2] = {u01(x.x, x.y), u01(x.z, x.w)};
+    uint32_t id[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        if (Np == 0) id[h] = 0;
+        else if (uni) {
+            id[h] = (uint32_t)(u[h] * (double)Np);
+            if (id[h] >= Np) id[h] = Np - 1u;
+        }
+    }
+    if (Np != 0 && !uni) {
+        // first i with cdf[i] > target (both >= +0: integer compares); the two searches go side by side
+        const double t0 = u[0] * total, t1 = u[1] * total;
+        uint32_t lo0 = 0, hi0 = Np, lo1 = 0, hi1 = Np;
+        while ((lo0 < hi0) | (lo1 < hi1)) {
+            const uint32_t m0 = (lo0 + hi0) >> 1, m1 = (lo1 + hi1) >> 1;
+            const double c0 = P.cdf[min(m0, Np - 1u)], c1 = P.cdf[min(m1, Np - 1u)];
+            if (lo0 < hi0) {
+                if (lt_nonneg(t0, c0)) hi0 = m0; else lo0 = m0 + 1u;
+            }
+            if (lo1 < hi1) {
+                if (lt_nonneg(t1, c1)) hi1 = m1; else lo1 = m1 + 1u;
+            }
+        }
+        id[0] = lo0 >= Np ? Np - 1u : lo0;
+        id[1] = lo1 >= Np ? Np - 1u : lo1;
+    }
+    return make_uint2(id[0], id[1]);
+}
+
+// Blocks [0, a) of a population's gridDim.x take the first of a kernel's two independent jobs, the rest the
+// second; a single block takes both.
+struct Share {
+    uint32_t i, n;
+    bool on;
+};
+__device__ __forceinline__ Share first_share(uint32_t a) {
+    if (gridDim.x == 1u) return Share{0u, 1u, true};
+    return Share{blockIdx.x, a, blockIdx.x < a};
+}
+__device__ __forceinline__ Share second_share(uint32_t a) {
+    if (gridDim.x == 1u) return Share{0u, 1u, true};
+    return Share{blockIdx.x - a, gridDim.x - a, blockIdx.x >= a};
+}
+
+}  // namespace
+
+// ---------------------------------------------------------------------------
+// Stage 1.  Block 0 of a population: the step header (the child becomes the parent,
+// engine_batched_task.hpp:164; the sizes of the parent move to pN, pA, pW here, those of
+// the child are written by stage 2, so that nobody reads what another block writes) and
+// the free-space analysis of the parent.  The other blocks: device-drawn mutation counts
+// with their chunk sums, or the tape's counted per row; parents, counted per parent for
+// the rows' processing order.
+//
+// Device-drawn mutation counts are Poisson(mu) per offspring row.  The sum over
+// rows is Poisson(2N mu) and, given the total, the rows are uniform -- the
+// same law as M ~ Poisson(mu * 2N) with uniform target rows
+// (mutation_allocator.hpp:41-47, batch_mutation_task_population_space_row.hpp:77).
+__global__ void __launch_bounds__(1024) k_stage1(const PopDev* __restrict__ pops, uint32_t npops,
+                                                 const uint32_t* __restrict__ hdr, WorkCtl* ctl, uint32_t what,
+                                                 uint32_t count_on) {
+    __shared__ uint32_t s_u32[33];
+    pdl_wait();
+    pdl_go();
+    for (uint32_t p = blockIdx.z; p < npops; p += gridDim.z) {
+        const PopDev& P = pops[p];
+        DevStatus* st = P.st;
+        const bool philox = P.mode == kModePhilox;
+        const uint32_t N = step_N(P, hdr, p), S = 2u * N;
+        if (blockIdx.x == 0) {
+            if (!(what & kStepBegin)) continue;
+            const uint32_t pN = st->N, pA = st->A, pW = st->W;
+            fs_finalize_block(P, pN, pA, pW, count_on != 0u);
+            if (threadIdx.x == 0) {
+                uint32_t err = 0, M = hdr[2u * p + 1u];
+                if (hdr[2u * p] > P.Ncap) err |= kErrAlleles;
+                if (M > P.Mcap) { err |= kErrMut; M = P.Mcap; }
+                if (err) atomicOr(&st->err, err);
+                st->pN = pN;
+                st->pA = pA;
+                st->pW = pW;
+                st->M = M;
+                st->ev_used = 0;
+            }
+            __syncthreads();
+            continue;
+        }
+        const uint32_t bx = blockIdx.x - 1u, nb = gridDim.x - 1u;
+        if (p == 0 && bx == 0 && (what & kStepBegin)) begin_items(pops, npops, hdr, ctl);
+        if (what & kStepMut) {
+            if (philox) {
+                const uint32_t gen = st->gen;
+                const double* cdf = P.pois_mu;
+                for (uint32_t c = bx; c * kChunk < S; c += nb) {
+                    const uint32_t r = c * kChunk + threadIdx.x;
+                    uint32_t n = 0;
+                    if (r < S) {
+                        const U4 x = philox4x32(r, 0u, gen, kStreamMutCount, P.seed);
+                        n = poisson_tab(u01(x.x, x.y), cdf, cdf[kPoisTab], P.mu);
+                        P.row_cnt[r] = n;
+                    }
+                    n = __reduce_add_sync(0xffffffffu, n);
+                    if ((threadIdx.x & 31u) == 0u) s_u32[threadIdx.x >> 5] = n;
+                    __syncthreads();
+                    if (threadIdx.x < 32u) {
+                        n = __reduce_add_sync(0xffffffffu, s_u32[threadIdx.x]);
+                        if (threadIdx.x == 0) P.scan_upart[c] = n;
+                    }
+                    __syncthreads();
+                }
+            } else {
+                const uint32_t M = min(hdr[2u * p + 1u], P.Mcap);
+                for (uint32_t i = bx * 1024u + threadIdx.x; i < M; i += nb * 1024u) {
+                    const uint32_t s = P.mut_seq[i];
+                    if (s >= S) { atomicOr(&st->err, kErrSeq); continue; }
+                    atomicAdd(&P.row_cnt[s], 1u);
+                }
+            }
+        }
+        if (what & kStepOrder) {
+            const uint32_t Np = hdr ? st->N : st->pN;  // staged calls have moved the sizes already
+            uint32_t* const cnt = P.plan_row ? P.ord_cnt : nullptr;
+            if (philox && (what & kStepSelect)) {
+                const bool uni = st->fit_const != 0u || !(st->fit_total > 0.0);
+                const double total = st->fit_total;
+                const uint32_t gen = st->gen;
+                for (uint32_t k = bx * 1024u + threadIdx.x; k < N; k += nb * 1024u) {
+                    const uint2 id = draw_parents(P, k, Np, gen, uni, total);
+                    *reinterpret_cast<uint2*>(P.pairs + 2u * k) = id;
+                    if (cnt) {
+                        atomicAdd(cnt + id.x, 1u);
+                        atomicAdd(cnt + id.y, 1u);
+                    }
+                }
+            } else if (cnt) {
+                for (uint32_t g = bx * 1024u + threadIdx.x; g < S; g += nb * 1024u) {
+                    const uint32_t id = P.pairs[g];
+                    atomicAdd(cnt + (id < Np ? id : 0u), 1u);
+                }
+            }
+        }
+    }
+}
+
+// Chunk sums of the counts that a scan cannot sum by itself (which == 0: new alleles per row, 1: rows per
+// parent, 2: positions per bucket).
+__global__ void __launch_bounds__(256) k_chunk_sums(const PopDev* __restrict__ pops, uint32_t npops,
+                                                    const uint32_t* __restrict__ hdr, uint32_t which) {
+    __shared__ uint32_t s8[8];
+    pdl_wait();
+    pdl_go();
+    for (uint32_t p = blockIdx.z; p < npops; p += gridDim.z) {
+        const PopDev& P = pops[p];
+        const uint32_t L = which == 0 ? 2u * step_N(P, hdr, p) : which == 1 ? order_keys(P.st->pN) : P.NB;
+        const uint32_t* cnt = which == 0 ? P.row_cnt : which == 1 ? P.ord_cnt : P.bcnt;
+        uint32_t* part = which == 1 ? P.scan_opart : P.scan_upart;
+        if (!cnt) continue;
+        for (uint32_t c = blockIdx.x; c * kChunk < L; c += gridDim.x) {
+            uint32_t v = 0;
+#pragma unroll
+            for (uint32_t k = 0; k < 4; ++k) {
+                const uint32_t i = c * kChunk + 256u * k + threadIdx.x;
+                if (i < L) v += cnt[i];
+            }
+            v = block_sum_256(v, s8);
+            if (threadIdx.x == 0) part[c] = v;
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------
+// Stage 2.  The prefix sums of the new alleles per row and of the rows per parent, and
+// the new alleles themselves: mutation i takes free_indices[i]; beyond the free list new
+// slots are appended at the parent allele count (batch_mutation_mt.hpp:69-80).  Writes
+// the allele table (AlleleGenerator, allele_generator_vector.hpp:76-83) and the trait
+// table (TraitSpaceGenerator2, trait_space_generator.hpp:118-129).  One thread per new
+// allele and trait, neighbours in different blocks: a drawn effect is about a hundred
+// operations of the narrow FP64 pipe, so they are spread over all SMs.
+__global__ void __launch_bounds__(256) k_stage2(const PopDev* __restrict__ pops, uint32_t npops,
+                                                const uint32_t* __restrict__ hdr, uint32_t what, uint32_t direct_max,
+                                                uint32_t nres) {
+    __shared__ uint32_t s8[8];
+    pdl_wait();
+    pdl_go();
+    for (uint32_t p = blockIdx.z; p < npops; p += gridDim.z) {
+        const PopDev& P = pops[p];
+        DevStatus* st = P.st;
+        const bool philox = P.mode == kModePhilox;
+        const uint32_t N = step_N(P, hdr, p), S = 2u * N;
+        const Share res = first_share(nres), scan = second_share(nres);
+        if (res.on && (what & kStepMut)) {
+            uint32_t M = 0;
+            if (philox) {  // stage 1 left the chunk sums
+                for (uint32_t i = threadIdx.x; i * kChunk < S; i += 256u) M += P.scan_upart[i];
+                M = block_sum_256(M, s8);
+            } else {
+                M = st->M;
+            }
+            const uint32_t Mraw = M;
+            M = min(M, P.Mcap);
+            const uint32_t fr = st->free_cnt, pA = st->pA, gen = st->gen, T = P.T;
+            const uint32_t Ac = pA + (M > fr ? M - fr : 0u), A = min(Ac, P.Acap);
+            if (res.i == 0 && threadIdx.x == 0) {
+                if (Ac > P.Acap) atomicOr(&st->err, kErrAlleles);
+                if (Mraw > P.Mcap) atomicOr(&st->err, kErrMut);
+                st->N = N;
+                st->A = A;
+                st->W = ref_width(A);
+                st->cur ^= 1u;
+                if (philox) st->M = M;
+            }
+            int nz_delta = 0;
+            for (uint64_t q = (uint64_t)threadIdx.x * res.n + res.i; q < (uint64_t)M * T; q += 256ull * res.n) {
+                const uint32_t i = (uint32_t)(q / T), t = (uint32_t)(q % T);
+                nz_delta += resolve_mutation(P, i, t, gen, fr, pA, A);
+            }
+            if (nz_delta) atomicAdd(&st->nz_eff, nz_delta);
+            __syncthreads();
+        }
+        if (!scan.on) continue;
+        // units: the row chunks, then the parent chunks
+        const uint32_t keys = order_keys(st->pN);
+        const uint32_t nr = (what & kStepMut) ? S / kChunk + 1u : 0u;
+        const uint32_t no = ((what & kStepOrder) && P.plan_row) ? (keys + kChunk - 1u) / kChunk : 0u;
+        for (uint32_t u = scan.i; u < nr + no; u += scan.n) {
+            if (u < nr) {
+                const uint32_t total = scan_chunk(P.row_cnt, P.scan_upart, !philox && S <= direct_max, S, u, P.row_off,
+                                                  philox ? nullptr : P.row_cur, s8);
+                if (u == nr - 1u && threadIdx.x == 0) P.row_off[S] = total;
+            } else {
+                scan_chunk(P.ord_cnt, P.scan_opart, keys <= direct_max, keys, u - nr, nullptr, P.ord_cur, s8);
+            }
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------
+// Stage 3.  Positions per bucket (the first step of the slots' ranks), the rows' processing
+// positions (parent-major order: rows sorted by parent individual, so rows reading the
+// same parent strands run side by side and the second read of a strand is an L2 hit;
+// the order inside one parent does not matter), the tape's new alleles grouped by row;
+// the counts of stage 1 go back to zero.
+__global__ void __launch_bounds__(256) k_stage3(const PopDev* __restrict__ pops, uint32_t npops, uint32_t what) {
+    pdl_wait();
+    pdl_go();
+    for (uint32_t p = blockIdx.z; p < npops; p += gridDim.z) {
+        const PopDev& P = pops[p];
+        const DevStatus* st = P.st;
+        const uint32_t at = blockIdx.x * 256u + threadIdx.x, step = gridDim.x * 256u;
+        const uint32_t A = st->A, N = st->N, pN = st->pN, S = 2u * N;
+        for (uint32_t s = at; s < A; s += step) atomicAdd(&P.bcnt[pos_bucket(P.pos[s], P.NB)], 1u);
+        if ((what & kStepOrder) && P.plan_row) {
+            for (uint32_t g = at; g < S; g += step) {
+                const uint32_t id = P.pairs[g];
+                P.ord_pos[g] = atomicAdd(&P.ord_cur[id < pN ? id : 0u], 1u);
+            }
+            for (uint32_t k = at; k < order_keys(pN); k += step) P.ord_cnt[k] = 0u;
+        }
+        if (what & kStepMut) {
+            if (P.mode != kModePhilox) {
+                const uint32_t M = st->M;
+                for (uint32_t i = at; i < M; i += step) {
+                    const uint32_t s = P.mut_seq[i];
+                    if (s < S) P.row_mut[atomicAdd(&P.row_cur[s], 1u)] = i;
+                }
+            }
+            for (uint32_t r = at; r < S; r += step) P.row_cnt[r] = 0u;
+        }
+    }
+}
+
+// Ascending order of a[0..n): insertion sort for short lists, heapsort beyond
+// (a tape may send many mutations to one row).
+static __device__ void sort_ascending(uint32_t* a, uint32_t n) {
+    if (n <= 16u) {
+        for (uint32_t i = 1; i < n; ++i) {
+            const uint32_t x = a[i];
+            uint32_t j = i;
+            for (; j > 0 && a[j - 1] > x; --j) a[j] = a[j - 1];
+            a[j] = x;
+        }
+        return;
+    }
+    auto sift = [a](uint32_t r, uint32_t end) {
+        const uint32_t x = a[r];
+        for (uint32_t c = 2u * r + 1u; c < end; c = 2u * r + 1u) {
+            if (c + 1u < end && a[c + 1u] > a[c]) ++c;
+            if (a[c] <= x) break;
+            a[r] = a[c];
+            r = c;
+        }
+        a[r] = x;
+    };
+    for (uint32_t r = n / 2u; r-- > 0;) sift(r, n);
+    for (uint32_t end = n - 1u; end > 0; --end) {
+        const uint32_t x = a[0];
+        a[0] = a[end];
+        a[end] = x;
+        sift(0, end);
+    }
+}
+
+// ---------------------------------------------------------------------------
+// Stage 4.  The prefix sum of the positions per bucket, and each tape row's new alleles in
+// ascending mutation index (the list order is the order in which their FP32 effects
+// enter the row's carried phenotype, so it must not depend on the order of the
+// scatter's atomics).  One thread per list position; the thread at a row's first
+// position sorts the row's list: ownership is decided by position, which never moves,
+// and every entry of a row's segment names that row, so no other thread acts on it.
+__global__ void __launch_bounds__(256) k_stage4(const PopDev* __restrict__ pops, uint32_t npops, uint32_t what,
+                                                uint32_t direct_max) {
+    __shared__ uint32_t s8[8];
+    pdl_wait();
+    pdl_go();
+    for (uint32_t p = blockIdx.z; p < npops; p += gridDim.z) {
+        const PopDev& P = pops[p];
+        for (uint32_t c = blockIdx.x; c * kChunk < P.NB; c += gridDim.x) {
+            const uint32_t total = scan_chunk(P.bcnt, P.scan_upart, P.NB <= direct_max, P.NB, c, P.boff, P.bcur, s8);
+            if ((c + 1u) * kChunk >= P.NB && threadIdx.x == 0) P.boff[P.NB] = total;
+        }
+        if ((what & kStepMut) && P.mode != kModePhilox) {
+            const uint32_t listed = P.row_off[2u * P.st->N];
+            for (uint32_t t = blockIdx.x * 256u + threadIdx.x; t < listed; t += gridDim.x * 256u) {
+                const uint32_t s = P.mut_seq[P.row_mut[t]];
+                const uint32_t off = P.row_off[s], n = P.row_off[s + 1u] - off;
+                if (t == off && n >= 2u) sort_ascending(P.row_mut + off, n);
+            }
+        }
+    }
+}
+
+// Stage 5.  Positions and slots grouped by bucket; the bucket counts go back to zero.
+__global__ void __launch_bounds__(256) k_stage5(const PopDev* __restrict__ pops, uint32_t npops) {
+    pdl_wait();
+    pdl_go();
+    for (uint32_t p = blockIdx.z; p < npops; p += gridDim.z) {
+        const PopDev& P = pops[p];
+        const uint32_t at = blockIdx.x * 256u + threadIdx.x, step = gridDim.x * 256u;
+        const uint32_t A = P.st->A;
+        for (uint32_t s = at; s < A; s += step) {
+            const double x = P.pos[s];
+            const uint32_t k = atomicAdd(&P.bcur[pos_bucket(x, P.NB)], 1u);
+            P.bpos[k] = x;
+            P.bslot[k] = s;
+        }
+        for (uint32_t b = at; b < P.NB; b += step) P.bcnt[b] = 0u;
+    }
+}
+
+uint32_t launch_prep(const LaunchCfg& L, const PopDev* pops, uint32_t npops, const PrepSizes& z, const uint32_t* hdr,
+                     WorkCtl* ctl, uint32_t what, bool count_on) {
+    // up to this many counts a scan block sums what lies before its chunk by itself: at 32,768 counts the last
+    // block reads 128 KB of L2, about as long as the extra launch that it saves
+    constexpr uint32_t kDirectScan = 32768;
+    uint32_t n = 0;
+    if (what & (kStepBegin | kStepMut | kStepOrder)) {
+        dim3 g = pop_grid(npops, blocks_for(z.maxS, kChunk), L.num_sms, std::max(1u, L.ind_per_sm / 4u));
+        g.x += 1u;
+        launch_k(L, k_stage1, g, dim3(1024), pops, npops, hdr, ctl, what, count_on ? 1u : 0u);
+        ++n;
+        // chunk sums: of the tape's counts (device draws leave their own in stage 1), of the rows per parent
+        if ((what & kStepMut) && (what & kStepTape) && z.maxS > kDirectScan) {
+            launch_k(L, k_chunk_sums, pop_grid(npops, blocks_for(z.maxS, kChunk), L.num_sms, 4), dim3(256), pops, npops,
+                     hdr, 0u);
+            ++n;
+        }
+        if ((what & kStepOrder) && z.tables && z.maxN > kDirectScan) {
+            launch_k(L, k_chunk_sums, pop_grid(npops, blocks_for(z.maxN, kChunk), L.num_sms, 4), dim3(256), pops, npops,
+                     hdr, 1u);
+            ++n;
+        }
+        const uint32_t units = blocks_for(z.maxS + 1u, kChunk) + blocks_for(z.maxN, kChunk);
+        g = pop_grid(npops, units + (uint32_t)L.num_sms, L.num_sms, 6);
+        launch_k(L, k_stage2, g, dim3(256), pops, npops, hdr, what, kDirectScan, std::max(1u, g.x / 3u));
+        ++n;
+    }
+    launch_k(L, k_stage3, pop_grid(npops, blocks_for(std::max(z.maxS, z.maxA), 256), L.num_sms, 8), dim3(256), pops,
+             npops, what);
+    if (z.maxNB > kDirectScan) {
+        launch_k(L, k_chunk_sums, pop_grid(npops, blocks_for(z.maxNB, kChunk), L.num_sms, 4), dim3(256), pops, npops,
+                 hdr, 2u);
+        ++n;
+    }
+    launch_k(L, k_stage4, pop_grid(npops, blocks_for(z.maxNB, kChunk), L.num_sms, 4), dim3(256), pops, npops, what,
+             kDirectScan);
+    launch_k(L, k_stage5, pop_grid(npops, blocks_for(std::max(z.maxNB, z.maxA), 256), L.num_sms, 8), dim3(256), pops,
+             npops);
+    return n + 3u;
+}
+
+// ---------------------------------------------------------------------------
+// A population's Poisson CDF tables, made once with it (thread 0: breakpoints per gamete, thread 1: new alleles
+// per row): 64 dependent FP64 steps, 10 us, that a block of the plan kernel would otherwise spend each generation.
+__global__ void k_pois_tables(PopDev P) {
+    if (threadIdx.x > 1u) return;
+    const double lambda = threadIdx.x ? P.mu : P.rho;
+    double* t = threadIdx.x ? P.pois_mu : P.pois_rho;
+    double pk = threadIdx.x ? P.exp_neg_mu : P.exp_neg_rho, F = pk;
+    t[0] = F;
+    for (uint32_t k = 1; k < kPoisTab; ++k) {
+        poisson_step(pk, F, lambda, k);
+        t[k] = F;
+    }
+    t[kPoisTab] = pk;
+}
+void launch_pois_tables(cudaStream_t s, const PopDev& P) { k_pois_tables<<<1, 32, 0, s>>>(P); }
+
+int init_recip_prep() { return fill_recip_table(); }
+
+// ---------------------------------------------------------------------------
+// Parent sampling on its own (staged API).
+__global__ void k_select_philox(const PopDev* __restrict__ pops, uint32_t npops) {
+    for (uint32_t p = blockIdx.z; p < npops; p += gridDim.z) {
+        const PopDev& P = pops[p];
+        const DevStatus* st = P.st;
+        const bool uni = st->fit_const != 0u || !(st->fit_total > 0.0);
+        for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < st->N; k += gridDim.x * blockDim.x)
+            *reinterpret_cast<uint2*>(P.pairs + 2u * k) = draw_parents(P, k, st->pN, st->gen, uni, st->fit_total);
+    }
+}
+void launch_select_philox(const LaunchCfg& L, const PopDev* pops, uint32_t npops) {
+    k_select_philox<<<pop_grid(npops, L.num_sms * 2u, L.num_sms, L.ind_per_sm), 256, 0, L.stream>>>(pops, npops);
+}
+
+}  // namespace clotho
