@@ -1055,6 +1055,311 @@ __device__ __forceinline__ bool gen_row_suf(const PopDev& P, const DevStatus& st
 }
 
 // ---------------------------------------------------------------------------
+// Short rows (parent and child at most 32 words): several rows a warp.
+//
+// A row of 8, 16 or 32 words fills 4, 8 or 16 lanes of two words each; one row a warp
+// leaves the other lanes idle and pays the row's set-up (plan, breakpoints, corrections,
+// reductions: several hundred instructions) for them as well.  Here L lanes take a row and
+// a warp 32 / L rows.  The switch mask stays in the lanes' registers, the corrections and
+// the new alleles go through a 2L-word bitmap per row, the AND/OR of the children is kept in registers
+// until the rows run out.  What bounds it is instruction issue: the set-up per warp, now shared.
+//
+// The phenotype is the one-row-a-warp form's to the bit: that form's lane v adds the row's
+// entries v, v + 32, ... one after another and then the lanes are summed by a butterfly; here
+// lane l holds the partial sums of the lanes l, l + L, ... and adds them in the same tree.
+template <uint32_t L>
+__device__ __forceinline__ void group_loop(const PopDev& P, uint32_t r0, uint32_t r1, uint32_t* next, uint32_t u0,
+                                           uint32_t us, uint32_t* crows, const uint64_t* sfix, uint32_t* gm,
+                                           uint32_t* Qw, uint64_t* sF, uint64_t* sV, uint64_t* cnt, uint32_t stride,
+                                           uint32_t fuse) {
+    constexpr uint32_t VL = 32u / L;        // rows a warp, and lanes of the one-row form that a lane stands for
+    constexpr uint32_t kWin = 16u * L;      // queue entries of a row (a multiple of 32)
+    constexpr uint32_t kFull = 0xffffffffu;
+    const uint32_t lane = threadIdx.x & 31u, l = lane & (L - 1u), sub = lane / L;
+    const bool do_mut = (fuse & kFuseMut) != 0, do_ph = (fuse & kFusePheno) != 0, do_fs = (fuse & kFuseFs) != 0;
+    const uint32_t Wc = P.st->W, Wp = P.st->pW, M = P.st->M, T = P.T;
+    const bool gather = do_ph && P.st->nz_eff != 0;
+    const bool philox = P.mode == kModePhilox;
+    const uint64_t* const prow = P.rows[P.st->cur ^ 1u];
+    uint64_t* const crow = P.rows[P.st->cur];
+    double* const zout = P.zg[P.st->cur];
+    const float4* const eff4 = reinterpret_cast<const float4*>(P.eff);
+    uint32_t* const gb = gm + sub * (4u * L);   // the row's bitmap, zero between uses
+    uint32_t* const Q = Qw + sub * kWin;
+    const uint32_t w = 2u * l;
+    ulonglong2 fm = make_ulonglong2(0, 0);
+    if (w < Wp) fm = *reinterpret_cast<const ulonglong2*>(sfix + w);
+    uint64_t F0 = ~0ull, F1 = ~0ull, V0 = 0ull, V1 = 0ull;
+    const uint32_t units = (r1 - r0 + VL - 1u) / VL;
+    uint32_t u = u0;
+    if (next) {
+        if (lane == 0) u = atomicAdd(next, 1u);
+        u = __shfl_sync(kFull, u, 0);
+    }
+    while (u < units) {
+        // the next rows are claimed, and their plans fetched into L1, behind these
+        uint32_t un = u + us;
+        if (next && lane == 0) un = atomicAdd(next, 1u);
+        const uint32_t v = r0 + u * VL + sub;
+        const bool live = v < r1;
+        uint4 pr = make_uint4(0, 0, 0, 0);
+        uint2 pm = make_uint2(0, 0);
+        double pz = 0.0;
+        if (live) {
+            pr = __ldg(P.plan_row + v);
+            if (do_mut) pm = __ldg(P.plan_mut + v);
+            if (do_ph && l < kMaxTraits) pz = __ldg(P.plan_z + (size_t)v * 4u + l);
+        }
+        un = __shfl_sync(kFull, un, 0);
+        if (r0 + un * VL + sub < r1 && un < units && l < 3u) {
+            const uint32_t vn = r0 + un * VL + sub;
+            const void* a = l == 0   ? (const void*)(P.plan_row + vn)
+                            : l == 1 ? (const void*)(P.plan_mut + vn)
+                                     : (const void*)(P.plan_z + (size_t)vn * 4u);
+            asm volatile("prefetch.global.L1 [%0];" ::"l"(a));
+        }
+        const uint32_t topr = pr.y, base = pr.z, E = pr.w & kPlanMaxEvents, flags = pr.w >> kPlanFlagShift;
+        const bool inv = gather && (flags & kPlanInv) != 0, isl = (flags & kPlanLong) != 0;
+        ulonglong2 t = make_ulonglong2(0, 0), b = make_ulonglong2(0, 0);
+        if (live && w < Wp) {
+            t = __ldg(reinterpret_cast<const ulonglong2*>(prow + (size_t)topr * P.Wcap + w));
+            if (E) b = __ldg(reinterpret_cast<const ulonglong2*>(prow + (size_t)(topr ^ 1u) * P.Wcap + w));
+        }
+        // the new alleles' effects
+        float acc[VL][kMaxTraits];
+#pragma unroll
+        for (uint32_t j = 0; j < VL; ++j)
+#pragma unroll
+            for (uint32_t k = 0; k < kMaxTraits; ++k) acc[j][k] = 0.f;
+        const uint32_t mo = pm.x, mc = pm.y;
+        const uint32_t mcm = __reduce_max_sync(kFull, mc);
+        bool any = false;
+        auto add_effects = [&](float (&d)[kMaxTraits], const float4& e) {
+            d[0] += e.x;
+            d[1] += e.y;
+            d[2] += e.z;
+            d[3] += e.w;
+        };
+        auto new_slot = [&](uint32_t j) {
+            const uint32_t i = mo + j, mi = philox ? i : P.row_mut[i];
+            return mi < M ? P.mut_slot[mi] : 0xffffffffu;
+        };
+        uint32_t ms0 = 0xffffffffu;   // the lane's first new allele
+        if (mcm) {
+#pragma unroll
+            for (uint32_t j = 0; j < VL; ++j) {
+                if (l + L * j < mc) {
+                    const uint32_t s = new_slot(l + L * j);
+                    if (j == 0) ms0 = s;
+                    if (gather && s != 0xffffffffu) add_effects(acc[j], __ldg(eff4 + s));
+                }
+                if (L * (j + 1u) >= mcm) break;
+            }
+            if (gather && mc > 32u && l == 0)
+                for (uint32_t j = 32; j < mc; ++j) {
+                    const uint32_t s = new_slot(j);
+                    if (s != 0xffffffffu) add_effects(acc[0], __ldg(eff4 + s));
+                }
+            any = gather;
+        }
+        // the switch mask: table rows in registers, correction slots through the bitmap
+        uint64_t m0 = 0, m1 = 0;
+        const uint32_t Em = __reduce_max_sync(kFull, isl ? 0u : E);
+        if (Em) {
+            for (uint32_t k0 = 0; k0 < Em; k0 += L) {
+                const bool mine = !isl && k0 + l < E;
+                const uint32_t go = mine ? __ldg(P.plan_go + base + k0 + l) : 0u;
+                const uint32_t cr = mine ? __ldg(P.plan_cr + base + k0 + l) : 0u;
+                const uint32_t ke = min(L, Em - k0);
+#pragma unroll 2
+                for (uint32_t k = 0; k < ke; ++k) {
+                    const uint32_t gk = __shfl_sync(kFull, go, k, L), ck = __shfl_sync(kFull, cr, k, L);
+                    if (!isl && k0 + k < E && w < Wp) {
+                        const ulonglong2 x = __ldg(reinterpret_cast<const ulonglong2*>(P.suf + gk + w));
+                        m0 ^= x.x;
+                        m1 ^= x.y;
+                    }
+                    const uint32_t n = ck >> 20, c0 = ck & 0xfffffu;
+                    uint32_t cs[VL];
+#pragma unroll
+                    for (uint32_t j = 0; j < VL; ++j)
+                        cs[j] = l + L * j < n ? __ldg(P.inv + c0 + l + L * j) : 0xffffffffu;
+#pragma unroll
+                    for (uint32_t j = 0; j < VL; ++j)
+                        if (cs[j] != 0xffffffffu) atomicXor(gb + (cs[j] >> 5), 1u << (cs[j] & 31u));
+                }
+            }
+            __syncwarp();
+            ulonglong2* mw = reinterpret_cast<ulonglong2*>(gb + 4u * l);
+            const ulonglong2 x = *mw;
+            *mw = make_ulonglong2(0, 0);
+            m0 ^= x.x;
+            m1 ^= x.y;
+            __syncwarp();
+        }
+        const uint64_t t0 = t.x & ~fm.x, t1 = t.y & ~fm.y, b0 = b.x & ~fm.x, b1 = b.y & ~fm.y;
+        const uint64_t h0 = E ? t0 ^ b0 : 0ull, h1 = E ? t1 ^ b1 : 0ull;
+        if (isl) {
+            m0 = sw_mask_events(h0, w * 64u, P.pos, P.ev_pos + base, E);
+            m1 = sw_mask_events(h1, w * 64u + 64u, P.pos, P.ev_pos + base, E);
+        }
+        const uint64_t sw0 = m0 & h0, sw1 = m1 & h1;
+        uint64_t x0 = t0 ^ sw0, x1 = t1 ^ sw1;
+        if (gather) {
+            // gathered bits in the one-row form's order: lane after lane, its four 32-bit parts one after
+            // another, highest bit first
+            const uint64_t g0 = inv ? h0 ^ sw0 : sw0, g1 = inv ? h1 ^ sw1 : sw1;
+            const uint32_t c = (uint32_t)(__popcll(g0) + __popcll(g1));
+            uint32_t incl = c;
+#pragma unroll
+            for (uint32_t o = 1; o < L; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(kFull, incl, o, L);
+                if (l >= o) incl += y;
+            }
+            uint32_t H = __shfl_sync(kFull, incl, L - 1u, L);
+            const uint64_t s0 = inv ? t0 : b0, s1 = inv ? t1 : b1;
+            float d[kMaxTraits] = {0.f, 0.f, 0.f, 0.f};
+            const bool add_late = isl;   // rows of very long event lists sum their entries apart from the new alleles
+            float keep[VL][kMaxTraits];
+            const bool late = __any_sync(kFull, add_late);
+            if (late) {
+#pragma unroll
+                for (uint32_t j = 0; j < VL; ++j)
+#pragma unroll
+                    for (uint32_t k = 0; k < kMaxTraits; ++k) {
+                        keep[j][k] = add_late ? acc[j][k] : 0.f;
+                        if (add_late) acc[j][k] = 0.f;
+                    }
+            }
+            if (H > kQueueCap - kRound) {   // denser than the one-row form queues: per-lane chains
+                switched_effects(g0, g1, s0, s1, w * 64u, eff4, d);
+#pragma unroll
+                for (uint32_t k = 0; k < kMaxTraits; ++k) acc[0][k] += d[k];
+                any = true;
+                H = 0;
+            }
+            const uint32_t Hm = __reduce_max_sync(kFull, H);
+            any |= Hm != 0u;
+            const uint32_t gg[4] = {(uint32_t)g0, (uint32_t)(g0 >> 32), (uint32_t)g1, (uint32_t)(g1 >> 32)};
+            const uint32_t ss[4] = {(uint32_t)s0, (uint32_t)(s0 >> 32), (uint32_t)s1, (uint32_t)(s1 >> 32)};
+            for (uint32_t q0 = 0; q0 < Hm; q0 += kWin) {
+                if (H > q0) {
+                    uint32_t i = incl - c - q0;   // entries of other windows fall outside [0, kWin)
+#pragma unroll
+                    for (uint32_t k = 0; k < 4; ++k) {
+                        for (uint32_t x = gg[k]; x;) {
+                            const uint32_t z = (uint32_t)__clz(x);
+                            if (i < kWin) Q[i] = (w * 64u + 32u * k + 31u - z) | ((ss[k] << z) & 0x80000000u);
+                            x ^= 0x80000000u >> z;
+                            ++i;
+                        }
+                    }
+                }
+                __syncwarp();
+                for (uint32_t q = 0; q < kWin && q0 + q < Hm; q += 32u) {
+                    float4 ef[VL];
+                    uint32_t sg = 0;
+#pragma unroll
+                    for (uint32_t j = 0; j < VL; ++j) {
+                        const uint32_t i = q + l + L * j;
+                        const bool ok = q0 + i < H;
+                        const uint32_t e = ok ? Q[i] : 0u;
+                        sg |= (e >> 31) << j;
+                        ef[j] = ok ? __ldg(eff4 + (e & 0x7fffffffu)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    }
+#pragma unroll
+                    for (uint32_t j = 0; j < VL; ++j) {
+                        const float sj = ((sg >> j) & 1u) ? 1.0f : -1.0f;
+                        acc[j][0] = fmaf(sj, ef[j].x, acc[j][0]);
+                        acc[j][1] = fmaf(sj, ef[j].y, acc[j][1]);
+                        acc[j][2] = fmaf(sj, ef[j].z, acc[j][2]);
+                        acc[j][3] = fmaf(sj, ef[j].w, acc[j][3]);
+                    }
+                }
+                __syncwarp();
+            }
+            if (late) {
+#pragma unroll
+                for (uint32_t j = 0; j < VL; ++j)
+#pragma unroll
+                    for (uint32_t k = 0; k < kMaxTraits; ++k)
+                        if (add_late) acc[j][k] = keep[j][k] + acc[j][k];
+            }
+        }
+        if (mcm) {   // the new alleles' bits
+            if (l < mc && ms0 != 0xffffffffu) atomicXor(gb + (ms0 >> 5), 1u << (ms0 & 31u));
+            for (uint32_t j = l + L; j < mc; j += L) {
+                const uint32_t s = new_slot(j);
+                if (s != 0xffffffffu) atomicXor(gb + (s >> 5), 1u << (s & 31u));
+            }
+            __syncwarp();
+            ulonglong2* mw = reinterpret_cast<ulonglong2*>(gb + 4u * l);
+            const ulonglong2 x = *mw;
+            *mw = make_ulonglong2(0, 0);
+            x0 ^= x.x;
+            x1 ^= x.y;
+            __syncwarp();
+        }
+        if (live && w < Wc) {
+            *reinterpret_cast<ulonglong2*>(crow + (size_t)pr.x * P.Wcap + w) = make_ulonglong2(x0, x1);
+            F0 &= x0;
+            F1 &= x1;
+            V0 |= x0;
+            V1 |= x1;
+        }
+        if (cnt) {
+            if (crows) {   // one population: a block counts at most kCountMax rows
+                uint32_t n = 0;
+                if (lane == 0) n = atomicAdd(crows, VL);
+                if (__shfl_sync(kFull, n, 0) + VL > kCountMax) {
+                    if (lane == 0) atomicAnd(&P.st->cols_valid, 0u);
+                    cnt = nullptr;
+                }
+            }
+            if (cnt && live && w < Wc) count_add(cnt, stride, w, x0, x1);
+        }
+        if (do_ph) {
+            float z = 0.f;
+            if (__any_sync(kFull, any)) {
+#pragma unroll
+                for (uint32_t k = 0; k < kMaxTraits; ++k) {
+                    if (k >= T) break;
+#pragma unroll
+                    for (uint32_t o = VL / 2u; o > 0; o >>= 1)
+#pragma unroll
+                        for (uint32_t j = 0; j < o; ++j) acc[j][k] += acc[j + o][k];
+                    float x = acc[0][k];
+#pragma unroll
+                    for (uint32_t o = L / 2u; o > 0; o >>= 1) x += __shfl_xor_sync(kFull, x, o);
+                    if (l == k) z = x;
+                }
+            }
+            if (live && l < kMaxTraits) zout[(size_t)pr.x * 4u + l] = pz + (double)z;
+        }
+        u = un;
+    }
+    if (do_fs && w < Wc) {
+        if (~F0) atomicAnd((unsigned long long*)&sF[w], (unsigned long long)F0);
+        if (~F1) atomicAnd((unsigned long long*)&sF[w + 1u], (unsigned long long)F1);
+        if (V0) atomicOr((unsigned long long*)&sV[w], (unsigned long long)V0);
+        if (V1) atomicOr((unsigned long long*)&sV[w + 1u], (unsigned long long)V1);
+    }
+}
+
+constexpr uint32_t kGroupWords = 32;   // widest rows that share a warp
+
+// The rows [r0, r1) of the processing order, units of 32 / L rows claimed from *next, or u0, u0 + us, ....
+__device__ __noinline__ void group_rows(const PopDev& P, uint32_t r0, uint32_t r1, uint32_t* next, uint32_t u0,
+                                        uint32_t us, uint32_t* crows, const uint64_t* sfix, uint64_t* mask, uint32_t* Q,
+                                        uint64_t* sF, uint64_t* sV, uint64_t* cnt, uint32_t stride, uint32_t fuse) {
+    const uint32_t W = max(P.st->W, P.st->pW);
+    uint32_t* gm = reinterpret_cast<uint32_t*>(mask);
+    if (W <= 8u) group_loop<4>(P, r0, r1, next, u0, us, crows, sfix, gm, Q, sF, sV, cnt, stride, fuse);
+    else if (W <= 16u) group_loop<8>(P, r0, r1, next, u0, us, crows, sfix, gm, Q, sF, sV, cnt, stride, fuse);
+    else group_loop<16>(P, r0, r1, next, u0, us, crows, sfix, gm, Q, sF, sV, cnt, stride, fuse);
+}
+
+// ---------------------------------------------------------------------------
 // Interval classifier (allele spaces beyond the suffix table).
 
 // Sorted breakpoint thresholds of one gamete as half-open rank intervals:
@@ -1409,8 +1714,15 @@ k_generation(const PopDev* __restrict__ pops, uint32_t npops, WorkCtl* __restric
         // the next claim is taken before the current rows run, so its
         // round trip to the counter is hidden behind them
         uint32_t claim = 0;
-        if (lane == 0) claim = atomicAdd(&ctl->gen_counter, kWarpChunk);
-        for (;;) {
+        const bool group = SUF && NARROW && !PROF && max(st.W, st.pW) <= kGroupWords;
+        if (group) {   // rows that share a warp cost about the same: no claims
+            group_rows(P, 0u, S, nullptr, warp * gridDim.x + blockIdx.x, gridDim.x * kWarps, cur_cnt ? &s_crows : nullptr,
+                       sfix, mask, ws.q, sF, sV, fo.cnt, maxW, fuse);
+            if (profile && blockIdx.x == 0 && threadIdx.x == 0) { rows_done = S; words_done = (uint64_t)S * st.W; }
+        } else if (lane == 0) {
+            claim = atomicAdd(&ctl->gen_counter, kWarpChunk);
+        }
+        for (; !group;) {
             const uint32_t k = __shfl_sync(0xffffffffu, claim, 0);
             if (k >= S) break;
             if (lane == 0) claim = atomicAdd(&ctl->gen_counter, kWarpChunk);
@@ -1518,8 +1830,14 @@ k_generation(const PopDev* __restrict__ pops, uint32_t npops, WorkCtl* __restric
         // narrow build: each warp claims its next row one ahead and fetches that row's plan entries into L1
         // behind the current row (narrow rows are bound by their chains of dependent loads)
         uint32_t kc = 0;
-        if (NARROW && lane == 0) kc = atomicAdd(&s_next, 1u);
-        for (;;) {
+        const bool group = SUF && NARROW && !PROF && max(st.W, st.pW) <= kGroupWords;
+        if (group) {
+            group_rows(P, r0, r1, &s_next, 0u, 0u, nullptr, sfix, mask, ws.q, sF, sV, fo.cnt, maxW, fuse);
+            if (profile && threadIdx.x == 0) { rows_done += r1 - r0; words_done += (uint64_t)(r1 - r0) * st.W; }
+        } else if (NARROW && lane == 0) {
+            kc = atomicAdd(&s_next, 1u);
+        }
+        for (; !group;) {
             uint32_t k = 0;
             if (NARROW) {
                 k = kc;
