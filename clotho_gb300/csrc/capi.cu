@@ -1197,45 +1197,46 @@ static int stats_of(clotho_ctx* ctx, uint32_t idx, clotho_stats* out, uint32_t* 
     DevStatus s = read_status(ctx, p, &rc);
     if (rc) return rc;
     const PopDev& D = p->dev[0];
-    const uint32_t A = s.A, S = 2 * s.N;
-    std::vector<uint32_t> counts(std::max<size_t>(1, (size_t)s.W * 64), 0);
-    if (s.cols_valid) {
-        // the last fused step counted the columns of these rows: no pass over the rows
-        if (A) CK(cudaMemcpyAsync(counts.data(), D.colcnt, (size_t)A * 4, cudaMemcpyDeviceToHost, ctx->stream));
-    } else {
-        // scratch column counts from the context's pool: stream-ordered, no device-wide synchronisation
-        uint32_t* d_counts = nullptr;
-        CK(pool_alloc(ctx, &d_counts, counts.size() * 4));
-        CK(cudaMemsetAsync(d_counts, 0, counts.size() * 4, ctx->stream));
-        launch_margins(cfg(ctx), ctx->d_pops[0], idx, S, s.W, d_counts, nullptr);
-        CK(cudaMemcpyAsync(counts.data(), d_counts, counts.size() * 4, cudaMemcpyDeviceToHost, ctx->stream));
-        CK(cudaFreeAsync(d_counts, ctx->stream));
-        ctx->launches += 1;
-    }
-    std::vector<double> zi((size_t)s.N * 4);
-    if (s.N) CK(cudaMemcpyAsync(zi.data(), D.zi, (size_t)s.N * 32, cudaMemcpyDeviceToHost, ctx->stream));
-    CK(cudaStreamSynchronize(ctx->stream));
-    *out = clotho_stats{};
-    if (sfs)
-        for (uint32_t k = 0; k < sfs_len; ++k) sfs[k] = 0;
-    double het = 0.0;
-    for (uint32_t a = 0; a < A; ++a) {
-        const uint32_t c = counts[a];
-        if (c > 0 && c < S) out->segregating += 1;
-        if (S && c == S) out->fixed_now += 1;
-        if (S) {
-            const double f = (double)c / (double)S;
-            het += 2.0 * f * (1.0 - f);
+    const uint32_t S = 2 * s.N;
+    // one scratch block from the context's pool (stream-ordered, no device-wide synchronisation): the results,
+    // the spectrum, and the column counts unless the last fused step counted the columns of these rows
+    const size_t head = align256(sizeof(StatsOut)), len = sfs ? sfs_len : 0;
+    const size_t spectrum = align256(len * 4), cols = s.cols_valid ? 0 : (size_t)s.W * 256;
+    char* d = nullptr;
+    CK(pool_alloc(ctx, &d, head + spectrum + cols));
+    StatsOut* d_out = reinterpret_cast<StatsOut*>(d);
+    uint32_t* d_sfs = reinterpret_cast<uint32_t*>(d + head);
+    uint32_t* d_counts = s.cols_valid ? D.colcnt : reinterpret_cast<uint32_t*>(d + head + spectrum);
+    std::vector<char> h(head + len * 4);
+    auto body = [&]() -> int {
+        CK(cudaMemsetAsync(d, 0, head + spectrum + cols, ctx->stream));
+        if (cols) {
+            launch_margins(cfg(ctx), ctx->d_pops[0], idx, S, s.W, d_counts, nullptr);
+            ctx->launches += 1;
         }
-        if (sfs && sfs_len) sfs[c < sfs_len ? c : sfs_len - 1] += 1;
-    }
-    out->heterozygosity = het;
+        launch_stats(cfg(ctx), ctx->d_pops[0], idx, d_counts, (uint32_t)len, d_out, d_sfs);
+        ctx->launches += 1;
+        if (int r = check_launch(ctx, "stats")) return r;
+        CK(cudaMemcpyAsync(h.data(), d, h.size(), cudaMemcpyDeviceToHost, ctx->stream));
+        return 0;
+    };
+    rc = body();
+    const cudaError_t e_free = cudaFreeAsync(d, ctx->stream);
+    const cudaError_t e_sync = cudaStreamSynchronize(ctx->stream);
+    if (rc) return rc;
+    CK(e_free);
+    CK(e_sync);
+    const StatsOut& o = *reinterpret_cast<const StatsOut*>(h.data());
+    double sum[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+    for (uint32_t i = 0; i < kStatBlocks; ++i)
+        for (uint32_t t = 0; t < 5; ++t) sum[t] += o.part[i][t];
+    *out = clotho_stats{};
+    out->segregating = o.segregating;
+    out->fixed_now = o.fixed_now;
+    out->heterozygosity = sum[4];
     out->mean_fitness = s.N ? s.fit_total / (double)s.N : 0.0;
-    for (uint32_t t = 0; t < 4; ++t) {
-        double m = 0.0;
-        for (uint32_t i = 0; i < s.N; ++i) m += zi[(size_t)i * 4 + t];
-        out->mean_phenotype[t] = s.N ? m / s.N : 0.0;
-    }
+    for (uint32_t t = 0; t < 4; ++t) out->mean_phenotype[t] = s.N ? sum[t] / s.N : 0.0;
+    if (len) std::memcpy(sfs, h.data() + head, len * 4);
     return 0;
 }
 

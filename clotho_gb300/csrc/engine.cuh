@@ -373,6 +373,15 @@ void launch_seed_rows(const LaunchCfg&, const PopDev* pops, uint32_t npops, cons
                       uint64_t seed, uint32_t A);
 void launch_margins(const LaunchCfg&, const PopDev* pops, uint32_t p, uint32_t S, uint32_t W, uint32_t* colc,
                     uint32_t* rowc);
+// sums over the current child for clotho_stats_compute, per block: traits 0..3, heterozygosity
+constexpr uint32_t kStatBlocks = 128;
+struct StatsOut {
+    uint32_t segregating, fixed_now;
+    double part[kStatBlocks][5];
+};
+// out and sfs (sfs_len counts) zero on entry; counts: carriers of every slot
+void launch_stats(const LaunchCfg&, const PopDev* pops, uint32_t p, const uint32_t* counts, uint32_t sfs_len,
+                  StatsOut* out, uint32_t* sfs);
 // device accumulators of the pairwise-difference kernel
 struct PairwiseOut {
     unsigned long long count, total, sumsq;

@@ -434,14 +434,26 @@ __global__ void __launch_bounds__(256) k_margins(const PopDev* __restrict__ pops
             c1.add8(y);
         }
         if (ROW) {
+            // two rows' counts (at most 4,096 each) share a word; lane j < 4 of a row's lanes keeps rows 2j, 2j + 1
+            uint32_t mine = 0;
+            const uint32_t j = lane & (lpr - 1u);
 #pragma unroll
-            for (uint32_t k = 0; k < 8; ++k) {
-                uint32_t n = (uint32_t)(__popcll(x[k]) + __popcll(y[k]));
-                for (uint32_t o = lpr >> 1; o > 0; o >>= 1) n += __shfl_xor_sync(0xffffffffu, n, o);
-                const uint32_t r = b + k * rpl + sub;
-                if ((lane & (lpr - 1u)) == 0u && r < r1) {
-                    if (gridDim.x == 1u) rowc[r] = n;
-                    else if (n) atomicAdd(rowc + r, n);
+            for (uint32_t k = 0; k < 4; ++k) {
+                uint32_t n = (uint32_t)(__popcll(x[2 * k]) + __popcll(y[2 * k])) |
+                             (uint32_t)(__popcll(x[2 * k + 1]) + __popcll(y[2 * k + 1])) << 16;
+                if (lpr == 32u) n = __reduce_add_sync(0xffffffffu, n);
+                else
+                    for (uint32_t o = lpr >> 1; o > 0; o >>= 1) n += __shfl_xor_sync(0xffffffffu, n, o);
+                if (j == k) mine = n;
+            }
+            if (j < 4u) {
+#pragma unroll
+                for (uint32_t k = 0; k < 2; ++k) {
+                    const uint32_t r = b + (2u * j + k) * rpl + sub, n = (mine >> (16u * k)) & 0xffffu;
+                    if (r < r1) {
+                        if (gridDim.x == 1u) rowc[r] = n;
+                        else if (n) atomicAdd(rowc + r, n);
+                    }
                 }
             }
         }
@@ -476,6 +488,75 @@ void launch_margins(const LaunchCfg& L, const PopDev* pops, uint32_t p, uint32_t
     if (colc && rowc) k_margins<true, true><<<grid, 256, 0, L.stream>>>(pops, p, colc, rowc, lpr, strip);
     else if (colc) k_margins<true, false><<<grid, 256, 0, L.stream>>>(pops, p, colc, nullptr, lpr, strip);
     else k_margins<false, true><<<grid, 256, 0, L.stream>>>(pops, p, nullptr, rowc, lpr, strip);
+}
+
+
+// ---------------------------------------------------------------------------
+// Summary statistics from the column counts and the individual phenotypes: segregating and fixed sites, the
+// spectrum, and per block the sums of 2 f (1 - f) and of each trait (fixed order in a block; the host adds the
+// blocks in order, so the sums do not depend on timing).  FP64 adds and quotients, spread over the GPU; on the
+// host these were 4 N dependent adds behind a copy of the phenotypes (0.6 ms of a 1.0 ms call at N = 1e5).
+constexpr uint32_t kStatBins = 2048;   // spectrum bins counted in shared memory
+
+__global__ void __launch_bounds__(256) k_stats(const PopDev* __restrict__ pops, uint32_t p,
+                                               const uint32_t* __restrict__ counts, uint32_t sfs_len,
+                                               StatsOut* __restrict__ out, uint32_t* __restrict__ sfs) {
+    __shared__ uint32_t s_bin[kStatBins];
+    __shared__ double s_sum[8][5];
+    const PopDev& P = pops[p];
+    const DevStatus* st = P.st;
+    const uint32_t A = st->A, N = st->N, S = 2u * N, bins = min(sfs_len, kStatBins);
+    for (uint32_t i = threadIdx.x; i < bins; i += 256u) s_bin[i] = 0u;
+    __syncthreads();
+    double v[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+    uint32_t seg = 0, fix = 0;
+    for (uint32_t a = blockIdx.x * 256u + threadIdx.x; a < A; a += gridDim.x * 256u) {
+        const uint32_t c = counts[a];
+        seg += (c > 0u && c < S) ? 1u : 0u;
+        fix += (S && c == S) ? 1u : 0u;
+        if (S && c) {
+            const double f = (double)c / (double)S;
+            v[4] += 2.0 * f * (1.0 - f);
+        }
+        if (sfs_len) {
+            const uint32_t b = min(c, sfs_len - 1u);
+            if (b < kStatBins) atomicAdd(&s_bin[b], 1u);
+            else atomicAdd(sfs + b, 1u);
+        }
+    }
+    for (uint32_t i = blockIdx.x * 256u + threadIdx.x; i < N; i += gridDim.x * 256u) {
+        const double2* z = reinterpret_cast<const double2*>(P.zi + (size_t)i * 4u);
+        const double2 a = z[0], b = z[1];
+        v[0] += a.x;
+        v[1] += a.y;
+        v[2] += b.x;
+        v[3] += b.y;
+    }
+    seg = __reduce_add_sync(0xffffffffu, seg);
+    fix = __reduce_add_sync(0xffffffffu, fix);
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    if (lane == 0) {
+        if (seg) atomicAdd(&out->segregating, seg);
+        if (fix) atomicAdd(&out->fixed_now, fix);
+    }
+#pragma unroll
+    for (uint32_t t = 0; t < 5; ++t) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v[t] += __shfl_xor_sync(0xffffffffu, v[t], o);
+        if (lane == 0) s_sum[warp][t] = v[t];
+    }
+    __syncthreads();
+    if (threadIdx.x < 5u) {
+        double x = 0.0;
+        for (uint32_t i = 0; i < 8; ++i) x += s_sum[i][threadIdx.x];
+        out->part[blockIdx.x][threadIdx.x] = x;
+    }
+    for (uint32_t i = threadIdx.x; i < bins; i += 256u)
+        if (s_bin[i]) atomicAdd(sfs + i, s_bin[i]);
+}
+void launch_stats(const LaunchCfg& L, const PopDev* pops, uint32_t p, const uint32_t* counts, uint32_t sfs_len,
+                  StatsOut* out, uint32_t* sfs) {
+    k_stats<<<kStatBlocks, 256, 0, L.stream>>>(pops, p, counts, sfs_len, out, sfs);
 }
 
 }  // namespace clotho
