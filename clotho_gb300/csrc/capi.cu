@@ -1287,26 +1287,35 @@ static int pairwise_of(clotho_ctx* ctx, uint32_t idx, const uint32_t* sample, ui
     *out = clotho_pairwise{};
     const uint64_t pairs = n > 1 ? (uint64_t)n * (n - 1) / 2 : 0;
     if (!pairs) return 0;
-    uint32_t* d_smp = nullptr;
-    uint32_t* d_dist = nullptr;
-    PairwiseOut* d_out = nullptr;
-    CK(pool_alloc(ctx, &d_smp, (size_t)n * 4));
-    CK(pool_alloc(ctx, &d_out, sizeof(PairwiseOut)));
-    if (dist) CK(pool_alloc(ctx, &d_dist, pairs * 4));
+    // one scratch block: accumulators, sample, row sums and, when the slots are split over CTAs, tile counts
+    const PairwisePlan z = pairwise_plan(cfg(ctx), n, s.W);
+    const size_t at_smp = align256(sizeof(PairwiseOut)), at_ones = at_smp + align256((size_t)n * 4);
+    const size_t at_dist = align256(at_ones + z.ones_bytes + z.sum_bytes);
+    std::vector<char> head(at_smp + (size_t)n * 4);
     PairwiseOut h{};
     h.min = 0xffffffffu;
-    CK(cudaMemcpyAsync(d_smp, smp.data(), (size_t)n * 4, cudaMemcpyHostToDevice, ctx->stream));
-    CK(cudaMemcpyAsync(d_out, &h, sizeof(h), cudaMemcpyHostToDevice, ctx->stream));
-    launch_pairwise(cfg(ctx), ctx->d_pops[0], idx, d_smp, n, d_dist, d_out);
-    rc = check_launch(ctx, "pairwise difference");
-    CK(cudaMemcpyAsync(&h, d_out, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream));
-    if (dist) CK(cudaMemcpyAsync(dist, d_dist, pairs * 4, cudaMemcpyDeviceToHost, ctx->stream));
-    CK(cudaFreeAsync(d_smp, ctx->stream));
-    CK(cudaFreeAsync(d_out, ctx->stream));
-    if (d_dist) CK(cudaFreeAsync(d_dist, ctx->stream));
-    CK(cudaStreamSynchronize(ctx->stream));
-    ctx->launches += 1;
+    std::memcpy(head.data(), &h, sizeof(h));
+    std::memcpy(head.data() + at_smp, smp.data(), (size_t)n * 4);
+    char* d = nullptr;
+    CK(pool_alloc(ctx, &d, at_dist + (dist ? pairs * 4 : 0)));
+    auto body = [&]() -> int {
+        CK(cudaMemcpyAsync(d, head.data(), head.size(), cudaMemcpyHostToDevice, ctx->stream));
+        if (z.sum_bytes) CK(cudaMemsetAsync(d + at_ones + z.ones_bytes, 0, z.sum_bytes, ctx->stream));
+        CK(launch_pairwise(cfg(ctx), ctx->d_pops[0], idx, reinterpret_cast<uint32_t*>(d + at_smp), n, z, d + at_ones,
+                           dist ? reinterpret_cast<uint32_t*>(d + at_dist) : nullptr, reinterpret_cast<PairwiseOut*>(d)));
+        ctx->launches += 2;
+        if (int r = check_launch(ctx, "pairwise difference")) return r;
+        CK(cudaMemcpyAsync(&h, d, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream));
+        if (dist) CK(cudaMemcpyAsync(dist, d + at_dist, pairs * 4, cudaMemcpyDeviceToHost, ctx->stream));
+        return 0;
+    };
+    rc = body();
+    const cudaError_t e_free = cudaFreeAsync(d, ctx->stream);
+    const cudaError_t e_sync = cudaStreamSynchronize(ctx->stream);
     if (rc) return rc;
+    CK(e_free);
+    CK(e_sync);
+    if (h.err) return fail(ctx, CLOTHO_E_DEVICE, "pairwise difference: a tile's multiplications did not end");
     out->count = h.count;
     out->total = h.total;
     out->min = h.count ? h.min : 0;

@@ -386,9 +386,16 @@ void launch_stats(const LaunchCfg&, const PopDev* pops, uint32_t p, const uint32
 struct PairwiseOut {
     unsigned long long count, total, sumsq;
     unsigned int min, max;
+    unsigned int err;   // a CTA gave up waiting for its multiplications
 };
-void launch_pairwise(const LaunchCfg&, const PopDev* pops, uint32_t p, const uint32_t* sample, uint32_t n,
-                     uint32_t* dist, PairwiseOut* out);
+// how the pairs of n rows of W words are cut into CTAs, and the scratch that takes
+struct PairwisePlan {
+    uint32_t tiles, splits, per;       // per: 128-slot stages a CTA
+    size_t ones_bytes, sum_bytes;
+};
+PairwisePlan pairwise_plan(const LaunchCfg&, uint32_t n, uint32_t W);
+cudaError_t launch_pairwise(const LaunchCfg&, const PopDev* pops, uint32_t p, const uint32_t* sample, uint32_t n,
+                            const PairwisePlan&, void* scratch, uint32_t* dist, PairwiseOut* out);
 // After launch_prep: the slots' ranks, the suffix tables and (tables: some population has one) the rows' plans.
 // Returns the launches made.
 uint32_t launch_plan(const LaunchCfg&, const PopDev* pops, uint32_t npops, const PrepSizes&, uint32_t maxW);

@@ -7,81 +7,231 @@
 // count, total, min, max, mean and variance (and, from the distances, the
 // median).
 //
-// One CTA takes a 64 x 64 tile of the pair matrix (tiles on or above the
-// diagonal only); the two row groups are staged 16 words at a time in shared
-// memory and every thread accumulates a 4 x 4 block of pair distances.
+// popcount(a XOR b) = |a| + |b| - 2 |a AND b|, and |a AND b| over all pairs is the product of the
+// sample's 0/1 matrix with its transpose: a contraction, so it runs on the tensor cores.
 #include "engine.cuh"
+
+#include <algorithm>
 
 namespace clotho {
 
 namespace {
-constexpr uint32_t kTile = 64;    // rows per tile side
-constexpr uint32_t kStageW = 16;  // words per stage
-constexpr uint32_t kPad = kStageW + 1;
+constexpr uint32_t kTM = 128, kTN = 256;        // pairs a CTA takes: rows i of the tile, rows j
+constexpr uint32_t kPairThreads = kTM + kTN;    // one expanded row a thread
+constexpr uint32_t kRing = 4;                   // stages of 128 slots in shared memory
+constexpr uint32_t kStageBytes = (kTM + kTN) * 128u;
+constexpr uint32_t kMaxSlots = 1u << 19;        // slots a CTA sums up: counts stay far below 2^24 units
+constexpr uint32_t kPairWait = 1u << 20;        // try_wait rounds before a CTA gives up
+
+__device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
+__device__ __forceinline__ bool wait_parity(uint32_t bar, uint32_t parity) {
+    for (uint32_t it = 0; it < kPairWait; ++it) {
+        uint32_t ok;
+        asm volatile(
+            "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
+            : "=r"(ok)
+            : "r"(bar), "r"(parity)
+            : "memory");
+        if (ok) return true;
+    }
+    return false;
+}
+
+// Shared-memory operand of K-major rows of 128 bytes in the 128-byte swizzle: groups of eight rows 1,024 bytes apart.
+__device__ __forceinline__ uint64_t operand(uint32_t addr) {
+    return (uint64_t)((addr & 0x3FFFFu) >> 4) | (1ull << 16) | ((uint64_t)(1024u >> 4) << 32) | (1ull << 46) | (2ull << 61);
+}
+
+__device__ __forceinline__ void mma_f8(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, bool accumulate) {
+    asm volatile(
+        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+        " tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n}" ::"r"(d),
+        "l"(a), "l"(b), "r"(idesc), "r"((uint32_t)accumulate)
+        : "memory");
+}
+__device__ __forceinline__ void mma_commit(uint32_t bar) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+
+__device__ __forceinline__ void load_32_columns(uint32_t taddr, uint32_t (&v)[32]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
+          "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]),
+          "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]),
+          "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
+        : "r"(taddr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
 }  // namespace
 
-__global__ void __launch_bounds__(256) k_pairwise(const PopDev* __restrict__ pops, uint32_t p,
-                                                  const uint32_t* __restrict__ sample, uint32_t n,
-                                                  uint32_t* __restrict__ dist, PairwiseOut* __restrict__ out) {
-    __shared__ uint64_t sA[kTile][kPad];
-    __shared__ uint64_t sB[kTile][kPad];
-    __shared__ unsigned long long s_sum[8], s_sq[8], s_cnt[8];
-    __shared__ unsigned int s_min[8], s_max[8];
+// Alleles of each sampled row, one warp a row.
+__global__ void __launch_bounds__(256) k_sample_ones(const PopDev* __restrict__ pops, uint32_t p,
+                                                     const uint32_t* __restrict__ sample, uint32_t n,
+                                                     uint32_t* __restrict__ ones) {
     const PopDev& P = pops[p];
-    const DevStatus* st = P.st;
-    const uint32_t W = st->W;
-    const uint64_t* rows = P.rows[st->cur];
-    // tile (ti, tj), ti <= tj, from the linear block index
-    const uint32_t T = (n + kTile - 1) / kTile;
-    uint32_t b = blockIdx.x, ti = 0;
-    while (b >= T - ti) {
-        b -= T - ti;
+    const uint32_t W = P.st->W, lane = threadIdx.x & 31u;
+    const uint64_t* rows = P.rows[P.st->cur];
+    for (uint32_t i = (blockIdx.x * 256u + threadIdx.x) >> 5; i < n; i += gridDim.x * 8u) {
+        const uint64_t* r = rows + (size_t)sample[i] * P.Wcap;
+        uint32_t c = 0;
+        for (uint32_t w = 2u * lane; w < W; w += 64u) {
+            const ulonglong2 x = __ldg(reinterpret_cast<const ulonglong2*>(r + w));
+            c += (uint32_t)(__popcll(x.x) + __popcll(x.y));
+        }
+        c = __reduce_add_sync(0xffffffffu, c);
+        if (lane == 0) ones[i] = c;
+    }
+}
+
+// One CTA takes a 128 x 256 tile of the pair matrix (tiles with a pair i < j only) and a range of the slots.
+// Every thread expands one row, 128 slots a stage: bit k of each byte of a 32-bit word becomes a byte of 0 or 1
+// (two operations for four slots; the order of the slots is the same for all rows, which is all a sum needs) in the
+// 128-byte swizzle that the tensor core reads.  A byte of 1 is the e4m3 value 2^-9, so products are 2^-18
+// and sums are whole multiples of it, exact in FP32.  One thread issues the four K = 32 steps of a stage; four stages
+// in flight let expansion and multiplication overlap.  Bound by shared-memory bandwidth: 48 KB written and
+// 48 KB read for a stage's 512 clocks of multiplication.
+// splits > 1 (few tiles): the CTAs of a tile add their counts into tile_sum, the last one to come finishes the
+// tile; no CTA waits for another.  (popcount of 64 x 64 tiles: 1.1 ms for 4,001 rows of 320 words, the popcount
+// unit's 16 words a clock and SM.)
+__global__ void __launch_bounds__(kPairThreads, 1)
+k_pairwise(const PopDev* __restrict__ pops, uint32_t p, const uint32_t* __restrict__ sample, uint32_t n,
+           const uint32_t* __restrict__ ones, uint32_t splits, uint32_t per, uint32_t* __restrict__ tile_sum,
+           uint32_t* __restrict__ tile_done, uint32_t* __restrict__ dist, PairwiseOut* __restrict__ out) {
+    extern __shared__ uint8_t s_raw[];
+    __shared__ __align__(8) unsigned long long s_bar[kRing + 1];
+    __shared__ uint32_t s_tmem, s_last;
+    __shared__ uint32_t s_ones[kPairThreads];
+    __shared__ unsigned long long s_sum[12], s_sq[12], s_cnt[12];
+    __shared__ uint32_t s_min[12], s_max[12];
+    const PopDev& P = pops[p];
+    const uint64_t* rows = P.rows[P.st->cur];
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    // tile (ti, tj): of tile row ti, the tile columns from its first row on
+    const uint32_t tile = blockIdx.x / splits, split = blockIdx.x % splits;
+    const uint32_t TJ = (n + kTN - 1u) / kTN;
+    uint32_t ti = 0, left = tile;
+    while (left >= TJ - ti * kTM / kTN) {
+        left -= TJ - ti * kTM / kTN;
         ++ti;
     }
-    const uint32_t tj = ti + b;
-    const uint32_t tx = threadIdx.x & 15u, ty = threadIdx.x >> 4;
-    uint32_t acc[4][4] = {};
-    for (uint32_t w0 = 0; w0 < W; w0 += kStageW) {
-        __syncthreads();
-        for (uint32_t e = threadIdx.x; e < kTile * kStageW; e += blockDim.x) {
-            const uint32_t r = e / kStageW, c = e % kStageW, w = w0 + c;
-            const uint32_t ia = ti * kTile + r, ib = tj * kTile + r;
-            sA[r][c] = (ia < n && w < W) ? rows[(size_t)sample[ia] * P.Wcap + w] : 0ull;
-            sB[r][c] = (ib < n && w < W) ? rows[(size_t)sample[ib] * P.Wcap + w] : 0ull;
-        }
-        __syncthreads();
-#pragma unroll 4
-        for (uint32_t c = 0; c < kStageW; ++c) {
-            uint64_t a[4], bb[4];
+    const uint32_t tj = ti * kTM / kTN + left;
+    const uint32_t nst = P.st->W / 2u, st0 = min(nst, split * per), cnt = min(nst, st0 + per) - st0;
+    const uint32_t row = tid < kTM ? ti * kTM + tid : tj * kTN + (tid - kTM);
+    const bool ok_row = row < n;
+    const uint4* src = ok_row ? reinterpret_cast<const uint4*>(rows + (size_t)sample[row] * P.Wcap) + st0 : nullptr;
+    s_ones[tid] = ok_row ? ones[row] : 0u;
+    uint8_t* const ring = s_raw + ((1024u - (smem_addr(s_raw) & 1023u)) & 1023u);
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&s_tmem)),
+                     "r"(kTN)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+    if (tid == 0) {
+        for (uint32_t i = 0; i <= kRing; ++i)
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&s_bar[i])) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = s_tmem;
+    // e4m3 x e4m3 -> f32, K-major operands; columns up to the sample's end
+    const uint32_t ncol = min(kTN, (n - tj * kTN + 15u) & ~15u);
+    const uint32_t idesc = (1u << 4) | ((ncol >> 3) << 17) | ((kTM >> 4) << 24);
+    const uint4 zero = make_uint4(0, 0, 0, 0);
+    uint4 q0 = ok_row && cnt > 0 ? __ldg(src) : zero, q1 = ok_row && cnt > 1 ? __ldg(src + 1) : zero;
+    bool ok = true;
+    uint32_t issued = 0;
+    for (uint32_t it = 0; it < cnt; ++it) {
+        const uint32_t s = it % kRing;
+        const uint4 q = q0;
+        q0 = q1;
+        q1 = ok_row && it + 2u < cnt ? __ldg(src + it + 2u) : zero;
+        if (it >= kRing) ok = wait_parity(smem_addr(&s_bar[s]), (it / kRing - 1u) & 1u);
+        if (ok && (ok_row || it < kRing)) {   // rows past the sample stay zero
+            uint8_t* dst = ring + s * kStageBytes + (tid < kTM ? tid : tid - kTM) * 128u + (tid < kTM ? 0u : kTM * 128u);
+            const uint32_t x[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
-            for (uint32_t k = 0; k < 4; ++k) {
-                a[k] = sA[ty * 4u + k][c];
-                bb[k] = sB[tx * 4u + k][c];
+            for (uint32_t c = 0; c < 8; ++c) {
+                const uint32_t v = x[c >> 1] >> (4u * (c & 1u));
+                const uint4 b = make_uint4(v & 0x01010101u, (v >> 1) & 0x01010101u, (v >> 2) & 0x01010101u,
+                                           (v >> 3) & 0x01010101u);
+                *reinterpret_cast<uint4*>(dst + ((c ^ (tid & 7u)) << 4)) = b;
+            }
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        if (!__syncthreads_and(ok)) {
+            ok = false;
+            break;
+        }
+        if (tid == 0) {
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t a = smem_addr(ring + s * kStageBytes), b = a + kTM * 128u;
+#pragma unroll
+            for (uint32_t k = 0; k < 4; ++k) mma_f8(tmem, operand(a + 32u * k), operand(b + 32u * k), idesc, (it | k) != 0u);
+            mma_commit(smem_addr(&s_bar[s]));
+        }
+        issued = it + 1u;
+    }
+    if (issued) {   // everything issued has ended, whether the loop ran through or not
+        if (tid == 0) mma_commit(smem_addr(&s_bar[kRing]));
+        ok = __syncthreads_and(wait_parity(smem_addr(&s_bar[kRing]), 0u)) && ok;
+    }
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    // TMEM lanes are the tile's rows: a warp reads the 32 of its place in its warpgroup, a third of the columns
+    const uint32_t i_tile = (warp & 3u) * 32u + lane, i = ti * kTM + i_tile;
+    const uint32_t taddr = tmem + (((warp & 3u) * 32u) << 16);
+    uint32_t* const sums = tile_sum ? tile_sum + (size_t)tile * kTM * kTN : nullptr;   // [column][row]
+    bool finish = ok;
+    if (splits > 1u) {
+        for (uint32_t c0 = (warp >> 2) * 32u; c0 < ncol; c0 += 96u) {
+            uint32_t v[32];
+            load_32_columns(taddr + c0, v);
+            if (ok && cnt)
+#pragma unroll
+                for (uint32_t k = 0; k < 32; ++k) {
+                    const uint32_t x = __float2uint_rn(__uint_as_float(v[k]) * 262144.0f);
+                    if (x && c0 + k < ncol) atomicAdd(sums + (c0 + k) * kTM + i_tile, x);
+                }
+        }
+        __threadfence();
+        __syncthreads();
+        if (tid == 0) s_last = atomicAdd(tile_done + tile, 1u) == splits - 1u;
+        __syncthreads();
+        finish = ok && s_last;
+        __threadfence();
+    }
+    unsigned long long sum = 0, sq = 0, pairs = 0;
+    uint32_t mn = 0xffffffffu, mx = 0;
+    if (finish) {
+        for (uint32_t c0 = (warp >> 2) * 32u; c0 < ncol; c0 += 96u) {
+            uint32_t v[32];
+            if (splits > 1u) {
+#pragma unroll
+                for (uint32_t k = 0; k < 32; ++k) v[k] = c0 + k < ncol ? __ldcg(sums + (c0 + k) * kTM + i_tile) : 0u;
+            } else {
+                load_32_columns(taddr + c0, v);
+#pragma unroll
+                for (uint32_t k = 0; k < 32; ++k)
+                    v[k] = cnt ? __float2uint_rn(__uint_as_float(v[k]) * 262144.0f) : 0u;
             }
 #pragma unroll
-            for (uint32_t k = 0; k < 4; ++k)
-#pragma unroll
-                for (uint32_t l = 0; l < 4; ++l) acc[k][l] += (uint32_t)__popcll(a[k] ^ bb[l]);
-        }
-    }
-    unsigned long long sum = 0, sq = 0, cnt = 0;
-    unsigned int mn = 0xffffffffu, mx = 0;
-#pragma unroll
-    for (uint32_t k = 0; k < 4; ++k) {
-#pragma unroll
-        for (uint32_t l = 0; l < 4; ++l) {
-            const uint32_t i = ti * kTile + ty * 4u + k, j = tj * kTile + tx * 4u + l;
-            if (i < j && j < n) {
-                const uint32_t d = acc[k][l];
-                if (dist) {
-                    const uint64_t at = (uint64_t)i * n - (uint64_t)i * (i + 1) / 2 + (j - i - 1);
-                    dist[at] = d;
+            for (uint32_t k = 0; k < 32; ++k) {
+                const uint32_t j = tj * kTN + c0 + k;
+                if (i < j && j < n) {
+                    const uint32_t d = s_ones[i_tile] + s_ones[kTM + c0 + k] - 2u * v[k];
+                    if (dist) dist[(uint64_t)i * n - (uint64_t)i * (i + 1) / 2 + (j - i - 1)] = d;
+                    sum += d;
+                    sq += (unsigned long long)d * d;
+                    pairs += 1;
+                    mn = min(mn, d);
+                    mx = max(mx, d);
                 }
-                sum += d;
-                sq += (unsigned long long)d * d;
-                cnt += 1;
-                mn = min(mn, d);
-                mx = max(mx, d);
             }
         }
     }
@@ -89,29 +239,32 @@ __global__ void __launch_bounds__(256) k_pairwise(const PopDev* __restrict__ pop
     for (int o = 16; o > 0; o >>= 1) {
         sum += __shfl_xor_sync(0xffffffffu, sum, o);
         sq += __shfl_xor_sync(0xffffffffu, sq, o);
-        cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
-        mn = min(mn, __shfl_xor_sync(0xffffffffu, mn, o));
-        mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        pairs += __shfl_xor_sync(0xffffffffu, pairs, o);
     }
-    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    mn = __reduce_min_sync(0xffffffffu, mn);
+    mx = __reduce_max_sync(0xffffffffu, mx);
     if (lane == 0) {
         s_sum[warp] = sum;
         s_sq[warp] = sq;
-        s_cnt[warp] = cnt;
+        s_cnt[warp] = pairs;
         s_min[warp] = mn;
         s_max[warp] = mx;
     }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (threadIdx.x == 0) {
-        for (uint32_t i = 1; i < blockDim.x / 32u; ++i) {
-            sum += s_sum[i];
-            sq += s_sq[i];
-            cnt += s_cnt[i];
-            mn = min(mn, s_min[i]);
-            mx = max(mx, s_max[i]);
+    if (warp == 0)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTN) : "memory");
+    if (tid == 0) {
+        for (uint32_t k = 1; k < kPairThreads / 32u; ++k) {
+            sum += s_sum[k];
+            sq += s_sq[k];
+            pairs += s_cnt[k];
+            mn = min(mn, s_min[k]);
+            mx = max(mx, s_max[k]);
         }
-        if (cnt) {
-            atomicAdd(&out->count, cnt);
+        if (!ok) atomicOr(&out->err, 1u);
+        if (pairs) {
+            atomicAdd(&out->count, pairs);
             atomicAdd(&out->total, sum);
             atomicAdd(&out->sumsq, sq);
             atomicMin(&out->min, mn);
@@ -120,13 +273,44 @@ __global__ void __launch_bounds__(256) k_pairwise(const PopDev* __restrict__ pop
     }
 }
 
-// Blocks: one per tile on or above the diagonal of the pair matrix.
-void launch_pairwise(const LaunchCfg& L, const PopDev* pops, uint32_t p, const uint32_t* sample, uint32_t n,
-                     uint32_t* dist, PairwiseOut* out) {
-    const uint32_t T = (n + kTile - 1) / kTile;
-    const uint32_t blocks = T * (T + 1) / 2;
-    if (blocks)
-        k_pairwise<<<blocks, 256, 0, L.stream>>>(pops, p, sample, n, dist, out);
+PairwisePlan pairwise_plan(const LaunchCfg& L, uint32_t n, uint32_t W) {
+    PairwisePlan z{};
+    const uint32_t TI = (n + kTM - 1u) / kTM, TJ = (n + kTN - 1u) / kTN, nst = W / 2u;
+    for (uint32_t ti = 0; ti < TI; ++ti) z.tiles += TJ - ti * kTM / kTN;
+    // Slots over several CTAs where the tiles alone leave SMs idle: the count with the least work on the busiest SM
+    // (rounds of tiles x splits over the SMs, each 1/splits of the slots plus about six stages' time to start and
+    // to add up), at least eight stages each, and as many as keep a CTA's sums in range
+    const uint32_t least = std::max(1u, (nst * 128u + kMaxSlots - 1u) / kMaxSlots);
+    double best = 1e30;
+    for (uint32_t s = least; s <= std::max(least, std::min(nst / 8u, 64u)); ++s) {
+        const double rounds = (double)((z.tiles * (uint64_t)s + L.num_sms - 1u) / L.num_sms);
+        const double cost = rounds * ((double)nst / s + 6.0 + (s > 1u ? 6.0 : 0.0));
+        if (cost < best * 0.98) {
+            best = cost;
+            z.splits = s;
+        }
+    }
+    z.per = (nst + z.splits - 1u) / z.splits;
+    z.ones_bytes = ((size_t)n * 4 + 255) & ~(size_t)255;
+    z.sum_bytes = z.splits > 1u ? (size_t)z.tiles * (kTM * kTN + 64u) * 4 : 0;
+    return z;
+}
+
+// scratch: ones_bytes, then sum_bytes zero on entry.
+cudaError_t launch_pairwise(const LaunchCfg& L, const PopDev* pops, uint32_t p, const uint32_t* sample, uint32_t n,
+                            const PairwisePlan& z, void* scratch, uint32_t* dist, PairwiseOut* out) {
+    uint32_t* ones = static_cast<uint32_t*>(scratch);
+    uint32_t* sums = z.sum_bytes ? reinterpret_cast<uint32_t*>(static_cast<char*>(scratch) + z.ones_bytes) : nullptr;
+    uint32_t* done = z.sum_bytes ? sums + (size_t)z.tiles * kTM * kTN : nullptr;
+    const size_t smem = kRing * kStageBytes + 1024u;
+    // a property of the function on the current device; setting it again is harmless
+    const cudaError_t e =
+        cudaFuncSetAttribute((const void*)k_pairwise, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    k_sample_ones<<<std::min(blocks_for(n, 8), (uint32_t)L.num_sms * 8u), 256, 0, L.stream>>>(pops, p, sample, n, ones);
+    k_pairwise<<<z.tiles * z.splits, kPairThreads, smem, L.stream>>>(pops, p, sample, n, ones, z.splits, z.per, sums,
+                                                                    done, dist, out);
+    return cudaSuccess;
 }
 
 }  // namespace clotho
