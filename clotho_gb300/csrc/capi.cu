@@ -67,7 +67,7 @@ std::vector<size_t> sizes_of(const Geometry& g) {
         A * 4, A * 8, A * 4, A * 16,     // free_list, pos, age, eff (traits padded to 4)
         g.FXcap * 8ull, g.FXcap * 4ull, g.FXcap * T * 4ull,
         S * 32, S * 32, N * 32, N * 8, N * 8,    // zg[0], zg[1], zi, fit, cdf
-        (N / 1024 + 8) * 8, (N / 128 + 64) * 8, (kPoisTab + 1) * 8, (kPoisTab + 1) * 8, ((S > g.NB ? S : g.NB) / 1024 + 8) * 4ull, ((S > g.NB ? S : g.NB) / 1024 + 8) * 4ull,
+        (N / 1024 + 8) * 8, (N / 128 + 64) * 8, (kPoisTab + 1) * 8, (kPoisTab + 1) * 8, ((S > g.NB ? S : g.NB) / 1024 + 32) * 4ull, (N / 1024 + 32) * 4ull,
         (S + 1) * 4, (S + 1) * 4,        // row_cnt, row_off
         S * 4, g.Mcap * 4ull, g.Mcap * 4ull,  // row_cur, row_mut, mut_slot
         (g.NB + 1ull) * 4, (g.NB + 1ull) * 4, g.NB * 4ull, A * 8, A * 4, A * 4,  // bcnt, boff, bcur, bpos, bslot, rank
@@ -160,8 +160,10 @@ int fail(clotho_ctx* c, int code, const std::string& m) {
             return fail(ctx, CLOTHO_E_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_)); \
     } while (0)
 
-LaunchCfg cfg(clotho_ctx* ctx) {
+// set: the descriptors that the launch takes (tape set 0 or 1, or 2 for device draws)
+LaunchCfg cfg(clotho_ctx* ctx, uint32_t set = 0) {
     LaunchCfg L{ctx->stream, ctx->num_sms};
+    if (!ctx->pops.empty()) L.one = &ctx->pops[0]->dev[set];  // taken by launches over the first population alone
     L.ind_per_sm = ctx->ind_per_sm;
     L.narrow_ok = ctx->narrow_ok;
     return L;
@@ -386,7 +388,7 @@ bool count_on(clotho_ctx* ctx, uint32_t fuse) {
 // The generation kernel over every population: one launch when all populations use the same build; in a
 // batch that mixes them, one launch per build (bitmap, chunk-mask, interval), each over its own populations,
 // so every population runs the build it runs alone.
-void launch_gen(clotho_ctx* ctx, const PopDev* pops, uint32_t npops, uint32_t fuse) {
+void launch_gen(clotho_ctx* ctx, const LaunchCfg& L, const PopDev* pops, uint32_t npops, uint32_t fuse) {
     const int prof = ctx->profiling ? (ctx->phase_clocks ? 2 : 1) : 0;
     const uint32_t kinds = (ctx->n_bm > 0) + (ctx->n_cm > 0) + (ctx->n_iv > 0);
     const bool mixed = kinds > 1;
@@ -401,7 +403,7 @@ void launch_gen(clotho_ctx* ctx, const PopDev* pops, uint32_t npops, uint32_t fu
         const uint32_t A = mixed ? pA[pass] : ctx->maxA;
         prof_begin(ctx);
         const cudaError_t e =
-            launch_generation(cfg(ctx), pops, npops, ctx->d_ctl, W, A, fuse, prof, builds[pass], cnt, mixed);
+            launch_generation(L, pops, npops, ctx->d_ctl, W, A, fuse, prof, builds[pass], cnt, mixed);
         if (e != cudaSuccess && ctx->launch_err == cudaSuccess) ctx->launch_err = e;
         prof_end(ctx);
         ctx->launches += 1;
@@ -465,15 +467,15 @@ void ensure_parent_acc(clotho_ctx* ctx, const PopDev* pops, uint32_t npops) {
 void enqueue_fused_step(clotho_ctx* ctx, uint32_t set, bool philox) {
     const uint32_t n = (uint32_t)ctx->pops.size();
     const PopDev* pops = ctx->d_pops[set];
-    LaunchCfg L = cfg(ctx);
+    const LaunchCfg L = cfg(ctx, set);
     ctx->pairs_set = set == 1u ? 1u : 0u;  // the device-drawn set (2) shares set 0's buffers
     ensure_parent_acc(ctx, pops, n);
     const PrepSizes z = prep_sizes(ctx);
+    const bool cnt = count_on(ctx, kFuseMut | kFusePheno | kFuseFs);
     const uint32_t what = kStepBegin | kStepMut | kStepOrder | (philox ? kStepSelect : kStepTape);
-    ctx->launches += launch_prep(L, pops, n, z, ctx->d_hdr[set], ctx->d_ctl, what,
-                                 count_on(ctx, kFuseMut | kFusePheno | kFuseFs));
-    ctx->launches += launch_plan(L, pops, n, z, ctx->maxW_suf);
-    launch_gen(ctx, pops, n, kFuseMut | kFusePheno | kFuseFs);
+    ctx->launches += launch_prep(L, pops, n, z, ctx->d_hdr[set], ctx->d_ctl, what, cnt);
+    ctx->launches += launch_plan(L, pops, n, z, ctx->maxW_suf, what);
+    launch_gen(ctx, L, pops, n, kFuseMut | kFusePheno | kFuseFs);
     ctx->launches += launch_fitness(L, pops, n, ctx->maxN, true);
     for (PopHost* p : ctx->pops) p->acc_valid = true;
 }
@@ -948,8 +950,8 @@ int clotho_crossover(clotho_ctx* ctx, const uint8_t* swap, const uint32_t* ev_of
     // item prefix is already set by begin; the rows' order, ranks over the current positions
     const PrepSizes z = prep_sizes(ctx);
     ctx->launches += launch_prep(cfg(ctx), ctx->d_pops[0], 1, z, nullptr, ctx->d_ctl, kStepOrder, false);
-    ctx->launches += launch_plan(cfg(ctx), ctx->d_pops[0], 1, z, ctx->maxW);
-    launch_gen(ctx, ctx->d_pops[0], 1, 0u);
+    ctx->launches += launch_plan(cfg(ctx), ctx->d_pops[0], 1, z, ctx->maxW, kStepOrder);
+    launch_gen(ctx, cfg(ctx), ctx->d_pops[0], 1, 0u);
     if ((rc = check_launch(ctx, "crossover"))) return rc;
     CK(cudaStreamSynchronize(ctx->stream));
     return 0;

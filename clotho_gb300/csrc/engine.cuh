@@ -81,8 +81,8 @@ struct PopDev {
     double*   scan_wsum;   // [Ncap / 128 + 64] fitness sums of 128 individuals
     double*   pois_mu;     // [kPoisTab + 1] Poisson(mu) CDF F_0 .. F_{kPoisTab-1}, then p_{kPoisTab-1}
     double*   pois_rho;    // [kPoisTab + 1] the same of Poisson(rho)
-    uint32_t* scan_upart;  // [max(Scap, NB) / 1024 + 2] chunk sums
-    uint32_t* scan_opart;  // [Scap / 1024 + 2] the row-ordering scan's own chunk sums (it runs beside the others)
+    uint32_t* scan_upart;  // [max(Scap, NB) / 1024 + 32] chunk sums
+    uint32_t* scan_opart;  // [Ncap / 1024 + 32] the row-ordering scan's own chunk sums (it runs beside the others)
     uint32_t* pairs;       // [2 * Ncap]
     uint8_t*  swap;        // [Scap]
     uint32_t* ev_off;      // [Scap + 1]
@@ -254,12 +254,13 @@ __device__ __forceinline__ uint32_t poisson_tab(double u, const double* cdf, dou
     return k;
 }
 
-// Programmatic dependent launch: a kernel launched with launch_k may be resident before its predecessor in the
-// stream ends.  pdl_wait returns when the predecessor has ended and its writes are visible; every block of every
-// such kernel calls it before it touches memory (so a predecessor's end means that all before it ended, too).
-// pdl_go lets the successor's blocks in as this kernel's leave.
+// Programmatic dependent launch: a kernel launched with launch_k is set up while its predecessor in the stream ends.
+// pdl_wait returns when the predecessor has ended and its writes are visible; every block of every such kernel
+// calls it before it touches memory (so a predecessor's end means that all before it ended, too).  No kernel
+// triggers its successor early (griddepcontrol.launch_dependents): blocks that are resident and wait cost the running
+// ones more than their start (a generation of 10,000 individuals 67.6 us with early triggers, 61.5 without; without
+// the programmatic dependency 65.6, and 84 against 71 us launched one by one).
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_go() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // Monotone bucket of a position in [0,1) (values outside are clamped).
 // floor(x * NB) for x in (0, 1), from the bits with integer operations: 0 for
@@ -295,6 +296,7 @@ struct LaunchCfg {
     int num_sms;
     uint32_t ind_per_sm = 16;     // blocks per SM of the per-individual kernels (selection, fitness)
     bool narrow_ok = true;        // the narrow build of k_generation may run when every row fits it
+    const PopDev* one = nullptr;  // host copy of the descriptor of a launch's only population
 };
 
 // Population-parallel launches: blockIdx.z walks the populations, so small
@@ -311,7 +313,7 @@ inline uint32_t blocks_for(uint64_t n, uint32_t per_block) {
     const uint64_t b = (n + per_block - 1) / per_block;
     return b < 1 ? 1u : (b > 0x7fffffffull ? 0x7fffffffu : (uint32_t)b);
 }
-// Launch with the programmatic dependency of pdl_wait / pdl_go.
+// Launch with the programmatic dependency of pdl_wait.
 template <class... P, class... A>
 inline cudaError_t launch_smem_k(const LaunchCfg& L, void (*k)(P...), dim3 grid, dim3 block, size_t smem, A... a) {
     cudaLaunchAttribute at{};
@@ -329,6 +331,27 @@ inline cudaError_t launch_smem_k(const LaunchCfg& L, void (*k)(P...), dim3 grid,
 template <class... P, class... A>
 inline cudaError_t launch_k(const LaunchCfg& L, void (*k)(P...), dim3 grid, dim3 block, A... a) {
     return launch_smem_k(L, k, grid, block, 0, a...);
+}
+
+// The kernels of a step are templates over ONE: with one population its descriptor comes in the kernel's parameters
+// (the constant bank) instead of an array in memory, which takes a round trip to L2 off each kernel's chain of
+// dependent loads.
+template <class K, class... A>
+inline cudaError_t launch_pops_smem(const LaunchCfg& L, K one, K all, dim3 grid, dim3 block, size_t smem,
+                                    const PopDev* pops, uint32_t npops, A... a) {
+    const bool single = npops == 1u && L.one;
+    const K k = single ? one : all;
+    if (smem > 48u * 1024u) {  // a property of the function on the current device; setting it again is harmless
+        const cudaError_t e =
+            cudaFuncSetAttribute((const void*)k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+    }
+    return launch_smem_k(L, k, grid, block, smem, single ? *L.one : PopDev{}, pops, npops, a...);
+}
+template <class K, class... A>
+inline cudaError_t launch_pops(const LaunchCfg& L, K one, K all, dim3 grid, dim3 block, const PopDev* pops,
+                               uint32_t npops, A... a) {
+    return launch_pops_smem(L, one, all, grid, block, 0, pops, npops, a...);
 }
 
 // which: 0 = current child rows, 1 = parent rows of the step in progress
@@ -349,6 +372,9 @@ struct PrepSizes {
 // valid.  Returns the launches made.
 uint32_t launch_prep(const LaunchCfg&, const PopDev* pops, uint32_t npops, const PrepSizes&, const uint32_t* hdr,
                      WorkCtl* ctl, uint32_t what, bool count_on);
+// Allele capacity up to which one block ranks a population's slots in shared memory (k_prep.cu)
+constexpr uint32_t kDirectRanks = 8192;
+inline bool direct_ranks(const PrepSizes& z) { return z.maxA <= kDirectRanks && z.tables; }
 // Poisson tables of one population (the device copy of its descriptor)
 void launch_pois_tables(cudaStream_t s, const PopDev& P);
 void launch_mut_resolve(const LaunchCfg&, const PopDev* pops, uint32_t npops);
@@ -398,7 +424,8 @@ cudaError_t launch_pairwise(const LaunchCfg&, const PopDev* pops, uint32_t p, co
                             const PairwisePlan&, void* scratch, uint32_t* dist, PairwiseOut* out);
 // After launch_prep: the slots' ranks, the suffix tables and (tables: some population has one) the rows' plans.
 // Returns the launches made.
-uint32_t launch_plan(const LaunchCfg&, const PopDev* pops, uint32_t npops, const PrepSizes&, uint32_t maxW);
+uint32_t launch_plan(const LaunchCfg&, const PopDev* pops, uint32_t npops, const PrepSizes&, uint32_t maxW,
+                     uint32_t what);
 int init_recip_prep();  // k_prep.cu's copy of the reciprocal table
 int init_recip_gen();   // k_generation.cu's copy
 

@@ -29,7 +29,7 @@
 //   suffix table (A <= 524,288 slots): the switch mask of a gamete with rank
 //              thresholds r_1..r_E is XOR_k G(r_k), G(r) = {slots with rank >= r}.
 //              G at every multiple of 64 is a per-generation table in L2
-//              (suf[g * Wcap + w], built by k_suf_build); G(r) differs from the
+//              (suf[g * Wcap + w], built by k_prep.cu); G(r) differs from the
 //              nearest table row by at most 32 slots, which the warp toggles in
 //              its own correction bitmap in shared memory.  Per word: E table
 //              loads and XORs, no per-bit work.  Rows too wide for a bitmap per
@@ -46,7 +46,7 @@
 // balanced.  The kernel is persistent, one CTA per SM: with one population each
 // warp claims rows one at a time from a device counter; a batch hands each CTA
 // items of rows, which its warps claim one at a time.
-#include "engine.cuh"
+#include "plan.cuh"
 
 #include <algorithm>
 #include <mutex>
@@ -115,15 +115,6 @@ __device__ __forceinline__ uint64_t sw_mask_events(uint64_t h, uint32_t base, co
         m |= (uint64_t)(c & 1u) << j;
     }
     return m;
-}
-
-// r(e) = #{slots with position < e} through the position buckets.
-__device__ __forceinline__ uint32_t threshold_rank(const PopDev& P, double e) {
-    const uint32_t b = pos_bucket(e, P.NB);
-    const uint32_t k0 = __ldg(P.boff + b), k1 = __ldg(P.boff + b + 1u);
-    uint32_t r = k0;
-    for (uint32_t k = k0; k < k1; ++k) r += pos_lt(__ldg(P.bpos + k), e) ? 1u : 0u;
-    return r;
 }
 
 struct RowArgs {
@@ -494,7 +485,6 @@ constexpr uint32_t kRound = 32u * kRoundLane;
 constexpr uint32_t kTableInflight = CLOTHO_TABLE_INFLIGHT;
 constexpr uint32_t kFlatLoads = 4;   // table loads per lane when a narrow row's whole mask is built at once
 constexpr uint32_t kDirectCopyChunks = 2;   // copy rows up to 128 words load their strand directly
-constexpr uint32_t kCmMaxEv = 16;           // chunk-mask build: breakpoints a row takes through the table
 constexpr uint32_t kCmCorr = 32u * kCmMaxEv;   // chunk-mask build: correction slots a warp holds
 constexpr uint32_t kCmAccWords = 3072;      // chunk-mask build: widest rows folded in shared memory
 #ifndef CLOTHO_WARP_CHUNK
@@ -859,16 +849,6 @@ __device__ CLOTHO_COLD float4 row_body_events(const PopDev& P, uint32_t M, const
     float d[kMaxTraits] = {0.f, 0.f, 0.f, 0.f};
     row_body_suf<1>(P, M, R, sfix, nullptr, Q, inv, do_mut, gather, do_fs, fo, d);
     return make_float4(d[0], d[1], d[2], d[3]);
-}
-
-// Nearest suffix-table row b (a multiple of 64) of rank threshold r and the
-// ranks between them: [c0, c0 + n), n <= 32.
-__device__ __forceinline__ uint32_t table_row(uint32_t r, uint32_t A, uint32_t& c0, uint32_t& n) {
-    const uint32_t lo = r & ~63u;
-    const uint32_t b = (r - lo <= 32u) ? lo : lo + 64u;
-    c0 = min(r, b);
-    n = min(max(r, b), A) - c0;
-    return b;
 }
 
 // Phase cycles of the profiling build, kept by every lane, flushed by lane 0.
@@ -1629,8 +1609,8 @@ __device__ __forceinline__ void gen_row_iv(const PopDev& P, const DevStatus& st,
 // PopDev::colcnt when the block moves to another population and at the kernel's end.
 template <bool SUF, bool PROF, bool NARROW, bool CNT = false, bool CM = false>
 __global__ void __launch_bounds__(kGenThreads, 1)
-k_generation(const PopDev* __restrict__ pops, uint32_t npops, WorkCtl* __restrict__ ctl, uint32_t fuse,
-             int profile, uint32_t maxW, uint32_t acc_words, uint32_t mixed) {
+k_generation(const __grid_constant__ PopDev one, const PopDev* __restrict__ pops, uint32_t npops,
+             WorkCtl* __restrict__ ctl, uint32_t fuse, int profile, uint32_t maxW, uint32_t acc_words, uint32_t mixed) {
     const long long c_start = PROF ? clock64() : 0;
     PhaseClk pc;
     if (PROF)
@@ -1671,7 +1651,6 @@ k_generation(const PopDev* __restrict__ pops, uint32_t npops, WorkCtl* __restric
         __syncwarp();
     }
     pdl_wait();
-    pdl_go();
     const bool do_mut = (fuse & kFuseMut) != 0, do_ph = (fuse & kFusePheno) != 0, do_fs = (fuse & kFuseFs) != 0;
     uint64_t* const cplanes =
         CNT ? reinterpret_cast<uint64_t*>(reinterpret_cast<WarpSmem*>(s_dyn + (3u + kWarps) * maxW) + kWarps) : nullptr;
@@ -1690,7 +1669,7 @@ k_generation(const PopDev* __restrict__ pops, uint32_t npops, WorkCtl* __restric
         // One population: each warp takes kWarpChunk rows at a time from the
         // step's counter, with no block barrier between them, so no warp waits
         // for the slowest warp of its block until the kernel's end.
-        const PopDev& P = pops[0];
+        const PopDev& P = one;   // in the kernel's parameters: no round trip for its pointers
         const DevStatus st = *P.st;
         cur_pop = 0;
         cur_W = st.W;
@@ -1716,7 +1695,7 @@ k_generation(const PopDev* __restrict__ pops, uint32_t npops, WorkCtl* __restric
         uint32_t claim = 0;
         const bool group = SUF && NARROW && !PROF && max(st.W, st.pW) <= kGroupWords;
         if (group) {   // rows that share a warp cost about the same: no claims
-            group_rows(P, 0u, S, nullptr, warp * gridDim.x + blockIdx.x, gridDim.x * kWarps, cur_cnt ? &s_crows : nullptr,
+            group_rows(pops[0], 0u, S, nullptr, warp * gridDim.x + blockIdx.x, gridDim.x * kWarps, cur_cnt ? &s_crows : nullptr,
                        sfix, mask, ws.q, sF, sV, fo.cnt, maxW, fuse);
             if (profile && blockIdx.x == 0 && threadIdx.x == 0) { rows_done = S; words_done = (uint64_t)S * st.W; }
         } else if (lane == 0) {
@@ -1941,7 +1920,7 @@ cudaError_t launch_generation(const LaunchCfg& L, const PopDev* pops, uint32_t n
     // 128 words: its narrow build (copy rows by direct loads)
     const bool narrow = L.narrow_ok && maxW <= 64u * kDirectCopyChunks;
     const int si = cm ? 7 : suf ? (profile == 2 ? (narrow ? 4 : 2) : cnt ? (narrow ? 6 : 5) : narrow ? 3 : 1) : 0;
-    using Kernel = void (*)(const PopDev*, uint32_t, WorkCtl*, uint32_t, int, uint32_t, uint32_t, uint32_t);
+    using Kernel = void (*)(PopDev, const PopDev*, uint32_t, WorkCtl*, uint32_t, int, uint32_t, uint32_t, uint32_t);
     static const Kernel fns[8] = {k_generation<false, false, false>,      k_generation<true, false, false>,
                                   k_generation<true, true, false>,        k_generation<true, false, true>,
                                   k_generation<true, true, true>,         k_generation<true, false, false, true>,
@@ -1963,227 +1942,12 @@ cudaError_t launch_generation(const LaunchCfg& L, const PopDev* pops, uint32_t n
             c = smem > 0 ? smem : 1;
         }
     }
-    return launch_smem_k(L, fns[si], dim3(L.num_sms), dim3(kGenThreads), smem, pops, npops, ctl, fuse, profile, maxW,
+    return launch_smem_k(L, fns[si], dim3(L.num_sms), dim3(kGenThreads), smem, npops == 1u ? *L.one : PopDev{}, pops, npops,
+                         ctl, fuse, profile, maxW,
                          (suf && !cm) ? 0u : acc_words, mx);
 }
 
-// ---------------------------------------------------------------------------
-constexpr uint32_t kPlanSmemEv = 16;  // breakpoints of a row the plan kernel ranks in shared memory
-// ---------------------------------------------------------------------------
-// Position ranks of the slots [0, A) and the rows' plans, side by side (both need only the
-// position buckets).
-//
-// A slot's rank = slots in lower buckets + slots of its own bucket with a smaller position
-// (or the same position and a lower slot index).  inv is the inverse map (rank -> slot).
-//
-// Per-row crossover plans for the suffix-table classifier, one thread per row:
-// the top strand (parent individual and strand swap), the breakpoint count,
-// and for every breakpoint its nearest table row and correction ranks; plus
-// the direction of the phenotype gather.  Device-drawn breakpoints get their
-// plan entries from a warp-aggregated counter; tape rows use the tape's own
-// event offsets.
-__device__ __forceinline__ void slot_ranks(const PopDev& P, uint32_t block, uint32_t blocks) {
-    const uint32_t A = P.st->A;
-    for (uint32_t s = block * 256u + threadIdx.x; s < A; s += blocks * 256u) {
-        const double x = P.pos[s];
-        const uint32_t b = pos_bucket(x, P.NB);
-        const uint32_t k0 = P.boff[b], k1 = P.boff[b + 1u];
-        uint32_t r = k0;
-        for (uint32_t k = k0; k < k1; ++k) {
-            const double y = P.bpos[k];
-            r += (y < x || (y == x && P.bslot[k] < s)) ? 1u : 0u;
-        }
-        P.rank[s] = r;
-        if (P.inv) P.inv[r] = s;
-    }
-}
-
-__global__ void __launch_bounds__(256, 4) k_plan(const PopDev* __restrict__ pops, uint32_t npops, uint32_t nrank) {
-    const uint32_t lane = threadIdx.x & 31u;
-    // a thread's thresholds (up to kPlanSmemEv) stay in shared memory while they are ranked
-    // against each other; longer lists use their global slots
-    __shared__ uint32_t s_cr[256][kPlanSmemEv + 1];
-    // the population's Poisson(rho) CDF, searched with integer compares, so a breakpoint count costs no FP64 work
-    __shared__ double s_cdf[kPoisTab + 1];
-    pdl_wait();
-    pdl_go();
-    for (uint32_t p = blockIdx.z; p < npops; p += gridDim.z) {
-        const PopDev& P = pops[p];
-        // blocks [0, nrank) rank the slots, the rest (a single block: the same) plan the rows
-        const bool alone = gridDim.x == 1u;
-        if (alone || blockIdx.x < nrank) slot_ranks(P, alone ? 0u : blockIdx.x, alone ? 1u : nrank);
-        if (!P.plan_row || (!alone && blockIdx.x < nrank)) continue;
-        const uint32_t bx = alone ? 0u : blockIdx.x - nrank, nb = alone ? 1u : gridDim.x - nrank;
-        __syncthreads();  // the previous population's table is no longer read
-        if (threadIdx.x <= kPoisTab) s_cdf[threadIdx.x] = P.pois_rho[threadIdx.x];
-        __syncthreads();
-        const DevStatus st = *P.st;
-        const uint32_t S = 2u * st.N, A = st.A, Se = (S + 1u) >> 1;
-        const bool philox = P.mode == kModePhilox;
-        const bool q1 = (P.flags & 1u) != 0;
-        for (uint32_t v0 = bx * 256u; v0 < S; v0 += nb * 256u) {
-            const uint32_t v = v0 + threadIdx.x;
-            const bool live = v < S;
-            // even gametes on the first half of the threads, odd ones on the second:
-            // under the reference's crossover rule odd gametes are copy rows, so a
-            // warp holds one kind of row
-            const uint32_t g = v < Se ? 2u * v : 2u * (v - Se) + 1u;
-            uint32_t pind = 0, E = 0, base = 0, flags = 0;
-            bool swap = false;
-            if (live) {
-                pind = P.pairs[g];
-                if (pind >= st.pN) {
-                    atomicOr(&P.st->err, kErrParent);
-                    pind = 0;
-                }
-                if (philox) {
-                    const U4 x = philox4x32(g, 0u, st.gen, kStreamGamete, P.seed);
-                    E = (q1 && (g & 1u)) ? 0u : poisson_tab(u01(x.x, x.y), s_cdf, s_cdf[kPoisTab], P.rho);
-                    swap = lt_nonneg(u01(x.z, x.w), P.bias);
-                    if (E > kMaxEvDevice) {
-                        atomicOr(&P.st->err, kErrEvents);
-                        E = kMaxEvDevice;
-                    }
-                } else {
-                    swap = P.swap[g] != 0;
-                    base = P.ev_off[g];
-                    E = (q1 && (g & 1u)) ? 0u : P.ev_off[g + 1u] - base;
-                }
-            }
-            if (philox) {  // warp-aggregated allocation of the plan entries
-                uint32_t incl = E;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
-                    if (lane >= (uint32_t)o) incl += y;
-                }
-                const uint32_t tot = __shfl_sync(0xffffffffu, incl, 31);
-                uint32_t b0 = 0;
-                if (lane == 0 && tot) b0 = atomicAdd(&P.st->ev_used, tot);
-                base = __shfl_sync(0xffffffffu, b0, 0) + incl - E;
-                if (E && base + E > P.EVcap) {
-                    atomicOr(&P.st->err, kErrEvents);
-                    E = 0;
-                }
-            }
-            if (!live) continue;
-            // what the plan entry needs besides the breakpoints, fetched before the breakpoint work so that
-            // their round trips overlap it: the processing position, the new alleles' CSR range, and the
-            // carried phenotypes of both parent strands (one 64-byte line; the gather direction picks one)
-            const uint32_t at = P.ord_pos[g];
-            const uint32_t mo = P.row_off[g], mend = P.row_off[g + 1u];
-            const uint32_t topr = 2u * pind + (swap ? 1u : 0u);
-            asm volatile("prefetch.global.L1 [%0];" ::"l"(P.zg[st.cur ^ 1u] + (size_t)(topr & ~1u) * 4u));
-            if (E > kMaxEvDevice) {
-                flags = kPlanLong;  // tape rows with very long event lists: direct compares
-            } else if (E > 0) {
-                uint32_t* cr = E <= kPlanSmemEv ? s_cr[threadIdx.x] : P.plan_cr + base;
-                // the chunk-mask build classifies rows of more than kCmMaxEv breakpoints by direct compares
-                // against their positions, which device-drawn rows keep in the event list for it (every
-                // population's, to keep the plan kernel uniform; rare: E > 16)
-                const bool keep_pos = philox && E > kCmMaxEv;
-                for (uint32_t k = 0; k < E; k += 2u) {
-                    double e0, e1 = 0.0;
-                    if (philox) {
-                        const U4 a = philox4x32(g, 1u + (k >> 1), st.gen, kStreamGamete, P.seed);
-                        e0 = u01(a.x, a.y);
-                        e1 = u01(a.z, a.w);
-                        if (keep_pos) {
-                            P.ev_pos[base + k] = e0;
-                            if (k + 1u < E) P.ev_pos[base + k + 1u] = e1;
-                        }
-                    } else {
-                        e0 = __ldg(P.ev_pos + base + k);
-                        if (k + 1u < E) e1 = __ldg(P.ev_pos + base + k + 1u);
-                    }
-                    cr[k] = threshold_rank(P, e0);
-                    if (k + 1u < E) cr[k + 1u] = threshold_rank(P, e1);
-                }
-                // share of the rank space the breakpoints switch: sorted thresholds pair into intervals
-                int64_t len = (E & 1u) ? (int64_t)A : 0;
-                for (uint32_t k = 0; k < E; ++k) {
-                    const uint32_t rk = cr[k];
-                    uint32_t posn = 0;
-                    for (uint32_t j = 0; j < E; ++j) {
-                        const uint32_t rj = cr[j];
-                        posn += (rj < rk || (rj == rk && j < k)) ? 1u : 0u;
-                    }
-                    len += (posn & 1u) ? (int64_t)rk : -(int64_t)rk;
-                }
-                if (2 * len > (int64_t)A) flags |= kPlanInv;
-                for (uint32_t k = 0; k < E; ++k) {
-                    uint32_t c0, n;
-                    const uint32_t b = table_row(cr[k], A, c0, n);
-                    P.plan_go[base + k] = (b >> 6) * P.Wcap;
-                    P.plan_cr[base + k] = c0 | (n << 20);
-                }
-            }
-            if (E > kPlanMaxEvents) {
-                atomicOr(&P.st->err, kErrEvents);
-                E = 0;
-                flags = 0;
-            }
-            P.plan_row[at] = make_uint4(g, topr, base, E | (flags << kPlanFlagShift));
-            // what the row's set-up would otherwise fetch after its plan: the new alleles' CSR
-            // range and the carried phenotype's base strand value less the fixed effects
-            P.plan_mut[at] = make_uint2(mo, mend - mo);
-            const uint32_t zs = ((flags & kPlanInv) && st.nz_eff != 0) ? topr ^ 1u : topr;
-            const double* zp = P.zg[st.cur ^ 1u] + (size_t)zs * 4u;
-#pragma unroll
-            for (uint32_t t = 0; t < kMaxTraits; ++t) P.plan_z[(size_t)at * 4u + t] = zp[t] - P.st->fixsum[t];
-        }
-    }
-}
-
 int init_recip_gen() { return fill_recip_table(); }
-
-// suf[g * Wcap + w] = bits of word w whose slot has rank >= 64 g, for
-// g = 0 .. ceil(A/64) (the last row is empty).  A unit of work is 32 words and
-// every kSufSlices-th table row; the units are spread over the whole grid from
-// the current width, so the blocks are busy however wide the capacity is.
-constexpr uint32_t kSufSlices = 16;
-__global__ void __launch_bounds__(256) k_suf_build(const PopDev* __restrict__ pops, uint32_t npops) {
-    __shared__ uint32_t s_grp[32][65];  // (rank >> 6) + 1 per slot, 0 beyond A
-    const uint32_t tx = threadIdx.x & 31u, ty = threadIdx.x >> 5;
-    pdl_wait();
-    pdl_go();
-    for (uint32_t p = blockIdx.z; p < npops; p += gridDim.z) {
-        const PopDev& P = pops[p];
-        if (!P.suf) continue;
-        const uint32_t A = P.st->A, W = P.st->W;
-        const uint32_t Gt = (A + 63u) >> 6;
-        const uint32_t wblocks = (W + 31u) / 32u;
-        for (uint32_t u = blockIdx.x; u < wblocks * kSufSlices; u += gridDim.x) {
-            const uint32_t wb = (u % wblocks) * 32u, slice = u / wblocks;
-            __syncthreads();
-            for (uint32_t i = threadIdx.x; i < 2048u; i += blockDim.x) {
-                const uint32_t s = wb * 64u + i;
-                s_grp[i >> 6][i & 63u] = (s < A) ? (P.rank[s] >> 6) + 1u : 0u;
-            }
-            __syncthreads();
-            const uint32_t w = wb + tx;
-            if (w >= W) continue;
-            for (uint32_t g = slice * 8u + ty; g <= Gt; g += kSufSlices * 8u) {
-                uint64_t m = 0;
-#pragma unroll 16
-                for (uint32_t b = 0; b < 64u; ++b) m |= (uint64_t)(s_grp[tx][b] > g) << b;
-                P.suf[(size_t)g * P.Wcap + w] = m;
-            }
-        }
-    }
-}
-
-uint32_t launch_plan(const LaunchCfg& L, const PopDev* pops, uint32_t npops, const PrepSizes& z, uint32_t maxW) {
-    const uint32_t nr = blocks_for(z.maxA, 256), np = z.tables ? blocks_for(z.maxS, 256) : 0u;
-    const dim3 g = pop_grid(npops, nr + np, L.num_sms, 8);
-    // a slot's rank is a quarter of a row's plan at most
-    const uint32_t nrank = z.tables ? std::max(1u, std::min(nr, g.x / 4u)) : g.x;
-    launch_k(L, k_plan, g, dim3(256), pops, npops, nrank);
-    if (!z.tables) return 1u;
-    const uint32_t units = (maxW + 31u) / 32u * kSufSlices;
-    launch_k(L, k_suf_build, pop_grid(npops, units, L.num_sms, 4), dim3(256), pops, npops);
-    return 2u;
-}
 
 // ---------------------------------------------------------------------------
 // Full per-genome phenotype (staged API and population set-up):

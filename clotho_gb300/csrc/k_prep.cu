@@ -1,7 +1,7 @@
-// k_prep.cu -- everything a generation needs before its rows are written, in six
+// k_prep.cu -- everything a generation needs before its rows are written, in seven
 // kernels: step header, free space, mutation counts and slots, parents, the rows'
-// processing order, and the position buckets of the crossover ranks (the ranks
-// themselves and the rows' plans are k_plan, k_generation.cu).
+// processing order, the position buckets; then the slots' ranks with the rows'
+// crossover plans, and the suffix tables.
 //
 // A small population's step is bound by its launches: every dependent launch costs
 // 3 to 4 us however little it does.  So work that does not depend on each other
@@ -9,11 +9,11 @@
 // prefix sums beside the new alleles; the rows' order beside the bucket counts), a
 // scan is one kernel (each block sums what lies before its chunk itself, as long as
 // that is at most kDirectScan counts; above, one more launch leaves chunk sums), and
-// every kernel is launched with programmatic dependent launch: its blocks are
-// resident when their predecessor ends.
+// every kernel is launched with programmatic dependent launch.
 //
 // All kernels walk every population of the batch on blockIdx.z; sizes are read from
 // the device status words.
+#include "plan.cuh"
 #include "step.cuh"
 
 #include <algorithm>
@@ -166,14 +166,14 @@ __device__ __forceinline__ Share second_share(uint32_t a) {
 // rows is Poisson(2N mu) and, given the total, the rows are uniform -- the
 // same law as M ~ Poisson(mu * 2N) with uniform target rows
 // (mutation_allocator.hpp:41-47, batch_mutation_task_population_space_row.hpp:77).
-__global__ void __launch_bounds__(1024) k_stage1(const PopDev* __restrict__ pops, uint32_t npops,
+template <bool ONE>
+__global__ void __launch_bounds__(1024) k_stage1(const __grid_constant__ PopDev one, const PopDev* __restrict__ pops, uint32_t npops,
                                                  const uint32_t* __restrict__ hdr, WorkCtl* ctl, uint32_t what,
                                                  uint32_t count_on) {
     __shared__ uint32_t s_u32[33];
     pdl_wait();
-    pdl_go();
     for (uint32_t p = blockIdx.z; p < npops; p += gridDim.z) {
-        const PopDev& P = pops[p];
+        const PopDev& P = ONE ? one : pops[p];
         DevStatus* st = P.st;
         const bool philox = P.mode == kModePhilox;
         const uint32_t N = step_N(P, hdr, p), S = 2u * N;
@@ -254,13 +254,13 @@ __global__ void __launch_bounds__(1024) k_stage1(const PopDev* __restrict__ pops
 
 // Chunk sums of the counts that a scan cannot sum by itself (which == 0: new alleles per row, 1: rows per
 // parent, 2: positions per bucket).
-__global__ void __launch_bounds__(256) k_chunk_sums(const PopDev* __restrict__ pops, uint32_t npops,
+template <bool ONE>
+__global__ void __launch_bounds__(256) k_chunk_sums(const __grid_constant__ PopDev one, const PopDev* __restrict__ pops, uint32_t npops,
                                                     const uint32_t* __restrict__ hdr, uint32_t which) {
     __shared__ uint32_t s8[8];
     pdl_wait();
-    pdl_go();
     for (uint32_t p = blockIdx.z; p < npops; p += gridDim.z) {
-        const PopDev& P = pops[p];
+        const PopDev& P = ONE ? one : pops[p];
         const uint32_t L = which == 0 ? 2u * step_N(P, hdr, p) : which == 1 ? order_keys(P.st->pN) : P.NB;
         const uint32_t* cnt = which == 0 ? P.row_cnt : which == 1 ? P.ord_cnt : P.bcnt;
         uint32_t* part = which == 1 ? P.scan_opart : P.scan_upart;
@@ -286,14 +286,14 @@ __global__ void __launch_bounds__(256) k_chunk_sums(const PopDev* __restrict__ p
 // table (TraitSpaceGenerator2, trait_space_generator.hpp:118-129).  One thread per new
 // allele and trait, neighbours in different blocks: a drawn effect is about a hundred
 // operations of the narrow FP64 pipe, so they are spread over all SMs.
-__global__ void __launch_bounds__(256) k_stage2(const PopDev* __restrict__ pops, uint32_t npops,
+template <bool ONE>
+__global__ void __launch_bounds__(256) k_stage2(const __grid_constant__ PopDev one, const PopDev* __restrict__ pops, uint32_t npops,
                                                 const uint32_t* __restrict__ hdr, uint32_t what, uint32_t direct_max,
                                                 uint32_t nres) {
     __shared__ uint32_t s8[8];
     pdl_wait();
-    pdl_go();
     for (uint32_t p = blockIdx.z; p < npops; p += gridDim.z) {
-        const PopDev& P = pops[p];
+        const PopDev& P = ONE ? one : pops[p];
         DevStatus* st = P.st;
         const bool philox = P.mode == kModePhilox;
         const uint32_t N = step_N(P, hdr, p), S = 2u * N;
@@ -345,20 +345,116 @@ __global__ void __launch_bounds__(256) k_stage2(const PopDev* __restrict__ pops,
 }
 
 // ---------------------------------------------------------------------------
-// Stage 3.  Positions per bucket (the first step of the slots' ranks), the rows' processing
+// Stage 3.  The first step of the slots' ranks, the rows' processing
 // positions (parent-major order: rows sorted by parent individual, so rows reading the
 // same parent strands run side by side and the second read of a strand is an L2 hit;
 // the order inside one parent does not matter), the tape's new alleles grouped by row;
 // the counts of stage 1 go back to zero.
-__global__ void __launch_bounds__(256) k_stage3(const PopDev* __restrict__ pops, uint32_t npops, uint32_t what) {
+//
+// Ranks of many slots: positions per bucket here, grouped by stages 4 and 5, ranked beside the plans.  Of few
+// (DIRECT, at most kDirectRanks slots of capacity): all of it here, by one block in shared memory, which saves three
+// launches.
+struct RankSmem {   // dynamic shared memory of the DIRECT form
+    uint64_t key[kDirectRanks];       // positions grouped by bucket, as integers of the same order
+    uint32_t off[kDirectRanks + 4];   // counts, then offsets, per bucket
+    uint16_t slot[kDirectRanks];
+    uint32_t s32[32];
+};
+
+__device__ __forceinline__ void rank_block(const PopDev& P, uint32_t A, RankSmem& z) {
+    constexpr uint32_t kItems = kDirectRanks / 1024u;
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, NB = P.NB, per = NB >> 10;
+    for (uint32_t i = tid; i < NB; i += 1024u) z.off[i] = 0u;
+    double x[kItems];
+#pragma unroll
+    for (uint32_t j = 0; j < kItems; ++j) x[j] = tid + 1024u * j < A ? P.pos[tid + 1024u * j] : 0.0;
+    __syncthreads();
+    uint32_t at[kItems];   // bucket, and the place in it
+#pragma unroll
+    for (uint32_t j = 0; j < kItems; ++j)
+        if (tid + 1024u * j < A) {
+            const uint32_t b = pos_bucket(x[j], NB);
+            at[j] = b | atomicAdd(&z.off[b], 1u) << 16;
+        }
+    __syncthreads();
+    // exclusive prefix of the counts, NB / 1024 buckets a thread (NB is a power of two, 1,024 to 8,192)
+    uint32_t n[kItems], s = 0;
+#pragma unroll
+    for (uint32_t j = 0; j < kItems; ++j) {
+        n[j] = j < per ? z.off[tid * per + j] : 0u;
+        s += n[j];
+    }
+    uint32_t incl = s;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= (uint32_t)o) incl += y;
+    }
+    if (lane == 31u) z.s32[warp] = incl;
+    __syncthreads();
+    uint32_t t = z.s32[lane];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, t, o);
+        if (lane >= (uint32_t)o) t += y;
+    }
+    const uint32_t before = __shfl_sync(0xffffffffu, t, warp ? warp - 1u : 0u);
+    uint32_t run = (warp ? before : 0u) + incl - s;
+#pragma unroll
+    for (uint32_t j = 0; j < kItems; ++j)
+        if (j < per) {
+            z.off[tid * per + j] = run;
+            P.boff[tid * per + j] = run;
+            run += n[j];
+        }
+    if (tid == 1023u) {
+        z.off[NB] = A;
+        P.boff[NB] = A;
+    }
+    __syncthreads();
+#pragma unroll
+    for (uint32_t j = 0; j < kItems; ++j)
+        if (tid + 1024u * j < A) {
+            const uint32_t k = z.off[at[j] & 0xffffu] + (at[j] >> 16);
+            z.key[k] = pos_key(x[j]);
+            z.slot[k] = (uint16_t)(tid + 1024u * j);
+            P.bpos[k] = x[j];
+        }
+    __syncthreads();
+#pragma unroll
+    for (uint32_t j = 0; j < kItems; ++j) {
+        const uint32_t me = tid + 1024u * j;
+        if (me >= A) break;
+        const uint64_t key = pos_key(x[j]);
+        const uint32_t b = at[j] & 0xffffu, k1 = z.off[b + 1u];
+        uint32_t r = z.off[b];
+        for (uint32_t k = r; k < k1; ++k) r += (z.key[k] < key || (z.key[k] == key && z.slot[k] < me)) ? 1u : 0u;
+        P.rank[me] = r;
+        P.inv[r] = me;
+    }
+    __syncthreads();   // the next population's counts
+}
+
+template <bool ONE, bool DIRECT>
+__global__ void __launch_bounds__(DIRECT ? 1024 : 256)
+k_stage3(const __grid_constant__ PopDev one, const PopDev* __restrict__ pops, uint32_t npops, uint32_t what) {
+    extern __shared__ __align__(16) uint8_t s_raw[];
+    constexpr uint32_t kThreads = DIRECT ? 1024u : 256u;
     pdl_wait();
-    pdl_go();
     for (uint32_t p = blockIdx.z; p < npops; p += gridDim.z) {
-        const PopDev& P = pops[p];
+        const PopDev& P = ONE ? one : pops[p];
         const DevStatus* st = P.st;
-        const uint32_t at = blockIdx.x * 256u + threadIdx.x, step = gridDim.x * 256u;
-        const uint32_t A = st->A, N = st->N, pN = st->pN, S = 2u * N;
-        for (uint32_t s = at; s < A; s += step) atomicAdd(&P.bcnt[pos_bucket(P.pos[s], P.NB)], 1u);
+        const uint32_t A = st->A;
+        // DIRECT: the first block ranks the slots, the others do the rest
+        if (DIRECT && blockIdx.x == 0) {
+            rank_block(P, A, *reinterpret_cast<RankSmem*>(s_raw));
+            continue;
+        }
+        const uint32_t at = (blockIdx.x - (DIRECT ? 1u : 0u)) * kThreads + threadIdx.x;
+        const uint32_t step = (gridDim.x - (DIRECT ? 1u : 0u)) * kThreads;
+        const uint32_t N = st->N, pN = st->pN, S = 2u * N;
+        if (!DIRECT)
+            for (uint32_t s = at; s < A; s += step) atomicAdd(&P.bcnt[pos_bucket(P.pos[s], P.NB)], 1u);
         if ((what & kStepOrder) && P.plan_row) {
             for (uint32_t g = at; g < S; g += step) {
                 const uint32_t id = P.pairs[g];
@@ -410,41 +506,43 @@ static __device__ void sort_ascending(uint32_t* a, uint32_t n) {
     }
 }
 
+// Each tape row's new alleles in ascending mutation index (the list order is the order in which their FP32 effects
+// enter the row's carried phenotype, so it must not depend on the order of the scatter's atomics).  One thread per
+// list position; the thread at a row's first position sorts the row's list: ownership is decided by position, which
+// never moves, and every entry of a row's segment names that row, so no other thread acts on it.
+__device__ __forceinline__ void sort_tape_lists(const PopDev& P, uint32_t at, uint32_t step) {
+    const uint32_t listed = P.row_off[2u * P.st->N];
+    for (uint32_t t = at; t < listed; t += step) {
+        const uint32_t s = P.mut_seq[P.row_mut[t]];
+        const uint32_t off = P.row_off[s], n = P.row_off[s + 1u] - off;
+        if (t == off && n >= 2u) sort_ascending(P.row_mut + off, n);
+    }
+}
+
 // ---------------------------------------------------------------------------
-// Stage 4.  The prefix sum of the positions per bucket, and each tape row's new alleles in
-// ascending mutation index (the list order is the order in which their FP32 effects
-// enter the row's carried phenotype, so it must not depend on the order of the
-// scatter's atomics).  One thread per list position; the thread at a row's first
-// position sorts the row's list: ownership is decided by position, which never moves,
-// and every entry of a row's segment names that row, so no other thread acts on it.
-__global__ void __launch_bounds__(256) k_stage4(const PopDev* __restrict__ pops, uint32_t npops, uint32_t what,
-                                                uint32_t direct_max) {
+// Stage 4.  The prefix sum of the positions per bucket, and the tape rows' lists in order.
+template <bool ONE>
+__global__ void __launch_bounds__(256) k_stage4(const __grid_constant__ PopDev one, const PopDev* __restrict__ pops,
+                                                uint32_t npops, uint32_t what, uint32_t direct_max) {
     __shared__ uint32_t s8[8];
     pdl_wait();
-    pdl_go();
     for (uint32_t p = blockIdx.z; p < npops; p += gridDim.z) {
-        const PopDev& P = pops[p];
+        const PopDev& P = ONE ? one : pops[p];
         for (uint32_t c = blockIdx.x; c * kChunk < P.NB; c += gridDim.x) {
             const uint32_t total = scan_chunk(P.bcnt, P.scan_upart, P.NB <= direct_max, P.NB, c, P.boff, P.bcur, s8);
             if ((c + 1u) * kChunk >= P.NB && threadIdx.x == 0) P.boff[P.NB] = total;
         }
-        if ((what & kStepMut) && P.mode != kModePhilox) {
-            const uint32_t listed = P.row_off[2u * P.st->N];
-            for (uint32_t t = blockIdx.x * 256u + threadIdx.x; t < listed; t += gridDim.x * 256u) {
-                const uint32_t s = P.mut_seq[P.row_mut[t]];
-                const uint32_t off = P.row_off[s], n = P.row_off[s + 1u] - off;
-                if (t == off && n >= 2u) sort_ascending(P.row_mut + off, n);
-            }
-        }
+        if ((what & kStepMut) && P.mode != kModePhilox)
+            sort_tape_lists(P, blockIdx.x * 256u + threadIdx.x, gridDim.x * 256u);
     }
 }
 
 // Stage 5.  Positions and slots grouped by bucket; the bucket counts go back to zero.
-__global__ void __launch_bounds__(256) k_stage5(const PopDev* __restrict__ pops, uint32_t npops) {
+template <bool ONE>
+__global__ void __launch_bounds__(256) k_stage5(const __grid_constant__ PopDev one, const PopDev* __restrict__ pops, uint32_t npops) {
     pdl_wait();
-    pdl_go();
     for (uint32_t p = blockIdx.z; p < npops; p += gridDim.z) {
-        const PopDev& P = pops[p];
+        const PopDev& P = ONE ? one : pops[p];
         const uint32_t at = blockIdx.x * 256u + threadIdx.x, step = gridDim.x * 256u;
         const uint32_t A = P.st->A;
         for (uint32_t s = at; s < A; s += step) {
@@ -457,44 +555,141 @@ __global__ void __launch_bounds__(256) k_stage5(const PopDev* __restrict__ pops,
     }
 }
 
+// ---------------------------------------------------------------------------
+// The rows' plans, and beside them what does not depend on them: the slots' ranks (both need only the position
+// buckets), or, with DIRECT ranks, the suffix table and the tape rows' lists.
+
+// suf[g * Wcap + w] = bits of word w whose slot has rank >= 64 g, for
+// g = 0 .. ceil(A/64) (the last row is empty).  A unit of work is 32 words and
+// every kSufSlices-th table row; the units are spread over the blocks from
+// the current width, so the blocks are busy however wide the capacity is.
+constexpr uint32_t kSufSlices = 16;
+__device__ __forceinline__ void build_suffix_table(const PopDev& P, uint32_t block, uint32_t blocks,
+                                                   uint32_t (*s_grp)[65]) {   // (rank >> 6) + 1 per slot, 0 beyond A
+    const uint32_t tx = threadIdx.x & 31u, ty = threadIdx.x >> 5;
+    const uint32_t A = P.st->A, W = P.st->W;
+    const uint32_t Gt = (A + 63u) >> 6;
+    const uint32_t wblocks = (W + 31u) / 32u;
+    for (uint32_t u = block; u < wblocks * kSufSlices; u += blocks) {
+        const uint32_t wb = (u % wblocks) * 32u, slice = u / wblocks;
+        __syncthreads();
+        for (uint32_t i = threadIdx.x; i < 2048u; i += 256u) {
+            const uint32_t s = wb * 64u + i;
+            s_grp[i >> 6][i & 63u] = (s < A) ? (P.rank[s] >> 6) + 1u : 0u;
+        }
+        __syncthreads();
+        const uint32_t w = wb + tx;
+        if (w >= W) continue;
+        for (uint32_t g = slice * 8u + ty; g <= Gt; g += kSufSlices * 8u) {
+            uint64_t m = 0;
+#pragma unroll 16
+            for (uint32_t b = 0; b < 64u; ++b) m |= (uint64_t)(s_grp[tx][b] > g) << b;
+            P.suf[(size_t)g * P.Wcap + w] = m;
+        }
+    }
+}
+
+template <bool ONE, bool DIRECT>
+__global__ void __launch_bounds__(256, 4) k_plan(const __grid_constant__ PopDev one, const PopDev* __restrict__ pops,
+                                                 uint32_t npops, uint32_t what, uint32_t nside) {
+    __shared__ uint32_t s_cr[256][kPlanSmemEv + 1];
+    __shared__ double s_cdf[kPoisTab + 1];
+    __shared__ uint32_t s_grp[DIRECT ? 32 : 1][65];
+    pdl_wait();
+    for (uint32_t p = blockIdx.z; p < npops; p += gridDim.z) {
+        const PopDev& P = ONE ? one : pops[p];
+        const DevStatus st = *P.st;
+        const Share side = first_share(nside), plan = second_share(nside);
+        if (side.on) {
+            if (DIRECT) {
+                if ((what & kStepMut) && P.mode != kModePhilox)
+                    sort_tape_lists(P, side.i * 256u + threadIdx.x, side.n * 256u);
+                build_suffix_table(P, side.i, side.n, s_grp);
+            } else {
+                for (uint32_t s = side.i * 256u + threadIdx.x; s < st.A; s += side.n * 256u) slot_rank(P, s);
+            }
+        }
+        if (!P.plan_row || !plan.on) continue;
+        __syncthreads();  // the previous population's tables are no longer read
+        if (threadIdx.x <= kPoisTab) s_cdf[threadIdx.x] = P.pois_rho[threadIdx.x];
+        __syncthreads();
+        for (uint32_t v0 = plan.i * 256u; v0 < 2u * st.N; v0 += plan.n * 256u) {
+            plan_row(P, st, v0 + threadIdx.x, s_cdf, s_cr[threadIdx.x]);
+        }
+    }
+}
+
+// The suffix tables of populations whose ranks k_plan has made.
+template <bool ONE>
+__global__ void __launch_bounds__(256) k_suf_build(const __grid_constant__ PopDev one, const PopDev* __restrict__ pops,
+                                                   uint32_t npops) {
+    __shared__ uint32_t s_grp[32][65];
+    pdl_wait();
+    for (uint32_t p = blockIdx.z; p < npops; p += gridDim.z) {
+        const PopDev& P = ONE ? one : pops[p];
+        if (P.suf) build_suffix_table(P, blockIdx.x, gridDim.x, s_grp);
+    }
+}
+
+uint32_t launch_plan(const LaunchCfg& L, const PopDev* pops, uint32_t npops, const PrepSizes& z, uint32_t maxW,
+                     uint32_t what) {
+    const uint32_t np = z.tables ? blocks_for(z.maxS, 256) : 0u, units = (maxW + 31u) / 32u * kSufSlices;
+    if (direct_ranks(z)) {
+        const dim3 g = pop_grid(npops, units + np, L.num_sms, 8);
+        launch_pops(L, k_plan<true, true>, k_plan<false, true>, g, dim3(256), pops, npops, what,
+                    std::max(1u, std::min(units, g.x / 3u)));
+        return 1u;
+    }
+    const uint32_t nr = blocks_for(z.maxA, 256);
+    const dim3 g = pop_grid(npops, nr + np, L.num_sms, 8);
+    // a slot's rank is a quarter of a row's plan at most
+    const uint32_t nrank = z.tables ? std::max(1u, std::min(nr, g.x / 4u)) : g.x;
+    launch_pops(L, k_plan<true, false>, k_plan<false, false>, g, dim3(256), pops, npops, what, nrank);
+    if (!z.tables) return 1u;
+    launch_pops(L, k_suf_build<true>, k_suf_build<false>, pop_grid(npops, units, L.num_sms, 4), dim3(256), pops, npops);
+    return 2u;
+}
+
 uint32_t launch_prep(const LaunchCfg& L, const PopDev* pops, uint32_t npops, const PrepSizes& z, const uint32_t* hdr,
                      WorkCtl* ctl, uint32_t what, bool count_on) {
     // up to this many counts a scan block sums what lies before its chunk by itself: at 32,768 counts the last
     // block reads 128 KB of L2, about as long as the extra launch that it saves
     constexpr uint32_t kDirectScan = 32768;
     uint32_t n = 0;
+    auto sums = [&](uint32_t most, uint32_t which) {
+        launch_pops(L, k_chunk_sums<true>, k_chunk_sums<false>, pop_grid(npops, blocks_for(most, kChunk), L.num_sms, 4),
+                    dim3(256), pops, npops, hdr, which);
+        ++n;
+    };
     if (what & (kStepBegin | kStepMut | kStepOrder)) {
         dim3 g = pop_grid(npops, blocks_for(z.maxS, kChunk), L.num_sms, std::max(1u, L.ind_per_sm / 4u));
         g.x += 1u;
-        launch_k(L, k_stage1, g, dim3(1024), pops, npops, hdr, ctl, what, count_on ? 1u : 0u);
+        launch_pops(L, k_stage1<true>, k_stage1<false>, g, dim3(1024), pops, npops, hdr, ctl, what, count_on ? 1u : 0u);
         ++n;
         // chunk sums: of the tape's counts (device draws leave their own in stage 1), of the rows per parent
-        if ((what & kStepMut) && (what & kStepTape) && z.maxS > kDirectScan) {
-            launch_k(L, k_chunk_sums, pop_grid(npops, blocks_for(z.maxS, kChunk), L.num_sms, 4), dim3(256), pops, npops,
-                     hdr, 0u);
-            ++n;
-        }
-        if ((what & kStepOrder) && z.tables && z.maxN > kDirectScan) {
-            launch_k(L, k_chunk_sums, pop_grid(npops, blocks_for(z.maxN, kChunk), L.num_sms, 4), dim3(256), pops, npops,
-                     hdr, 1u);
-            ++n;
-        }
+        if ((what & kStepMut) && (what & kStepTape) && z.maxS > kDirectScan) sums(z.maxS, 0u);
+        if ((what & kStepOrder) && z.tables && z.maxN > kDirectScan) sums(z.maxN, 1u);
         const uint32_t units = blocks_for(z.maxS + 1u, kChunk) + blocks_for(z.maxN, kChunk);
         g = pop_grid(npops, units + (uint32_t)L.num_sms, L.num_sms, 6);
-        launch_k(L, k_stage2, g, dim3(256), pops, npops, hdr, what, kDirectScan, std::max(1u, g.x / 3u));
+        launch_pops(L, k_stage2<true>, k_stage2<false>, g, dim3(256), pops, npops, hdr, what, kDirectScan,
+                    std::max(1u, g.x / 3u));
         ++n;
     }
-    launch_k(L, k_stage3, pop_grid(npops, blocks_for(std::max(z.maxS, z.maxA), 256), L.num_sms, 8), dim3(256), pops,
-             npops, what);
-    if (z.maxNB > kDirectScan) {
-        launch_k(L, k_chunk_sums, pop_grid(npops, blocks_for(z.maxNB, kChunk), L.num_sms, 4), dim3(256), pops, npops,
-                 hdr, 2u);
-        ++n;
+    const uint32_t rest = blocks_for(z.maxS, 256);
+    if (direct_ranks(z)) {
+        dim3 g = pop_grid(npops, blocks_for(z.maxS, 1024), L.num_sms, 2);
+        g.x += 1u;
+        launch_pops_smem(L, k_stage3<true, true>, k_stage3<false, true>, g, dim3(1024), sizeof(RankSmem), pops, npops,
+                         what);
+        return n + 1u;
     }
-    launch_k(L, k_stage4, pop_grid(npops, blocks_for(z.maxNB, kChunk), L.num_sms, 4), dim3(256), pops, npops, what,
-             kDirectScan);
-    launch_k(L, k_stage5, pop_grid(npops, blocks_for(std::max(z.maxNB, z.maxA), 256), L.num_sms, 8), dim3(256), pops,
-             npops);
+    launch_pops(L, k_stage3<true, false>, k_stage3<false, false>,
+                pop_grid(npops, std::max(rest, blocks_for(z.maxA, 256)), L.num_sms, 8), dim3(256), pops, npops, what);
+    if (z.maxNB > kDirectScan) sums(z.maxNB, 2u);
+    launch_pops(L, k_stage4<true>, k_stage4<false>, pop_grid(npops, blocks_for(z.maxNB, kChunk), L.num_sms, 4), dim3(256),
+                pops, npops, what, kDirectScan);
+    launch_pops(L, k_stage5<true>, k_stage5<false>,
+                pop_grid(npops, blocks_for(std::max(z.maxNB, z.maxA), 256), L.num_sms, 8), dim3(256), pops, npops);
     return n + 3u;
 }
 

@@ -109,14 +109,14 @@ void launch_mut_scatter(const LaunchCfg& L, const PopDev* pops, uint32_t npops) 
 // Bound by the FP64 pipe (about two operations a clock and SM): the exponential and the sum's adds.  So every
 // warp of the GPU takes 128 individuals, and what is the same for all of them (the root, the quotients) is
 // computed once a block.
-__global__ void __launch_bounds__(256) k_individuals(const PopDev* __restrict__ pops, uint32_t npops) {
+template <bool ONE>
+__global__ void __launch_bounds__(256) k_individuals(const __grid_constant__ PopDev one, const PopDev* __restrict__ pops, uint32_t npops) {
     __shared__ double s_k[4];
     __shared__ double s_f[8][128];
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     pdl_wait();
-    pdl_go();
     for (uint32_t p = blockIdx.z; p < npops; p += gridDim.z) {
-        const PopDev& P = pops[p];
+        const PopDev& P = ONE ? one : pops[p];
         DevStatus* st = P.st;
         const uint32_t N = st->N, T = P.T;
         const uint32_t nw = (N + kScanChunk - 1u) / kScanChunk * 32u;  // whole chunks: empty warps sum to zero
@@ -209,7 +209,6 @@ __global__ void __launch_bounds__(256) k_cdf_offsets(const PopDev* __restrict__ 
     __shared__ double s_acc;
     const PopDev& P = pops[blockIdx.x];
     pdl_wait();
-    pdl_go();
     const uint32_t nch = (P.st->N + kScanChunk - 1u) / kScanChunk;
     if (nch <= kInlineChunks) return;
     if (threadIdx.x == 0) s_acc = 0.0;
@@ -232,15 +231,15 @@ __global__ void __launch_bounds__(256) k_cdf_offsets(const PopDev* __restrict__ 
 }
 
 // A unit is 8 warps of 128 individuals: a quarter of a chunk.
-__global__ void __launch_bounds__(256) k_cdf(const PopDev* __restrict__ pops, uint32_t npops, uint32_t end) {
+template <bool ONE>
+__global__ void __launch_bounds__(256) k_cdf(const __grid_constant__ PopDev one, const PopDev* __restrict__ pops, uint32_t npops, uint32_t end) {
     __shared__ double s_tot[kInlineChunks];
     __shared__ double s_woff[32];
     __shared__ double s_part, s_last;
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     pdl_wait();
-    pdl_go();
     for (uint32_t p = blockIdx.z; p < npops; p += gridDim.z) {
-        const PopDev& P = pops[p];
+        const PopDev& P = ONE ? one : pops[p];
         DevStatus* st = P.st;
         const uint32_t N = st->N;
         const uint32_t nch = (N + kScanChunk - 1u) / kScanChunk;
@@ -309,10 +308,10 @@ __global__ void __launch_bounds__(256) k_cdf(const PopDev* __restrict__ pops, ui
 }
 uint32_t launch_fitness(const LaunchCfg& L, const PopDev* pops, uint32_t npops, uint32_t maxN, bool end) {
     const uint32_t units = std::max(1u, (maxN + kScanChunk - 1u) / kScanChunk * 4u);
-    launch_k(L, k_individuals, pop_grid(npops, units, L.num_sms, L.ind_per_sm), dim3(256), pops, npops);
+    launch_pops(L, k_individuals<true>, k_individuals<false>, pop_grid(npops, units, L.num_sms, L.ind_per_sm), dim3(256), pops, npops);
     const bool offsets = maxN > kInlineChunks * kScanChunk;
     if (offsets) launch_k(L, k_cdf_offsets, dim3(npops), dim3(256), pops);
-    launch_k(L, k_cdf, pop_grid(npops, units, L.num_sms, 8), dim3(256), pops, npops, end ? 1u : 0u);
+    launch_pops(L, k_cdf<true>, k_cdf<false>, pop_grid(npops, units, L.num_sms, 8), dim3(256), pops, npops, end ? 1u : 0u);
     return offsets ? 3u : 2u;
 }
 
