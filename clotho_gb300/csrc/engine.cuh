@@ -375,6 +375,17 @@ uint32_t launch_prep(const LaunchCfg&, const PopDev* pops, uint32_t npops, const
 // Allele capacity up to which one block ranks a population's slots in shared memory (k_prep.cu)
 constexpr uint32_t kDirectRanks = 8192;
 inline bool direct_ranks(const PrepSizes& z) { return z.maxA <= kDirectRanks && z.tables; }
+// One generation's tape from a pinned staging block into a population's tape arrays, and the step's header: pieces
+// of n16 16-byte words (the last one padded; arrays and staging start on 16-byte boundaries).
+struct TapePieces {
+    const void* src[7];
+    void* dst[7];
+    uint32_t end[7];      // 16-byte words up to and with this piece
+    uint32_t N, M;
+};
+void launch_tape_upload(const LaunchCfg&, const TapePieces&, uint32_t* hdr);
+// dst[i * T + t] = src[i * 4 + t]
+void launch_pack_traits(const LaunchCfg&, const double* src, double* dst, uint32_t n, uint32_t T);
 // Poisson tables of one population (the device copy of its descriptor)
 void launch_pois_tables(cudaStream_t s, const PopDev& P);
 void launch_mut_resolve(const LaunchCfg&, const PopDev* pops, uint32_t npops);

@@ -377,13 +377,10 @@ __device__ __forceinline__ void rank_block(const PopDev& P, uint32_t A, RankSmem
             at[j] = b | atomicAdd(&z.off[b], 1u) << 16;
         }
     __syncthreads();
-    // exclusive prefix of the counts, NB / 1024 buckets a thread (NB is a power of two, 1,024 to 8,192)
-    uint32_t n[kItems], s = 0;
-#pragma unroll
-    for (uint32_t j = 0; j < kItems; ++j) {
-        n[j] = j < per ? z.off[tid * per + j] : 0u;
-        s += n[j];
-    }
+    // exclusive prefix of the counts: four or eight buckets a thread (capacities come in steps of 4,096 slots)
+    uint4* const off4 = reinterpret_cast<uint4*>(z.off) + tid * (per >> 2);
+    uint4 n0 = off4[0], n1 = per > 4u ? off4[1] : make_uint4(0, 0, 0, 0);
+    const uint32_t s = n0.x + n0.y + n0.z + n0.w + n1.x + n1.y + n1.z + n1.w;
     uint32_t incl = s;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -400,18 +397,18 @@ __device__ __forceinline__ void rank_block(const PopDev& P, uint32_t A, RankSmem
     }
     const uint32_t before = __shfl_sync(0xffffffffu, t, warp ? warp - 1u : 0u);
     uint32_t run = (warp ? before : 0u) + incl - s;
-#pragma unroll
-    for (uint32_t j = 0; j < kItems; ++j)
-        if (j < per) {
-            z.off[tid * per + j] = run;
-            P.boff[tid * per + j] = run;
-            run += n[j];
-        }
-    if (tid == 1023u) {
-        z.off[NB] = A;
-        P.boff[NB] = A;
-    }
+    auto advance = [&run](uint4& q) {
+        const uint4 c = q;
+        q = make_uint4(run, run + c.x, run + c.x + c.y, run + c.x + c.y + c.z);
+        run = q.w + c.w;
+    };
+    advance(n0);
+    advance(n1);
+    off4[0] = n0;
+    if (per > 4u) off4[1] = n1;
+    if (tid == 1023u) z.off[NB] = A;
     __syncthreads();
+    for (uint32_t i = tid; i <= NB; i += 1024u) P.boff[i] = z.off[i];
 #pragma unroll
     for (uint32_t j = 0; j < kItems; ++j)
         if (tid + 1024u * j < A) {
@@ -691,6 +688,41 @@ uint32_t launch_prep(const LaunchCfg& L, const PopDev* pops, uint32_t npops, con
     launch_pops(L, k_stage5<true>, k_stage5<false>,
                 pop_grid(npops, blocks_for(std::max(z.maxNB, z.maxA), 256), L.num_sms, 8), dim3(256), pops, npops);
     return n + 3u;
+}
+
+// ---------------------------------------------------------------------------
+// A small tape's arrays in one launch: the host has packed them into one pinned block, which the threads read over
+// the chip-to-chip link, 16 bytes each.  (Seven copies from pageable memory cost 10 us each on the host, 88 us a
+// call at 10,007 individuals, where the bytes take 3.)
+__global__ void __launch_bounds__(256) k_tape_upload(const TapePieces z, uint32_t* __restrict__ hdr) {
+    pdl_wait();
+    const uint32_t at = blockIdx.x * 256u + threadIdx.x, step = gridDim.x * 256u;
+    if (at == 0) {
+        hdr[0] = z.N;
+        hdr[1] = z.M;
+    }
+    for (uint32_t i = at; i < z.end[6]; i += step) {
+        uint32_t begin = 0;
+#pragma unroll
+        for (uint32_t k = 0; k < 7; ++k) {
+            if (i >= begin && i < z.end[k])
+                static_cast<uint4*>(z.dst[k])[i - begin] = __ldcv(static_cast<const uint4*>(z.src[k]) + (i - begin));
+            begin = z.end[k];
+        }
+    }
+}
+void launch_tape_upload(const LaunchCfg& L, const TapePieces& z, uint32_t* hdr) {
+    const uint32_t g = std::min(blocks_for(z.end[6], 256), (uint32_t)L.num_sms * 2u);
+    launch_k(L, k_tape_upload, dim3(g), dim3(256), z, hdr);
+}
+
+__global__ void __launch_bounds__(256) k_pack_traits(const double* __restrict__ src, double* __restrict__ dst, uint32_t n,
+                                                     uint32_t T) {
+    for (uint32_t i = blockIdx.x * 256u + threadIdx.x; i < n; i += gridDim.x * 256u)
+        for (uint32_t t = 0; t < T; ++t) dst[(size_t)i * T + t] = src[(size_t)i * 4u + t];
+}
+void launch_pack_traits(const LaunchCfg& L, const double* src, double* dst, uint32_t n, uint32_t T) {
+    k_pack_traits<<<std::min(blocks_for(n, 256), (uint32_t)L.num_sms * 8u), 256, 0, L.stream>>>(src, dst, n, T);
 }
 
 // ---------------------------------------------------------------------------
