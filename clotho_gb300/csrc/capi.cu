@@ -105,6 +105,9 @@ struct clotho_ctx {
     std::vector<PopHost*> pops;
     PopDev* d_pops[3] = {nullptr, nullptr, nullptr};  // per set: npops contiguous PopDev
     WorkCtl* d_ctl = nullptr;
+    BlockPart* d_parts = nullptr;      // a batch's block tables (BlockTable), kMaxParts entries each
+    uint32_t n_parts[3] = {0, 0, 0};
+    bool parts_stale = true;
     uint32_t* d_hdr[3] = {nullptr, nullptr, nullptr}; // per set: [2*npops]
     // step headers (N, M per population) are staged in a ring of pinned slots:
     // a slot is reused only after the copy that read it has completed
@@ -148,6 +151,7 @@ struct clotho_ctx {
 namespace {
 
 constexpr uint32_t kHdrRing = 64;
+constexpr uint32_t kMaxParts = 4096;   // blocks of a batch's launch at most
 constexpr uint32_t kStatRing = 8;   // outstanding asynchronous status reads (clotho_info_request)
 static_assert(sizeof(((clotho_ctx*)nullptr)->ring_ev) / sizeof(cudaEvent_t) == kHdrRing, "header ring size");
 static_assert(sizeof(((clotho_ctx*)nullptr)->stat_ev) / sizeof(cudaEvent_t) == kStatRing, "status ring size");
@@ -168,6 +172,10 @@ int fail(clotho_ctx* c, int code, const std::string& m) {
 LaunchCfg cfg(clotho_ctx* ctx, uint32_t set = 0) {
     LaunchCfg L{ctx->stream, ctx->num_sms};
     if (!ctx->pops.empty()) L.one = &ctx->pops[0]->dev[set];  // taken by launches over the first population alone
+    for (uint32_t k = 0; k < 3; ++k) {
+        L.parts[k] = ctx->d_parts ? ctx->d_parts + k * kMaxParts : nullptr;
+        L.blocks[k] = ctx->n_parts[k];
+    }
     L.ind_per_sm = ctx->ind_per_sm;
     L.narrow_ok = ctx->narrow_ok;
     return L;
@@ -336,7 +344,36 @@ int sync_pop_arrays(clotho_ctx* ctx, uint32_t from = 0) {
         }
     }
     if (ctx->graph) { cudaGraphExecDestroy(ctx->graph); ctx->graph = nullptr; }
+    ctx->parts_stale = true;
     CK(cudaStreamSynchronize(ctx->stream));
+    return 0;
+}
+
+// The block tables of a batch, made anew before the first step after its populations (or the tuning) changed: blocks
+// in proportion to the populations' rows (plans: rows and breakpoints), a few an SM (by the tuning; two of 1,024
+// threads), so that blocks that come later even out what the proportions miss.
+int block_tables(clotho_ctx* ctx) {
+    const size_t n = ctx->pops.size();
+    if (!ctx->parts_stale || n < 2) return 0;
+    if (!ctx->d_parts) CK(cudaMalloc(&ctx->d_parts, sizeof(BlockPart) * 3 * kMaxParts));
+    std::vector<BlockPart> h(3 * kMaxParts);
+    for (uint32_t k = 0; k < 3; ++k) {
+        auto work = [k](const PopHost* p) { return p->dev[0].Scap * (k == kTablePlan ? 1.0 + 0.4 * p->desc.rho : 1.0); };
+        double sum = 0.0;
+        for (const PopHost* p : ctx->pops) sum += work(p);
+        const uint32_t least = k == kTable1024 ? 2u : 1u;   // there a population's first block has a job of its own
+        const double all = std::min<double>(
+            (double)ctx->num_sms * (k == kTable1024 ? 2u : std::max(1u, ctx->ind_per_sm / 2u)), kMaxParts - (double)n * least);
+        uint32_t at = 0;
+        for (uint32_t p = 0; p < n; ++p) {
+            const uint32_t b = std::max(least, (uint32_t)(all * work(ctx->pops[p]) / sum));
+            for (uint32_t i = 0; i < b; ++i) h[k * kMaxParts + at++] = BlockPart{p, i, b, 0u};
+        }
+        ctx->n_parts[k] = at;
+    }
+    CK(cudaMemcpyAsync(ctx->d_parts, h.data(), h.size() * sizeof(BlockPart), cudaMemcpyHostToDevice, ctx->stream));
+    CK(cudaStreamSynchronize(ctx->stream));
+    ctx->parts_stale = false;
     return 0;
 }
 
@@ -495,6 +532,7 @@ void ensure_parent_acc(clotho_ctx* ctx, const PopDev* pops, uint32_t npops) {
 
 // The fused step shared by tape and device-drawn modes, for every population.
 void enqueue_fused_step(clotho_ctx* ctx, uint32_t set, bool philox) {
+    // (block_tables has run: the callers that can hold several populations see to it)
     const uint32_t n = (uint32_t)ctx->pops.size();
     const PopDev* pops = ctx->d_pops[set];
     const LaunchCfg L = cfg(ctx, set);
@@ -514,6 +552,7 @@ void enqueue_fused_step(clotho_ctx* ctx, uint32_t set, bool philox) {
 // with the same key is reused).  Whatever fails between the start of the capture and the graph's
 // instantiation, the capture is ended and the partial graph discarded, so the stream stays usable.
 int capture_step_graph(clotho_ctx* ctx, std::vector<uint32_t> key) {
+    if (int rc = block_tables(ctx)) return rc;
     key.push_back(ctx->tuning_epoch);
     if (ctx->graph && ctx->graph_key == key) return 0;
     if (ctx->graph) {
@@ -663,6 +702,7 @@ int clotho_destroy(clotho_ctx* ctx) {
     for (uint32_t k = 0; k < kHdrRing; ++k)
         if (ctx->ring_ev[k]) cudaEventDestroy(ctx->ring_ev[k]);
     if (ctx->d_ctl) cudaFree(ctx->d_ctl);
+    if (ctx->d_parts) cudaFree(ctx->d_parts);
     if (ctx->graph) cudaGraphExecDestroy(ctx->graph);
     for (cudaEvent_t e : ctx->prof_ev) cudaEventDestroy(e);
     for (int i = 0; i < 2; ++i) {
@@ -886,6 +926,7 @@ int clotho_generation_tape(clotho_ctx* ctx, const clotho_gen_tape* tape) {
 int clotho_generation_philox(clotho_ctx* ctx, uint32_t N) {
     int rc = require_ready(ctx);
     if (rc) return rc;
+    if ((rc = block_tables(ctx))) return rc;
     if (ctx->in_step) return fail(ctx, CLOTHO_E_STATE, "a staged generation is in progress");
     for (size_t i = 0; i < ctx->pops.size(); ++i)
         if (N > ctx->pops[i]->dev[2].Ncap) return fail(ctx, CLOTHO_E_CAPACITY, "N exceeds max_individuals");
@@ -1365,10 +1406,10 @@ static int pairwise_of(clotho_ctx* ctx, uint32_t idx, const uint32_t* sample, ui
     *out = clotho_pairwise{};
     const uint64_t pairs = n > 1 ? (uint64_t)n * (n - 1) / 2 : 0;
     if (!pairs) return 0;
-    // one scratch block: accumulators, sample, row sums and, when the slots are split over CTAs, tile counts
+    // one scratch block: accumulators, sample and, when the slots are split over CTAs, tile counts
     const PairwisePlan z = pairwise_plan(cfg(ctx), n, s.W);
-    const size_t at_smp = align256(sizeof(PairwiseOut)), at_ones = at_smp + align256((size_t)n * 4);
-    const size_t at_dist = align256(at_ones + z.ones_bytes + z.sum_bytes);
+    const size_t at_smp = align256(sizeof(PairwiseOut)), at_sums = at_smp + align256((size_t)n * 4);
+    const size_t at_dist = align256(at_sums + z.sum_bytes);
     std::vector<char> head(at_smp + (size_t)n * 4);
     PairwiseOut h{};
     h.min = 0xffffffffu;
@@ -1378,10 +1419,10 @@ static int pairwise_of(clotho_ctx* ctx, uint32_t idx, const uint32_t* sample, ui
     CK(pool_alloc(ctx, &d, at_dist + (dist ? pairs * 4 : 0)));
     auto body = [&]() -> int {
         CK(cudaMemcpyAsync(d, head.data(), head.size(), cudaMemcpyHostToDevice, ctx->stream));
-        if (z.sum_bytes) CK(cudaMemsetAsync(d + at_ones + z.ones_bytes, 0, z.sum_bytes, ctx->stream));
-        CK(launch_pairwise(cfg(ctx), ctx->d_pops[0], idx, reinterpret_cast<uint32_t*>(d + at_smp), n, z, d + at_ones,
+        if (z.sum_bytes) CK(cudaMemsetAsync(d + at_sums, 0, z.sum_bytes, ctx->stream));
+        CK(launch_pairwise(cfg(ctx), ctx->d_pops[0], idx, reinterpret_cast<uint32_t*>(d + at_smp), n, z, d + at_sums,
                            dist ? reinterpret_cast<uint32_t*>(d + at_dist) : nullptr, reinterpret_cast<PairwiseOut*>(d)));
-        ctx->launches += 2;
+        ctx->launches += 1;
         if (int r = check_launch(ctx, "pairwise difference")) return r;
         CK(cudaMemcpyAsync(&h, d, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream));
         if (dist) host_pages(dist, pairs * 4);
@@ -1775,6 +1816,7 @@ int clotho_pop_stats(clotho_ctx* ctx, uint32_t index, clotho_stats* out, uint32_
 int clotho_batch_generation_philox(clotho_ctx* ctx, const uint32_t* N) {
     int rc = require_ready(ctx);
     if (rc) return rc;
+    if ((rc = block_tables(ctx))) return rc;
     if (!N) return fail(ctx, CLOTHO_E_ARG, "null N");
     if (ctx->pops.empty()) return 0;
     if (ctx->in_step) return fail(ctx, CLOTHO_E_STATE, "a staged generation is in progress");
@@ -1817,6 +1859,7 @@ int clotho_batch_run_philox(clotho_ctx* ctx, const uint32_t* N, uint32_t G) {
 int clotho_run_philox_schedule(clotho_ctx* ctx, const uint32_t* N, uint32_t G) {
     int rc = require_ready(ctx);
     if (rc) return rc;
+    if ((rc = block_tables(ctx))) return rc;
     if (!N) return fail(ctx, CLOTHO_E_ARG, "null schedule");
     if (ctx->in_step) return fail(ctx, CLOTHO_E_STATE, "a staged generation is in progress");
     const uint32_t n = (uint32_t)ctx->pops.size();
@@ -1883,6 +1926,7 @@ int clotho_set_tuning(clotho_ctx* ctx, const clotho_tuning* t) {
     }
     ctx->ind_per_sm = t->row_blocks_per_sm ? t->row_blocks_per_sm : 16u;
     ctx->narrow_ok = t->narrow_build != 0u;
+    ctx->parts_stale = true;
     ctx->tuning_epoch += 1;  // graphs captured under the old launch shapes are not replayed
     return 0;
 }

@@ -297,6 +297,19 @@ struct LaunchCfg {
     uint32_t ind_per_sm = 16;     // blocks per SM of the per-individual kernels (selection, fitness)
     bool narrow_ok = true;        // the narrow build of k_generation may run when every row fits it
     const PopDev* one = nullptr;  // host copy of the descriptor of a launch's only population
+    // which block works on which population of a batch (device tables, by BlockTable)
+    const struct BlockPart* parts[3] = {nullptr, nullptr, nullptr};
+    uint32_t blocks[3] = {0, 0, 0};
+};
+// Kernels of 256 threads, of 1,024 (every population has at least two blocks), and the row plans, whose work goes with
+// the breakpoints as well.
+enum BlockTable : uint32_t { kTable256 = 0, kTable1024 = 1, kTablePlan = 2 };
+// A block's population and its place among that population's blocks.  A batch's blocks are dealt out in proportion to
+// the populations' work by their capacities: with as many for each, the largest population's blocks ran when the
+// others' were done (64 populations of 1,000 to 20,000 individuals, a generation: plans 119 -> 64 us, fitness
+// 73 -> 62, first stage 47 -> 36).
+struct BlockPart {
+    uint32_t pop, i, n, pad;
 };
 
 // Population-parallel launches: blockIdx.z walks the populations, so small
@@ -313,6 +326,11 @@ inline uint32_t blocks_for(uint64_t n, uint32_t per_block) {
     const uint64_t b = (n + per_block - 1) / per_block;
     return b < 1 ? 1u : (b > 0x7fffffffull ? 0x7fffffffu : (uint32_t)b);
 }
+template <bool ONE>
+__device__ __forceinline__ BlockPart block_part(const BlockPart* map) {
+    return ONE ? BlockPart{0u, blockIdx.x, gridDim.x, 0u} : map[blockIdx.x];
+}
+
 // Launch with the programmatic dependency of pdl_wait.
 template <class... P, class... A>
 inline cudaError_t launch_smem_k(const LaunchCfg& L, void (*k)(P...), dim3 grid, dim3 block, size_t smem, A... a) {
@@ -336,22 +354,29 @@ inline cudaError_t launch_k(const LaunchCfg& L, void (*k)(P...), dim3 grid, dim3
 // The kernels of a step are templates over ONE: with one population its descriptor comes in the kernel's parameters
 // (the constant bank) instead of an array in memory, which takes a round trip to L2 off each kernel's chain of
 // dependent loads.
+// grid: blocks for one population; a batch takes its table's.
 template <class K, class... A>
-inline cudaError_t launch_pops_smem(const LaunchCfg& L, K one, K all, dim3 grid, dim3 block, size_t smem,
+inline cudaError_t launch_pops_smem(const LaunchCfg& L, BlockTable table, K one, K all, uint32_t grid, size_t smem,
                                     const PopDev* pops, uint32_t npops, A... a) {
-    const bool single = npops == 1u && L.one;
+    const bool single = npops == 1u;
     const K k = single ? one : all;
     if (smem > 48u * 1024u) {  // a property of the function on the current device; setting it again is harmless
         const cudaError_t e =
             cudaFuncSetAttribute((const void*)k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
     }
-    return launch_smem_k(L, k, grid, block, smem, single ? *L.one : PopDev{}, pops, npops, a...);
+    return launch_smem_k(L, k, dim3(single ? grid : L.blocks[table]), dim3(table == kTable1024 ? 1024u : 256u), smem,
+                         single ? *L.one : PopDev{}, pops, single ? nullptr : L.parts[table], a...);
 }
 template <class K, class... A>
-inline cudaError_t launch_pops(const LaunchCfg& L, K one, K all, dim3 grid, dim3 block, const PopDev* pops,
+inline cudaError_t launch_pops(const LaunchCfg& L, BlockTable table, K one, K all, uint32_t grid, const PopDev* pops,
                                uint32_t npops, A... a) {
-    return launch_pops_smem(L, one, all, grid, block, 0, pops, npops, a...);
+    return launch_pops_smem(L, table, one, all, grid, 0, pops, npops, a...);
+}
+// Blocks of one population's launch: per_pop useful ones, at most per_sm an SM.
+inline uint32_t blocks_of(const LaunchCfg& L, uint32_t per_pop, uint32_t per_sm) {
+    const uint32_t most = (uint32_t)L.num_sms * per_sm;
+    return per_pop < 1u ? 1u : per_pop < most ? per_pop : most;
 }
 
 // which: 0 = current child rows, 1 = parent rows of the step in progress
@@ -428,7 +453,7 @@ struct PairwiseOut {
 // how the pairs of n rows of W words are cut into CTAs, and the scratch that takes
 struct PairwisePlan {
     uint32_t tiles, splits, per;       // per: 128-slot stages a CTA
-    size_t ones_bytes, sum_bytes;
+    size_t sum_bytes;
 };
 PairwisePlan pairwise_plan(const LaunchCfg&, uint32_t n, uint32_t W);
 cudaError_t launch_pairwise(const LaunchCfg&, const PopDev* pops, uint32_t p, const uint32_t* sample, uint32_t n,

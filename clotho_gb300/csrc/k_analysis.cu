@@ -21,6 +21,7 @@ constexpr uint32_t kPairThreads = kTM + kTN;    // one expanded row a thread
 constexpr uint32_t kRing = 4;                   // stages of 128 slots in shared memory
 constexpr uint32_t kStageBytes = (kTM + kTN) * 128u;
 constexpr uint32_t kMaxSlots = 1u << 19;        // slots a CTA sums up: counts stay far below 2^24 units
+constexpr uint32_t kTileSums = kTM * kTN + kPairThreads;   // counts of a tile whose slots several CTAs share
 constexpr uint32_t kPairWait = 1u << 20;        // try_wait rounds before a CTA gives up
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -68,25 +69,6 @@ __device__ __forceinline__ void load_32_columns(uint32_t taddr, uint32_t (&v)[32
 }
 }  // namespace
 
-// Alleles of each sampled row, one warp a row.
-__global__ void __launch_bounds__(256) k_sample_ones(const PopDev* __restrict__ pops, uint32_t p,
-                                                     const uint32_t* __restrict__ sample, uint32_t n,
-                                                     uint32_t* __restrict__ ones) {
-    const PopDev& P = pops[p];
-    const uint32_t W = P.st->W, lane = threadIdx.x & 31u;
-    const uint64_t* rows = P.rows[P.st->cur];
-    for (uint32_t i = (blockIdx.x * 256u + threadIdx.x) >> 5; i < n; i += gridDim.x * 8u) {
-        const uint64_t* r = rows + (size_t)sample[i] * P.Wcap;
-        uint32_t c = 0;
-        for (uint32_t w = 2u * lane; w < W; w += 64u) {
-            const ulonglong2 x = __ldg(reinterpret_cast<const ulonglong2*>(r + w));
-            c += (uint32_t)(__popcll(x.x) + __popcll(x.y));
-        }
-        c = __reduce_add_sync(0xffffffffu, c);
-        if (lane == 0) ones[i] = c;
-    }
-}
-
 // One CTA takes a 128 x 256 tile of the pair matrix (tiles with a pair i < j only) and a range of the slots.
 // Every thread expands one row, 128 slots a stage: bit k of each byte of a 32-bit word becomes a byte of 0 or 1
 // (two operations for four slots; the order of the slots is the same for all rows, which is all a sum needs) in the
@@ -99,7 +81,7 @@ __global__ void __launch_bounds__(256) k_sample_ones(const PopDev* __restrict__ 
 // unit's 16 words a clock and SM.)
 __global__ void __launch_bounds__(kPairThreads, 1)
 k_pairwise(const PopDev* __restrict__ pops, uint32_t p, const uint32_t* __restrict__ sample, uint32_t n,
-           const uint32_t* __restrict__ ones, uint32_t splits, uint32_t per, uint32_t* __restrict__ tile_sum,
+           uint32_t splits, uint32_t per, uint32_t* __restrict__ tile_sum,
            uint32_t* __restrict__ tile_done, uint32_t* __restrict__ dist, PairwiseOut* __restrict__ out) {
     extern __shared__ uint8_t s_raw[];
     __shared__ __align__(8) unsigned long long s_bar[kRing + 1];
@@ -123,7 +105,6 @@ k_pairwise(const PopDev* __restrict__ pops, uint32_t p, const uint32_t* __restri
     const uint32_t row = tid < kTM ? ti * kTM + tid : tj * kTN + (tid - kTM);
     const bool ok_row = row < n;
     const uint4* src = ok_row ? reinterpret_cast<const uint4*>(rows + (size_t)sample[row] * P.Wcap) + st0 : nullptr;
-    s_ones[tid] = ok_row ? ones[row] : 0u;
     uint8_t* const ring = s_raw + ((1024u - (smem_addr(s_raw) & 1023u)) & 1023u);
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&s_tmem)),
@@ -146,12 +127,13 @@ k_pairwise(const PopDev* __restrict__ pops, uint32_t p, const uint32_t* __restri
     const uint4 zero = make_uint4(0, 0, 0, 0);
     uint4 q0 = ok_row && cnt > 0 ? __ldg(src) : zero, q1 = ok_row && cnt > 1 ? __ldg(src + 1) : zero;
     bool ok = true;
-    uint32_t issued = 0;
+    uint32_t issued = 0, ones = 0;   // the row's alleles in this CTA's slots
     for (uint32_t it = 0; it < cnt; ++it) {
         const uint32_t s = it % kRing;
         const uint4 q = q0;
         q0 = q1;
         q1 = ok_row && it + 2u < cnt ? __ldg(src + it + 2u) : zero;
+        ones += (uint32_t)(__popc(q.x) + __popc(q.y) + __popc(q.z) + __popc(q.w));
         if (it >= kRing) ok = wait_parity(smem_addr(&s_bar[s]), (it / kRing - 1u) & 1u);
         if (ok && (ok_row || it < kRing)) {   // rows past the sample stay zero
             uint8_t* dst = ring + s * kStageBytes + (tid < kTM ? tid : tid - kTM) * 128u + (tid < kTM ? 0u : kTM * 128u);
@@ -182,11 +164,13 @@ k_pairwise(const PopDev* __restrict__ pops, uint32_t p, const uint32_t* __restri
         if (tid == 0) mma_commit(smem_addr(&s_bar[kRing]));
         ok = __syncthreads_and(wait_parity(smem_addr(&s_bar[kRing]), 0u)) && ok;
     }
+    s_ones[tid] = ones;
+    __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     // TMEM lanes are the tile's rows: a warp reads the 32 of its place in its warpgroup, a third of the columns
     const uint32_t i_tile = (warp & 3u) * 32u + lane, i = ti * kTM + i_tile;
     const uint32_t taddr = tmem + (((warp & 3u) * 32u) << 16);
-    uint32_t* const sums = tile_sum ? tile_sum + (size_t)tile * kTM * kTN : nullptr;   // [column][row]
+    uint32_t* const sums = tile_sum ? tile_sum + (size_t)tile * kTileSums : nullptr;   // [column][row], then the rows' alleles
     bool finish = ok;
     if (splits > 1u) {
         for (uint32_t c0 = (warp >> 2) * 32u; c0 < ncol; c0 += 96u) {
@@ -199,12 +183,15 @@ k_pairwise(const PopDev* __restrict__ pops, uint32_t p, const uint32_t* __restri
                     if (x && c0 + k < ncol) atomicAdd(sums + (c0 + k) * kTM + i_tile, x);
                 }
         }
+        if (ones) atomicAdd(sums + kTM * kTN + tid, ones);
         __threadfence();
         __syncthreads();
         if (tid == 0) s_last = atomicAdd(tile_done + tile, 1u) == splits - 1u;
         __syncthreads();
         finish = ok && s_last;
         __threadfence();
+        if (finish) s_ones[tid] = __ldcg(sums + kTM * kTN + tid);
+        __syncthreads();
     }
     unsigned long long sum = 0, sq = 0, pairs = 0;
     uint32_t mn = 0xffffffffu, mx = 0;
@@ -291,25 +278,22 @@ PairwisePlan pairwise_plan(const LaunchCfg& L, uint32_t n, uint32_t W) {
         }
     }
     z.per = (nst + z.splits - 1u) / z.splits;
-    z.ones_bytes = ((size_t)n * 4 + 255) & ~(size_t)255;
-    z.sum_bytes = z.splits > 1u ? (size_t)z.tiles * (kTM * kTN + 64u) * 4 : 0;
+    z.sum_bytes = z.splits > 1u ? (size_t)z.tiles * (kTileSums + 1u) * 4 : 0;
     return z;
 }
 
-// scratch: ones_bytes, then sum_bytes zero on entry.
+// scratch: sum_bytes, zero on entry.
 cudaError_t launch_pairwise(const LaunchCfg& L, const PopDev* pops, uint32_t p, const uint32_t* sample, uint32_t n,
                             const PairwisePlan& z, void* scratch, uint32_t* dist, PairwiseOut* out) {
-    uint32_t* ones = static_cast<uint32_t*>(scratch);
-    uint32_t* sums = z.sum_bytes ? reinterpret_cast<uint32_t*>(static_cast<char*>(scratch) + z.ones_bytes) : nullptr;
-    uint32_t* done = z.sum_bytes ? sums + (size_t)z.tiles * kTM * kTN : nullptr;
+    uint32_t* sums = z.sum_bytes ? static_cast<uint32_t*>(scratch) : nullptr;
+    uint32_t* done = z.sum_bytes ? sums + (size_t)z.tiles * kTileSums : nullptr;
     const size_t smem = kRing * kStageBytes + 1024u;
     // a property of the function on the current device; setting it again is harmless
     const cudaError_t e =
         cudaFuncSetAttribute((const void*)k_pairwise, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    k_sample_ones<<<std::min(blocks_for(n, 8), (uint32_t)L.num_sms * 8u), 256, 0, L.stream>>>(pops, p, sample, n, ones);
-    k_pairwise<<<z.tiles * z.splits, kPairThreads, smem, L.stream>>>(pops, p, sample, n, ones, z.splits, z.per, sums,
-                                                                    done, dist, out);
+    k_pairwise<<<z.tiles * z.splits, kPairThreads, smem, L.stream>>>(pops, p, sample, n, z.splits, z.per, sums, done,
+                                                                    dist, out);
     return cudaSuccess;
 }
 

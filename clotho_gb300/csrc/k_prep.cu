@@ -11,8 +11,8 @@
 // that is at most kDirectScan counts; above, one more launch leaves chunk sums), and
 // every kernel is launched with programmatic dependent launch.
 //
-// All kernels walk every population of the batch on blockIdx.z; sizes are read from
-// the device status words.
+// A block works on one population (block_part); sizes are read from the device status
+// words.
 #include "plan.cuh"
 #include "step.cuh"
 
@@ -137,19 +137,17 @@ __device__ __forceinline__ uint2 draw_parents(const PopDev& P, uint32_t k, uint3
     return make_uint2(id[0], id[1]);
 }
 
-// Blocks [0, a) of a population's gridDim.x take the first of a kernel's two independent jobs, the rest the
-// second; a single block takes both.
+// The first blocks of a population take the first of a kernel's two independent jobs, the rest the second; a single
+// block takes both.
 struct Share {
     uint32_t i, n;
     bool on;
 };
-__device__ __forceinline__ Share first_share(uint32_t a) {
-    if (gridDim.x == 1u) return Share{0u, 1u, true};
-    return Share{blockIdx.x, a, blockIdx.x < a};
+__device__ __forceinline__ Share first_share(const BlockPart& b, uint32_t first) {
+    return b.n == 1u ? Share{0u, 1u, true} : Share{b.i, first, b.i < first};
 }
-__device__ __forceinline__ Share second_share(uint32_t a) {
-    if (gridDim.x == 1u) return Share{0u, 1u, true};
-    return Share{blockIdx.x - a, gridDim.x - a, blockIdx.x >= a};
+__device__ __forceinline__ Share second_share(const BlockPart& b, uint32_t first) {
+    return b.n == 1u ? Share{0u, 1u, true} : Share{b.i - first, b.n - first, b.i >= first};
 }
 
 }  // namespace
@@ -167,86 +165,85 @@ __device__ __forceinline__ Share second_share(uint32_t a) {
 // same law as M ~ Poisson(mu * 2N) with uniform target rows
 // (mutation_allocator.hpp:41-47, batch_mutation_task_population_space_row.hpp:77).
 template <bool ONE>
-__global__ void __launch_bounds__(1024) k_stage1(const __grid_constant__ PopDev one, const PopDev* __restrict__ pops, uint32_t npops,
+__global__ void __launch_bounds__(1024) k_stage1(const __grid_constant__ PopDev one, const PopDev* __restrict__ pops,
+                                                 const BlockPart* __restrict__ map, uint32_t npops,
                                                  const uint32_t* __restrict__ hdr, WorkCtl* ctl, uint32_t what,
                                                  uint32_t count_on) {
     __shared__ uint32_t s_u32[33];
+    const BlockPart part = block_part<ONE>(map);
+    const PopDev& P = ONE ? one : pops[part.pop];
     pdl_wait();
-    for (uint32_t p = blockIdx.z; p < npops; p += gridDim.z) {
-        const PopDev& P = ONE ? one : pops[p];
-        DevStatus* st = P.st;
-        const bool philox = P.mode == kModePhilox;
-        const uint32_t N = step_N(P, hdr, p), S = 2u * N;
-        if (blockIdx.x == 0) {
-            if (!(what & kStepBegin)) continue;
-            const uint32_t pN = st->N, pA = st->A, pW = st->W;
-            fs_finalize_block(P, pN, pA, pW, count_on != 0u);
-            if (threadIdx.x == 0) {
-                uint32_t err = 0, M = hdr[2u * p + 1u];
-                if (hdr[2u * p] > P.Ncap) err |= kErrAlleles;
-                if (M > P.Mcap) { err |= kErrMut; M = P.Mcap; }
-                if (err) atomicOr(&st->err, err);
-                st->pN = pN;
-                st->pA = pA;
-                st->pW = pW;
-                st->M = M;
-                st->ev_used = 0;
-            }
-            __syncthreads();
-            continue;
+    DevStatus* st = P.st;
+    const bool philox = P.mode == kModePhilox;
+    const uint32_t N = step_N(P, hdr, part.pop), S = 2u * N;
+    if (part.i == 0) {
+        if (!(what & kStepBegin)) return;
+        const uint32_t pN = st->N, pA = st->A, pW = st->W;
+        fs_finalize_block(P, pN, pA, pW, count_on != 0u);
+        if (threadIdx.x == 0) {
+            uint32_t err = 0, M = hdr[2u * part.pop + 1u];
+            if (hdr[2u * part.pop] > P.Ncap) err |= kErrAlleles;
+            if (M > P.Mcap) { err |= kErrMut; M = P.Mcap; }
+            if (err) atomicOr(&st->err, err);
+            st->pN = pN;
+            st->pA = pA;
+            st->pW = pW;
+            st->M = M;
+            st->ev_used = 0;
         }
-        const uint32_t bx = blockIdx.x - 1u, nb = gridDim.x - 1u;
-        if (p == 0 && bx == 0 && (what & kStepBegin)) begin_items(pops, npops, hdr, ctl);
-        if (what & kStepMut) {
-            if (philox) {
-                const uint32_t gen = st->gen;
-                const double* cdf = P.pois_mu;
-                for (uint32_t c = bx; c * kChunk < S; c += nb) {
-                    const uint32_t r = c * kChunk + threadIdx.x;
-                    uint32_t n = 0;
-                    if (r < S) {
-                        const U4 x = philox4x32(r, 0u, gen, kStreamMutCount, P.seed);
-                        n = poisson_tab(u01(x.x, x.y), cdf, cdf[kPoisTab], P.mu);
-                        P.row_cnt[r] = n;
-                    }
-                    n = __reduce_add_sync(0xffffffffu, n);
-                    if ((threadIdx.x & 31u) == 0u) s_u32[threadIdx.x >> 5] = n;
-                    __syncthreads();
-                    if (threadIdx.x < 32u) {
-                        n = __reduce_add_sync(0xffffffffu, s_u32[threadIdx.x]);
-                        if (threadIdx.x == 0) P.scan_upart[c] = n;
-                    }
-                    __syncthreads();
+        return;
+    }
+    const uint32_t bx = part.i - 1u, nb = part.n - 1u, p = part.pop;
+    if (p == 0 && bx == 0 && (what & kStepBegin)) begin_items(pops, npops, hdr, ctl);
+    if (what & kStepMut) {
+        if (philox) {
+            const uint32_t gen = st->gen;
+            const double* cdf = P.pois_mu;
+            for (uint32_t c = bx; c * kChunk < S; c += nb) {
+                const uint32_t r = c * kChunk + threadIdx.x;
+                uint32_t n = 0;
+                if (r < S) {
+                    const U4 x = philox4x32(r, 0u, gen, kStreamMutCount, P.seed);
+                    n = poisson_tab(u01(x.x, x.y), cdf, cdf[kPoisTab], P.mu);
+                    P.row_cnt[r] = n;
                 }
-            } else {
-                const uint32_t M = min(hdr[2u * p + 1u], P.Mcap);
-                for (uint32_t i = bx * 1024u + threadIdx.x; i < M; i += nb * 1024u) {
-                    const uint32_t s = P.mut_seq[i];
-                    if (s >= S) { atomicOr(&st->err, kErrSeq); continue; }
-                    atomicAdd(&P.row_cnt[s], 1u);
+                n = __reduce_add_sync(0xffffffffu, n);
+                if ((threadIdx.x & 31u) == 0u) s_u32[threadIdx.x >> 5] = n;
+                __syncthreads();
+                if (threadIdx.x < 32u) {
+                    n = __reduce_add_sync(0xffffffffu, s_u32[threadIdx.x]);
+                    if (threadIdx.x == 0) P.scan_upart[c] = n;
                 }
+                __syncthreads();
+            }
+        } else {
+            const uint32_t M = min(hdr[2u * p + 1u], P.Mcap);
+            for (uint32_t i = bx * 1024u + threadIdx.x; i < M; i += nb * 1024u) {
+                const uint32_t s = P.mut_seq[i];
+                if (s >= S) { atomicOr(&st->err, kErrSeq); continue; }
+                atomicAdd(&P.row_cnt[s], 1u);
             }
         }
-        if (what & kStepOrder) {
-            const uint32_t Np = hdr ? st->N : st->pN;  // staged calls have moved the sizes already
-            uint32_t* const cnt = P.plan_row ? P.ord_cnt : nullptr;
-            if (philox && (what & kStepSelect)) {
-                const bool uni = st->fit_const != 0u || !(st->fit_total > 0.0);
-                const double total = st->fit_total;
-                const uint32_t gen = st->gen;
-                for (uint32_t k = bx * 1024u + threadIdx.x; k < N; k += nb * 1024u) {
-                    const uint2 id = draw_parents(P, k, Np, gen, uni, total);
-                    *reinterpret_cast<uint2*>(P.pairs + 2u * k) = id;
-                    if (cnt) {
-                        atomicAdd(cnt + id.x, 1u);
-                        atomicAdd(cnt + id.y, 1u);
-                    }
+    }
+    if (what & kStepOrder) {
+        const uint32_t Np = hdr ? st->N : st->pN;  // staged calls have moved the sizes already
+        uint32_t* const cnt = P.plan_row ? P.ord_cnt : nullptr;
+        if (philox && (what & kStepSelect)) {
+            const bool uni = st->fit_const != 0u || !(st->fit_total > 0.0);
+            const double total = st->fit_total;
+            const uint32_t gen = st->gen;
+            for (uint32_t k = bx * 1024u + threadIdx.x; k < N; k += nb * 1024u) {
+                const uint2 id = draw_parents(P, k, Np, gen, uni, total);
+                *reinterpret_cast<uint2*>(P.pairs + 2u * k) = id;
+                if (cnt) {
+                    atomicAdd(cnt + id.x, 1u);
+                    atomicAdd(cnt + id.y, 1u);
                 }
-            } else if (cnt) {
-                for (uint32_t g = bx * 1024u + threadIdx.x; g < S; g += nb * 1024u) {
-                    const uint32_t id = P.pairs[g];
-                    atomicAdd(cnt + (id < Np ? id : 0u), 1u);
-                }
+            }
+        } else if (cnt) {
+            for (uint32_t g = bx * 1024u + threadIdx.x; g < S; g += nb * 1024u) {
+                const uint32_t id = P.pairs[g];
+                atomicAdd(cnt + (id < Np ? id : 0u), 1u);
             }
         }
     }
@@ -255,26 +252,27 @@ __global__ void __launch_bounds__(1024) k_stage1(const __grid_constant__ PopDev 
 // Chunk sums of the counts that a scan cannot sum by itself (which == 0: new alleles per row, 1: rows per
 // parent, 2: positions per bucket).
 template <bool ONE>
-__global__ void __launch_bounds__(256) k_chunk_sums(const __grid_constant__ PopDev one, const PopDev* __restrict__ pops, uint32_t npops,
+__global__ void __launch_bounds__(256) k_chunk_sums(const __grid_constant__ PopDev one,
+                                                    const PopDev* __restrict__ pops,
+                                                    const BlockPart* __restrict__ map,
                                                     const uint32_t* __restrict__ hdr, uint32_t which) {
     __shared__ uint32_t s8[8];
+    const BlockPart part = block_part<ONE>(map);
+    const PopDev& P = ONE ? one : pops[part.pop];
     pdl_wait();
-    for (uint32_t p = blockIdx.z; p < npops; p += gridDim.z) {
-        const PopDev& P = ONE ? one : pops[p];
-        const uint32_t L = which == 0 ? 2u * step_N(P, hdr, p) : which == 1 ? order_keys(P.st->pN) : P.NB;
-        const uint32_t* cnt = which == 0 ? P.row_cnt : which == 1 ? P.ord_cnt : P.bcnt;
-        uint32_t* part = which == 1 ? P.scan_opart : P.scan_upart;
-        if (!cnt) continue;
-        for (uint32_t c = blockIdx.x; c * kChunk < L; c += gridDim.x) {
-            uint32_t v = 0;
+    const uint32_t L = which == 0 ? 2u * step_N(P, hdr, part.pop) : which == 1 ? order_keys(P.st->pN) : P.NB;
+    const uint32_t* cnt = which == 0 ? P.row_cnt : which == 1 ? P.ord_cnt : P.bcnt;
+    uint32_t* sums = which == 1 ? P.scan_opart : P.scan_upart;
+    if (!cnt) return;
+    for (uint32_t c = part.i; c * kChunk < L; c += part.n) {
+        uint32_t v = 0;
 #pragma unroll
-            for (uint32_t k = 0; k < 4; ++k) {
-                const uint32_t i = c * kChunk + 256u * k + threadIdx.x;
-                if (i < L) v += cnt[i];
-            }
-            v = block_sum_256(v, s8);
-            if (threadIdx.x == 0) part[c] = v;
+        for (uint32_t k = 0; k < 4; ++k) {
+            const uint32_t i = c * kChunk + 256u * k + threadIdx.x;
+            if (i < L) v += cnt[i];
         }
+        v = block_sum_256(v, s8);
+        if (threadIdx.x == 0) sums[c] = v;
     }
 }
 
@@ -287,59 +285,59 @@ __global__ void __launch_bounds__(256) k_chunk_sums(const __grid_constant__ PopD
 // allele and trait, neighbours in different blocks: a drawn effect is about a hundred
 // operations of the narrow FP64 pipe, so they are spread over all SMs.
 template <bool ONE>
-__global__ void __launch_bounds__(256) k_stage2(const __grid_constant__ PopDev one, const PopDev* __restrict__ pops, uint32_t npops,
-                                                const uint32_t* __restrict__ hdr, uint32_t what, uint32_t direct_max,
-                                                uint32_t nres) {
+__global__ void __launch_bounds__(256) k_stage2(const __grid_constant__ PopDev one, const PopDev* __restrict__ pops,
+                                                const BlockPart* __restrict__ map, const uint32_t* __restrict__ hdr,
+                                                uint32_t what, uint32_t direct_max) {
     __shared__ uint32_t s8[8];
+    const BlockPart part = block_part<ONE>(map);
+    const PopDev& P = ONE ? one : pops[part.pop];
     pdl_wait();
-    for (uint32_t p = blockIdx.z; p < npops; p += gridDim.z) {
-        const PopDev& P = ONE ? one : pops[p];
-        DevStatus* st = P.st;
-        const bool philox = P.mode == kModePhilox;
-        const uint32_t N = step_N(P, hdr, p), S = 2u * N;
-        const Share res = first_share(nres), scan = second_share(nres);
-        if (res.on && (what & kStepMut)) {
-            uint32_t M = 0;
-            if (philox) {  // stage 1 left the chunk sums
-                for (uint32_t i = threadIdx.x; i * kChunk < S; i += 256u) M += P.scan_upart[i];
-                M = block_sum_256(M, s8);
-            } else {
-                M = st->M;
-            }
-            const uint32_t Mraw = M;
-            M = min(M, P.Mcap);
-            const uint32_t fr = st->free_cnt, pA = st->pA, gen = st->gen, T = P.T;
-            const uint32_t Ac = pA + (M > fr ? M - fr : 0u), A = min(Ac, P.Acap);
-            if (res.i == 0 && threadIdx.x == 0) {
-                if (Ac > P.Acap) atomicOr(&st->err, kErrAlleles);
-                if (Mraw > P.Mcap) atomicOr(&st->err, kErrMut);
-                st->N = N;
-                st->A = A;
-                st->W = ref_width(A);
-                st->cur ^= 1u;
-                if (philox) st->M = M;
-            }
-            int nz_delta = 0;
-            for (uint64_t q = (uint64_t)threadIdx.x * res.n + res.i; q < (uint64_t)M * T; q += 256ull * res.n) {
-                const uint32_t i = (uint32_t)(q / T), t = (uint32_t)(q % T);
-                nz_delta += resolve_mutation(P, i, t, gen, fr, pA, A);
-            }
-            if (nz_delta) atomicAdd(&st->nz_eff, nz_delta);
-            __syncthreads();
+    DevStatus* st = P.st;
+    const bool philox = P.mode == kModePhilox;
+    const uint32_t N = step_N(P, hdr, part.pop), S = 2u * N;
+    const uint32_t a = max(1u, part.n / 3u);
+    const Share res = first_share(part, a), scan = second_share(part, a);
+    if (res.on && (what & kStepMut)) {
+        uint32_t M = 0;
+        if (philox) {  // stage 1 left the chunk sums
+            for (uint32_t i = threadIdx.x; i * kChunk < S; i += 256u) M += P.scan_upart[i];
+            M = block_sum_256(M, s8);
+        } else {
+            M = st->M;
         }
-        if (!scan.on) continue;
-        // units: the row chunks, then the parent chunks
-        const uint32_t keys = order_keys(st->pN);
-        const uint32_t nr = (what & kStepMut) ? S / kChunk + 1u : 0u;
-        const uint32_t no = ((what & kStepOrder) && P.plan_row) ? (keys + kChunk - 1u) / kChunk : 0u;
-        for (uint32_t u = scan.i; u < nr + no; u += scan.n) {
-            if (u < nr) {
-                const uint32_t total = scan_chunk(P.row_cnt, P.scan_upart, !philox && S <= direct_max, S, u, P.row_off,
-                                                  philox ? nullptr : P.row_cur, s8);
-                if (u == nr - 1u && threadIdx.x == 0) P.row_off[S] = total;
-            } else {
-                scan_chunk(P.ord_cnt, P.scan_opart, keys <= direct_max, keys, u - nr, nullptr, P.ord_cur, s8);
-            }
+        const uint32_t Mraw = M;
+        M = min(M, P.Mcap);
+        const uint32_t fr = st->free_cnt, pA = st->pA, gen = st->gen, T = P.T;
+        const uint32_t Ac = pA + (M > fr ? M - fr : 0u), A = min(Ac, P.Acap);
+        if (res.i == 0 && threadIdx.x == 0) {
+            if (Ac > P.Acap) atomicOr(&st->err, kErrAlleles);
+            if (Mraw > P.Mcap) atomicOr(&st->err, kErrMut);
+            st->N = N;
+            st->A = A;
+            st->W = ref_width(A);
+            st->cur ^= 1u;
+            if (philox) st->M = M;
+        }
+        int nz_delta = 0;
+        for (uint64_t q = (uint64_t)threadIdx.x * res.n + res.i; q < (uint64_t)M * T; q += 256ull * res.n) {
+            const uint32_t i = (uint32_t)(q / T), t = (uint32_t)(q % T);
+            nz_delta += resolve_mutation(P, i, t, gen, fr, pA, A);
+        }
+        if (nz_delta) atomicAdd(&st->nz_eff, nz_delta);
+        __syncthreads();
+    }
+    if (!scan.on) return;
+    // units: the row chunks, then the parent chunks
+    const uint32_t keys = order_keys(st->pN);
+    const uint32_t nr = (what & kStepMut) ? S / kChunk + 1u : 0u;
+    const uint32_t no = ((what & kStepOrder) && P.plan_row) ? (keys + kChunk - 1u) / kChunk : 0u;
+    for (uint32_t u = scan.i; u < nr + no; u += scan.n) {
+        if (u < nr) {
+            const uint32_t total = scan_chunk(P.row_cnt, P.scan_upart, !philox && S <= direct_max, S, u, P.row_off,
+                                              philox ? nullptr : P.row_cur, s8);
+            if (u == nr - 1u && threadIdx.x == 0) P.row_off[S] = total;
+        } else {
+            scan_chunk(P.ord_cnt, P.scan_opart, keys <= direct_max, keys, u - nr, nullptr, P.ord_cur, s8);
         }
     }
 }
@@ -429,46 +427,45 @@ __device__ __forceinline__ void rank_block(const PopDev& P, uint32_t A, RankSmem
         P.rank[me] = r;
         P.inv[r] = me;
     }
-    __syncthreads();   // the next population's counts
 }
 
 template <bool ONE, bool DIRECT>
 __global__ void __launch_bounds__(DIRECT ? 1024 : 256)
-k_stage3(const __grid_constant__ PopDev one, const PopDev* __restrict__ pops, uint32_t npops, uint32_t what) {
+k_stage3(const __grid_constant__ PopDev one, const PopDev* __restrict__ pops, const BlockPart* __restrict__ map,
+         uint32_t what) {
     extern __shared__ __align__(16) uint8_t s_raw[];
     constexpr uint32_t kThreads = DIRECT ? 1024u : 256u;
+    const BlockPart part = block_part<ONE>(map);
+    const PopDev& P = ONE ? one : pops[part.pop];
     pdl_wait();
-    for (uint32_t p = blockIdx.z; p < npops; p += gridDim.z) {
-        const PopDev& P = ONE ? one : pops[p];
-        const DevStatus* st = P.st;
-        const uint32_t A = st->A;
-        // DIRECT: the first block ranks the slots, the others do the rest
-        if (DIRECT && blockIdx.x == 0) {
-            rank_block(P, A, *reinterpret_cast<RankSmem*>(s_raw));
-            continue;
+    const DevStatus* st = P.st;
+    const uint32_t A = st->A;
+    // DIRECT: the first block ranks the slots, the others do the rest
+    if (DIRECT && part.i == 0) {
+        rank_block(P, A, *reinterpret_cast<RankSmem*>(s_raw));
+        return;
+    }
+    const uint32_t at = (part.i - (DIRECT ? 1u : 0u)) * kThreads + threadIdx.x;
+    const uint32_t step = (part.n - (DIRECT ? 1u : 0u)) * kThreads;
+    const uint32_t N = st->N, pN = st->pN, S = 2u * N;
+    if (!DIRECT)
+        for (uint32_t s = at; s < A; s += step) atomicAdd(&P.bcnt[pos_bucket(P.pos[s], P.NB)], 1u);
+    if ((what & kStepOrder) && P.plan_row) {
+        for (uint32_t g = at; g < S; g += step) {
+            const uint32_t id = P.pairs[g];
+            P.ord_pos[g] = atomicAdd(&P.ord_cur[id < pN ? id : 0u], 1u);
         }
-        const uint32_t at = (blockIdx.x - (DIRECT ? 1u : 0u)) * kThreads + threadIdx.x;
-        const uint32_t step = (gridDim.x - (DIRECT ? 1u : 0u)) * kThreads;
-        const uint32_t N = st->N, pN = st->pN, S = 2u * N;
-        if (!DIRECT)
-            for (uint32_t s = at; s < A; s += step) atomicAdd(&P.bcnt[pos_bucket(P.pos[s], P.NB)], 1u);
-        if ((what & kStepOrder) && P.plan_row) {
-            for (uint32_t g = at; g < S; g += step) {
-                const uint32_t id = P.pairs[g];
-                P.ord_pos[g] = atomicAdd(&P.ord_cur[id < pN ? id : 0u], 1u);
+        for (uint32_t k = at; k < order_keys(pN); k += step) P.ord_cnt[k] = 0u;
+    }
+    if (what & kStepMut) {
+        if (P.mode != kModePhilox) {
+            const uint32_t M = st->M;
+            for (uint32_t i = at; i < M; i += step) {
+                const uint32_t s = P.mut_seq[i];
+                if (s < S) P.row_mut[atomicAdd(&P.row_cur[s], 1u)] = i;
             }
-            for (uint32_t k = at; k < order_keys(pN); k += step) P.ord_cnt[k] = 0u;
         }
-        if (what & kStepMut) {
-            if (P.mode != kModePhilox) {
-                const uint32_t M = st->M;
-                for (uint32_t i = at; i < M; i += step) {
-                    const uint32_t s = P.mut_seq[i];
-                    if (s < S) P.row_mut[atomicAdd(&P.row_cur[s], 1u)] = i;
-                }
-            }
-            for (uint32_t r = at; r < S; r += step) P.row_cnt[r] = 0u;
-        }
+        for (uint32_t r = at; r < S; r += step) P.row_cnt[r] = 0u;
     }
 }
 
@@ -520,36 +517,36 @@ __device__ __forceinline__ void sort_tape_lists(const PopDev& P, uint32_t at, ui
 // Stage 4.  The prefix sum of the positions per bucket, and the tape rows' lists in order.
 template <bool ONE>
 __global__ void __launch_bounds__(256) k_stage4(const __grid_constant__ PopDev one, const PopDev* __restrict__ pops,
-                                                uint32_t npops, uint32_t what, uint32_t direct_max) {
+                                                const BlockPart* __restrict__ map, uint32_t what,
+                                                uint32_t direct_max) {
     __shared__ uint32_t s8[8];
+    const BlockPart part = block_part<ONE>(map);
+    const PopDev& P = ONE ? one : pops[part.pop];
     pdl_wait();
-    for (uint32_t p = blockIdx.z; p < npops; p += gridDim.z) {
-        const PopDev& P = ONE ? one : pops[p];
-        for (uint32_t c = blockIdx.x; c * kChunk < P.NB; c += gridDim.x) {
-            const uint32_t total = scan_chunk(P.bcnt, P.scan_upart, P.NB <= direct_max, P.NB, c, P.boff, P.bcur, s8);
-            if ((c + 1u) * kChunk >= P.NB && threadIdx.x == 0) P.boff[P.NB] = total;
-        }
-        if ((what & kStepMut) && P.mode != kModePhilox)
-            sort_tape_lists(P, blockIdx.x * 256u + threadIdx.x, gridDim.x * 256u);
+    for (uint32_t c = part.i; c * kChunk < P.NB; c += part.n) {
+        const uint32_t total = scan_chunk(P.bcnt, P.scan_upart, P.NB <= direct_max, P.NB, c, P.boff, P.bcur, s8);
+        if ((c + 1u) * kChunk >= P.NB && threadIdx.x == 0) P.boff[P.NB] = total;
     }
+    if ((what & kStepMut) && P.mode != kModePhilox)
+        sort_tape_lists(P, part.i * 256u + threadIdx.x, part.n * 256u);
 }
 
 // Stage 5.  Positions and slots grouped by bucket; the bucket counts go back to zero.
 template <bool ONE>
-__global__ void __launch_bounds__(256) k_stage5(const __grid_constant__ PopDev one, const PopDev* __restrict__ pops, uint32_t npops) {
+__global__ void __launch_bounds__(256) k_stage5(const __grid_constant__ PopDev one, const PopDev* __restrict__ pops,
+                                                const BlockPart* __restrict__ map) {
+    const BlockPart part = block_part<ONE>(map);
+    const PopDev& P = ONE ? one : pops[part.pop];
     pdl_wait();
-    for (uint32_t p = blockIdx.z; p < npops; p += gridDim.z) {
-        const PopDev& P = ONE ? one : pops[p];
-        const uint32_t at = blockIdx.x * 256u + threadIdx.x, step = gridDim.x * 256u;
-        const uint32_t A = P.st->A;
-        for (uint32_t s = at; s < A; s += step) {
-            const double x = P.pos[s];
-            const uint32_t k = atomicAdd(&P.bcur[pos_bucket(x, P.NB)], 1u);
-            P.bpos[k] = x;
-            P.bslot[k] = s;
-        }
-        for (uint32_t b = at; b < P.NB; b += step) P.bcnt[b] = 0u;
+    const uint32_t at = part.i * 256u + threadIdx.x, step = part.n * 256u;
+    const uint32_t A = P.st->A;
+    for (uint32_t s = at; s < A; s += step) {
+        const double x = P.pos[s];
+        const uint32_t k = atomicAdd(&P.bcur[pos_bucket(x, P.NB)], 1u);
+        P.bpos[k] = x;
+        P.bslot[k] = s;
     }
+    for (uint32_t b = at; b < P.NB; b += step) P.bcnt[b] = 0u;
 }
 
 // ---------------------------------------------------------------------------
@@ -588,62 +585,62 @@ __device__ __forceinline__ void build_suffix_table(const PopDev& P, uint32_t blo
 
 template <bool ONE, bool DIRECT>
 __global__ void __launch_bounds__(256, 4) k_plan(const __grid_constant__ PopDev one, const PopDev* __restrict__ pops,
-                                                 uint32_t npops, uint32_t what, uint32_t nside) {
+                                                 const BlockPart* __restrict__ map, uint32_t what, uint32_t first) {
     __shared__ uint32_t s_cr[256][kPlanSmemEv + 1];
     __shared__ double s_cdf[kPoisTab + 1];
     __shared__ uint32_t s_grp[DIRECT ? 32 : 1][65];
+    const BlockPart part = block_part<ONE>(map);
+    const PopDev& P = ONE ? one : pops[part.pop];
     pdl_wait();
-    for (uint32_t p = blockIdx.z; p < npops; p += gridDim.z) {
-        const PopDev& P = ONE ? one : pops[p];
-        const DevStatus st = *P.st;
-        const Share side = first_share(nside), plan = second_share(nside);
-        if (side.on) {
-            if (DIRECT) {
-                if ((what & kStepMut) && P.mode != kModePhilox)
-                    sort_tape_lists(P, side.i * 256u + threadIdx.x, side.n * 256u);
-                build_suffix_table(P, side.i, side.n, s_grp);
-            } else {
-                for (uint32_t s = side.i * 256u + threadIdx.x; s < st.A; s += side.n * 256u) slot_rank(P, s);
-            }
+    const DevStatus st = *P.st;
+    const uint32_t a = ONE ? first : max(1u, part.n / first);
+    const Share side = first_share(part, a), plan = second_share(part, a);
+    if (side.on) {
+        if (DIRECT) {
+            if ((what & kStepMut) && P.mode != kModePhilox)
+                sort_tape_lists(P, side.i * 256u + threadIdx.x, side.n * 256u);
+            build_suffix_table(P, side.i, side.n, s_grp);
+        } else {
+            for (uint32_t s = side.i * 256u + threadIdx.x; s < st.A; s += side.n * 256u) slot_rank(P, s);
         }
-        if (!P.plan_row || !plan.on) continue;
-        __syncthreads();  // the previous population's tables are no longer read
-        if (threadIdx.x <= kPoisTab) s_cdf[threadIdx.x] = P.pois_rho[threadIdx.x];
-        __syncthreads();
-        for (uint32_t v0 = plan.i * 256u; v0 < 2u * st.N; v0 += plan.n * 256u) {
-            plan_row(P, st, v0 + threadIdx.x, s_cdf, s_cr[threadIdx.x]);
-        }
+    }
+    if (!P.plan_row || !plan.on) return;
+    if (threadIdx.x <= kPoisTab) s_cdf[threadIdx.x] = P.pois_rho[threadIdx.x];
+    __syncthreads();
+    for (uint32_t v0 = plan.i * 256u; v0 < 2u * st.N; v0 += plan.n * 256u) {
+        plan_row(P, st, v0 + threadIdx.x, s_cdf, s_cr[threadIdx.x]);
     }
 }
 
 // The suffix tables of populations whose ranks k_plan has made.
 template <bool ONE>
-__global__ void __launch_bounds__(256) k_suf_build(const __grid_constant__ PopDev one, const PopDev* __restrict__ pops,
-                                                   uint32_t npops) {
+__global__ void __launch_bounds__(256) k_suf_build(const __grid_constant__ PopDev one,
+                                                   const PopDev* __restrict__ pops,
+                                                   const BlockPart* __restrict__ map) {
     __shared__ uint32_t s_grp[32][65];
+    const BlockPart part = block_part<ONE>(map);
+    const PopDev& P = ONE ? one : pops[part.pop];
     pdl_wait();
-    for (uint32_t p = blockIdx.z; p < npops; p += gridDim.z) {
-        const PopDev& P = ONE ? one : pops[p];
-        if (P.suf) build_suffix_table(P, blockIdx.x, gridDim.x, s_grp);
-    }
+    if (P.suf) build_suffix_table(P, part.i, part.n, s_grp);
 }
 
 uint32_t launch_plan(const LaunchCfg& L, const PopDev* pops, uint32_t npops, const PrepSizes& z, uint32_t maxW,
                      uint32_t what) {
     const uint32_t np = z.tables ? blocks_for(z.maxS, 256) : 0u, units = (maxW + 31u) / 32u * kSufSlices;
+    // Blocks for the tables: as many as there are units, at most half as many as for the rows, but eight (a unit is a
+    // dependent chain of its own: 16 of them in one block made a generation of 100 individuals 29.7 us, in eight
+    // 25.7); in a batch an eighth of each population's.
     if (direct_ranks(z)) {
-        const dim3 g = pop_grid(npops, units + np, L.num_sms, 8);
-        launch_pops(L, k_plan<true, true>, k_plan<false, true>, g, dim3(256), pops, npops, what,
-                    std::max(1u, std::min(units, g.x / 3u)));
+        const uint32_t ns = std::min(units, std::max(np / 2u, 8u)), g = blocks_of(L, ns + np, 8);
+        launch_pops(L, kTablePlan, k_plan<true, true>, k_plan<false, true>, g, pops, npops, what,
+                    npops == 1u ? ns : 8u);
         return 1u;
     }
-    const uint32_t nr = blocks_for(z.maxA, 256);
-    const dim3 g = pop_grid(npops, nr + np, L.num_sms, 8);
-    // a slot's rank is a quarter of a row's plan at most
-    const uint32_t nrank = z.tables ? std::max(1u, std::min(nr, g.x / 4u)) : g.x;
-    launch_pops(L, k_plan<true, false>, k_plan<false, false>, g, dim3(256), pops, npops, what, nrank);
+    const uint32_t nr = blocks_for(z.maxA, 256), g = blocks_of(L, nr + np, 8);
+    const uint32_t ns = npops > 1u ? (z.tables ? 4u : 1u) : (z.tables ? std::max(1u, g / 4u) : g);
+    launch_pops(L, kTablePlan, k_plan<true, false>, k_plan<false, false>, g, pops, npops, what, ns);
     if (!z.tables) return 1u;
-    launch_pops(L, k_suf_build<true>, k_suf_build<false>, pop_grid(npops, units, L.num_sms, 4), dim3(256), pops, npops);
+    launch_pops(L, kTable256, k_suf_build<true>, k_suf_build<false>, blocks_of(L, units, 4), pops, npops);
     return 2u;
 }
 
@@ -654,39 +651,36 @@ uint32_t launch_prep(const LaunchCfg& L, const PopDev* pops, uint32_t npops, con
     constexpr uint32_t kDirectScan = 32768;
     uint32_t n = 0;
     auto sums = [&](uint32_t most, uint32_t which) {
-        launch_pops(L, k_chunk_sums<true>, k_chunk_sums<false>, pop_grid(npops, blocks_for(most, kChunk), L.num_sms, 4),
-                    dim3(256), pops, npops, hdr, which);
+        launch_pops(L, kTable256, k_chunk_sums<true>, k_chunk_sums<false>, blocks_of(L, blocks_for(most, kChunk), 4), pops, npops,
+                    hdr, which);
         ++n;
     };
     if (what & (kStepBegin | kStepMut | kStepOrder)) {
-        dim3 g = pop_grid(npops, blocks_for(z.maxS, kChunk), L.num_sms, std::max(1u, L.ind_per_sm / 4u));
-        g.x += 1u;
-        launch_pops(L, k_stage1<true>, k_stage1<false>, g, dim3(1024), pops, npops, hdr, ctl, what, count_on ? 1u : 0u);
+        launch_pops(L, kTable1024, k_stage1<true>, k_stage1<false>,
+                    1u + blocks_of(L, blocks_for(z.maxS, kChunk), std::max(1u, L.ind_per_sm / 4u)), pops, npops, npops,
+                    hdr, ctl, what, count_on ? 1u : 0u);
         ++n;
         // chunk sums: of the tape's counts (device draws leave their own in stage 1), of the rows per parent
         if ((what & kStepMut) && (what & kStepTape) && z.maxS > kDirectScan) sums(z.maxS, 0u);
         if ((what & kStepOrder) && z.tables && z.maxN > kDirectScan) sums(z.maxN, 1u);
         const uint32_t units = blocks_for(z.maxS + 1u, kChunk) + blocks_for(z.maxN, kChunk);
-        g = pop_grid(npops, units + (uint32_t)L.num_sms, L.num_sms, 6);
-        launch_pops(L, k_stage2<true>, k_stage2<false>, g, dim3(256), pops, npops, hdr, what, kDirectScan,
-                    std::max(1u, g.x / 3u));
+        launch_pops(L, kTable256, k_stage2<true>, k_stage2<false>, blocks_of(L, units + (uint32_t)L.num_sms, 6), pops, npops, hdr,
+                    what, kDirectScan);
         ++n;
     }
     const uint32_t rest = blocks_for(z.maxS, 256);
     if (direct_ranks(z)) {
-        dim3 g = pop_grid(npops, blocks_for(z.maxS, 1024), L.num_sms, 2);
-        g.x += 1u;
-        launch_pops_smem(L, k_stage3<true, true>, k_stage3<false, true>, g, dim3(1024), sizeof(RankSmem), pops, npops,
-                         what);
+        launch_pops_smem(L, kTable1024, k_stage3<true, true>, k_stage3<false, true>, 1u + blocks_of(L, blocks_for(z.maxS, 1024), 2),
+                         sizeof(RankSmem), pops, npops, what);
         return n + 1u;
     }
-    launch_pops(L, k_stage3<true, false>, k_stage3<false, false>,
-                pop_grid(npops, std::max(rest, blocks_for(z.maxA, 256)), L.num_sms, 8), dim3(256), pops, npops, what);
+    launch_pops(L, kTable256, k_stage3<true, false>, k_stage3<false, false>,
+                blocks_of(L, std::max(rest, blocks_for(z.maxA, 256)), 8), pops, npops, what);
     if (z.maxNB > kDirectScan) sums(z.maxNB, 2u);
-    launch_pops(L, k_stage4<true>, k_stage4<false>, pop_grid(npops, blocks_for(z.maxNB, kChunk), L.num_sms, 4), dim3(256),
-                pops, npops, what, kDirectScan);
-    launch_pops(L, k_stage5<true>, k_stage5<false>,
-                pop_grid(npops, blocks_for(std::max(z.maxNB, z.maxA), 256), L.num_sms, 8), dim3(256), pops, npops);
+    launch_pops(L, kTable256, k_stage4<true>, k_stage4<false>, blocks_of(L, blocks_for(z.maxNB, kChunk), 4), pops, npops, what,
+                kDirectScan);
+    launch_pops(L, kTable256, k_stage5<true>, k_stage5<false>, blocks_of(L, blocks_for(std::max(z.maxNB, z.maxA), 256), 8), pops,
+                npops);
     return n + 3u;
 }
 

@@ -110,84 +110,87 @@ void launch_mut_scatter(const LaunchCfg& L, const PopDev* pops, uint32_t npops) 
 // warp of the GPU takes 128 individuals, and what is the same for all of them (the root, the quotients) is
 // computed once a block.
 template <bool ONE>
-__global__ void __launch_bounds__(256) k_individuals(const __grid_constant__ PopDev one, const PopDev* __restrict__ pops, uint32_t npops) {
+__global__ void __launch_bounds__(256) k_individuals(const __grid_constant__ PopDev one,
+                                                     const PopDev* __restrict__ pops,
+                                                     const BlockPart* __restrict__ map) {
     __shared__ double s_k[4];
     __shared__ double s_f[8][128];
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     pdl_wait();
-    for (uint32_t p = blockIdx.z; p < npops; p += gridDim.z) {
-        const PopDev& P = ONE ? one : pops[p];
-        DevStatus* st = P.st;
-        const uint32_t N = st->N, T = P.T;
-        const uint32_t nw = (N + kScanChunk - 1u) / kScanChunk * 32u;  // whole chunks: empty warps sum to zero
-        if (blockIdx.x * 8u >= nw && blockIdx.x) continue;
-        const bool neutral = st->nz_eff == 0;
-        const int fitness = P.fitness;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            if (blockIdx.x == 0) {
-                st->all_neutral = neutral ? 1u : 0u;
-                st->fit_const = 1u;  // k_cdf clears it
-            }
-            if (fitness == 1 || fitness == 2) {
-                const double sig = sqrt(4.0 * (double)N * P.mu);  // normal/quadratic generators
-                s_k[0] = (1.0 / sig) * 0.398942280401432677939946059934;
-                s_k[1] = 2.0 * sig * sig;
-                s_k[2] = P.fit_param * sig;
-            }
+    const BlockPart part = block_part<ONE>(map);
+    const PopDev& P = ONE ? one : pops[part.pop];
+    pdl_wait();
+    DevStatus* st = P.st;
+    const uint32_t N = st->N, T = P.T;
+    const uint32_t nw = (N + kScanChunk - 1u) / kScanChunk * 32u;  // whole chunks: empty warps sum to zero
+    if (part.i >= nw && part.i) return;
+    const bool neutral = st->nz_eff == 0;
+    const int fitness = P.fitness;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        if (part.i == 0) {
+            st->all_neutral = neutral ? 1u : 0u;
+            st->fit_const = 1u;  // k_cdf clears it
         }
-        __syncthreads();
-        const double* zg = P.zg[st->cur];
-        for (uint32_t w = blockIdx.x * 8u + warp; w < nw; w += gridDim.x * 8u) {
+        if (fitness == 1 || fitness == 2) {
+            const double sig = sqrt(4.0 * (double)N * P.mu);  // normal/quadratic generators
+            s_k[0] = (1.0 / sig) * 0.398942280401432677939946059934;
+            s_k[1] = 2.0 * sig * sig;
+            s_k[2] = P.fit_param * sig;
+        }
+    }
+    __syncthreads();
+    const double* zg = P.zg[st->cur];
+    // neighbouring units in different blocks: as even a share of the FP64 pipes as there are units
+    for (uint32_t w = warp * part.n + part.i; w < nw; w += part.n * 8u) {
 #pragma unroll
-            for (uint32_t k = 0; k < 4; ++k) {
-                const uint32_t i = w * 128u + 32u * k + lane;
-                double f = 0.0;
-                if (i < N) {
-                    const double2* a = reinterpret_cast<const double2*>(zg + (size_t)i * 8u);  // genomes 2i, 2i + 1
-                    double z[4] = {1.0, 1.0, 1.0, 1.0};
-                    if (!neutral) {
-                        const double2 a0 = a[0], b0 = a[2];
-                        z[0] = a0.x + b0.x;
-                        if (T > 1) z[1] = a0.y + b0.y;
-                        if (T > 2) {
-                            const double2 a1 = a[1], b1 = a[3];
-                            z[2] = a1.x + b1.x;
-                            z[3] = a1.y + b1.y;
-                        }
+        for (uint32_t k = 0; k < 4; ++k) {
+            const uint32_t i = w * 128u + 32u * k + lane;
+            double f = 0.0;
+            if (i < N) {
+                const double2* a = reinterpret_cast<const double2*>(zg + (size_t)i * 8u);  // genomes 2i, 2i + 1
+                double z[4] = {1.0, 1.0, 1.0, 1.0};
+                if (!neutral) {
+                    const double2 a0 = a[0], b0 = a[2];
+                    z[0] = a0.x + b0.x;
+                    if (T > 1) z[1] = a0.y + b0.y;
+                    if (T > 2) {
+                        const double2 a1 = a[1], b1 = a[3];
+                        z[2] = a1.x + b1.x;
+                        z[3] = a1.y + b1.y;
                     }
-                    for (uint32_t t = 1; t < 4; ++t)
-                        if (t >= T) z[t] = 0.0;
-                    double2* zi = reinterpret_cast<double2*>(P.zi + (size_t)i * 4u);
-                    zi[0] = make_double2(z[0], z[1]);
-                    zi[1] = make_double2(z[2], z[3]);
-                    f = 1.0;
-                    const double z0 = z[0];
-                    switch (fitness) {
-                        case 1:  // gaussian (normal_fitness_metric.cpp:25-31)
-                            f = s_k[0] * exp(-(z0 * z0) / s_k[1]);
-                            break;
-                        case 2: {  // quadratic (quadratic_fitness_metric.cpp:23-28)
-                            double r = z0 / s_k[2];
-                            r *= r;
-                            f = (r >= 1.0) ? 0.0 : 1.0 - r;
-                        } break;
-                        case 3: {  // gaussian_vs
-                            const double ss = z[0] * z[0] + z[1] * z[1] + z[2] * z[2] + z[3] * z[3];
-                            f = exp(-ss / (2.0 * P.fit_param));
-                        } break;
-                        default: f = 1.0;
-                    }
-                    P.fit[i] = f;
                 }
-                s_f[warp][32u * k + lane] = f;
+                for (uint32_t t = 1; t < 4; ++t)
+                    if (t >= T) z[t] = 0.0;
+                double2* zi = reinterpret_cast<double2*>(P.zi + (size_t)i * 4u);
+                zi[0] = make_double2(z[0], z[1]);
+                zi[1] = make_double2(z[2], z[3]);
+                f = 1.0;
+                const double z0 = z[0];
+                switch (fitness) {
+                    case 1:  // gaussian (normal_fitness_metric.cpp:25-31)
+                        f = s_k[0] * exp(-(z0 * z0) / s_k[1]);
+                        break;
+                    case 2: {  // quadratic (quadratic_fitness_metric.cpp:23-28)
+                        double r = z0 / s_k[2];
+                        r *= r;
+                        f = (r >= 1.0) ? 0.0 : 1.0 - r;
+                    } break;
+                    case 3: {  // gaussian_vs
+                        const double ss = z[0] * z[0] + z[1] * z[1] + z[2] * z[2] + z[3] * z[3];
+                        f = exp(-ss / (2.0 * P.fit_param));
+                    } break;
+                    default: f = 1.0;
+                }
+                P.fit[i] = f;
             }
-            __syncwarp();
-            const double* v = &s_f[warp][4u * lane];
-            const double s = warp_incl_f64(((v[0] + v[1]) + v[2]) + v[3]);
-            if (lane == 31u) P.scan_wsum[w] = s;
-            __syncwarp();
+            s_f[warp][32u * k + lane] = f;
         }
+        __syncwarp();
+        const double* v = &s_f[warp][4u * lane];
+        const double s = warp_incl_f64(((v[0] + v[1]) + v[2]) + v[3]);
+        if (lane == 31u) P.scan_wsum[w] = s;
+        __syncwarp();
     }
 }
 
@@ -232,86 +235,87 @@ __global__ void __launch_bounds__(256) k_cdf_offsets(const PopDev* __restrict__ 
 
 // A unit is 8 warps of 128 individuals: a quarter of a chunk.
 template <bool ONE>
-__global__ void __launch_bounds__(256) k_cdf(const __grid_constant__ PopDev one, const PopDev* __restrict__ pops, uint32_t npops, uint32_t end) {
+__global__ void __launch_bounds__(256) k_cdf(const __grid_constant__ PopDev one, const PopDev* __restrict__ pops,
+                                             const BlockPart* __restrict__ map, uint32_t end) {
     __shared__ double s_tot[kInlineChunks];
     __shared__ double s_woff[32];
     __shared__ double s_part, s_last;
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     pdl_wait();
-    for (uint32_t p = blockIdx.z; p < npops; p += gridDim.z) {
-        const PopDev& P = ONE ? one : pops[p];
-        DevStatus* st = P.st;
-        const uint32_t N = st->N;
-        const uint32_t nch = (N + kScanChunk - 1u) / kScanChunk;
-        if (blockIdx.x == 0 && threadIdx.x == 0) {
-            if (end) {
-                st->last_M = st->M;
-                st->gen += 1u;
-            }
-            if (N == 0) st->fit_total = 0.0;
+    const BlockPart part = block_part<ONE>(map);
+    const PopDev& P = ONE ? one : pops[part.pop];
+    pdl_wait();
+    DevStatus* st = P.st;
+    const uint32_t N = st->N;
+    const uint32_t nch = (N + kScanChunk - 1u) / kScanChunk;
+    if (part.i == 0 && threadIdx.x == 0) {
+        if (end) {
+            st->last_M = st->M;
+            st->gen += 1u;
         }
-        const double f0 = N ? P.fit[0] : 0.0;
-        for (uint32_t u = blockIdx.x; u < nch * 4u; u += gridDim.x) {
-            const uint32_t c = u >> 2, w = u * 8u + warp;
-            const bool last = u == nch * 4u - 1u;
-            const uint32_t b = w * 128u + lane * 4u;
-            double v[4], s = 0.0;
-            bool same = true;
+        if (N == 0) st->fit_total = 0.0;
+    }
+    const double f0 = N ? P.fit[0] : 0.0;
+    for (uint32_t u = part.i; u < nch * 4u; u += part.n) {
+        const uint32_t c = u >> 2, w = u * 8u + warp;
+        const bool last = u == nch * 4u - 1u;
+        const uint32_t b = w * 128u + lane * 4u;
+        double v[4], s = 0.0;
+        bool same = true;
 #pragma unroll
-            for (uint32_t k = 0; k < 4; ++k) {
-                v[k] = (b + k < N) ? P.fit[b + k] : 0.0;
-                if (b + k < N && v[k] != f0) same = false;
-                s += v[k];
-            }
-            if (!__all_sync(0xffffffffu, same) && lane == 0u) atomicAnd(&st->fit_const, 0u);
-            __syncthreads();  // the previous unit's offsets are read
-            if (nch <= kInlineChunks) {
-                if (threadIdx.x < c) s_tot[threadIdx.x] = chunk_total(P.scan_wsum, threadIdx.x);
-                __syncthreads();
-            }
-            if (threadIdx.x == 0) {
-                double acc = 0.0;
-                if (nch <= kInlineChunks)
-                    for (uint32_t j = 0; j < c; ++j) acc += s_tot[j];
-                else
-                    acc = P.scan_part[c];
-                s_part = acc;
-            }
-            if (warp == 1u) {  // offsets of the chunk's warps: lane i adds the i before it one after another
-                const double ws = P.scan_wsum[32u * c + lane];
-                double acc = 0.0;
-                for (uint32_t j = 0; j < 31u; ++j) {
-                    const double x = __shfl_sync(0xffffffffu, ws, j);
-                    if (j < lane) acc += x;
-                }
-                s_woff[lane] = acc;
-                if (lane == 31u) s_last = acc + ws;  // the chunk's total
-            }
-            const double incl = warp_incl_f64(s);
+        for (uint32_t k = 0; k < 4; ++k) {
+            v[k] = (b + k < N) ? P.fit[b + k] : 0.0;
+            if (b + k < N && v[k] != f0) same = false;
+            s += v[k];
+        }
+        if (!__all_sync(0xffffffffu, same) && lane == 0u) atomicAnd(&st->fit_const, 0u);
+        __syncthreads();  // the previous unit's offsets are read
+        if (nch <= kInlineChunks) {
+            if (threadIdx.x < c) s_tot[threadIdx.x] = chunk_total(P.scan_wsum, threadIdx.x);
             __syncthreads();
-            // exclusive prefix inside the warp = inclusive value of the previous lane
-            const double prev = __shfl_up_sync(0xffffffffu, incl, 1);
-            const double excl_w = lane ? prev : 0.0;
-            double r = s_part + (s_woff[w & 31u] + excl_w);
+        }
+        if (threadIdx.x == 0) {
+            double acc = 0.0;
+            if (nch <= kInlineChunks)
+                for (uint32_t j = 0; j < c; ++j) acc += s_tot[j];
+            else
+                acc = P.scan_part[c];
+            s_part = acc;
+        }
+        if (warp == 1u) {  // offsets of the chunk's warps: lane i adds the i before it one after another
+            const double ws = P.scan_wsum[32u * c + lane];
+            double acc = 0.0;
+            for (uint32_t j = 0; j < 31u; ++j) {
+                const double x = __shfl_sync(0xffffffffu, ws, j);
+                if (j < lane) acc += x;
+            }
+            s_woff[lane] = acc;
+            if (lane == 31u) s_last = acc + ws;  // the chunk's total
+        }
+        const double incl = warp_incl_f64(s);
+        __syncthreads();
+        // exclusive prefix inside the warp = inclusive value of the previous lane
+        const double prev = __shfl_up_sync(0xffffffffu, incl, 1);
+        const double excl_w = lane ? prev : 0.0;
+        double r = s_part + (s_woff[w & 31u] + excl_w);
 #pragma unroll
-            for (uint32_t k = 0; k < 4; ++k) {
-                r += v[k];
-                if (b + k < N) P.cdf[b + k] = r;
-            }
-            if (last && threadIdx.x == 0) {
-                const double total = s_part + s_last;
-                st->fit_total = total;
-                if (!(total > 0.0)) atomicOr(&st->err, kErrFitness);
-            }
+        for (uint32_t k = 0; k < 4; ++k) {
+            r += v[k];
+            if (b + k < N) P.cdf[b + k] = r;
+        }
+        if (last && threadIdx.x == 0) {
+            const double total = s_part + s_last;
+            st->fit_total = total;
+            if (!(total > 0.0)) atomicOr(&st->err, kErrFitness);
         }
     }
 }
 uint32_t launch_fitness(const LaunchCfg& L, const PopDev* pops, uint32_t npops, uint32_t maxN, bool end) {
     const uint32_t units = std::max(1u, (maxN + kScanChunk - 1u) / kScanChunk * 4u);
-    launch_pops(L, k_individuals<true>, k_individuals<false>, pop_grid(npops, units, L.num_sms, L.ind_per_sm), dim3(256), pops, npops);
+    launch_pops(L, kTable256, k_individuals<true>, k_individuals<false>, blocks_of(L, units, L.ind_per_sm), pops, npops);
     const bool offsets = maxN > kInlineChunks * kScanChunk;
     if (offsets) launch_k(L, k_cdf_offsets, dim3(npops), dim3(256), pops);
-    launch_pops(L, k_cdf<true>, k_cdf<false>, pop_grid(npops, units, L.num_sms, 8), dim3(256), pops, npops, end ? 1u : 0u);
+    launch_pops(L, kTable256, k_cdf<true>, k_cdf<false>, blocks_of(L, units, 8), pops, npops, end ? 1u : 0u);
     return offsets ? 3u : 2u;
 }
 

@@ -153,16 +153,32 @@ __device__ __forceinline__ void plan_row(const PopDev& P, const DevStatus& st, u
                 cr[k] = threshold_rank(P, e0);
             }
         }
-        // share of the rank space the breakpoints switch: sorted thresholds pair into intervals
+        // share of the rank space the breakpoints switch: sorted thresholds pair into intervals.  A threshold counts
+        // by the parity of its place in the order (equal ones in list order); each pair is compared once.
         int64_t len = (E & 1u) ? (int64_t)A : 0;
-        for (uint32_t k = 0; k < E; ++k) {
-            const uint32_t rk = cr[k];
-            uint32_t posn = 0;
-            for (uint32_t j = 0; j < E; ++j) {
-                const uint32_t rj = cr[j];
-                posn += (rj < rk || (rj == rk && j < k)) ? 1u : 0u;
+        if (E <= kPlanSmemEv) {
+            uint32_t odd = 0;
+            for (uint32_t k = 1; k < E; ++k) {
+                const uint32_t rk = cr[k];
+                uint32_t here = 0;
+                for (uint32_t j = 0; j < k; ++j) {
+                    const uint32_t before = cr[j] <= rk ? 1u : 0u;
+                    here ^= before;
+                    odd ^= (before ^ 1u) << j;
+                }
+                odd |= here << k;
             }
-            len += (posn & 1u) ? (int64_t)rk : -(int64_t)rk;
+            for (uint32_t k = 0; k < E; ++k) len += ((odd >> k) & 1u) ? (int64_t)cr[k] : -(int64_t)cr[k];
+        } else {
+            for (uint32_t k = 0; k < E; ++k) {
+                const uint32_t rk = cr[k];
+                uint32_t posn = 0;
+                for (uint32_t j = 0; j < E; ++j) {
+                    const uint32_t rj = cr[j];
+                    posn += (rj < rk || (rj == rk && j < k)) ? 1u : 0u;
+                }
+                len += (posn & 1u) ? (int64_t)rk : -(int64_t)rk;
+            }
         }
         if (2 * len > (int64_t)A) flags |= kPlanInv;
         for (uint32_t k = 0; k < E; ++k) {
