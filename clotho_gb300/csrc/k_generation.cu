@@ -140,15 +140,20 @@ __device__ __forceinline__ void load_pair(ulonglong2& t, ulonglong2& b, const Ro
     }
 }
 
-// AND/OR into the CTA accumulators; the atomic is issued only when it would
-// change the word (both operations are monotone, so skipping is exact).
+// AND/OR into the CTA accumulators; the atomics are issued only when they would
+// change a word (both operations are monotone, so skipping is exact).  One test covers all four: rarely true once a
+// few rows are in.
+template <bool ONE_TEST>
 __device__ __forceinline__ void fold_fs(uint64_t* sF, uint64_t* sV, uint32_t w, uint64_t x0, uint64_t x1) {
     const ulonglong2 f = *reinterpret_cast<const ulonglong2*>(sF + w);
     const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(sV + w);
-    if (f.x & ~x0) atomicAnd((unsigned long long*)&sF[w], (unsigned long long)x0);
-    if (f.y & ~x1) atomicAnd((unsigned long long*)&sF[w + 1u], (unsigned long long)x1);
-    if (x0 & ~v.x) atomicOr((unsigned long long*)&sV[w], (unsigned long long)x0);
-    if (x1 & ~v.y) atomicOr((unsigned long long*)&sV[w + 1u], (unsigned long long)x1);
+    const uint64_t c0 = (f.x & ~x0) | (x0 & ~v.x), c1 = (f.y & ~x1) | (x1 & ~v.y);
+    if (!ONE_TEST || (c0 | c1)) {
+        if (f.x & ~x0) atomicAnd((unsigned long long*)&sF[w], (unsigned long long)x0);
+        if (f.y & ~x1) atomicAnd((unsigned long long*)&sF[w + 1u], (unsigned long long)x1);
+        if (x0 & ~v.x) atomicOr((unsigned long long*)&sV[w], (unsigned long long)x0);
+        if (x1 & ~v.y) atomicOr((unsigned long long*)&sV[w + 1u], (unsigned long long)x1);
+    }
 }
 
 // Per-column counts of the finished child words, bit-sliced: plane b (cnt + b * stride) holds bit b of every
@@ -174,8 +179,9 @@ struct Fold {
     uint64_t* cnt;
     uint32_t stride;
 };
+template <bool ONE_TEST = true>
 __device__ __forceinline__ void fold(const Fold& fo, uint32_t w, uint64_t x0, uint64_t x1) {
-    fold_fs(fo.F, fo.V, w, x0, x1);
+    fold_fs<ONE_TEST>(fo.F, fo.V, w, x0, x1);
     if (fo.cnt) count_add(fo.cnt, fo.stride, w, x0, x1);
 }
 constexpr uint32_t kCountMax = (1u << kCountPlanes) - 1u;   // rows a CTA may add between flushes
@@ -392,7 +398,7 @@ struct WarpSmem {
 };
 
 // Copy rows of the bitmap builds: 1 = one bulk copy of the parent strand into the warp's bitmap,
-// 0 = register streaming six chunks deep (what the chunk-mask build, which has no bitmaps, always does)
+// 0 = register streaming a few chunks deep (what the chunk-mask build, which has no bitmaps, always does)
 #ifndef CLOTHO_COPY_BULK
 #define CLOTHO_COPY_BULK 1
 #endif
@@ -477,12 +483,14 @@ __device__ CLOTHO_COLD float4 effects_direct(uint64_t m0, uint64_t m1, uint64_t 
 #ifndef CLOTHO_ROUND_LANE
 #define CLOTHO_ROUND_LANE 3
 #endif
-#ifndef CLOTHO_TABLE_INFLIGHT
-#define CLOTHO_TABLE_INFLIGHT 16
-#endif
 constexpr uint32_t kRoundLane = CLOTHO_ROUND_LANE;   // queue entries gathered per lane per round
 constexpr uint32_t kRound = 32u * kRoundLane;
-constexpr uint32_t kTableInflight = CLOTHO_TABLE_INFLIGHT;
+// Table rows and 64-word chunks of a step of the mask's building: 4 x 3 16-byte loads a lane in flight.  A row's whole
+// width of one table row at a time (16 loads) read and wrote the bitmap once a breakpoint: N = 400,000 of the
+// large population 5.77 ms, 200,000 individuals of 320-word rows 1.51 ms; 4 x 3 5.42 and 1.32; 4 x 4 spills (5.70),
+// 3 x 3 5.47, 5 x 2 5.47, 6 x 2 5.63.
+constexpr uint32_t kTableEv = 4, kTableChunks = 3;
+constexpr uint32_t kCorrAhead = 3;       // breakpoints whose correction slots are fetched before the table rows
 constexpr uint32_t kFlatLoads = 4;   // table loads per lane when a narrow row's whole mask is built at once
 constexpr uint32_t kDirectCopyChunks = 2;   // copy rows up to 128 words load their strand directly
 constexpr uint32_t kCmCorr = 32u * kCmMaxEv;   // chunk-mask build: correction slots a warp holds
@@ -611,12 +619,12 @@ __device__ __forceinline__ void row_mutations(const PopDev& P, uint32_t M, const
 }
 
 // Copy rows (no breakpoint): the top strand with the fixed columns cleared and
-// the new alleles added, streamed through registers six chunks ahead (the
+// the new alleles added, streamed through registers a few chunks ahead (the
 // chunk-mask build, whose warps have no bitmap for a bulk copy to land in).
 __device__ __forceinline__ void row_body_copy(const PopDev& P, uint32_t M, const RowArgs& R, const uint64_t* sfix,
                                               bool do_mut, bool do_fs, const Fold& fo) {
     const uint32_t lane = threadIdx.x & 31u;
-    constexpr uint32_t D = 6;
+    constexpr uint32_t D = 3;   // the rows are prefetched into L2 as a whole: six chunks 2.07 ms, three 2.04
     ulonglong2 t[D];
 #pragma unroll
     for (uint32_t j = 0; j < D; ++j) {
@@ -666,7 +674,7 @@ __device__ __forceinline__ void row_body_copy_direct(const PopDev& P, uint32_t M
                 w < R.Wp ? *reinterpret_cast<const ulonglong2*>(sfix + w) : make_ulonglong2(0, 0);
             const uint64_t x0 = (t[j].x & ~fm.x) ^ mx0, x1 = (t[j].y & ~fm.y) ^ mx1;
             *reinterpret_cast<ulonglong2*>(R.out + w) = make_ulonglong2(x0, x1);
-            if (do_fs) fold(fo, w, x0, x1);
+            if (do_fs) fold<false>(fo, w, x0, x1);
         }
     }
     if (R.Wc > 64u * kDirectCopyChunks) {  // a child wider than its parent: the rest is new alleles only
@@ -676,7 +684,7 @@ __device__ __forceinline__ void row_body_copy_direct(const PopDev& P, uint32_t M
             if (do_mut && R.mc) row_mutations(P, M, R, w, mx0, mx1);
             if (w < R.Wc) {
                 *reinterpret_cast<ulonglong2*>(R.out + w) = make_ulonglong2(mx0, mx1);
-                if (do_fs) fold(fo, w, mx0, mx1);
+                if (do_fs) fold<false>(fo, w, mx0, mx1);
             }
         }
     }
@@ -715,7 +723,6 @@ __device__ __forceinline__ bool row_body_copy_bulk(const PopDev& P, uint32_t M, 
             if (w < R.Wp) {
                 ulonglong2* bw = reinterpret_cast<ulonglong2*>(buf + w);
                 if (ok) t = *bw;
-                *bw = make_ulonglong2(0, 0);  // crossover rows expect the bitmap at zero
                 fm = *reinterpret_cast<const ulonglong2*>(sfix + w);
             }
             const uint64_t x0 = (t.x & ~fm.x) ^ mx0, x1 = (t.y & ~fm.y) ^ mx1;
@@ -733,7 +740,7 @@ __device__ __forceinline__ bool row_body_copy_bulk(const PopDev& P, uint32_t M, 
 // of the breakpoints (lane k < E holds row k's offset in my_go) and toggled at
 // the row's correction slots (cs[32 k + lane], 0xffffffff for none).
 // PROF: clock the effect gather into *gcyc (profiling build).
-template <int MODE, bool PROF = false>
+template <int MODE, bool PROF = false, bool CLEAR = false>
 __device__ __forceinline__ void row_body_suf(const PopDev& P, uint32_t M, const RowArgs& R, const uint64_t* sfix,
                                              uint64_t* mask, uint32_t* Q, bool inv, bool do_mut, bool gather,
                                              bool do_fs, const Fold& fo, float (&d)[kMaxTraits],
@@ -768,7 +775,7 @@ __device__ __forceinline__ void row_body_suf(const PopDev& P, uint32_t M, const 
                 if (live) {
                     ulonglong2* mw = reinterpret_cast<ulonglong2*>(mask + w);
                     const ulonglong2 m = *mw;
-                    *mw = make_ulonglong2(0, 0);  // the bitmap starts every row at zero
+                    if (CLEAR) *mw = make_ulonglong2(0, 0);  // narrow build: the bitmap starts every row at zero
                     m0 = m.x;
                     m1 = m.y;
                 }
@@ -826,7 +833,7 @@ __device__ __forceinline__ void row_body_suf(const PopDev& P, uint32_t M, const 
             x0 ^= mx0;
             x1 ^= mx1;
             *reinterpret_cast<ulonglong2*>(R.out + w) = make_ulonglong2(x0, x1);
-            if (do_fs) fold(fo, w, x0, x1);
+            if (do_fs) fold<!CLEAR>(fo, w, x0, x1);
         }
         t_a = t_b; b_a = b_b;
     }
@@ -930,6 +937,10 @@ __device__ __forceinline__ bool gen_row_suf(const PopDev& P, const DevStatus& st
             // costs one table round trip instead of one per breakpoint
             const uint32_t my_cr = lane < E ? __ldg(P.plan_cr + base + lane) : 0u;
             const uint32_t my_go = lane < E ? __ldg(P.plan_go + base + lane) : 0u;
+            if (!NARROW) {   // the wide builds' bitmap holds anything
+                for (uint32_t i = lane; i < np; i += 32u) reinterpret_cast<ulonglong2*>(mask)[i] = make_ulonglong2(0, 0);
+                __syncwarp();
+            }
             ulonglong2 v[kFlatLoads];
             uint32_t at[kFlatLoads];
 #pragma unroll
@@ -961,14 +972,66 @@ __device__ __forceinline__ bool gen_row_suf(const PopDev& P, const DevStatus& st
                 }
             }
         } else {
-            // corrections: toggle the slots whose rank lies between threshold and table row (the table-row
-            // offsets of the first 32 breakpoints are fetched with their correction ranks)
+            // the bitmap takes the XOR of the breakpoints' table rows, then the corrections: the slots whose rank lies
+            // between threshold and table row are toggled.  The correction slots of the first kCorrAhead breakpoints
+            // are fetched before the table rows.
             const uint32_t go0 = lane < E ? __ldg(P.plan_go + base + lane) : 0u;
+            const uint32_t cr0 = lane < E ? __ldg(P.plan_cr + base + lane) : 0u;
+            uint32_t cs0[kCorrAhead];
+#pragma unroll
+            for (uint32_t k = 0; k < kCorrAhead; ++k) {
+                const uint32_t pc = __shfl_sync(0xffffffffu, cr0, k);
+                cs0[k] = lane < (pc >> 20) ? __ldg(P.inv + (pc & 0xfffffu) + lane) : 0xffffffffu;
+            }
+            // kTableEv rows of kTableChunks 64-word chunks at a time: 16-byte loads in flight, one access of the
+            // bitmap for all rows of a step (the first one only writes: the wide builds' bitmap holds anything)
+            ulonglong2* m2 = reinterpret_cast<ulonglong2*>(mask);
             for (uint32_t k0 = 0; k0 < E; k0 += 32u) {
-                const uint32_t my_cr = (k0 + lane < E) ? __ldg(P.plan_cr + base + k0 + lane) : 0u;
+                const uint32_t my_go = k0 == 0 ? go0 : (k0 + lane < E) ? __ldg(P.plan_go + base + k0 + lane) : 0u;
                 const uint32_t ke = min(32u, E - k0);
-    #pragma unroll 4
-                for (uint32_t k = 0; k < ke; ++k) {
+                for (uint32_t kq = 0; kq < ke; kq += kTableEv) {
+                    const bool fresh = !NARROW && k0 + kq == 0u;
+                    const uint64_t* tk[kTableEv];
+#pragma unroll
+                    for (uint32_t q = 0; q < kTableEv; ++q)
+                        tk[q] = suf + __shfl_sync(0xffffffffu, my_go, (kq + q) & 31u) + 2u * lane;
+                    for (uint32_t wb = 0; wb < R.Wp; wb += 64u * kTableChunks) {
+                        ulonglong2 v[kTableEv][kTableChunks];
+#pragma unroll
+                        for (uint32_t q = 0; q < kTableEv; ++q) {
+#pragma unroll
+                            for (uint32_t j = 0; j < kTableChunks; ++j) {
+                                const uint32_t w = wb + 64u * j;
+                                v[q][j] = (kq + q < ke && w + 2u * lane < R.Wp)
+                                              ? __ldg(reinterpret_cast<const ulonglong2*>(tk[q] + w))
+                                              : make_ulonglong2(0, 0);
+                            }
+                        }
+#pragma unroll
+                        for (uint32_t j = 0; j < kTableChunks; ++j) {
+                            const uint32_t w = wb + 64u * j + 2u * lane;
+                            if (w < R.Wp) {
+                                ulonglong2 x = fresh ? make_ulonglong2(0, 0) : m2[w >> 1];
+#pragma unroll
+                                for (uint32_t q = 0; q < kTableEv; ++q) {
+                                    x.x ^= v[q][j].x;
+                                    x.y ^= v[q][j].y;
+                                }
+                                m2[w >> 1] = x;
+                            }
+                        }
+                    }
+                }
+            }
+            __syncwarp();
+#pragma unroll
+            for (uint32_t k = 0; k < kCorrAhead; ++k)
+                if (cs0[k] != 0xffffffffu) atomicXor(m32 + (cs0[k] >> 5), 1u << (cs0[k] & 31u));
+            for (uint32_t k0 = 0; k0 < E; k0 += 32u) {
+                const uint32_t my_cr = k0 == 0 ? cr0 : (k0 + lane < E) ? __ldg(P.plan_cr + base + k0 + lane) : 0u;
+                const uint32_t ke = min(32u, E - k0);
+#pragma unroll 4
+                for (uint32_t k = k0 ? 0u : kCorrAhead; k < ke; ++k) {
                     const uint32_t pc = __shfl_sync(0xffffffffu, my_cr, k);
                     if (lane < (pc >> 20)) {
                         const uint32_t s = __ldg(P.inv + (pc & 0xfffffu) + lane);
@@ -976,39 +1039,10 @@ __device__ __forceinline__ bool gen_row_suf(const PopDev& P, const DevStatus& st
                     }
                 }
             }
-            __syncwarp();
-            // XOR of the events' table rows, kTableInflight 16-byte loads per lane in flight
-            ulonglong2* m2 = reinterpret_cast<ulonglong2*>(mask);
-            for (uint32_t k0 = 0; k0 < E; k0 += 32u) {
-                const uint32_t my_go = k0 == 0 ? go0 : (k0 + lane < E) ? __ldg(P.plan_go + base + k0 + lane) : 0u;
-                const uint32_t ke = min(32u, E - k0);
-                for (uint32_t k = 0; k < ke; ++k) {
-                    const uint64_t* tk = suf + __shfl_sync(0xffffffffu, my_go, k);
-                    for (uint32_t wb = 0; wb < R.Wp; wb += 64u * kTableInflight) {
-                        ulonglong2 v[kTableInflight];
-    #pragma unroll
-                        for (uint32_t j = 0; j < kTableInflight; ++j) {
-                            const uint32_t w = wb + 64u * j + 2u * lane;
-                            v[j] = (w < R.Wp) ? __ldg(reinterpret_cast<const ulonglong2*>(tk + w))
-                                              : make_ulonglong2(0, 0);
-                        }
-    #pragma unroll
-                        for (uint32_t j = 0; j < kTableInflight; ++j) {
-                            const uint32_t w = wb + 64u * j + 2u * lane;
-                            if (w < R.Wp) {
-                                ulonglong2 x = m2[w >> 1];
-                                x.x ^= v[j].x;
-                                x.y ^= v[j].y;
-                                m2[w >> 1] = x;
-                            }
-                        }
-                    }
-                }
-            }
         }
         __syncwarp();
         if (PROF) c2 = clock64();
-        row_body_suf<0, PROF>(P, st.M, R, sfix, mask, ws.q, inv, do_mut, gather, do_fs, fo, d,
+        row_body_suf<0, PROF, NARROW>(P, st.M, R, sfix, mask, ws.q, inv, do_mut, gather, do_fs, fo, d,
                               &pc.c[kPhXoGather]);
     }
     if (PROF) c3 = clock64();
@@ -1035,12 +1069,12 @@ __device__ __forceinline__ bool gen_row_suf(const PopDev& P, const DevStatus& st
 }
 
 // ---------------------------------------------------------------------------
-// Short rows (parent and child at most 32 words): several rows a warp.
+// Short rows (parent and child at most 64 words): a row in the lanes it fills.
 //
 // A row of 8, 16 or 32 words fills 4, 8 or 16 lanes of two words each; one row a warp
 // leaves the other lanes idle and pays the row's set-up (plan, breakpoints, corrections,
 // reductions: several hundred instructions) for them as well.  Here L lanes take a row and
-// a warp 32 / L rows.  The switch mask stays in the lanes' registers, the corrections and
+// a warp 32 / L rows (rows of up to 64 words: one).  The switch mask stays in the lanes' registers, the corrections and
 // the new alleles go through a 2L-word bitmap per row, the AND/OR of the children is kept in registers
 // until the rows run out.  What bounds it is instruction issue: the set-up per warp, now shared.
 //
@@ -1048,8 +1082,8 @@ __device__ __forceinline__ bool gen_row_suf(const PopDev& P, const DevStatus& st
 // entries v, v + 32, ... one after another and then the lanes are summed by a butterfly; here
 // lane l holds the partial sums of the lanes l, l + L, ... and adds them in the same tree.
 template <uint32_t L>
-__device__ __forceinline__ void group_loop(const PopDev& P, uint32_t r0, uint32_t r1, uint32_t* next, uint32_t u0,
-                                           uint32_t us, uint32_t* crows, const uint64_t* sfix, uint32_t* gm,
+__device__ __forceinline__ void group_loop(const PopDev& P, uint32_t r0, uint32_t r1, uint32_t* next, uint32_t chunk,
+                                           uint32_t u0, uint32_t us, uint32_t* crows, const uint64_t* sfix, uint32_t* gm,
                                            uint32_t* Qw, uint64_t* sF, uint64_t* sV, uint64_t* cnt, uint32_t stride,
                                            uint32_t fuse) {
     constexpr uint32_t VL = 32u / L;        // rows a warp, and lanes of the one-row form that a lane stands for
@@ -1071,15 +1105,19 @@ __device__ __forceinline__ void group_loop(const PopDev& P, uint32_t r0, uint32_
     if (w < Wp) fm = *reinterpret_cast<const ulonglong2*>(sfix + w);
     uint64_t F0 = ~0ull, F1 = ~0ull, V0 = 0ull, V1 = 0ull;
     const uint32_t units = (r1 - r0 + VL - 1u) / VL;
-    uint32_t u = u0;
+    uint32_t u = u0, left = chunk;   // units left of the claim
     if (next) {
-        if (lane == 0) u = atomicAdd(next, 1u);
+        if (lane == 0) u = atomicAdd(next, chunk);
         u = __shfl_sync(kFull, u, 0);
     }
     while (u < units) {
         // the next rows are claimed, and their plans fetched into L1, behind these
         uint32_t un = u + us;
-        if (next && lane == 0) un = atomicAdd(next, 1u);
+        if (next) {
+            if (--left) un = u + 1u;
+            else if (lane == 0) un = atomicAdd(next, chunk);
+            if (!left) left = chunk;
+        }
         const uint32_t v = r0 + u * VL + sub;
         const bool live = v < r1;
         uint4 pr = make_uint4(0, 0, 0, 0);
@@ -1326,17 +1364,19 @@ __device__ __forceinline__ void group_loop(const PopDev& P, uint32_t r0, uint32_
     }
 }
 
-constexpr uint32_t kGroupWords = 32;   // widest rows that share a warp
+constexpr uint32_t kGroupWords = 64;   // widest rows whose words are all in a warp's lanes at once
 
-// The rows [r0, r1) of the processing order, units of 32 / L rows claimed from *next, or u0, u0 + us, ....
-__device__ __noinline__ void group_rows(const PopDev& P, uint32_t r0, uint32_t r1, uint32_t* next, uint32_t u0,
-                                        uint32_t us, uint32_t* crows, const uint64_t* sfix, uint64_t* mask, uint32_t* Q,
+// The rows [r0, r1) of the processing order in units of 32 / L rows: chunk at a time claimed from *next, or u0, u0 +
+// us, ....
+__device__ __noinline__ void group_rows(const PopDev& P, uint32_t r0, uint32_t r1, uint32_t* next, uint32_t chunk,
+                                        uint32_t u0, uint32_t us, uint32_t* crows, const uint64_t* sfix, uint64_t* mask, uint32_t* Q,
                                         uint64_t* sF, uint64_t* sV, uint64_t* cnt, uint32_t stride, uint32_t fuse) {
     const uint32_t W = max(P.st->W, P.st->pW);
     uint32_t* gm = reinterpret_cast<uint32_t*>(mask);
-    if (W <= 8u) group_loop<4>(P, r0, r1, next, u0, us, crows, sfix, gm, Q, sF, sV, cnt, stride, fuse);
-    else if (W <= 16u) group_loop<8>(P, r0, r1, next, u0, us, crows, sfix, gm, Q, sF, sV, cnt, stride, fuse);
-    else group_loop<16>(P, r0, r1, next, u0, us, crows, sfix, gm, Q, sF, sV, cnt, stride, fuse);
+    if (W <= 8u) group_loop<4>(P, r0, r1, next, chunk, u0, us, crows, sfix, gm, Q, sF, sV, cnt, stride, fuse);
+    else if (W <= 16u) group_loop<8>(P, r0, r1, next, chunk, u0, us, crows, sfix, gm, Q, sF, sV, cnt, stride, fuse);
+    else if (W <= 32u) group_loop<16>(P, r0, r1, next, chunk, u0, us, crows, sfix, gm, Q, sF, sV, cnt, stride, fuse);
+    else group_loop<32>(P, r0, r1, next, chunk, u0, us, crows, sfix, gm, Q, sF, sV, cnt, stride, fuse);
 }
 
 // ---------------------------------------------------------------------------
@@ -1403,15 +1443,17 @@ __device__ __forceinline__ void classify_balanced(uint64_t h0, uint64_t h1, uint
     const uint32_t lane = threadIdx.x & 31u;
 #pragma unroll
     for (uint32_t k = 0; k < 4; ++k) SM[4u * lane + k] = 0u;
-    uint32_t q = off;
+    uint32_t* q = Q + off;
     const uint32_t hh[4] = {(uint32_t)h0, (uint32_t)(h0 >> 32), (uint32_t)h1, (uint32_t)(h1 >> 32)};
     const uint32_t bb[4] = {(uint32_t)b0, (uint32_t)(b0 >> 32), (uint32_t)b1, (uint32_t)(b1 >> 32)};
 #pragma unroll
     for (uint32_t k = 0; k < 4; ++k) {
-        const uint32_t base = w * 64u + 32u * k;
-        for (uint32_t x = hh[k]; x; x &= x - 1u) {
-            const uint32_t j = (uint32_t)(__ffs(x) - 1);
-            Q[q++] = (base + j) | (((bb[k] >> j) & 1u) << 31);
+        // lowest bit first: reversed once, then one leading-zero count per bit, the sign bit shifted into place by it
+        const uint32_t base = w * 64u + 32u * k, sign = __brev(bb[k]);
+        for (uint32_t x = __brev(hh[k]); x;) {
+            const uint32_t z = (uint32_t)__clz(x);
+            *q++ = (base + z) | ((sign << z) & 0x80000000u);
+            x ^= 0x80000000u >> z;
         }
     }
     __syncwarp();
@@ -1642,7 +1684,7 @@ k_generation(const __grid_constant__ PopDev one, const PopDev* __restrict__ pops
     uint32_t bphase = 0;  // parity of the warp's bulk-copy barrier
     const uint32_t* wait_limit = &ctl->wait_limit;  // read only when a copy is late
     if (SUF) {
-        if (!CM)
+        if (NARROW)
             for (uint32_t w = lane; w < maxW; w += 32u) mask[w] = 0ull;
         if (lane == 0) {
             mbar_init(&ws.mbar);
@@ -1692,20 +1734,25 @@ k_generation(const __grid_constant__ PopDev one, const PopDev* __restrict__ pops
         Fold fo{sF, sV, cur_cnt ? cplanes : nullptr, maxW};
         // the next claim is taken before the current rows run, so its
         // round trip to the counter is hidden behind them
+        constexpr uint32_t kChunkRows = SUF ? kWarpChunk : 2u;   // interval rows: 924 us with two, 959 with one, 940 with four
         uint32_t claim = 0;
         const bool group = SUF && NARROW && !PROF && max(st.W, st.pW) <= kGroupWords;
-        if (group) {   // rows that share a warp cost about the same: no claims
-            group_rows(pops[0], 0u, S, nullptr, warp * gridDim.x + blockIdx.x, gridDim.x * kWarps, cur_cnt ? &s_crows : nullptr,
-                       sfix, mask, ws.q, sF, sV, fo.cnt, maxW, fuse);
+        if (group) {
+            // copy rows cost about the same, so units in a fixed stride spare the claims (2e4 of them on one counter:
+            // 26.6 against 20.4 us); with a breakpoint on every eighth row or more, claims even the rows out
+            // (10,000 individuals at rho = 3: 37.4 against 43.5 us), a few units at a time where there are many
+            const uint32_t events = P.mode == kModePhilox ? st.ev_used : P.ev_off[S];
+            group_rows(pops[0], 0u, S, events > S / 8u ? &ctl->gen_counter : nullptr,
+                       max(1u, S / (gridDim.x * kWarps * 8u)), warp * gridDim.x + blockIdx.x, gridDim.x * kWarps, cur_cnt ? &s_crows : nullptr, sfix, mask, ws.q, sF, sV, fo.cnt, maxW, fuse);
             if (profile && blockIdx.x == 0 && threadIdx.x == 0) { rows_done = S; words_done = (uint64_t)S * st.W; }
         } else if (lane == 0) {
-            claim = atomicAdd(&ctl->gen_counter, kWarpChunk);
+            claim = atomicAdd(&ctl->gen_counter, kChunkRows);
         }
         for (; !group;) {
             const uint32_t k = __shfl_sync(0xffffffffu, claim, 0);
             if (k >= S) break;
-            if (lane == 0) claim = atomicAdd(&ctl->gen_counter, kWarpChunk);
-            const uint32_t k1 = min(S, k + kWarpChunk);
+            if (lane == 0) claim = atomicAdd(&ctl->gen_counter, kChunkRows);
+            const uint32_t k1 = min(S, k + kChunkRows);
             for (uint32_t v = k; v < k1; ++v) {
                 const uint32_t g = v < Se ? 2u * v : 2u * (v - Se) + 1u;
                 if (CNT && fo.cnt) {  // a block counts at most kCountMax rows (one flush, at the end)
@@ -1811,7 +1858,7 @@ k_generation(const __grid_constant__ PopDev one, const PopDev* __restrict__ pops
         uint32_t kc = 0;
         const bool group = SUF && NARROW && !PROF && max(st.W, st.pW) <= kGroupWords;
         if (group) {
-            group_rows(P, r0, r1, &s_next, 0u, 0u, nullptr, sfix, mask, ws.q, sF, sV, fo.cnt, maxW, fuse);
+            group_rows(P, r0, r1, &s_next, 1u, 0u, 0u, nullptr, sfix, mask, ws.q, sF, sV, fo.cnt, maxW, fuse);
             if (profile && threadIdx.x == 0) { rows_done += r1 - r0; words_done += (uint64_t)(r1 - r0) * st.W; }
         } else if (NARROW && lane == 0) {
             kc = atomicAdd(&s_next, 1u);

@@ -1,4 +1,4 @@
-"""Rows of at most 32 words share a warp (4, 8 or 16 lanes a row).  The form with one row a warp (narrow_build = 0)
+"""Rows of at most 64 words share a warp (4, 8, 16 or 32 lanes a row).  The form with one row a warp (narrow_build = 0)
 gives the same rows, phenotypes and fitness to the bit: rows that fill their lanes and rows that do not, parents
 narrower than their children, dense rows (more gathered alleles than a queue holds), breakpoint lists longer than
 the device draws, more new alleles a row than a warp has lanes."""
@@ -75,3 +75,9 @@ def test_short_rows_of_a_batch():
         b.close()
     for x, y in zip(*got):
         assert np.array_equal(x[0], y[0]) and np.array_equal(x[1], y[1]) and np.array_equal(x[2], y[2]) and x[3] == y[3]
+
+
+# 32 lanes a row: rows of 40 and 48 words and rows that grow from 56 words to 64
+@pytest.mark.parametrize("A0,T,dense,q1", [(2_049, 4, False, True), (3_000, 1, True, False), (3_300, 2, False, False)])
+def test_rows_of_33_to_64_words_change_nothing(A0, T, dense, q1):
+    test_short_rows_share_a_warp_and_change_nothing(A0, T, dense, q1)
