@@ -515,6 +515,14 @@ int require_ready(clotho_ctx* ctx) {
     return 0;
 }
 
+// None of the first n populations has a fitness metric (every fitness is 1).
+bool constant_fitness(const clotho_ctx* ctx, uint32_t n) {
+    for (uint32_t i = 0; i < n; ++i)
+        if (ctx->pops[i]->desc.fitness >= CLOTHO_FIT_GAUSSIAN && ctx->pops[i]->desc.fitness <= CLOTHO_FIT_GAUSSIAN_VS)
+            return false;
+    return true;
+}
+
 PrepSizes prep_sizes(const clotho_ctx* ctx) {
     return PrepSizes{ctx->maxS, ctx->maxN, ctx->maxNB, ctx->maxA, ctx->n_suf > 0};
 }
@@ -544,7 +552,7 @@ void enqueue_fused_step(clotho_ctx* ctx, uint32_t set, bool philox) {
     ctx->launches += launch_prep(L, pops, n, z, ctx->d_hdr[set], ctx->d_ctl, what, cnt);
     ctx->launches += launch_plan(L, pops, n, z, ctx->maxW_suf, what);
     launch_gen(ctx, L, pops, n, kFuseMut | kFusePheno | kFuseFs);
-    ctx->launches += launch_fitness(L, pops, n, ctx->maxN, true);
+    ctx->launches += launch_fitness(L, pops, n, ctx->maxN, constant_fitness(ctx, n), true);
     for (PopHost* p : ctx->pops) p->acc_valid = true;
 }
 
@@ -820,7 +828,7 @@ static int finish_start(clotho_ctx* ctx) {
     LaunchCfg L = cfg(ctx);
     launch_fs_reduce(L, ctx->d_pops[0], 1, ctx->maxW, 0u);
     launch_phenotype(L, ctx->d_pops[0], 1);
-    ctx->launches += 2 + launch_fitness(L, ctx->d_pops[0], 1, ctx->maxN, false);
+    ctx->launches += 2 + launch_fitness(L, ctx->d_pops[0], 1, ctx->maxN, constant_fitness(ctx, 1), false);
     int rc = check_launch(ctx, "start");
     if (rc) return rc;
     CK(cudaStreamSynchronize(ctx->stream));
@@ -1086,7 +1094,7 @@ int clotho_phenotype(clotho_ctx* ctx) {
 
 int clotho_fitness(clotho_ctx* ctx) {
     if (!ctx) return CLOTHO_E_ARG;
-    ctx->launches += launch_fitness(cfg(ctx), ctx->d_pops[0], 1, ctx->maxN, false);
+    ctx->launches += launch_fitness(cfg(ctx), ctx->d_pops[0], 1, ctx->maxN, constant_fitness(ctx, 1), false);
     return check_launch(ctx, "fitness");
 }
 

@@ -428,8 +428,9 @@ cudaError_t launch_generation(const LaunchCfg&, const PopDev* pops, uint32_t npo
 bool generation_counts_fit(uint32_t maxW, uint32_t maxA);
 void launch_mut_scatter(const LaunchCfg&, const PopDev* pops, uint32_t npops);
 void launch_phenotype(const LaunchCfg&, const PopDev* pops, uint32_t npops);
-// individual phenotypes, fitness and its prefix sum; end: and the step's end.  Returns the launches made.
-uint32_t launch_fitness(const LaunchCfg&, const PopDev* pops, uint32_t npops, uint32_t maxN, bool end);
+// individual phenotypes, fitness (constant: no population has a metric) and its prefix sum; end: and the step's end.
+// Returns the launches made.
+uint32_t launch_fitness(const LaunchCfg&, const PopDev* pops, uint32_t npops, uint32_t maxN, bool constant, bool end);
 void launch_end(const LaunchCfg&, const PopDev* pops, uint32_t npops);
 void launch_seed_rows(const LaunchCfg&, const PopDev* pops, uint32_t npops, const uint32_t* thr,
                       uint64_t seed, uint32_t A);

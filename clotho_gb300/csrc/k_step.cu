@@ -109,14 +109,16 @@ void launch_mut_scatter(const LaunchCfg& L, const PopDev* pops, uint32_t npops) 
 // Bound by the FP64 pipe (about two operations a clock and SM): the exponential and the sum's adds.  So every
 // warp of the GPU takes 128 individuals, and what is the same for all of them (the root, the quotients) is
 // computed once a block.
-template <bool ONE>
+//
+// CONSTANT (no population of the launch has a metric): every fitness is 1, so the prefix sum of individual i is i + 1
+// in any order of additions; it is written here and the step ends here, without k_cdf.
+template <bool ONE, bool CONSTANT>
 __global__ void __launch_bounds__(256) k_individuals(const __grid_constant__ PopDev one,
                                                      const PopDev* __restrict__ pops,
-                                                     const BlockPart* __restrict__ map) {
+                                                     const BlockPart* __restrict__ map, uint32_t end) {
     __shared__ double s_k[4];
     __shared__ double s_f[8][128];
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    pdl_wait();
     const BlockPart part = block_part<ONE>(map);
     const PopDev& P = ONE ? one : pops[part.pop];
     pdl_wait();
@@ -131,6 +133,13 @@ __global__ void __launch_bounds__(256) k_individuals(const __grid_constant__ Pop
         if (part.i == 0) {
             st->all_neutral = neutral ? 1u : 0u;
             st->fit_const = 1u;  // k_cdf clears it
+            if (CONSTANT) {
+                st->fit_total = (double)N;
+                if (end) {
+                    st->last_M = st->M;
+                    st->gen += 1u;
+                }
+            }
         }
         if (fitness == 1 || fitness == 2) {
             const double sig = sqrt(4.0 * (double)N * P.mu);  // normal/quadratic generators
@@ -167,7 +176,7 @@ __global__ void __launch_bounds__(256) k_individuals(const __grid_constant__ Pop
                 zi[1] = make_double2(z[2], z[3]);
                 f = 1.0;
                 const double z0 = z[0];
-                switch (fitness) {
+                if (!CONSTANT) switch (fitness) {
                     case 1:  // gaussian (normal_fitness_metric.cpp:25-31)
                         f = s_k[0] * exp(-(z0 * z0) / s_k[1]);
                         break;
@@ -183,9 +192,11 @@ __global__ void __launch_bounds__(256) k_individuals(const __grid_constant__ Pop
                     default: f = 1.0;
                 }
                 P.fit[i] = f;
+                if (CONSTANT) P.cdf[i] = (double)(i + 1u);
             }
             s_f[warp][32u * k + lane] = f;
         }
+        if (CONSTANT) continue;
         __syncwarp();
         const double* v = &s_f[warp][4u * lane];
         const double s = warp_incl_f64(((v[0] + v[1]) + v[2]) + v[3]);
@@ -241,7 +252,6 @@ __global__ void __launch_bounds__(256) k_cdf(const __grid_constant__ PopDev one,
     __shared__ double s_woff[32];
     __shared__ double s_part, s_last;
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    pdl_wait();
     const BlockPart part = block_part<ONE>(map);
     const PopDev& P = ONE ? one : pops[part.pop];
     pdl_wait();
@@ -310,12 +320,18 @@ __global__ void __launch_bounds__(256) k_cdf(const __grid_constant__ PopDev one,
         }
     }
 }
-uint32_t launch_fitness(const LaunchCfg& L, const PopDev* pops, uint32_t npops, uint32_t maxN, bool end) {
-    const uint32_t units = std::max(1u, (maxN + kScanChunk - 1u) / kScanChunk * 4u);
-    launch_pops(L, kTable256, k_individuals<true>, k_individuals<false>, blocks_of(L, units, L.ind_per_sm), pops, npops);
+uint32_t launch_fitness(const LaunchCfg& L, const PopDev* pops, uint32_t npops, uint32_t maxN, bool constant, bool end) {
+    const uint32_t units = std::max(1u, (maxN + kScanChunk - 1u) / kScanChunk * 4u), last = end ? 1u : 0u;
+    if (constant) {
+        launch_pops(L, kTable256, k_individuals<true, true>, k_individuals<false, true>, blocks_of(L, units, L.ind_per_sm),
+                    pops, npops, last);
+        return 1u;
+    }
+    launch_pops(L, kTable256, k_individuals<true, false>, k_individuals<false, false>, blocks_of(L, units, L.ind_per_sm),
+                pops, npops, 0u);
     const bool offsets = maxN > kInlineChunks * kScanChunk;
     if (offsets) launch_k(L, k_cdf_offsets, dim3(npops), dim3(256), pops);
-    launch_pops(L, kTable256, k_cdf<true>, k_cdf<false>, blocks_of(L, units, 8), pops, npops, end ? 1u : 0u);
+    launch_pops(L, kTable256, k_cdf<true>, k_cdf<false>, blocks_of(L, units, 8), pops, npops, last);
     return offsets ? 3u : 2u;
 }
 

@@ -140,6 +140,7 @@ __device__ inline uint64_t block_excl_scan_1024(uint64_t v, uint64_t* s_warp, ui
 __device__ inline void fs_finalize_block(const PopDev& P, uint32_t pN, uint32_t pA, uint32_t pW, bool count_on) {
     __shared__ uint64_t s_warp[32];
     __shared__ double s_fx[32][kMaxTraits];
+    __shared__ uint32_t s_any;   // warps that hold a fixed allele
     DevStatus* st = P.st;
     const uint32_t pS = 2u * pN;
     const uint32_t fx_base = st->fixed_total;
@@ -150,6 +151,7 @@ __device__ inline void fs_finalize_block(const PopDev& P, uint32_t pN, uint32_t 
         for (uint32_t a = threadIdx.x; a < P.Acap; a += 1024u) P.colcnt[a] = 0u;
     uint32_t totF = 0, totL = 0;
     double fsum[kMaxTraits] = {0.0, 0.0, 0.0, 0.0};
+    bool fixed_here = false;
     if (pA > 0) {
         if (pW > 1024u) {  // the lost list starts behind every fixed index
             uint32_t cf = 0;
@@ -172,6 +174,7 @@ __device__ inline void fs_finalize_block(const PopDev& P, uint32_t pN, uint32_t 
             if (pW <= 1024u) totF = (uint32_t)t;
             if (w < pW) {
                 uint32_t i = base_f + (uint32_t)o;
+                fixed_here |= F != 0ull;
                 for (uint64_t b = F; b; b &= b - 1ull) {
                     const uint32_t slot = w * 64u + (uint32_t)(__ffsll((long long)b) - 1);
                     P.free_list[i] = slot;
@@ -194,20 +197,22 @@ __device__ inline void fs_finalize_block(const PopDev& P, uint32_t pN, uint32_t 
     }
     // effect sum of the fixed alleles (every parent row carries them): the
     // generation pass subtracts it from the carried per-genome sums
-    if (totF) {
-#pragma unroll
-        for (uint32_t t = 0; t < kMaxTraits; ++t) {
-            double v = fsum[t];
+    if (threadIdx.x == 0) s_any = 0u;
+    __syncthreads();
+    if (totF && __any_sync(0xffffffffu, fixed_here)) {
+        for (uint32_t t = 0; t < P.T; ++t) {
+            double v = t == 0 ? fsum[0] : t == 1 ? fsum[1] : t == 2 ? fsum[2] : fsum[3];
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
             if ((threadIdx.x & 31u) == 0) s_fx[threadIdx.x >> 5][t] = v;
         }
-        __syncthreads();
+        if ((threadIdx.x & 31u) == 0) atomicOr(&s_any, 1u << (threadIdx.x >> 5));
     }
+    __syncthreads();
     if (threadIdx.x < kMaxTraits) {
         double v = 0.0;
-        if (totF)
-            for (int i = 0; i < 32; ++i) v += s_fx[i][threadIdx.x];
+        if (threadIdx.x < P.T)
+            for (uint32_t m = s_any; m; m &= m - 1u) v += s_fx[__ffs((int)m) - 1][threadIdx.x];
         st->fixsum[threadIdx.x] = v;
     }
     // reset the accumulators for the child of this step
