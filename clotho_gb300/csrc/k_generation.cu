@@ -1403,6 +1403,31 @@ __device__ __forceinline__ bool in_iv(uint32_t r, const RowXo& X) {
     return s;
 }
 
+// A round of the interval classifier, four heterozygous bits a lane, with the switched ones' effects in flight: folded
+// into the sums one round later, as an EffRound's (an entry that did not switch loads zeros).  Folded at once, the
+// kernel waited for L2 each round: 50,000 individuals of 464-word rows at rho = 5, 886 us against 836 (rounds of
+// three or two bits a lane 848, 900).
+constexpr uint32_t kIvLane = 4;
+struct IvRound {
+    float4 ef[kIvLane];
+    uint32_t sg;
+};
+__device__ __forceinline__ void iv_complete(const IvRound& r, float (&d)[kMaxTraits]) {
+#pragma unroll
+    for (uint32_t k = 0; k < kIvLane; ++k) {
+        const float g = ((r.sg >> k) & 1u) ? 1.0f : -1.0f;
+        d[0] = fmaf(g, r.ef[k].x, d[0]);
+        d[1] = fmaf(g, r.ef[k].y, d[1]);
+        d[2] = fmaf(g, r.ef[k].z, d[2]);
+        d[3] = fmaf(g, r.ef[k].w, d[3]);
+    }
+}
+__device__ __forceinline__ void iv_clear(IvRound& r) {
+    r.sg = 0u;
+#pragma unroll
+    for (uint32_t k = 0; k < kIvLane; ++k) r.ef[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+}
+
 // One branch-free step of a het-bit chain: classify the lowest bit of h.
 template <int NI>
 __device__ __forceinline__ void xo_step(uint32_t& h, uint32_t& m, uint32_t base, const uint32_t* __restrict__ grank,
@@ -1438,11 +1463,10 @@ template <int NI>
 __device__ __forceinline__ void classify_balanced(uint64_t h0, uint64_t h1, uint64_t b0, uint64_t b1, uint32_t w,
                                                   uint32_t w0, uint32_t off, uint32_t H, uint32_t* Q,
                                                   uint32_t* SM, const uint32_t* __restrict__ grank, const RowXo& X,
-                                                  const float4* __restrict__ eff4, bool gather,
+                                                  const float4* __restrict__ eff4, bool gather, IvRound& pend,
                                                   float (&d)[kMaxTraits], uint64_t& m0, uint64_t& m1) {
     const uint32_t lane = threadIdx.x & 31u;
-#pragma unroll
-    for (uint32_t k = 0; k < 4; ++k) SM[4u * lane + k] = 0u;
+    *reinterpret_cast<uint4*>(SM + 4u * lane) = make_uint4(0, 0, 0, 0);
     uint32_t* q = Q + off;
     const uint32_t hh[4] = {(uint32_t)h0, (uint32_t)(h0 >> 32), (uint32_t)h1, (uint32_t)(h1 >> 32)};
     const uint32_t bb[4] = {(uint32_t)b0, (uint32_t)(b0 >> 32), (uint32_t)b1, (uint32_t)(b1 >> 32)};
@@ -1458,41 +1482,37 @@ __device__ __forceinline__ void classify_balanced(uint64_t h0, uint64_t h1, uint
     }
     __syncwarp();
     const uint32_t sbase = w0 * 64u;
-    for (uint32_t ib = 0; ib < H; ib += 128u) {
-        uint32_t e[4];
-        bool sw[4];
+    for (uint32_t ib = 0; ib < H; ib += 32u * kIvLane) {
+        uint32_t e[kIvLane];
+        bool sw[kIvLane];
 #pragma unroll
-        for (uint32_t k = 0; k < 4; ++k) {
+        for (uint32_t k = 0; k < kIvLane; ++k) {
             const uint32_t i = ib + lane + 32u * k;
             e[k] = (i < H) ? Q[i] : 0u;
             const uint32_t r = __ldg(grank + (e[k] & 0x7fffffffu));
             sw[k] = (i < H) && in_iv<NI>(r, X);
         }
+        if (gather) {
+            iv_complete(pend, d);
+            pend.sg = 0u;
 #pragma unroll
-        for (uint32_t k = 0; k < 4; ++k) {
+            for (uint32_t k = 0; k < kIvLane; ++k) {
+                pend.sg |= (e[k] >> 31) << k;
+                pend.ef[k] = sw[k] ? __ldg(eff4 + (e[k] & 0x7fffffffu)) : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+        }
+#pragma unroll
+        for (uint32_t k = 0; k < kIvLane; ++k) {
             if (sw[k]) {
                 const uint32_t loc = (e[k] & 0x7fffffffu) - sbase;
                 atomicOr(&SM[loc >> 5], 1u << (loc & 31u));
             }
         }
-        if (gather) {
-            float4 ef[4];
-#pragma unroll
-            for (uint32_t k = 0; k < 4; ++k)
-                ef[k] = sw[k] ? __ldg(eff4 + (e[k] & 0x7fffffffu)) : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-            for (uint32_t k = 0; k < 4; ++k) {
-                const float g = sw[k] ? ((e[k] >> 31) ? 1.0f : -1.0f) : 0.0f;
-                d[0] = fmaf(g, ef[k].x, d[0]);
-                d[1] = fmaf(g, ef[k].y, d[1]);
-                d[2] = fmaf(g, ef[k].z, d[2]);
-                d[3] = fmaf(g, ef[k].w, d[3]);
-            }
-        }
     }
     __syncwarp();
-    m0 = (uint64_t)SM[4u * lane] | ((uint64_t)SM[4u * lane + 1u] << 32);
-    m1 = (uint64_t)SM[4u * lane + 2u] | ((uint64_t)SM[4u * lane + 3u] << 32);
+    const uint4 sm = *reinterpret_cast<const uint4*>(SM + 4u * lane);
+    m0 = (uint64_t)sm.x | ((uint64_t)sm.y << 32);
+    m1 = (uint64_t)sm.z | ((uint64_t)sm.w << 32);
     __syncwarp();
 }
 
@@ -1507,13 +1527,18 @@ __device__ __forceinline__ void row_body_iv(const PopDev& P, const DevStatus& st
     const uint32_t lane = threadIdx.x & 31u;
     constexpr bool xo = (KIND != kXoCopy);
     const float4* eff4 = reinterpret_cast<const float4*>(P.eff);
-    ulonglong2 t_a, b_a, t_b, b_b;
+    IvRound pend;
+    iv_clear(pend);
+    // parent words one chunk ahead, whole strands into L2 at row start (two chunks ahead without that: 875 us for the
+    // 836 above, the registers being the rounds')
+    prefetch_l2(R.top, R.Wp * 8u);
+    if (xo) prefetch_l2(R.bot, R.Wp * 8u);
+    ulonglong2 t_a, b_a;
     load_pair(t_a, b_a, R, 2u * lane, xo);
-    load_pair(t_b, b_b, R, 2u * lane + 64u, xo);
     for (uint32_t w0 = 0; w0 < R.Wc; w0 += 64u) {
         const uint32_t w = w0 + 2u * lane;
-        ulonglong2 t_c, b_c;
-        load_pair(t_c, b_c, R, w + 128u, xo);
+        ulonglong2 t_b, b_b;
+        load_pair(t_b, b_b, R, w + 64u, xo);
         uint64_t mx0 = 0, mx1 = 0;
         if (do_mut && R.mc) mutation_masks(P, st, R, w, mx0, mx1);
         const bool live = w < R.Wc;
@@ -1537,8 +1562,10 @@ __device__ __forceinline__ void row_body_iv(const PopDev& P, const DevStatus& st
                 const uint32_t H = __shfl_sync(0xffffffffu, incl, 31);
                 if (H <= kQueueCap) {
                     classify_balanced<(KIND > 0 ? KIND : 0)>(h0, h1, b0, b1, w, w0, incl - c, H, Q, SM, P.rank, X,
-                                                             eff4, gather, d, m0, m1);
+                                                             eff4, gather, pend, d, m0, m1);
                 } else {
+                    iv_complete(pend, d);
+                    iv_clear(pend);
                     classify<(KIND > 0 ? KIND : 0)>(h0, h1, w * 64u, P.rank, X, m0, m1);
                     if (gather) switched_effects(m0, m1, b0, b1, w * 64u, eff4, d);
                 }
@@ -1557,8 +1584,8 @@ __device__ __forceinline__ void row_body_iv(const PopDev& P, const DevStatus& st
             if (do_fs) fold(fo, w, x0, x1);
         }
         t_a = t_b; b_a = b_b;
-        t_b = t_c; b_b = b_c;
     }
+    if (xo && KIND != kXoEvents && gather) iv_complete(pend, d);
 }
 
 // One offspring row, the whole warp (interval classifier).
@@ -1662,7 +1689,7 @@ k_generation(const __grid_constant__ PopDev one, const PopDev* __restrict__ pops
     __shared__ uint2 s_iv[kIvWarps][kMaxIvSmem];
     __shared__ uint32_t s_thr[kIvWarps][kMaxEvDevice];
     __shared__ uint32_t s_q[kIvWarps][kQueueCap];
-    __shared__ uint32_t s_sm[kIvWarps][128];
+    __shared__ __align__(16) uint32_t s_sm[kIvWarps][128];
     __shared__ uint32_t s_item, s_next;
     __shared__ uint32_t s_crows;   // CNT, one population: rows the block has counted
     // the suffix-table builds keep their accumulators maxW words wide; the chunk-mask and interval builds
