@@ -17,17 +17,20 @@ namespace clotho {
 
 namespace {
 constexpr uint32_t kTM = 128, kTN = 256;        // pairs a CTA takes: rows i of the tile, rows j
-constexpr uint32_t kPairThreads = kTM + kTN;    // one expanded row a thread
+constexpr uint32_t kRowWarps = (kTM + kTN) / 32u;             // warps that expand rows, 32 each
+constexpr uint32_t kPairThreads = (kRowWarps + 1u) * 32u;     // and one that issues the multiplications
 constexpr uint32_t kRing = 4;                   // stages of 128 slots in shared memory
+constexpr uint32_t kRound = 8;                  // stages from one load of the rows: 128 bytes of each
 constexpr uint32_t kStageBytes = (kTM + kTN) * 128u;
 constexpr uint32_t kMaxSlots = 1u << 19;        // slots a CTA sums up: counts stay far below 2^24 units
-constexpr uint32_t kTileSums = kTM * kTN + kPairThreads;   // counts of a tile whose slots several CTAs share
+constexpr uint32_t kTileSums = kTM * kTN + kTM + kTN;   // counts of a tile whose slots several CTAs share
 constexpr uint32_t kPairWait = 1u << 20;        // try_wait rounds before a CTA gives up
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
-__device__ __forceinline__ bool wait_parity(uint32_t bar, uint32_t parity) {
-    for (uint32_t it = 0; it < kPairWait; ++it) {
+// false: given up, by this warp or (fail) by another one of the CTA
+__device__ __forceinline__ bool wait_parity(uint32_t bar, uint32_t parity, volatile uint32_t* fail) {
+    for (uint32_t it = 0; it < kPairWait && !*fail; ++it) {
         uint32_t ok;
         asm volatile(
             "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
@@ -36,7 +39,11 @@ __device__ __forceinline__ bool wait_parity(uint32_t bar, uint32_t parity) {
             : "memory");
         if (ok) return true;
     }
+    *fail = 1u;
     return false;
+}
+__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
 }
 
 // Shared-memory operand of K-major rows of 128 bytes in the 128-byte swizzle: groups of eight rows 1,024 bytes apart.
@@ -70,12 +77,14 @@ __device__ __forceinline__ void load_32_columns(uint32_t taddr, uint32_t (&v)[32
 }  // namespace
 
 // One CTA takes a 128 x 256 tile of the pair matrix (tiles with a pair i < j only) and a range of the slots.
-// Every thread expands one row, 128 slots a stage: bit k of each byte of a 32-bit word becomes a byte of 0 or 1
-// (two operations for four slots; the order of the slots is the same for all rows, which is all a sum needs) in the
+// A warp loads 128 bytes of each of its 32 rows, eight lanes a row, for eight stages; in a stage every lane turns 16
+// of a row's slots into 16 bytes of 0 or 1: bit k of each byte of a 32-bit word becomes a byte (two operations for
+// four slots; which slots make up a stage is the same for all rows, which is all a sum needs), in the
 // 128-byte swizzle that the tensor core reads.  A byte of 1 is the e4m3 value 2^-9, so products are 2^-18
-// and sums are whole multiples of it, exact in FP32.  One thread issues the four K = 32 steps of a stage; four stages
-// in flight let expansion and multiplication overlap.  Bound by shared-memory bandwidth: 48 KB written and
-// 48 KB read for a stage's 512 clocks of multiplication.
+// and sums are whole multiples of it, exact in FP32.  A warp of its own issues the four K = 32 steps of a stage when
+// the twelve others have arrived on its barrier; a stage is filled again when its multiplications have ended, so warps
+// run up to four stages apart (a block barrier a stage: 4,001 rows of 320 words 226 us, this 187).  Bound by
+// shared memory: 48 KB written and 48 KB read, 768 clocks, for a stage's 512 of multiplication; a stage takes 985.
 // splits > 1 (few tiles): the CTAs of a tile add their counts into tile_sum, the last one to come finishes the
 // tile; no CTA waits for another.  (popcount of 64 x 64 tiles: 1.1 ms for 4,001 rows of 320 words, the popcount
 // unit's 16 words a clock and SM.)
@@ -84,11 +93,11 @@ k_pairwise(const PopDev* __restrict__ pops, uint32_t p, const uint32_t* __restri
            uint32_t splits, uint32_t per, uint32_t* __restrict__ tile_sum,
            uint32_t* __restrict__ tile_done, uint32_t* __restrict__ dist, PairwiseOut* __restrict__ out) {
     extern __shared__ uint8_t s_raw[];
-    __shared__ __align__(8) unsigned long long s_bar[kRing + 1];
-    __shared__ uint32_t s_tmem, s_last;
-    __shared__ uint32_t s_ones[kPairThreads];
-    __shared__ unsigned long long s_sum[12], s_sq[12], s_cnt[12];
-    __shared__ uint32_t s_min[12], s_max[12];
+    __shared__ __align__(8) unsigned long long s_full[kRing], s_free[kRing], s_end;
+    __shared__ uint32_t s_tmem, s_last, s_fail, s_issued;
+    __shared__ uint32_t s_ones[kTM + kTN];
+    __shared__ unsigned long long s_sum[kRowWarps], s_sq[kRowWarps], s_cnt[kRowWarps];
+    __shared__ uint32_t s_min[kRowWarps], s_max[kRowWarps];
     const PopDev& P = pops[p];
     const uint64_t* rows = P.rows[P.st->cur];
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
@@ -101,10 +110,8 @@ k_pairwise(const PopDev* __restrict__ pops, uint32_t p, const uint32_t* __restri
         ++ti;
     }
     const uint32_t tj = ti * kTM / kTN + left;
-    const uint32_t nst = P.st->W / 2u, st0 = min(nst, split * per), cnt = min(nst, st0 + per) - st0;
-    const uint32_t row = tid < kTM ? ti * kTM + tid : tj * kTN + (tid - kTM);
-    const bool ok_row = row < n;
-    const uint4* src = ok_row ? reinterpret_cast<const uint4*>(rows + (size_t)sample[row] * P.Wcap) + st0 : nullptr;
+    const uint32_t quads = P.st->W / 2u;   // 16-byte pieces of a row
+    const uint32_t nr = (quads + kRound - 1u) / kRound, r0 = min(nr, split * per), cnt = min(nr, r0 + per) - r0;
     uint8_t* const ring = s_raw + ((1024u - (smem_addr(s_raw) & 1023u)) & 1023u);
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&s_tmem)),
@@ -113,8 +120,12 @@ k_pairwise(const PopDev* __restrict__ pops, uint32_t p, const uint32_t* __restri
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
     if (tid == 0) {
-        for (uint32_t i = 0; i <= kRing; ++i)
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&s_bar[i])) : "memory");
+        for (uint32_t i = 0; i < kRing; ++i) {
+            mbar_init(smem_addr(&s_full[i]), kRowWarps);
+            mbar_init(smem_addr(&s_free[i]), 1u);
+        }
+        mbar_init(smem_addr(&s_end), 1u);
+        s_fail = s_issued = 0u;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -124,56 +135,94 @@ k_pairwise(const PopDev* __restrict__ pops, uint32_t p, const uint32_t* __restri
     // e4m3 x e4m3 -> f32, K-major operands; columns up to the sample's end
     const uint32_t ncol = min(kTN, (n - tj * kTN + 15u) & ~15u);
     const uint32_t idesc = (1u << 4) | ((ncol >> 3) << 17) | ((kTM >> 4) << 24);
-    const uint4 zero = make_uint4(0, 0, 0, 0);
-    uint4 q0 = ok_row && cnt > 0 ? __ldg(src) : zero, q1 = ok_row && cnt > 1 ? __ldg(src + 1) : zero;
-    bool ok = true;
-    uint32_t issued = 0, ones = 0;   // the row's alleles in this CTA's slots
-    for (uint32_t it = 0; it < cnt; ++it) {
-        const uint32_t s = it % kRing;
-        const uint4 q = q0;
-        q0 = q1;
-        q1 = ok_row && it + 2u < cnt ? __ldg(src + it + 2u) : zero;
-        ones += (uint32_t)(__popc(q.x) + __popc(q.y) + __popc(q.z) + __popc(q.w));
-        if (it >= kRing) ok = wait_parity(smem_addr(&s_bar[s]), (it / kRing - 1u) & 1u);
-        if (ok && (ok_row || it < kRing)) {   // rows past the sample stay zero
-            uint8_t* dst = ring + s * kStageBytes + (tid < kTM ? tid : tid - kTM) * 128u + (tid < kTM ? 0u : kTM * 128u);
-            const uint32_t x[4] = {q.x, q.y, q.z, q.w};
+    if (warp < kRowWarps) {
+        // the thread's rows: warp's first + 4 j + lane / 8, of each the piece lane % 8 of a round
+        const uint32_t first = warp * 32u + (lane >> 3), piece = lane & 7u;
+        const ulonglong2* const base = reinterpret_cast<const ulonglong2*>(rows) + piece;
+        uint32_t at[8];   // row of the population; ~0 past the sample
 #pragma unroll
-            for (uint32_t c = 0; c < 8; ++c) {
-                const uint32_t v = x[c >> 1] >> (4u * (c & 1u));
-                const uint4 b = make_uint4(v & 0x01010101u, (v >> 1) & 0x01010101u, (v >> 2) & 0x01010101u,
-                                           (v >> 3) & 0x01010101u);
-                *reinterpret_cast<uint4*>(dst + ((c ^ (tid & 7u)) << 4)) = b;
+        for (uint32_t j = 0; j < 8; ++j) {
+            const uint32_t r = first + 4u * j, row = r < kTM ? ti * kTM + r : tj * kTN + (r - kTM);
+            at[j] = row < n ? sample[row] : ~0u;
+        }
+        auto load = [&](uint32_t r, ulonglong2 (&x)[8]) {
+            const uint32_t quad = r * kRound;
+#pragma unroll
+            for (uint32_t j = 0; j < 8; ++j)
+                x[j] = at[j] != ~0u && quad + piece < quads ? __ldg(base + (size_t)at[j] * (P.Wcap / 2u) + quad)
+                                                            : make_ulonglong2(0, 0);
+        };
+        ulonglong2 x[8], next[8];
+        if (cnt) load(r0, next);
+        bool ok = true;
+        uint32_t ones[8] = {0, 0, 0, 0, 0, 0, 0, 0};   // the rows' alleles in this lane's slots
+        for (uint32_t r = 0; r < cnt && ok; ++r) {
+#pragma unroll
+            for (uint32_t j = 0; j < 8; ++j) {
+                x[j] = next[j];
+                ones[j] += (uint32_t)(__popcll(x[j].x) + __popcll(x[j].y));
+            }
+            if (r + 1u < cnt) load(r0 + r + 1u, next);
+#pragma unroll
+            for (uint32_t t = 0; t < kRound; ++t) {
+                const uint32_t it = r * kRound + t, s = t % kRing;
+                if (it >= kRing) ok = wait_parity(smem_addr(&s_free[s]), (it / kRing - 1u) & 1u, &s_fail);
+                ok = __all_sync(0xffffffffu, ok);
+                if (!ok) break;
+                uint8_t* const dst = ring + s * kStageBytes + first * 128u;
+#pragma unroll
+                for (uint32_t j = 0; j < 8; ++j) {
+                    const uint64_t half = (t & 4u) ? x[j].y : x[j].x;
+                    const uint32_t v = (uint32_t)(half >> (32u * ((t >> 1) & 1u))) >> (4u * (t & 1u));
+                    const uint4 b = make_uint4(v & 0x01010101u, (v >> 1) & 0x01010101u, (v >> 2) & 0x01010101u,
+                                               (v >> 3) & 0x01010101u);
+                    if (at[j] != ~0u || it < kRing)   // rows past the sample stay zero
+                        *reinterpret_cast<uint4*>(dst + j * 512u + ((piece ^ ((first + 4u * j) & 7u)) << 4)) = b;
+                }
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                __syncwarp();
+                if (lane == 0)
+                    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(&s_full[s])) : "memory");
             }
         }
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        if (!__syncthreads_and(ok)) {
-            ok = false;
-            break;
+#pragma unroll
+        for (uint32_t j = 0; j < 8; ++j) {
+            uint32_t v = ones[j];
+            v += __shfl_xor_sync(0xffffffffu, v, 1);
+            v += __shfl_xor_sync(0xffffffffu, v, 2);
+            v += __shfl_xor_sync(0xffffffffu, v, 4);
+            if (piece == 0) s_ones[first + 4u * j] = v;
         }
-        if (tid == 0) {
+    } else if (lane == 0) {
+        uint32_t it = 0;
+        for (; it < cnt * kRound; ++it) {
+            const uint32_t s = it % kRing;
+            if (!wait_parity(smem_addr(&s_full[s]), (it / kRing) & 1u, &s_fail)) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t a = smem_addr(ring + s * kStageBytes), b = a + kTM * 128u;
 #pragma unroll
-            for (uint32_t k = 0; k < 4; ++k) mma_f8(tmem, operand(a + 32u * k), operand(b + 32u * k), idesc, (it | k) != 0u);
-            mma_commit(smem_addr(&s_bar[s]));
+            for (uint32_t k = 0; k < 4; ++k)
+                mma_f8(tmem, operand(a + 32u * k), operand(b + 32u * k), idesc, (it | k) != 0u);
+            mma_commit(smem_addr(&s_free[s]));
         }
-        issued = it + 1u;
+        s_issued = it;
+        if (it) mma_commit(smem_addr(&s_end));
     }
-    if (issued) {   // everything issued has ended, whether the loop ran through or not
-        if (tid == 0) mma_commit(smem_addr(&s_bar[kRing]));
-        ok = __syncthreads_and(wait_parity(smem_addr(&s_bar[kRing]), 0u)) && ok;
-    }
-    s_ones[tid] = ones;
     __syncthreads();
+    bool ok = !s_fail;
+    if (s_issued) {   // everything issued has ended, whether the loops ran through or not
+        uint32_t never = 0;
+        ok = __syncthreads_and(wait_parity(smem_addr(&s_end), 0u, &never)) && ok;
+    }
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    // TMEM lanes are the tile's rows: a warp reads the 32 of its place in its warpgroup, a third of the columns
+    // TMEM lanes are the tile's rows: a warp reads the 32 of its place in its warpgroup, a third of the columns (the
+    // issuing warp none)
     const uint32_t i_tile = (warp & 3u) * 32u + lane, i = ti * kTM + i_tile;
-    const uint32_t taddr = tmem + (((warp & 3u) * 32u) << 16);
+    const uint32_t taddr = tmem + (((warp & 3u) * 32u) << 16), col0 = warp < kRowWarps ? (warp >> 2) * 32u : ncol;
     uint32_t* const sums = tile_sum ? tile_sum + (size_t)tile * kTileSums : nullptr;   // [column][row], then the rows' alleles
     bool finish = ok;
     if (splits > 1u) {
-        for (uint32_t c0 = (warp >> 2) * 32u; c0 < ncol; c0 += 96u) {
+        for (uint32_t c0 = col0; c0 < ncol; c0 += 96u) {
             uint32_t v[32];
             load_32_columns(taddr + c0, v);
             if (ok && cnt)
@@ -183,20 +232,20 @@ k_pairwise(const PopDev* __restrict__ pops, uint32_t p, const uint32_t* __restri
                     if (x && c0 + k < ncol) atomicAdd(sums + (c0 + k) * kTM + i_tile, x);
                 }
         }
-        if (ones) atomicAdd(sums + kTM * kTN + tid, ones);
+        if (tid < kTM + kTN && s_ones[tid]) atomicAdd(sums + kTM * kTN + tid, s_ones[tid]);
         __threadfence();
         __syncthreads();
         if (tid == 0) s_last = atomicAdd(tile_done + tile, 1u) == splits - 1u;
         __syncthreads();
         finish = ok && s_last;
         __threadfence();
-        if (finish) s_ones[tid] = __ldcg(sums + kTM * kTN + tid);
+        if (finish && tid < kTM + kTN) s_ones[tid] = __ldcg(sums + kTM * kTN + tid);
         __syncthreads();
     }
     unsigned long long sum = 0, sq = 0, pairs = 0;
     uint32_t mn = 0xffffffffu, mx = 0;
     if (finish) {
-        for (uint32_t c0 = (warp >> 2) * 32u; c0 < ncol; c0 += 96u) {
+        for (uint32_t c0 = col0; c0 < ncol; c0 += 96u) {
             uint32_t v[32];
             if (splits > 1u) {
 #pragma unroll
@@ -230,7 +279,7 @@ k_pairwise(const PopDev* __restrict__ pops, uint32_t p, const uint32_t* __restri
     }
     mn = __reduce_min_sync(0xffffffffu, mn);
     mx = __reduce_max_sync(0xffffffffu, mx);
-    if (lane == 0) {
+    if (lane == 0 && warp < kRowWarps) {
         s_sum[warp] = sum;
         s_sq[warp] = sq;
         s_cnt[warp] = pairs;
@@ -242,7 +291,7 @@ k_pairwise(const PopDev* __restrict__ pops, uint32_t p, const uint32_t* __restri
     if (warp == 0)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTN) : "memory");
     if (tid == 0) {
-        for (uint32_t k = 1; k < kPairThreads / 32u; ++k) {
+        for (uint32_t k = 1; k < kRowWarps; ++k) {
             sum += s_sum[k];
             sq += s_sq[k];
             pairs += s_cnt[k];
@@ -262,22 +311,23 @@ k_pairwise(const PopDev* __restrict__ pops, uint32_t p, const uint32_t* __restri
 
 PairwisePlan pairwise_plan(const LaunchCfg& L, uint32_t n, uint32_t W) {
     PairwisePlan z{};
-    const uint32_t TI = (n + kTM - 1u) / kTM, TJ = (n + kTN - 1u) / kTN, nst = W / 2u;
+    const uint32_t TI = (n + kTM - 1u) / kTM, TJ = (n + kTN - 1u) / kTN, nr = (W / 2u + kRound - 1u) / kRound;
     for (uint32_t ti = 0; ti < TI; ++ti) z.tiles += TJ - ti * kTM / kTN;
     // Slots over several CTAs where the tiles alone leave SMs idle: the count with the least work on the busiest SM
-    // (rounds of tiles x splits over the SMs, each 1/splits of the slots plus about six stages' time to start and
-    // to add up), at least eight stages each, and as many as keep a CTA's sums in range
-    const uint32_t least = std::max(1u, (nst * 128u + kMaxSlots - 1u) / kMaxSlots);
+    // (tiles x splits over the SMs, each with its share of the rounds plus about six stages' time to start and
+    // to add up), and as many as keep a CTA's sums in range
+    const uint32_t least = std::max(1u, (nr * kRound * 128u + kMaxSlots - 1u) / kMaxSlots);
     double best = 1e30;
-    for (uint32_t s = least; s <= std::max(least, std::min(nst / 8u, 64u)); ++s) {
-        const double rounds = (double)((z.tiles * (uint64_t)s + L.num_sms - 1u) / L.num_sms);
-        const double cost = rounds * ((double)nst / s + 6.0 + (s > 1u ? 6.0 : 0.0));
+    z.splits = least;
+    for (uint32_t s = least; s <= std::max(least, std::min(nr, 64u)); ++s) {
+        const double waves = (double)((z.tiles * (uint64_t)s + L.num_sms - 1u) / L.num_sms);
+        const double cost = waves * ((double)((nr + s - 1u) / s * kRound) + 6.0 + (s > 1u ? 6.0 : 0.0));
         if (cost < best * 0.98) {
             best = cost;
             z.splits = s;
         }
     }
-    z.per = (nst + z.splits - 1u) / z.splits;
+    z.per = (nr + z.splits - 1u) / z.splits;
     z.sum_bytes = z.splits > 1u ? (size_t)z.tiles * (kTileSums + 1u) * 4 : 0;
     return z;
 }
