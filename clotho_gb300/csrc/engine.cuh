@@ -133,6 +133,8 @@ struct WorkCtl {
     uint32_t item_base[257];        // item prefix per population (<= 256 pops)
     uint32_t gen_counter_iv;        // item counter of the interval-classifier pass of a mixed batch
     uint32_t gen_counter_cm;        // item counter of the chunk-mask pass of a mixed batch
+    const uint32_t* sched;          // step headers of a size schedule
+    uint32_t sched_at;              // steps begun since the host set it
     uint64_t rows_done;             // profiling: rows processed
     uint64_t words_done;            // profiling: words written
     uint64_t phase[16];             // profiling: k_generation phase cycles (kPh*)
@@ -428,9 +430,17 @@ cudaError_t launch_generation(const LaunchCfg&, const PopDev* pops, uint32_t npo
 bool generation_counts_fit(uint32_t maxW, uint32_t maxA);
 void launch_mut_scatter(const LaunchCfg&, const PopDev* pops, uint32_t npops);
 void launch_phenotype(const LaunchCfg&, const PopDev* pops, uint32_t npops);
-// individual phenotypes, fitness (constant: no population has a metric) and its prefix sum; end: and the step's end.
+// How a step ends after the fitness: not here (a staged generation), with ++m_generation, or with that and the next
+// header of a schedule (2 * npops words a step) copied to where the next step reads it.
+struct StepEnd {
+    enum Mode : uint32_t { kNone = 0, kStep = 1, kSchedule = 2 };
+    uint32_t mode, npops;
+    uint32_t* hdr;
+    const WorkCtl* ctl;
+};
+// individual phenotypes, fitness (constant: no population has a metric) and its prefix sum, then the step's end.
 // Returns the launches made.
-uint32_t launch_fitness(const LaunchCfg&, const PopDev* pops, uint32_t npops, uint32_t maxN, bool constant, bool end);
+uint32_t launch_fitness(const LaunchCfg&, const PopDev* pops, uint32_t npops, uint32_t maxN, bool constant, StepEnd end);
 void launch_end(const LaunchCfg&, const PopDev* pops, uint32_t npops);
 void launch_seed_rows(const LaunchCfg&, const PopDev* pops, uint32_t npops, const uint32_t* thr,
                       uint64_t seed, uint32_t A);

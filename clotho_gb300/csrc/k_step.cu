@@ -112,10 +112,21 @@ void launch_mut_scatter(const LaunchCfg& L, const PopDev* pops, uint32_t npops) 
 //
 // CONSTANT (no population of the launch has a metric): every fitness is 1, so the prefix sum of individual i is i + 1
 // in any order of additions; it is written here and the step ends here, without k_cdf.
+__device__ __forceinline__ void end_step(const StepEnd& end, uint32_t pop, DevStatus* st) {
+    if (end.mode == StepEnd::kNone) return;
+    st->last_M = st->M;
+    st->gen += 1u;  // ++m_generation (engine_batched_task.hpp:222)
+    if (end.mode == StepEnd::kSchedule) {
+        const uint32_t* next = end.ctl->sched + (size_t)end.ctl->sched_at * 2u * end.npops + 2u * pop;
+        end.hdr[2u * pop] = next[0];
+        end.hdr[2u * pop + 1u] = next[1];
+    }
+}
+
 template <bool ONE, bool CONSTANT>
 __global__ void __launch_bounds__(256) k_individuals(const __grid_constant__ PopDev one,
                                                      const PopDev* __restrict__ pops,
-                                                     const BlockPart* __restrict__ map, uint32_t end) {
+                                                     const BlockPart* __restrict__ map, const StepEnd end) {
     __shared__ double s_k[4];
     __shared__ double s_f[8][128];
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
@@ -135,10 +146,7 @@ __global__ void __launch_bounds__(256) k_individuals(const __grid_constant__ Pop
             st->fit_const = 1u;  // k_cdf clears it
             if (CONSTANT) {
                 st->fit_total = (double)N;
-                if (end) {
-                    st->last_M = st->M;
-                    st->gen += 1u;
-                }
+                end_step(end, part.pop, st);
             }
         }
         if (fitness == 1 || fitness == 2) {
@@ -207,7 +215,7 @@ __global__ void __launch_bounds__(256) k_individuals(const __grid_constant__ Pop
 
 // Deterministic FP64 inclusive prefix sum of fitness with a fixed association order (four individuals a lane,
 // a shuffle scan over the warp, the 32 warps of a chunk and the chunks one after another), the total and the
-// all-equal check; end: the step's end (++m_generation, engine_batched_task.hpp:222).
+// all-equal check; then the step's end.
 constexpr uint32_t kInlineChunks = 64;   // up to here a block adds up the chunks before its own by itself
 
 __device__ __forceinline__ double chunk_total(const double* wsum, uint32_t c) {
@@ -247,7 +255,7 @@ __global__ void __launch_bounds__(256) k_cdf_offsets(const PopDev* __restrict__ 
 // A unit is 8 warps of 128 individuals: a quarter of a chunk.
 template <bool ONE>
 __global__ void __launch_bounds__(256) k_cdf(const __grid_constant__ PopDev one, const PopDev* __restrict__ pops,
-                                             const BlockPart* __restrict__ map, uint32_t end) {
+                                             const BlockPart* __restrict__ map, const StepEnd end) {
     __shared__ double s_tot[kInlineChunks];
     __shared__ double s_woff[32];
     __shared__ double s_part, s_last;
@@ -259,10 +267,7 @@ __global__ void __launch_bounds__(256) k_cdf(const __grid_constant__ PopDev one,
     const uint32_t N = st->N;
     const uint32_t nch = (N + kScanChunk - 1u) / kScanChunk;
     if (part.i == 0 && threadIdx.x == 0) {
-        if (end) {
-            st->last_M = st->M;
-            st->gen += 1u;
-        }
+        end_step(end, part.pop, st);
         if (N == 0) st->fit_total = 0.0;
     }
     const double f0 = N ? P.fit[0] : 0.0;
@@ -320,18 +325,18 @@ __global__ void __launch_bounds__(256) k_cdf(const __grid_constant__ PopDev one,
         }
     }
 }
-uint32_t launch_fitness(const LaunchCfg& L, const PopDev* pops, uint32_t npops, uint32_t maxN, bool constant, bool end) {
-    const uint32_t units = std::max(1u, (maxN + kScanChunk - 1u) / kScanChunk * 4u), last = end ? 1u : 0u;
+uint32_t launch_fitness(const LaunchCfg& L, const PopDev* pops, uint32_t npops, uint32_t maxN, bool constant, StepEnd end) {
+    const uint32_t units = std::max(1u, (maxN + kScanChunk - 1u) / kScanChunk * 4u);
     if (constant) {
         launch_pops(L, kTable256, k_individuals<true, true>, k_individuals<false, true>, blocks_of(L, units, L.ind_per_sm),
-                    pops, npops, last);
+                    pops, npops, end);
         return 1u;
     }
     launch_pops(L, kTable256, k_individuals<true, false>, k_individuals<false, false>, blocks_of(L, units, L.ind_per_sm),
-                pops, npops, 0u);
+                pops, npops, StepEnd{});
     const bool offsets = maxN > kInlineChunks * kScanChunk;
     if (offsets) launch_k(L, k_cdf_offsets, dim3(npops), dim3(256), pops);
-    launch_pops(L, kTable256, k_cdf<true>, k_cdf<false>, blocks_of(L, units, 8), pops, npops, last);
+    launch_pops(L, kTable256, k_cdf<true>, k_cdf<false>, blocks_of(L, units, 8), pops, npops, end);
     return offsets ? 3u : 2u;
 }
 

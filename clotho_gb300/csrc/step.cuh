@@ -14,6 +14,7 @@ __device__ inline void begin_items(const PopDev* pops, uint32_t npops, const uin
     __shared__ uint32_t s_items[kMaxPops / 32u];
     const uint32_t p = threadIdx.x, lane = p & 31u, warp = p >> 5;
     const uint32_t rpi = ctl->rows_per_item ? ctl->rows_per_item : kRowsPerItem;
+    if (p == 0) ctl->sched_at += 1u;
     const uint32_t n = p < npops ? (2u * min(hdr[2u * p], pops[p].Ncap) + rpi - 1u) / rpi : 0u;
     uint32_t incl = n;
 #pragma unroll
