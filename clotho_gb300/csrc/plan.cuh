@@ -35,6 +35,9 @@ __device__ __forceinline__ uint64_t pos_key(double x) {
     const uint64_t b = (uint64_t)__double_as_longlong(x);
     return b == 0x8000000000000000ull ? b : (b >> 63) ? ~b : b | 0x8000000000000000ull;
 }
+__device__ __forceinline__ double key_pos(uint64_t key) {   // both zeros: +0
+    return __longlong_as_double((long long)((key >> 63) ? key & 0x7fffffffffffffffull : ~key));
+}
 
 // Nearest suffix-table row b (a multiple of 64) of rank threshold r and the
 // ranks between them: [c0, c0 + n), n <= 32.
