@@ -8,7 +8,8 @@ Three knobs (clotho_set_tuning):
                      direct loads, every breakpoint's table words loaded at once)
                      may run when every row is at most 128 words;
   row_blocks_per_sm  blocks per SM of the per-individual kernels (parent
-                     sampling, phenotype and fitness).
+                     sampling, phenotype and fitness); a batch's kernels take
+                     half as many, dealt out by the populations' work.
 No knob changes a result (every kernel is deterministic in every shape), so the
 tuning runs on the live batch: a coordinate search times a few generations per
 candidate, one knob at a time with the others at their best so far, and keeps

@@ -44,8 +44,9 @@
 // is prefetched into L2 at row start.  Effects of switched alleles are gathered
 // from a per-warp queue, kRoundLane entries per lane a round, so lanes stay
 // balanced.  The kernel is persistent, one CTA per SM: with one population each
-// warp claims rows one at a time from a device counter; a batch hands each CTA
-// items of rows, which its warps claim one at a time.
+// warp claims rows one at a time from a device counter (short rows in units, by
+// a stride or a few units a claim); a batch hands each CTA items of rows, which
+// its warps claim one at a time.
 #include "plan.cuh"
 
 #include <algorithm>
@@ -864,7 +865,7 @@ struct PhaseClk {
 };
 
 // One offspring row, the whole warp (suffix-table classifier), from the plan
-// at processing position v (k_row_plan): row, top strand, breakpoints, table
+// at processing position v (k_plan): row, top strand, breakpoints, table
 // rows and correction ranks.  PROF: clock the row's phases into pc.
 // Returns false when the row's bulk copy was abandoned (the warp then stops working on rows).
 template <bool PROF, bool NARROW, bool CM = false>
