@@ -123,6 +123,7 @@ struct clotho_ctx {
     uint32_t set = 0;                                    // next tape set
     uint32_t pairs_set = 0;                              // the set whose pairs the last generation used
     cudaEvent_t copy_done[2]{}, kern_done[2]{};
+    bool drawn = false;   // device-drawn steps, which share set 0's buffers, enqueued since kern_done[0] was recorded
     std::string err;
     bool profiling = false;
     bool phase_clocks = false;      // profiling with the phase-clock build of k_generation
@@ -556,6 +557,7 @@ void enqueue_fused_step(clotho_ctx* ctx, uint32_t set, bool philox, StepEnd::Mod
     const PopDev* pops = ctx->d_pops[set];
     const LaunchCfg L = cfg(ctx, set);
     ctx->pairs_set = set == 1u ? 1u : 0u;  // the device-drawn set (2) shares set 0's buffers
+    ctx->drawn |= philox;
     ensure_parent_acc(ctx, pops, n);
     const PrepSizes z = prep_sizes(ctx);
     const bool cnt = count_on(ctx, kFuseMut | kFusePheno | kFuseFs);
@@ -633,6 +635,7 @@ int replay_generations(clotho_ctx* ctx, std::vector<uint32_t> key, uint32_t coun
     if (!ctx->graph_long && ctx->replayed >= kLongAfter && count >= kLongGraph)
         if (int rc = capture_generations(ctx, kLongGraph, end, &ctx->graph_long)) return rc;
     ctx->pairs_set = 0u;
+    ctx->drawn = true;
     while (count) {
         const bool many = ctx->graph_long && count >= kLongGraph;
         CK(cudaGraphLaunch(many ? ctx->graph_long : ctx->graph, ctx->stream));
@@ -959,7 +962,8 @@ int clotho_generation_tape(clotho_ctx* ctx, const clotho_gen_tape* tape) {
         launch_tape_upload(cfg(ctx, s), z, ctx->d_hdr[s]);
         ctx->launches += 1;
     } else {
-        // the tape set s was last read by the kernels of two steps ago
+        // the tape set s was last read by the kernels of two steps ago, set 0 by any device-drawn steps since
+        if (s == 0u && ctx->drawn) CK(cudaEventRecord(ctx->kern_done[0], ctx->stream));
         CK(cudaStreamWaitEvent(ctx->copy_stream, ctx->kern_done[s], 0));
         for (const TapeArray& a : arr)
             if (a.bytes) CK(cudaMemcpyAsync(a.dst, a.src, a.bytes, cudaMemcpyHostToDevice, ctx->copy_stream));
@@ -975,6 +979,7 @@ int clotho_generation_tape(clotho_ctx* ctx, const clotho_gen_tape* tape) {
     enqueue_fused_step(ctx, s, false);
     if ((rc = check_launch(ctx, "generation_tape"))) return rc;
     CK(cudaEventRecord(ctx->kern_done[s], ctx->stream));
+    if (s == 0u) ctx->drawn = false;
     // the caller's host arrays are free once the copies are done
     if (!staged) CK(cudaEventSynchronize(ctx->copy_done[s]));
     ctx->set ^= 1u;
