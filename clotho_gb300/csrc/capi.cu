@@ -520,6 +520,12 @@ int tape_arrays(clotho_ctx* ctx, PopHost* p, uint32_t s, const clotho_gen_tape* 
 // own copying (15 GB/s) takes longer than the copies' calls.
 constexpr size_t kTapeStage = 1u << 20;
 
+// Calls that work on the first population, or on all as if there were at least one.
+int require_pop(clotho_ctx* ctx) {
+    if (!ctx) return CLOTHO_E_ARG;
+    return ctx->pops.empty() ? fail(ctx, CLOTHO_E_ARG, "the context has no population") : 0;
+}
+
 int require_ready(clotho_ctx* ctx) {
     if (!ctx) return CLOTHO_E_ARG;
     for (PopHost* p : ctx->pops)
@@ -847,11 +853,12 @@ int clotho_init(clotho_ctx* ctx, uint32_t N0) { return init_pop(ctx, 0, N0); }
 // Shared set-up of an explicit or seeded start: status, allele tables, then
 // (after the caller fills the rows) reduction, phenotype and fitness.
 static int start_population(clotho_ctx* ctx, uint32_t N, uint32_t A, const double* pos, const float* eff) {
+    int rc = require_pop(ctx);
+    if (rc) return rc;
     PopHost* p = ctx->pops[0];
     const PopDev& D = p->dev[0];
     if (A > D.Acap || ref_width(A) > D.Wcap) return fail(ctx, CLOTHO_E_CAPACITY, "A exceeds max_alleles");
-    int rc = clotho_init(ctx, N);
-    if (rc) return rc;
+    if ((rc = clotho_init(ctx, N))) return rc;
     const uint32_t T = D.T;
     int32_t nz = 0;
     for (size_t i = 0; i < (size_t)A * T; ++i) nz += (eff[i] != 0.0f);
@@ -990,6 +997,7 @@ int clotho_generation_tape(clotho_ctx* ctx, const clotho_gen_tape* tape) {
 int clotho_generation_philox(clotho_ctx* ctx, uint32_t N) {
     int rc = require_ready(ctx);
     if (rc) return rc;
+    if ((rc = require_pop(ctx))) return rc;
     if ((rc = block_tables(ctx))) return rc;
     if (ctx->in_step) return fail(ctx, CLOTHO_E_STATE, "a staged generation is in progress");
     for (size_t i = 0; i < ctx->pops.size(); ++i)
@@ -1006,6 +1014,7 @@ int clotho_run_philox(clotho_ctx* ctx, uint32_t N, uint32_t G) {
     if (rc) return rc;
     if (ctx->in_step) return fail(ctx, CLOTHO_E_STATE, "a staged generation is in progress");
     if (G == 0) return 0;
+    if ((rc = require_pop(ctx))) return rc;
     for (const PopHost* p : ctx->pops)
         if (N > p->dev[2].Ncap) return fail(ctx, CLOTHO_E_CAPACITY, "N exceeds max_individuals");
     const std::vector<uint32_t> key(ctx->pops.size(), N);
@@ -1030,6 +1039,7 @@ int clotho_run_philox(clotho_ctx* ctx, uint32_t N, uint32_t G) {
 int clotho_begin_generation(clotho_ctx* ctx, uint32_t N, uint32_t M) {
     int rc = require_ready(ctx);
     if (rc) return rc;
+    if ((rc = require_pop(ctx))) return rc;
     if (ctx->in_step) return fail(ctx, CLOTHO_E_STATE, "generation already begun");
     PopHost* p = ctx->pops[0];
     if (N > p->dev[0].Ncap) return fail(ctx, CLOTHO_E_CAPACITY, "N exceeds max_individuals");
@@ -1138,14 +1148,14 @@ int clotho_mutate(clotho_ctx* ctx, const uint32_t* mut_seq, const double* mut_po
 }
 
 int clotho_phenotype(clotho_ctx* ctx) {
-    if (!ctx) return CLOTHO_E_ARG;
+    if (int rc = require_pop(ctx)) return rc;
     launch_phenotype(cfg(ctx), ctx->d_pops[0], 1);
     ctx->launches += 1;
     return check_launch(ctx, "phenotype");
 }
 
 int clotho_fitness(clotho_ctx* ctx) {
-    if (!ctx) return CLOTHO_E_ARG;
+    if (int rc = require_pop(ctx)) return rc;
     ctx->launches += launch_fitness(cfg(ctx), ctx->d_pops[0], 1, ctx->maxN, constant_fitness(ctx, 1), StepEnd{});
     return check_launch(ctx, "fitness");
 }
@@ -1261,8 +1271,8 @@ static int rows_of(clotho_ctx* ctx, uint32_t idx, uint64_t* dst, size_t dst_word
 int clotho_get_rows(clotho_ctx* ctx, uint64_t* dst, size_t dst_words) { return rows_of(ctx, 0, dst, dst_words); }
 
 int clotho_get_alleles(clotho_ctx* ctx, double* pos, uint32_t* age, float* eff) {
-    if (!ctx) return CLOTHO_E_ARG;
-    int rc;
+    int rc = require_pop(ctx);
+    if (rc) return rc;
     PopHost* p = ctx->pops[0];
     DevStatus s = read_status(ctx, p, &rc);
     if (rc) return rc;
@@ -1279,8 +1289,8 @@ int clotho_get_alleles(clotho_ctx* ctx, double* pos, uint32_t* age, float* eff) 
 }
 
 int clotho_get_fixed(clotho_ctx* ctx, double* pos, uint32_t* age, float* eff) {
-    if (!ctx) return CLOTHO_E_ARG;
-    int rc;
+    int rc = require_pop(ctx);
+    if (rc) return rc;
     PopHost* p = ctx->pops[0];
     DevStatus s = read_status(ctx, p, &rc);
     if (rc) return rc;
@@ -1294,8 +1304,8 @@ int clotho_get_fixed(clotho_ctx* ctx, double* pos, uint32_t* age, float* eff) {
 }
 
 int clotho_get_free(clotho_ctx* ctx, uint32_t* dst) {
-    if (!ctx) return CLOTHO_E_ARG;
-    int rc;
+    int rc = require_pop(ctx);
+    if (rc) return rc;
     PopHost* p = ctx->pops[0];
     DevStatus s = read_status(ctx, p, &rc);
     if (rc) return rc;
@@ -1332,8 +1342,8 @@ static int get_double4(clotho_ctx* ctx, const double* src, size_t n, double* dst
 }
 
 int clotho_get_genome_traits(clotho_ctx* ctx, double* dst) {
-    if (!ctx) return CLOTHO_E_ARG;
-    int rc;
+    int rc = require_pop(ctx);
+    if (rc) return rc;
     DevStatus s = read_status(ctx, ctx->pops[0], &rc);
     if (rc) return rc;
     return get_double4(ctx, ctx->pops[0]->dev[0].zg[s.cur], 2ull * s.N, dst);
@@ -1341,12 +1351,12 @@ int clotho_get_genome_traits(clotho_ctx* ctx, double* dst) {
 
 // The current size is the host's own view: every call that changes it brings it along.
 int clotho_get_phenotypes(clotho_ctx* ctx, double* dst) {
-    if (!ctx) return CLOTHO_E_ARG;
+    if (int rc = require_pop(ctx)) return rc;
     return get_double4(ctx, ctx->pops[0]->dev[0].zi, ctx->pops[0]->hostN, dst);
 }
 
 int clotho_get_fitness(clotho_ctx* ctx, double* dst) {
-    if (!ctx) return CLOTHO_E_ARG;
+    if (int rc = require_pop(ctx)) return rc;
     const PopHost* p = ctx->pops[0];
     host_pages(dst, (size_t)p->hostN * 8);
     if (p->hostN) CK(cudaMemcpyAsync(dst, p->dev[0].fit, (size_t)p->hostN * 8, cudaMemcpyDeviceToHost, ctx->stream));
@@ -1355,8 +1365,8 @@ int clotho_get_fitness(clotho_ctx* ctx, double* dst) {
 }
 
 int clotho_get_pairs(clotho_ctx* ctx, uint32_t* dst) {
-    if (!ctx) return CLOTHO_E_ARG;
-    int rc;
+    int rc = require_pop(ctx);
+    if (rc) return rc;
     DevStatus s = read_status(ctx, ctx->pops[0], &rc);
     if (rc) return rc;
     // tape steps alternate between sets 0 and 1; device draws and the staged calls use set 0's buffer

@@ -360,6 +360,7 @@ inline cudaError_t launch_k(const LaunchCfg& L, void (*k)(P...), dim3 grid, dim3
 template <class K, class... A>
 inline cudaError_t launch_pops_smem(const LaunchCfg& L, BlockTable table, K one, K all, uint32_t grid, size_t smem,
                                     const PopDev* pops, uint32_t npops, A... a) {
+    if (npops == 0u) return cudaErrorInvalidValue;   // the tables may hold an earlier batch's blocks
     const bool single = npops == 1u;
     const K k = single ? one : all;
     if (smem > 48u * 1024u) {  // a property of the function on the current device; setting it again is harmless

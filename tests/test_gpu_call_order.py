@@ -42,3 +42,36 @@ def test_queued_calls_do_not_disturb_each_other(order):
             got.append([pop.rows(), pop.genome_traits(), pop.pairs()])
     for a, b in zip(*got):
         assert a.shape == b.shape and a.tobytes() == b.tobytes()
+
+
+@pytest.mark.parametrize("before", [0, 1, 3])
+def test_calls_on_a_context_without_populations_are_refused(before):
+    import ctypes as C
+
+    import clotho_gb300 as cg
+    desc = [cg.make_desc(500, 2_000, 2, mu=0.01, rho=0.4, p_neutral=0.3, seed=i + 1) for i in range(3)]
+    b, fresh = cg.Batch(desc[:before]), cg.Batch(desc[:2])
+    b.init()
+    b.run(5)
+    while len(b):
+        b.remove(0)
+    L, h, launches = b.L, b.h, b.launches
+    buf = np.zeros(10_000, np.float64)
+    p, n0 = buf.ctypes.data_as(C.c_void_p), C.c_uint32(0)
+    for rc in (L.clotho_generation_philox(h, 500), L.clotho_run_philox(h, 500, 3), L.clotho_begin_generation(h, 500, 0),
+               L.clotho_phenotype(h), L.clotho_fitness(h), L.clotho_get_phenotypes(h, p), L.clotho_get_fitness(h, p),
+               L.clotho_get_genome_traits(h, p), L.clotho_get_pairs(h, p), L.clotho_get_free(h, p),
+               L.clotho_get_alleles(h, p, None, None), L.clotho_get_fixed(h, p, None, None),
+               L.clotho_seed_population(h, 10, 0, None, None, None, 1)):
+        assert rc != 0
+    assert L.clotho_batch_run_philox(h, C.byref(n0), 3) == 0 and L.clotho_run_philox(h, 500, 0) == 0
+    assert b.launches == launches and not buf.any()
+    for d in desc[:2]:
+        b.add(d, 500)
+    fresh.init()
+    for x in (b, fresh):
+        x.run(4)
+    for i in range(2):
+        assert b.rows(i).tobytes() == fresh.rows(i).tobytes() and b.info(i) == fresh.info(i)
+    b.close()
+    fresh.close()
