@@ -164,11 +164,15 @@ int fail(clotho_ctx* c, int code, const std::string& m) {
     return code;
 }
 
-#define CK(call)                                                                    \
-    do {                                                                            \
-        cudaError_t e_ = (call);                                                    \
-        if (e_ != cudaSuccess)                                                      \
-            return fail(ctx, CLOTHO_E_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_)); \
+// The runtime's record of the error goes with its report: left there, the next call that checks its launches would
+// report it again.
+#define CK(call)                                                                                      \
+    do {                                                                                              \
+        cudaError_t e_ = (call);                                                                      \
+        if (e_ != cudaSuccess) {                                                                      \
+            cudaGetLastError();                                                                       \
+            return fail(ctx, CLOTHO_E_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_));      \
+        }                                                                                             \
     } while (0)
 
 // set: the descriptors that the launch takes (tape set 0 or 1, or 2 for device draws)

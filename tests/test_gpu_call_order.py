@@ -75,3 +75,17 @@ def test_calls_on_a_context_without_populations_are_refused(before):
         assert b.rows(i).tobytes() == fresh.rows(i).tobytes() and b.info(i) == fresh.info(i)
     b.close()
     fresh.close()
+
+
+def test_a_refused_call_is_reported_once():
+    # the graph calls cannot capture on the legacy default stream
+    import clotho_gb300 as cg
+    with cg.Population(200, 2_000, 1, mu=0.02, rho=0.4, p_neutral=0.0, fitness="gaussian", seed=5) as pop:
+        pop.init(120)
+        for after in (pop.phenotypes, pop.margins, lambda: pop.simulate_philox(100)):
+            pop.set_stream(1)
+            with pytest.raises(cg.ClothoError, match="rc="):
+                pop.run_philox(110, 3)
+            pop.set_stream(None)
+            after()
+        pop.check()
