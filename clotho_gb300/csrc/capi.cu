@@ -28,7 +28,8 @@ struct PopHost {
     size_t bytes = 0;
     bool acc_valid = false;   // accF/accV hold AND/OR of the current child rows
     bool ready = false;       // init/seed done
-    uint32_t hostN = 0;       // host view of N after the last completed call
+    uint32_t hostN = 0;       // host view of N, while n_known
+    bool n_known = false;     // false from a step's enqueuing to its call's success: a call that fails leaves the size open
 };
 
 struct Geometry {
@@ -306,6 +307,18 @@ int alloc_pop(clotho_ctx* ctx, const clotho_desc& d, PopHost** out) {
     return 0;
 }
 
+// Steps were enqueued, and a call has succeeded: N(i) individuals in population i.
+void sizes_open(clotho_ctx* ctx) {
+    for (PopHost* p : ctx->pops) p->n_known = false;
+}
+template <class F>
+void sizes_are(clotho_ctx* ctx, F N) {
+    for (size_t i = 0; i < ctx->pops.size(); ++i) {
+        ctx->pops[i]->hostN = N(i);
+        ctx->pops[i]->n_known = true;
+    }
+}
+
 void drop_graphs(clotho_ctx* ctx) {
     for (cudaGraphExec_t* g : {&ctx->graph, &ctx->graph_long}) {
         if (*g) cudaGraphExecDestroy(*g);
@@ -399,6 +412,17 @@ DevStatus read_status(clotho_ctx* ctx, PopHost* p, int* rc) {
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     *rc = (e == cudaSuccess) ? 0 : fail(ctx, CLOTHO_E_CUDA, std::string("status read: ") + cudaGetErrorString(e));
     return s;
+}
+
+// The population's current size: the host's own view, or after a failed call the device's.
+uint32_t current_N(clotho_ctx* ctx, PopHost* p, int* rc) {
+    *rc = 0;
+    if (!p->n_known) {
+        const uint32_t N = read_status(ctx, p, rc).N;
+        if (*rc == 0) p->hostN = N;
+        p->n_known = *rc == 0;
+    }
+    return p->hostN;
 }
 
 // Backs a caller's buffer with memory before the device writes to it.  On a machine whose GPU walks the host's page
@@ -568,6 +592,7 @@ void enqueue_fused_step(clotho_ctx* ctx, uint32_t set, bool philox, StepEnd::Mod
     const LaunchCfg L = cfg(ctx, set);
     ctx->pairs_set = set == 1u ? 1u : 0u;  // the device-drawn set (2) shares set 0's buffers
     ctx->drawn |= philox;
+    sizes_open(ctx);
     ensure_parent_acc(ctx, pops, n);
     const PrepSizes z = prep_sizes(ctx);
     const bool cnt = count_on(ctx, kFuseMut | kFusePheno | kFuseFs);
@@ -646,6 +671,7 @@ int replay_generations(clotho_ctx* ctx, std::vector<uint32_t> key, uint32_t coun
         if (int rc = capture_generations(ctx, kLongGraph, end, &ctx->graph_long)) return rc;
     ctx->pairs_set = 0u;
     ctx->drawn = true;
+    sizes_open(ctx);
     while (count) {
         const bool many = ctx->graph_long && count >= kLongGraph;
         CK(cudaGraphLaunch(many ? ctx->graph_long : ctx->graph, ctx->stream));
@@ -823,6 +849,7 @@ static int init_pop(clotho_ctx* ctx, uint32_t idx, uint32_t N0) {
     const PopDev& D = p->dev[0];
     if (N0 > D.Ncap) return fail(ctx, CLOTHO_E_CAPACITY, "N0 exceeds max_individuals");
     CK(cudaStreamSynchronize(ctx->stream));
+    p->n_known = false;
     DevStatus s{};
     s.gen = 1;
     s.cur = 0;
@@ -849,6 +876,7 @@ static int init_pop(clotho_ctx* ctx, uint32_t idx, uint32_t N0) {
     p->acc_valid = true;  // A == 0: the first analysis is skipped (free_space_mt...:46)
     p->ready = true;
     p->hostN = N0;
+    p->n_known = true;
     return 0;
 }
 
@@ -994,7 +1022,7 @@ int clotho_generation_tape(clotho_ctx* ctx, const clotho_gen_tape* tape) {
     // the caller's host arrays are free once the copies are done
     if (!staged) CK(cudaEventSynchronize(ctx->copy_done[s]));
     ctx->set ^= 1u;
-    ctx->pops[0]->hostN = tape->N;
+    sizes_are(ctx, [tape](size_t) { return tape->N; });
     return 0;
 }
 
@@ -1009,7 +1037,7 @@ int clotho_generation_philox(clotho_ctx* ctx, uint32_t N) {
     if ((rc = put_header(ctx, [N](size_t) { return N; }))) return rc;
     enqueue_fused_step(ctx, 2, true);
     if ((rc = check_launch(ctx, "generation_philox"))) return rc;
-    for (PopHost* p : ctx->pops) p->hostN = N;
+    sizes_are(ctx, [N](size_t) { return N; });
     return 0;
 }
 
@@ -1025,7 +1053,6 @@ int clotho_run_philox(clotho_ctx* ctx, uint32_t N, uint32_t G) {
     uint32_t left = G;
     if (!ctx->profiling && graph_ready(ctx, key)) {
         if ((rc = put_header(ctx, [N](size_t) { return N; }))) return rc;
-        for (PopHost* p : ctx->pops) p->hostN = N;
     } else {
         // the first generation runs eagerly (it may need the parent reduction)
         if ((rc = clotho_generation_philox(ctx, N))) return rc;
@@ -1036,7 +1063,9 @@ int clotho_run_philox(clotho_ctx* ctx, uint32_t N, uint32_t G) {
             if ((rc = clotho_generation_philox(ctx, N))) return rc;
         return 0;
     }
-    return left ? replay_generations(ctx, key, left, StepEnd::kStep) : 0;
+    if (left && (rc = replay_generations(ctx, key, left, StepEnd::kStep))) return rc;
+    sizes_are(ctx, [N](size_t) { return N; });
+    return 0;
 }
 
 // ---- staged entry points -------------------------------------------------
@@ -1059,7 +1088,9 @@ int clotho_begin_generation(clotho_ctx* ctx, uint32_t N, uint32_t M) {
     ctx->launches += 1;
     ctx->in_step = true;
     p->hostN = N;
-    return check_launch(ctx, "begin");
+    rc = check_launch(ctx, "begin");
+    p->n_known = rc == 0;
+    return rc;
 }
 
 int clotho_free_space(clotho_ctx* ctx, uint32_t* counts) {
@@ -1353,17 +1384,20 @@ int clotho_get_genome_traits(clotho_ctx* ctx, double* dst) {
     return get_double4(ctx, ctx->pops[0]->dev[0].zg[s.cur], 2ull * s.N, dst);
 }
 
-// The current size is the host's own view: every call that changes it brings it along.
 int clotho_get_phenotypes(clotho_ctx* ctx, double* dst) {
     if (int rc = require_pop(ctx)) return rc;
-    return get_double4(ctx, ctx->pops[0]->dev[0].zi, ctx->pops[0]->hostN, dst);
+    int rc;
+    const uint32_t N = current_N(ctx, ctx->pops[0], &rc);
+    return rc ? rc : get_double4(ctx, ctx->pops[0]->dev[0].zi, N, dst);
 }
 
 int clotho_get_fitness(clotho_ctx* ctx, double* dst) {
     if (int rc = require_pop(ctx)) return rc;
-    const PopHost* p = ctx->pops[0];
-    host_pages(dst, (size_t)p->hostN * 8);
-    if (p->hostN) CK(cudaMemcpyAsync(dst, p->dev[0].fit, (size_t)p->hostN * 8, cudaMemcpyDeviceToHost, ctx->stream));
+    int rc;
+    const size_t N = current_N(ctx, ctx->pops[0], &rc);
+    if (rc) return rc;
+    host_pages(dst, N * 8);
+    if (N) CK(cudaMemcpyAsync(dst, ctx->pops[0]->dev[0].fit, N * 8, cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
     return 0;
 }
@@ -1723,7 +1757,6 @@ int clotho_restore(clotho_ctx* ctx, const void* src, size_t len) {
     }
     CK(cudaStreamSynchronize(s));
     p->acc_valid = false;  // the next step reduces the restored rows again
-    p->hostN = st.N;
     drop_graphs(ctx);
     return 0;
 }
@@ -1899,7 +1932,7 @@ int clotho_batch_generation_philox(clotho_ctx* ctx, const uint32_t* N) {
     if ((rc = put_header(ctx, [N](size_t i) { return N[i]; }))) return rc;
     enqueue_fused_step(ctx, 2, true);
     if ((rc = check_launch(ctx, "batch_generation_philox"))) return rc;
-    for (size_t i = 0; i < ctx->pops.size(); ++i) ctx->pops[i]->hostN = N[i];
+    sizes_are(ctx, [N](size_t i) { return N[i]; });
     return 0;
 }
 
@@ -1915,7 +1948,6 @@ int clotho_batch_run_philox(clotho_ctx* ctx, const uint32_t* N, uint32_t G) {
     uint32_t left = G;
     if (!ctx->profiling && graph_ready(ctx, key)) {
         if ((rc = put_header(ctx, [N](size_t i) { return N[i]; }))) return rc;
-        for (size_t i = 0; i < ctx->pops.size(); ++i) ctx->pops[i]->hostN = N[i];
     } else {
         if ((rc = clotho_batch_generation_philox(ctx, N))) return rc;
         left -= 1;
@@ -1925,7 +1957,9 @@ int clotho_batch_run_philox(clotho_ctx* ctx, const uint32_t* N, uint32_t G) {
             if ((rc = clotho_batch_generation_philox(ctx, N))) return rc;
         return 0;
     }
-    return left ? replay_generations(ctx, key, left, StepEnd::kStep) : 0;
+    if (left && (rc = replay_generations(ctx, key, left, StepEnd::kStep))) return rc;
+    sizes_are(ctx, [N](size_t i) { return N[i]; });
+    return 0;
 }
 
 int clotho_run_philox_schedule(clotho_ctx* ctx, const uint32_t* N, uint32_t G) {
@@ -1983,7 +2017,7 @@ int clotho_run_philox_schedule(clotho_ctx* ctx, const uint32_t* N, uint32_t G) {
     if (rc) return rc;
     CK(e_free);
     CK(e_sync);
-    for (uint32_t i = 0; i < n; ++i) ctx->pops[i]->hostN = N[(size_t)(G - 1) * n + i];
+    sizes_are(ctx, [=](size_t i) { return N[(size_t)(G - 1) * n + i]; });
     return 0;
 }
 

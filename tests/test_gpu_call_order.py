@@ -89,3 +89,27 @@ def test_a_refused_call_is_reported_once():
             pop.set_stream(None)
             after()
         pop.check()
+
+
+@pytest.mark.parametrize("N", [90, 150])
+def test_reads_after_a_call_that_failed_halfway(N):
+    # the graph calls cannot capture on the legacy default stream; they fail there behind their first generation
+    import ctypes as C
+
+    import clotho_gb300 as cg
+    with cg.Population(200, 2_000, 1, mu=0.02, rho=0.4, p_neutral=0.0, fitness="gaussian", seed=5) as pop:
+        pop.init(120)
+        pop.run_philox(120, 3)
+        for n, call in ((N, lambda: pop.run_philox_schedule([N] * 3)), (N + 7, lambda: pop.run_philox(N + 7, 3))):
+            pop.set_stream(1)
+            with pytest.raises(cg.ClothoError, match="rc="):
+                call()
+            pop.set_stream(None)
+            assert pop.info()["N"] == n
+            for read in (pop.L.clotho_get_fitness, pop.L.clotho_get_phenotypes):
+                buf = np.full(200, -7.0)
+                assert read(pop.h, buf.ctypes.data_as(C.c_void_p)) == 0
+                assert (buf[:n] != -7.0).all() and (buf[n:] == -7.0).all()
+            call()
+            assert pop.fitness().size == n
+        pop.check()
