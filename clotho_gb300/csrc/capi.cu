@@ -1016,11 +1016,12 @@ int clotho_generation_tape(clotho_ctx* ctx, const clotho_gen_tape* tape) {
         CK(cudaStreamWaitEvent(ctx->stream, ctx->copy_done[s], 0));
     }
     enqueue_fused_step(ctx, s, false);
-    if ((rc = check_launch(ctx, "generation_tape"))) return rc;
+    // recorded also when a launch was refused: those before it still read the tape
     CK(cudaEventRecord(ctx->kern_done[s], ctx->stream));
     if (s == 0u) ctx->drawn = false;
     // the caller's host arrays are free once the copies are done
     if (!staged) CK(cudaEventSynchronize(ctx->copy_done[s]));
+    if ((rc = check_launch(ctx, "generation_tape"))) return rc;
     ctx->set ^= 1u;
     sizes_are(ctx, [tape](size_t) { return tape->N; });
     return 0;
