@@ -554,6 +554,13 @@ int require_pop(clotho_ctx* ctx) {
     return ctx->pops.empty() ? fail(ctx, CLOTHO_E_ARG, "the context has no population") : 0;
 }
 
+// The context's stream is inside a graph capture of the caller's (false for the library's own: they end in their call).
+bool capturing(clotho_ctx* ctx) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(ctx->stream, &st) != cudaSuccess) cudaGetLastError();
+    return st != cudaStreamCaptureStatusNone;
+}
+
 int require_ready(clotho_ctx* ctx) {
     if (!ctx) return CLOTHO_E_ARG;
     for (PopHost* p : ctx->pops)
@@ -974,6 +981,8 @@ int clotho_generation_tape(clotho_ctx* ctx, const clotho_gen_tape* tape) {
     if (rc) return rc;
     if (!tape || ctx->pops.size() != 1) return fail(ctx, CLOTHO_E_ARG, "bad tape");
     if (ctx->in_step) return fail(ctx, CLOTHO_E_STATE, "a staged generation is in progress");
+    // a replay would read what the pinned block holds by then
+    if (capturing(ctx)) return fail(ctx, CLOTHO_E_STATE, "a tape cannot be captured in a graph");
     const uint32_t s = ctx->set;
     TapeArray arr[7];
     if ((rc = tape_arrays(ctx, ctx->pops[0], s, tape, arr))) return rc;
