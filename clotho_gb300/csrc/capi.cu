@@ -109,6 +109,8 @@ struct clotho_ctx {
     BlockPart* d_parts = nullptr;      // a batch's block tables (BlockTable), kMaxParts entries each
     uint32_t n_parts[3] = {0, 0, 0};
     bool parts_stale = true;
+    bool parts_captured = false;             // a caller's graph may read d_parts
+    std::vector<BlockPart*> parts_kept;      // tables that such graphs read, superseded
     uint32_t* d_hdr[3] = {nullptr, nullptr, nullptr}; // per set: [2*npops]
     // step headers (N, M per population) are staged in a ring of pinned slots:
     // a slot is reused only after the copy that read it has completed
@@ -378,13 +380,42 @@ int sync_pop_arrays(clotho_ctx* ctx, uint32_t from = 0) {
     return 0;
 }
 
+// The context's stream is inside a graph capture of the caller's (false for the library's own: they end in their call).
+bool capturing(clotho_ctx* ctx) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(ctx->stream, &st) != cudaSuccess) cudaGetLastError();
+    return st != cudaStreamCaptureStatusNone;
+}
+
+// Lets the thread allocate and wait on streams that are not captured, whatever the mode of its captures.
+struct RelaxedCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
 // The block tables of a batch, made anew before the first step after its populations (or the tuning) changed: blocks
 // in proportion to the populations' rows (plans: rows and breakpoints), a few an SM (by the tuning; two of 1,024
-// threads), so that blocks that come later even out what the proportions miss.
+// threads), so that blocks that come later even out what the proportions miss.  A step may be captured in a graph of
+// the caller's, so the tables are written on the copy stream (nothing on the context's stream reads stale tables: what
+// makes them stale waits for it), and tables that such a graph reads are left as they are.
 int block_tables(clotho_ctx* ctx) {
     const size_t n = ctx->pops.size();
-    if (!ctx->parts_stale || n < 2) return 0;
-    if (!ctx->d_parts) CK(cudaMalloc(&ctx->d_parts, sizeof(BlockPart) * 3 * kMaxParts));
+    if (n < 2) return 0;
+    const bool captured = capturing(ctx);
+    if (!ctx->parts_stale) {
+        ctx->parts_captured |= captured;
+        return 0;
+    }
+    const RelaxedCapture relaxed;
+    if (ctx->d_parts && ctx->parts_captured) {
+        ctx->parts_kept.push_back(ctx->d_parts);
+        ctx->d_parts = nullptr;
+    }
+    if (!ctx->d_parts)
+        CK(cudaMallocFromPoolAsync(reinterpret_cast<void**>(&ctx->d_parts), sizeof(BlockPart) * 3 * kMaxParts, ctx->pool,
+                                   ctx->copy_stream));
+    ctx->parts_captured = captured;
     std::vector<BlockPart> h(3 * kMaxParts);
     for (uint32_t k = 0; k < 3; ++k) {
         auto work = [k](const PopHost* p) { return p->dev[0].Scap * (k == kTablePlan ? 1.0 + 0.4 * p->desc.rho : 1.0); };
@@ -400,8 +431,8 @@ int block_tables(clotho_ctx* ctx) {
         }
         ctx->n_parts[k] = at;
     }
-    CK(cudaMemcpyAsync(ctx->d_parts, h.data(), h.size() * sizeof(BlockPart), cudaMemcpyHostToDevice, ctx->stream));
-    CK(cudaStreamSynchronize(ctx->stream));
+    CK(cudaMemcpyAsync(ctx->d_parts, h.data(), h.size() * sizeof(BlockPart), cudaMemcpyHostToDevice, ctx->copy_stream));
+    CK(cudaStreamSynchronize(ctx->copy_stream));
     ctx->parts_stale = false;
     return 0;
 }
@@ -552,13 +583,6 @@ constexpr size_t kTapeStage = 1u << 20;
 int require_pop(clotho_ctx* ctx) {
     if (!ctx) return CLOTHO_E_ARG;
     return ctx->pops.empty() ? fail(ctx, CLOTHO_E_ARG, "the context has no population") : 0;
-}
-
-// The context's stream is inside a graph capture of the caller's (false for the library's own: they end in their call).
-bool capturing(clotho_ctx* ctx) {
-    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(ctx->stream, &st) != cudaSuccess) cudaGetLastError();
-    return st != cudaStreamCaptureStatusNone;
 }
 
 int require_ready(clotho_ctx* ctx) {
@@ -792,6 +816,9 @@ int clotho_destroy(clotho_ctx* ctx) {
     if (ctx->copy_stream) cudaStreamSynchronize(ctx->copy_stream);
     for (PopHost* p : ctx->pops) free_pop(ctx, p);
     ctx->pops.clear();
+    ctx->parts_kept.push_back(ctx->d_parts);
+    for (BlockPart* t : ctx->parts_kept)
+        if (t) cudaFreeAsync(t, ctx->own_stream);
     if (ctx->own_stream) cudaStreamSynchronize(ctx->own_stream);
     if (ctx->pool) cudaMemPoolDestroy(ctx->pool);  // its blocks are back: free_pop returned them
     for (int s = 0; s < 3; ++s) {
@@ -807,7 +834,6 @@ int clotho_destroy(clotho_ctx* ctx) {
     for (uint32_t k = 0; k < kHdrRing; ++k)
         if (ctx->ring_ev[k]) cudaEventDestroy(ctx->ring_ev[k]);
     if (ctx->d_ctl) cudaFree(ctx->d_ctl);
-    if (ctx->d_parts) cudaFree(ctx->d_parts);
     drop_graphs(ctx);
     for (cudaEvent_t e : ctx->prof_ev) cudaEventDestroy(e);
     for (int i = 0; i < 2; ++i) {
@@ -2046,6 +2072,10 @@ int clotho_set_tuning(clotho_ctx* ctx, const clotho_tuning* t) {
     if (t->rows_per_item) {
         int rc = clotho_set_rows_per_item(ctx, t->rows_per_item);
         if (rc) return rc;
+    }
+    if (ctx->pops.size() > 1) {   // steps under way read the block tables
+        if (capturing(ctx)) ctx->parts_captured = true;
+        else CK(cudaStreamSynchronize(ctx->stream));
     }
     ctx->ind_per_sm = t->row_blocks_per_sm ? t->row_blocks_per_sm : 16u;
     ctx->narrow_ok = t->narrow_build != 0u;

@@ -72,3 +72,58 @@ def test_tapes_are_refused_and_leave_the_context_whole(N, mode):
             pop.check()
             got.append((pop.info(), pop.rows().tobytes(), pop.pairs().tobytes()))
     assert got[0] == got[1]
+
+
+def _descs(cg):
+    return [cg.make_desc(n, 2_000, 1, mu=0.01, rho=0.3, fitness=f, p_neutral=0.2, seed=n)
+            for n, f in ((400, "constant"), (37, "gaussian"), (900, "constant"), (1_500, "gaussian"))]
+
+
+def _states(b):
+    return [(b.info(i), b.rows(i).tobytes()) for i in range(len(b))]
+
+
+@pytest.mark.parametrize("mode,before", [(RELAXED, 0), (RELAXED, 1), (GLOBAL, 1), (THREAD, 1)])
+@pytest.mark.parametrize("change", ["add", "tune", "remove"])
+def test_first_batch_step_after_a_change_is_captured(mode, before, change):
+    # (in the stricter modes a context's first step of all is refused: it takes pinned memory)
+    import clotho_gb300 as cg
+    got = []
+    for capture in (True, False):
+        d = _descs(cg)
+        b = cg.Batch(d[:3])
+        b.init()
+        c = Capture()
+        b.set_stream(c.stream)
+        for _ in range(before):
+            b.step()
+        for tune in (3, 24):      # twice: the second change is one under a graph that exists
+            if change == "add" and len(b) < 4:
+                b.add(d[3], 1_500)
+            elif change == "remove" and len(b) > 2:
+                b.remove(0)
+            elif tune == 3 or not capture:
+                b.set_tuning(row_blocks_per_sm=tune)
+            if capture:
+                c.begin(mode)
+                try:
+                    if change == "tune" and tune != 3:
+                        b.set_tuning(row_blocks_per_sm=tune)
+                    b.step()
+                finally:
+                    x = c.end()
+                c.replay(x, 3)
+                if tune == 3:
+                    first = x
+            else:
+                for _ in range(3):
+                    b.step()
+        if change == "tune":      # the first graph's launch shapes still hold
+            if capture:
+                c.replay(first, 2)
+            else:
+                b.run(2)
+        b.run(2)
+        got.append(_states(b))
+        b.close()
+    assert got[0] == got[1]
