@@ -126,6 +126,7 @@ struct clotho_ctx {
     uint32_t set = 0;                                    // next tape set
     uint32_t pairs_set = 0;                              // the set whose pairs the last generation used
     cudaEvent_t copy_done[2]{}, kern_done[2]{};
+    bool captured = false;   // a step went into a graph of the caller's: replays run steps that no call here tells of
     bool drawn = false;   // device-drawn steps, which share set 0's buffers, enqueued since kern_done[0] was recorded
     std::string err;
     bool profiling = false;
@@ -191,6 +192,13 @@ LaunchCfg cfg(clotho_ctx* ctx, uint32_t set = 0) {
     return L;
 }
 
+// The context's stream is inside a graph capture of the caller's (false for the library's own: they end in their call).
+bool capturing(clotho_ctx* ctx) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(ctx->stream, &st) != cudaSuccess) cudaGetLastError();
+    return st != cudaStreamCaptureStatusNone;
+}
+
 // A pinned slot for one step header; nullptr if pinned memory is unavailable.
 uint32_t* hdr_stage(clotho_ctx* ctx, uint32_t* slot) {
     if (!ctx->h_ring) {
@@ -210,6 +218,7 @@ uint32_t* hdr_stage(clotho_ctx* ctx, uint32_t* slot) {
 
 // Copy n headers from slot into dst on stream s and mark the slot busy until then.
 int hdr_copy(clotho_ctx* ctx, uint32_t slot, uint32_t* dst, uint32_t n, cudaStream_t s) {
+    if (s == ctx->stream) ctx->captured |= capturing(ctx);
     CK(cudaMemcpyAsync(dst, ctx->h_ring + (size_t)slot * 2 * kMaxPops, 8ull * n, cudaMemcpyHostToDevice, s));
     CK(cudaEventRecord(ctx->ring_ev[slot], s));
     ctx->ring_used[slot] = true;
@@ -317,7 +326,7 @@ template <class F>
 void sizes_are(clotho_ctx* ctx, F N) {
     for (size_t i = 0; i < ctx->pops.size(); ++i) {
         ctx->pops[i]->hostN = N(i);
-        ctx->pops[i]->n_known = true;
+        ctx->pops[i]->n_known = !ctx->captured;
     }
 }
 
@@ -378,13 +387,6 @@ int sync_pop_arrays(clotho_ctx* ctx, uint32_t from = 0) {
     ctx->parts_stale = true;
     CK(cudaStreamSynchronize(ctx->stream));
     return 0;
-}
-
-// The context's stream is inside a graph capture of the caller's (false for the library's own: they end in their call).
-bool capturing(clotho_ctx* ctx) {
-    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(ctx->stream, &st) != cudaSuccess) cudaGetLastError();
-    return st != cudaStreamCaptureStatusNone;
 }
 
 // Lets the thread allocate and wait on streams that are not captured, whatever the mode of its captures.
@@ -451,7 +453,7 @@ uint32_t current_N(clotho_ctx* ctx, PopHost* p, int* rc) {
     if (!p->n_known) {
         const uint32_t N = read_status(ctx, p, rc).N;
         if (*rc == 0) p->hostN = N;
-        p->n_known = *rc == 0;
+        p->n_known = *rc == 0 && !ctx->captured;
     }
     return p->hostN;
 }
@@ -909,7 +911,7 @@ static int init_pop(clotho_ctx* ctx, uint32_t idx, uint32_t N0) {
     p->acc_valid = true;  // A == 0: the first analysis is skipped (free_space_mt...:46)
     p->ready = true;
     p->hostN = N0;
-    p->n_known = true;
+    p->n_known = !ctx->captured;
     return 0;
 }
 
@@ -1037,7 +1039,7 @@ int clotho_generation_tape(clotho_ctx* ctx, const clotho_gen_tape* tape) {
         ctx->launches += 1;
     } else {
         // the tape set s was last read by the kernels of two steps ago, set 0 by any device-drawn steps since
-        if (s == 0u && ctx->drawn) CK(cudaEventRecord(ctx->kern_done[0], ctx->stream));
+        if (s == 0u && (ctx->drawn || ctx->captured)) CK(cudaEventRecord(ctx->kern_done[0], ctx->stream));
         CK(cudaStreamWaitEvent(ctx->copy_stream, ctx->kern_done[s], 0));
         for (const TapeArray& a : arr)
             if (a.bytes) CK(cudaMemcpyAsync(a.dst, a.src, a.bytes, cudaMemcpyHostToDevice, ctx->copy_stream));
@@ -1125,7 +1127,7 @@ int clotho_begin_generation(clotho_ctx* ctx, uint32_t N, uint32_t M) {
     ctx->in_step = true;
     p->hostN = N;
     rc = check_launch(ctx, "begin");
-    p->n_known = rc == 0;
+    p->n_known = rc == 0 && !ctx->captured;
     return rc;
 }
 

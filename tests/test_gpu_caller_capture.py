@@ -127,3 +127,33 @@ def test_first_batch_step_after_a_change_is_captured(mode, before, change):
         got.append(_states(b))
         b.close()
     assert got[0] == got[1]
+
+
+def test_reads_between_replays_of_the_callers_graph():
+    import clotho_gb300 as cg
+    with cg.Population(200, 2_000, 1, mu=0.02, rho=0.4, p_neutral=0.0, fitness="gaussian", seed=5) as pop:
+        pop.init(120)
+        pop.run_philox(120, 3)
+        c = Capture()
+        pop.set_stream(c.stream)
+
+        def reads(N):
+            assert pop.info()["N"] == N
+            for read in (pop.L.clotho_get_fitness, pop.L.clotho_get_phenotypes):
+                buf = np.full(200, -7.0)
+                assert read(pop.h, buf.ctypes.data_as(C.c_void_p)) == 0
+                assert (buf[:N] != -7.0).all() and (buf[N:] == -7.0).all()
+
+        c.begin(RELAXED)
+        try:
+            pop.simulate_philox(80)
+        finally:
+            x = c.end()
+        reads(120)
+        c.replay(x, 1)
+        reads(80)
+        pop.run_philox(150, 2)
+        reads(150)
+        c.replay(x, 2)
+        reads(80)
+        pop.check()
