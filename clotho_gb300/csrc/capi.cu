@@ -1565,10 +1565,9 @@ static int pairwise_of(clotho_ctx* ctx, uint32_t idx, const uint32_t* sample, ui
     CK(pool_alloc(ctx, &d, at_dist + (dist ? pairs * 4 : 0)));
     auto body = [&]() -> int {
         CK(cudaMemcpyAsync(d, head.data(), head.size(), cudaMemcpyHostToDevice, ctx->stream));
-        if (z.sum_bytes) CK(cudaMemsetAsync(d + at_sums, 0, z.sum_bytes, ctx->stream));
         CK(launch_pairwise(cfg(ctx), ctx->d_pops[0], idx, reinterpret_cast<uint32_t*>(d + at_smp), n, z, d + at_sums,
                            dist ? reinterpret_cast<uint32_t*>(d + at_dist) : nullptr, reinterpret_cast<PairwiseOut*>(d)));
-        ctx->launches += 1;
+        ctx->launches += (z.tiles + z.group - 1u) / z.group;
         if (int r = check_launch(ctx, "pairwise difference")) return r;
         CK(cudaMemcpyAsync(&h, d, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream));
         if (dist) host_pages(dist, pairs * 4);

@@ -465,6 +465,7 @@ struct PairwiseOut {
 // how the pairs of n rows of W words are cut into CTAs, and the scratch that takes
 struct PairwisePlan {
     uint32_t tiles, splits, per;       // per: rounds of eight 128-slot stages a CTA
+    uint32_t group;                    // tiles a launch
     size_t sum_bytes;
 };
 PairwisePlan pairwise_plan(const LaunchCfg&, uint32_t n, uint32_t W);

@@ -24,6 +24,7 @@ constexpr uint32_t kRound = 8;                  // stages from one load of the r
 constexpr uint32_t kStageBytes = (kTM + kTN) * 128u;
 constexpr uint32_t kMaxSlots = 1u << 19;        // slots a CTA sums up: counts stay far below 2^24 units
 constexpr uint32_t kTileSums = kTM * kTN + kTM + kTN;   // counts of a tile whose slots several CTAs share
+constexpr uint32_t kSplitTiles = 1024;          // tiles whose slots are shared at a time: 136 MB of counts
 constexpr uint32_t kPairWait = 1u << 20;        // try_wait rounds before a CTA gives up
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -90,7 +91,7 @@ __device__ __forceinline__ void load_32_columns(uint32_t taddr, uint32_t (&v)[32
 // unit's 16 words a clock and SM.)
 __global__ void __launch_bounds__(kPairThreads, 1)
 k_pairwise(const PopDev* __restrict__ pops, uint32_t p, const uint32_t* __restrict__ sample, uint32_t n,
-           uint32_t splits, uint32_t per, uint32_t* __restrict__ tile_sum,
+           uint32_t tile0, uint32_t splits, uint32_t per, uint32_t* __restrict__ tile_sum,
            uint32_t* __restrict__ tile_done, uint32_t* __restrict__ dist, PairwiseOut* __restrict__ out) {
     extern __shared__ uint8_t s_raw[];
     __shared__ __align__(8) unsigned long long s_full[kRing], s_free[kRing], s_end;
@@ -101,10 +102,10 @@ k_pairwise(const PopDev* __restrict__ pops, uint32_t p, const uint32_t* __restri
     const PopDev& P = pops[p];
     const uint64_t* rows = P.rows[P.st->cur];
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-    // tile (ti, tj): of tile row ti, the tile columns from its first row on
+    // tile (ti, tj): of tile row ti, the tile columns from its first row on; tile0: the launch's first
     const uint32_t tile = blockIdx.x / splits, split = blockIdx.x % splits;
     const uint32_t TJ = (n + kTN - 1u) / kTN;
-    uint32_t ti = 0, left = tile;
+    uint32_t ti = 0, left = tile0 + tile;
     while (left >= TJ - ti * kTM / kTN) {
         left -= TJ - ti * kTM / kTN;
         ++ti;
@@ -315,12 +316,16 @@ PairwisePlan pairwise_plan(const LaunchCfg& L, uint32_t n, uint32_t W) {
     for (uint32_t ti = 0; ti < TI; ++ti) z.tiles += TJ - ti * kTM / kTN;
     // Slots over several CTAs where the tiles alone leave SMs idle: the count with the least work on the busiest SM
     // (tiles x splits over the SMs, each with its share of the rounds plus about six stages' time to start and
-    // to add up), and as many as keep a CTA's sums in range
+    // to add up), and as many as keep a CTA's sums in range.  Above kSplitTiles tiles the counts would take more
+    // memory (133 KB a tile, 8.7 GB for 65,536 rows) than the last wave's idle SMs are worth: one CTA a tile, or, where
+    // the sums' range asks for more, a launch for every kSplitTiles of them.
     const uint32_t least = std::max(1u, (nr * kRound * 128u + kMaxSlots - 1u) / kMaxSlots);
+    const bool many = z.tiles > kSplitTiles;
+    z.group = many && least > 1u ? kSplitTiles : z.tiles;
     double best = 1e30;
     z.splits = least;
-    for (uint32_t s = least; s <= std::max(least, std::min(nr, 64u)); ++s) {
-        const double waves = (double)((z.tiles * (uint64_t)s + L.num_sms - 1u) / L.num_sms);
+    for (uint32_t s = least; s <= std::max(least, many && least == 1u ? 1u : std::min(nr, 64u)); ++s) {
+        const double waves = (double)((z.group * (uint64_t)s + L.num_sms - 1u) / L.num_sms);
         const double cost = waves * ((double)((nr + s - 1u) / s * kRound) + 6.0 + (s > 1u ? 6.0 : 0.0));
         if (cost < best * 0.98) {
             best = cost;
@@ -328,23 +333,27 @@ PairwisePlan pairwise_plan(const LaunchCfg& L, uint32_t n, uint32_t W) {
         }
     }
     z.per = (nr + z.splits - 1u) / z.splits;
-    z.sum_bytes = z.splits > 1u ? (size_t)z.tiles * (kTileSums + 1u) * 4 : 0;
+    z.sum_bytes = z.splits > 1u ? (size_t)z.group * (kTileSums + 1u) * 4 : 0;
     return z;
 }
 
-// scratch: sum_bytes, zero on entry.
+// scratch: sum_bytes.
 cudaError_t launch_pairwise(const LaunchCfg& L, const PopDev* pops, uint32_t p, const uint32_t* sample, uint32_t n,
                             const PairwisePlan& z, void* scratch, uint32_t* dist, PairwiseOut* out) {
     uint32_t* sums = z.sum_bytes ? static_cast<uint32_t*>(scratch) : nullptr;
-    uint32_t* done = z.sum_bytes ? sums + (size_t)z.tiles * kTileSums : nullptr;
+    uint32_t* done = z.sum_bytes ? sums + (size_t)z.group * kTileSums : nullptr;
     const size_t smem = kRing * kStageBytes + 1024u;
     // a property of the function on the current device; setting it again is harmless
-    const cudaError_t e =
+    cudaError_t e =
         cudaFuncSetAttribute((const void*)k_pairwise, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    k_pairwise<<<z.tiles * z.splits, kPairThreads, smem, L.stream>>>(pops, p, sample, n, z.splits, z.per, sums, done,
-                                                                    dist, out);
-    return cudaSuccess;
+    for (uint32_t t = 0; t < z.tiles && e == cudaSuccess; t += z.group) {
+        if (sums) e = cudaMemsetAsync(sums, 0, z.sum_bytes, L.stream);
+        if (e != cudaSuccess) break;
+        k_pairwise<<<std::min(z.group, z.tiles - t) * z.splits, kPairThreads, smem, L.stream>>>(
+            pops, p, sample, n, t, z.splits, z.per, sums, done, dist, out);
+        e = cudaPeekAtLastError();
+    }
+    return e;
 }
 
 }  // namespace clotho
