@@ -432,7 +432,7 @@ struct Planes {
 template <bool COL, bool ROW>
 __global__ void __launch_bounds__(256, 3) k_margins(const PopDev* __restrict__ pops, uint32_t p,
                                                  uint32_t* __restrict__ colc, uint32_t* __restrict__ rowc,
-                                                 uint32_t lpr, uint32_t strip) {
+                                                 uint32_t lpr, uint32_t strip, uint32_t groups) {
     __shared__ uint32_t s_cnt[COL ? 64 * 65 : 1];   // [column of the word][word]
     const PopDev& P = pops[p];
     const DevStatus* st = P.st;
@@ -440,8 +440,10 @@ __global__ void __launch_bounds__(256, 3) k_margins(const PopDev* __restrict__ p
     const uint64_t* rows = P.rows[st->cur];
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t rpl = 32u / lpr, sub = lane / lpr;       // rows a load, this lane's row among them
-    const uint32_t wi = 2u * (lane & (lpr - 1u)), w = blockIdx.x * 64u + wi;
-    const uint32_t r0 = blockIdx.y * strip, r1 = min(S, r0 + strip);
+    // a block's 64-word group and strip of rows: in one grid dimension, which takes more strips than the others'
+    // 65,535 (130 million rows)
+    const uint32_t g = blockIdx.x % groups, wi = 2u * (lane & (lpr - 1u)), w = g * 64u + wi;
+    const uint32_t r0 = blockIdx.x / groups * strip, r1 = min(S, r0 + strip);
     if (COL) {
         for (uint32_t i = threadIdx.x; i < 64u * 65u; i += 256u) s_cnt[i] = 0u;
         __syncthreads();
@@ -450,7 +452,7 @@ __global__ void __launch_bounds__(256, 3) k_margins(const PopDev* __restrict__ p
     for (uint32_t b = r0 + warp * 8u * rpl; b < r1; b += 64u * rpl) {
         uint64_t x[8], y[8];
         if (lpr == 32u && lane < 8u) {   // the warp's next eight rows
-            const uint32_t r = b + 64u + lane, w0 = blockIdx.x * 64u;
+            const uint32_t r = b + 64u + lane, w0 = g * 64u;
             if (r < r1)
                 asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(rows + (size_t)r * P.Wcap + w0),
                              "r"(min(64u, W - w0) * 8u)
@@ -487,7 +489,7 @@ __global__ void __launch_bounds__(256, 3) k_margins(const PopDev* __restrict__ p
                 for (uint32_t k = 0; k < 2; ++k) {
                     const uint32_t r = b + (2u * j + k) * rpl + sub, n = (mine >> (16u * k)) & 0xffffu;
                     if (r < r1) {
-                        if (gridDim.x == 1u) rowc[r] = n;
+                        if (groups == 1u) rowc[r] = n;
                         else if (n) atomicAdd(rowc + r, n);
                     }
                 }
@@ -503,7 +505,7 @@ __global__ void __launch_bounds__(256, 3) k_margins(const PopDev* __restrict__ p
         for (uint32_t i = threadIdx.x; i < 4096u; i += 256u) {
             const uint32_t j = i & 63u, ww = i >> 6;
             const uint32_t c = s_cnt[j * 65u + ww];
-            if (c) atomicAdd(colc + (size_t)blockIdx.x * 4096u + i, c);
+            if (c) atomicAdd(colc + (size_t)g * 4096u + i, c);
         }
     }
 }
@@ -520,10 +522,10 @@ void launch_margins(const LaunchCfg& L, const PopDev* pops, uint32_t p, uint32_t
     const uint32_t want = std::max(1u, (uint32_t)L.num_sms * 4u / groups);
     uint32_t strip = (blocks_for(S, want) + unit - 1u) / unit * unit;
     strip = std::min(strip, kMarginRows * 8u * rpl);
-    const dim3 grid(groups, blocks_for(S, strip));
-    if (colc && rowc) k_margins<true, true><<<grid, 256, 0, L.stream>>>(pops, p, colc, rowc, lpr, strip);
-    else if (colc) k_margins<true, false><<<grid, 256, 0, L.stream>>>(pops, p, colc, nullptr, lpr, strip);
-    else k_margins<false, true><<<grid, 256, 0, L.stream>>>(pops, p, nullptr, rowc, lpr, strip);
+    const uint32_t grid = groups * blocks_for(S, strip);
+    if (colc && rowc) k_margins<true, true><<<grid, 256, 0, L.stream>>>(pops, p, colc, rowc, lpr, strip, groups);
+    else if (colc) k_margins<true, false><<<grid, 256, 0, L.stream>>>(pops, p, colc, nullptr, lpr, strip, groups);
+    else k_margins<false, true><<<grid, 256, 0, L.stream>>>(pops, p, nullptr, rowc, lpr, strip, groups);
 }
 
 
