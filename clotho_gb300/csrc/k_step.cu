@@ -407,10 +407,12 @@ struct Planes {
             c = t;
         }
     }
-    // cnt[j * 65] += count of column j
-    __device__ __forceinline__ void flush(uint32_t* cnt) const {
+    // cnt[j * 65] += count of column j.  The lanes of one word (rows that share a warp) go through its columns eight
+    // apart: side by side they would add to the same counts.
+    __device__ __forceinline__ void flush(uint32_t* cnt, uint32_t sub) const {
 #pragma unroll 1
-        for (uint32_t k = 0; k < 8; ++k) {
+        for (uint32_t k0 = 0; k0 < 8; ++k0) {
+            const uint32_t k = (k0 + sub) & 7u;
             uint64_t x = 0;  // byte i: digit i of columns 8k .. 8k + 7
 #pragma unroll
             for (int i = 0; i < 8; ++i) x |= ((d[i] >> (8u * k)) & 0xffull) << (8 * i);
@@ -497,9 +499,9 @@ __global__ void __launch_bounds__(256, 3) k_margins(const PopDev* __restrict__ p
         }
     }
     if (COL) {
-        if (w < W) {
-            c0.flush(s_cnt + wi);
-            c1.flush(s_cnt + wi + 1u);
+        if (w < W && r0 + warp * 8u * rpl < r1) {   // (warps that had rows)
+            c0.flush(s_cnt + wi, sub);
+            c1.flush(s_cnt + wi + 1u, sub);
         }
         __syncthreads();
         for (uint32_t i = threadIdx.x; i < 4096u; i += 256u) {
@@ -541,10 +543,12 @@ __global__ void __launch_bounds__(256) k_stats(const PopDev* __restrict__ pops, 
                                                StatsOut* __restrict__ out, uint32_t* __restrict__ sfs) {
     __shared__ uint32_t s_bin[kStatBins];
     __shared__ double s_sum[8][5];
+    const uint32_t bins = min(sfs_len, kStatBins);
+    for (uint32_t i = threadIdx.x; i < bins; i += 256u) s_bin[i] = 0u;
+    pdl_wait();
     const PopDev& P = pops[p];
     const DevStatus* st = P.st;
-    const uint32_t A = st->A, N = st->N, S = 2u * N, bins = min(sfs_len, kStatBins);
-    for (uint32_t i = threadIdx.x; i < bins; i += 256u) s_bin[i] = 0u;
+    const uint32_t A = st->A, N = st->N, S = 2u * N;
     __syncthreads();
     double v[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
     uint32_t seg = 0, fix = 0;
@@ -594,7 +598,7 @@ __global__ void __launch_bounds__(256) k_stats(const PopDev* __restrict__ pops, 
 }
 void launch_stats(const LaunchCfg& L, const PopDev* pops, uint32_t p, const uint32_t* counts, uint32_t sfs_len,
                   StatsOut* out, uint32_t* sfs) {
-    k_stats<<<kStatBlocks, 256, 0, L.stream>>>(pops, p, counts, sfs_len, out, sfs);
+    launch_k(L, k_stats, dim3(kStatBlocks), dim3(256), pops, p, counts, sfs_len, out, sfs);
 }
 
 }  // namespace clotho

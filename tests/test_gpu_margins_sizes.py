@@ -1,4 +1,5 @@
-"""Margins at the largest populations: more strips of rows than a grid's second dimension takes."""
+"""Margins at the largest populations (more strips of rows than a grid's second dimension takes), and around the size up
+to which both come in one copy."""
 import numpy as np
 import pytest
 
@@ -24,3 +25,24 @@ def test_more_than_130_million_rows():
     assert int(col.sum(dtype=np.uint64)) == int(row.sum(dtype=np.uint64))
     assert row.min() >= 0 and row.max() <= 6 and abs(float(row[-1_000_000:].mean()) - p.sum()) < 0.02
     assert st["segregating"] == int(((col > 0) & (col < 2 * N)).sum())
+
+
+@pytest.mark.parametrize("N,A", [(1, 1), (7_935, 400), (7_936, 400), (7_937, 400), (20, 16_383), (20, 15_872)])
+def test_margins_in_one_copy_or_two(N, A):
+    # 16,384 counts in all at N = 7,936 and A = 400 (512 columns and 15,872 rows)
+    import ctypes as C
+
+    import clotho_gb300 as cg
+    rng = np.random.default_rng(N + A)
+    W = (A + 511) // 512 * 8
+    rows = rng.integers(0, 2 ** 64, size=(2 * N, W), dtype=np.uint64)
+    bits = np.unpackbits(rows.view(np.uint8), axis=1, bitorder="little")[:, :A]
+    with cg.Population(N, A, 1) as pop:
+        pop.load_population(N, rows, rng.random(A), np.zeros(A, np.float32))
+        for want_col, want_row in ((True, True), (True, False), (False, True)):
+            col, row = np.full(A + 8, 77, np.uint32), np.full(2 * N + 8, 77, np.uint32)
+            p = [x.ctypes.data_as(C.c_void_p) if on else None for x, on in ((col, want_col), (row, want_row))]
+            assert pop.L.clotho_margins(pop.h, *p) == 0
+            assert np.array_equal(col[:A], bits.sum(0, dtype=np.uint32) if want_col else np.full(A, 77))
+            assert np.array_equal(row[:2 * N], bits.sum(1, dtype=np.uint32) if want_row else np.full(2 * N, 77))
+            assert (col[A:] == 77).all() and (row[2 * N:] == 77).all()
