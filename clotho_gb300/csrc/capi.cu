@@ -2,8 +2,10 @@
 //
 // A context owns a set of resident populations (one for the plain engine) and
 // two CUDA streams: a compute stream for every kernel and a copy stream for
-// tape uploads.  Tape buffers are double-buffered so the host->device copy of
-// generation g+1 overlaps the kernels of generation g.
+// the uploads of large tapes.  Tape buffers are double-buffered, so that the
+// host->device copies of generation g+1 overlap the kernels of generation g.
+// Tapes of at most 1 MB are packed into a pinned block (one a buffer) and
+// uploaded by a kernel on the compute stream.
 #include "engine.cuh"
 #include "../../include/clotho_gpu.h"
 
@@ -509,7 +511,7 @@ int prof_collect(clotho_ctx* ctx) {
 }
 
 // The fused step's generation kernel counts columns (its counting build) when a population asked and the
-// counters fit in shared memory; k_fs_finalize of the same step zeroes those counts and marks them valid.
+// counters fit in shared memory; the step's first kernel zeroes those counts and marks them valid.
 bool count_on(clotho_ctx* ctx, uint32_t fuse) {
     return ctx->counting > 0 && ctx->n_bm > 0 && (fuse & kFuseFs) && !(ctx->profiling && ctx->phase_clocks) &&
            generation_counts_fit(ctx->maxW_bm, ctx->maxA_bm);

@@ -400,11 +400,12 @@ struct PrepSizes {
 // valid.  Returns the launches made.
 uint32_t launch_prep(const LaunchCfg&, const PopDev* pops, uint32_t npops, const PrepSizes&, const uint32_t* hdr,
                      WorkCtl* ctl, uint32_t what, bool count_on);
-// Allele capacity up to which one block ranks a population's slots in shared memory (k_prep.cu)
+// Allele capacity up to which a population's slots are ranked in shared memory: by eight blocks, each its share of the
+// buckets, or in a batch by one (k_prep.cu)
 constexpr uint32_t kDirectRanks = 8192;
 inline bool direct_ranks(const PrepSizes& z) { return z.maxA <= kDirectRanks && z.tables; }
-// One generation's tape from a pinned staging block into a population's tape arrays, and the step's header: pieces
-// of n16 16-byte words (the last one padded; arrays and staging start on 16-byte boundaries).
+// One generation's tape from a pinned staging block into a population's tape arrays, and the step's header: seven pieces
+// of whole 16-byte words (their ends padded; arrays and staging start on 16-byte boundaries).
 struct TapePieces {
     const void* src[7];
     void* dst[7];

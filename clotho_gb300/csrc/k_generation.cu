@@ -1767,8 +1767,13 @@ k_generation(const __grid_constant__ PopDev one, const PopDev* __restrict__ pops
         const bool group = SUF && NARROW && !PROF && max(st.W, st.pW) <= kGroupWords;
         if (group) {
             // copy rows cost about the same, so units in a fixed stride spare the claims (2e4 of them on one counter:
-            // 26.6 against 20.4 us); with a breakpoint on every eighth row or more, claims even the rows out
-            // (10,000 individuals at rho = 3: 37.4 against 43.5 us), a few units at a time where there are many
+            // 26.6 against 20.4 us); with a breakpoint on every eighth row or more, claims even the rows out, a few
+            // units at a time where there are many.  They do where a row takes long: a generation of 10,000 individuals
+            // of 64-word rows with effects at rho = 0.5 / 1 / 3 takes 58.8 / 63.4 / 73.0 us with claims, 61.1 / 68.0 / 79.3
+            // with strides (of 100,000: 224 / 247 / 305 and 230 / 254 / 316).  Where rows are narrow or have no effects
+            // strides would be the better ones above the line as well, most for many rows (100,000 individuals of 8-word
+            // rows at rho = 0.5 / 3: 88 / 139 with claims, 75 / 112 with strides; 16 words 94 / 134, 85 / 118; 32 words
+            // 121 / 153, 114 / 145; 1,000 individuals of 64-word rows 36 / 44, 34 / 42): the line does not ask for either
             const uint32_t events = P.mode == kModePhilox ? st.ev_used : P.ev_off[S];
             group_rows(pops[0], 0u, S, events > S / 8u ? &ctl->gen_counter : nullptr,
                        max(1u, S / (gridDim.x * kWarps * 8u)), warp * gridDim.x + blockIdx.x, gridDim.x * kWarps, cur_cnt ? &s_crows : nullptr, sfix, mask, ws.q, sF, sV, fo.cnt, maxW, fuse);

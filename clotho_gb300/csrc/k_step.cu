@@ -519,7 +519,7 @@ void launch_margins(const LaunchCfg& L, const PopDev* pops, uint32_t p, uint32_t
     while (lpr < 32u && 2u * lpr < W) lpr <<= 1;
     const uint32_t rpl = 32u / lpr, unit = 64u * rpl;       // rows that a block's warps load together
     const uint32_t groups = (W + 63u) / 64u;
-    // about four blocks an SM: two are resident (their loads in flight cover the DRAM latency), the rest
+    // about four blocks an SM: three are resident (their loads in flight cover the DRAM latency), the rest
     // even out the end; narrow populations take fewer rows a block
     const uint32_t want = std::max(1u, (uint32_t)L.num_sms * 4u / groups);
     uint32_t strip = (blocks_for(S, want) + unit - 1u) / unit * unit;

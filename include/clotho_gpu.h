@@ -140,7 +140,10 @@ int  clotho_sync(clotho_ctx *ctx);
  * the previous stream is finished first.  The caller keeps ownership of its
  * stream and must not destroy it while the context uses it.  The graph calls
  * (clotho_run_philox*) capture on this stream, so it must not be the legacy
- * default stream for them. */
+ * default stream for them.  A caller that captures the stream itself can put
+ * single device-drawn generations (clotho_generation_philox,
+ * clotho_batch_generation_philox) into its graph; tapes and calls that wait are
+ * refused. */
 int  clotho_set_stream(clotho_ctx *ctx, void *stream);
 
 /* ---- population set-up ------------------------------------------------- */
@@ -180,14 +183,18 @@ int  clotho_restore(clotho_ctx *ctx, const void *src, size_t len);
 /* Engine::simulate() (engine_batched_task.hpp:163-223) with the tape standing
  * in for the RNG draws: free space + fixed removal (FreeSpaceAnalyzerMT,
  * updateFixedAlleles :303-345), crossover (BatchCrossoverMTWE), mutation
- * (BatchMutationMT), phenotype (BatchPhenotypeMT) and fitness (GeneralFitness),
- * with no host synchronisation. */
+ * (BatchMutationMT), phenotype (BatchPhenotypeMT) and fitness (GeneralFitness).
+ * The call waits for no step of its own: it returns when the tape's arrays are
+ * the caller's again, which may wait for the step before the last (it read the
+ * buffers that this tape goes into).  It cannot be captured in a graph of the
+ * caller's (CLOTHO_E_STATE). */
 int  clotho_generation_tape(clotho_ctx *ctx, const clotho_gen_tape *tape);
 /* The same step with every draw made on the device (Philox-4x32-10 keyed by
  * (seed, generation, stream, index)); parents are sampled by an FP64 inclusive
  * prefix sum of fitness.  N = offspring individuals. */
 int  clotho_generation_philox(clotho_ctx *ctx, uint32_t N);
-/* G device-drawn generations replayed from one captured CUDA graph. */
+/* G device-drawn generations replayed from captured CUDA graphs: of one
+ * generation and, once 64 of a size have been replayed, of eight. */
 int  clotho_run_philox(clotho_ctx *ctx, uint32_t N, uint32_t G);
 
 /* ---- staged entry points (one per reference policy) --------------------- */
@@ -340,14 +347,14 @@ int  clotho_pop_pairwise_difference(clotho_ctx *ctx, uint32_t index, const uint3
 int  clotho_pop_count_columns(clotho_ctx *ctx, uint32_t index, int enable);
 /* One device-drawn generation of every population (N[i] offspring). */
 int  clotho_batch_generation_philox(clotho_ctx *ctx, const uint32_t *N);
-/* G such generations, replayed from one captured CUDA graph. */
+/* G such generations, replayed from captured CUDA graphs (as clotho_run_philox). */
 int  clotho_batch_run_philox(clotho_ctx *ctx, const uint32_t *N, uint32_t G);
 /* G device-drawn generations with a size schedule: N[g * npops + i] offspring
  * individuals of population i in generation g (population growth,
  * predefined_population_growth.cpp:26-28, linear_population_growth.cpp:23-25).
- * One captured CUDA graph serves every generation; the sizes are copied to
- * the device once and each replay reads its own.  Works on single-population
- * and batched contexts. */
+ * The same graphs serve every generation; the sizes are copied to the device
+ * once and each step leaves the next one's.  Works on single-population and
+ * batched contexts. */
 int  clotho_run_philox_schedule(clotho_ctx *ctx, const uint32_t *N, uint32_t G);
 /* Rounds of mbarrier try_wait a copy row's bulk copy of its parent strand may
  * take before CLOTHO_DEVERR_STALL is raised (0 = the default, 2^22; at most
@@ -357,8 +364,8 @@ int  clotho_run_philox_schedule(clotho_ctx *ctx, const uint32_t *N, uint32_t G);
  * reference counterpart (the reference has no asynchronous copies). */
 int  clotho_set_copy_wait_limit(clotho_ctx *ctx, uint32_t rounds);
 /* Rows per scheduling item of the generation kernel (autotuner knob of
- * batched contexts; a single-population context has its warps claim one row
- * at a time and ignores it). */
+ * batched contexts; a single-population context ignores it: its warps claim a
+ * row or two at a time, or units of short rows, or take those by a stride). */
 int  clotho_set_rows_per_item(clotho_ctx *ctx, uint32_t rows);
 /* Launch shapes chosen by an autotuner (clotho_gb300/autotune.py).  None
  * changes a result: the kernels are deterministic in every shape.
@@ -370,8 +377,9 @@ int  clotho_set_rows_per_item(clotho_ctx *ctx, uint32_t rows);
  *   row_blocks_per_sm  blocks per SM of the per-individual kernels of a step
  *                      (parent sampling; phenotype and fitness); 0 = the
  *                      default, 16
- * No reference counterpart: the reference's work partition is its thread
- * pool's fixed batches (thread_pool.hpp:31-139). */
+ * On a batch clotho_set_tuning waits for the steps under way.  No reference
+ * counterpart: the reference's work partition is its thread pool's fixed
+ * batches (thread_pool.hpp:31-139). */
 typedef struct clotho_tuning {
     uint32_t rows_per_item;
     uint32_t narrow_build;
